@@ -347,13 +347,14 @@ int d2h_small(gsj_context* c, X* dst, const X* src, size_t count) {
 }
 
 // Entries a block-reserving pass may take for `real` entries: each warp
-// reserves blocks of kScreenBlockSlack entries and abandons its block (padding
-// the tail) when the next chunk of at most `max_chunk` entries does not fit,
-// so every abandoned block holds at least kScreenBlockSlack - (max_chunk - 1)
-// real entries; each of the `warps` warps may end with one partly filled block.
-uint64_t reserve_bound(uint64_t real, uint64_t warps, uint32_t max_chunk) {
-    const uint64_t per = kScreenBlockSlack - (max_chunk - 1u);
-    return ((real + per - 1u) / per + warps) * kScreenBlockSlack;
+// reserves blocks of `block` entries and abandons its block (padding the tail)
+// when the next chunk of at most `max_chunk` entries does not fit (1: chunks
+// are split over blocks), so every abandoned block holds at least block -
+// (max_chunk - 1) real entries; each of the `warps` warps may end with one
+// partly filled block.
+uint64_t reserve_bound(uint64_t real, uint64_t warps, uint64_t block, uint32_t max_chunk) {
+    const uint64_t per = block - (max_chunk - 1u);
+    return ((real + per - 1u) / per + warps) * block;
 }
 
 // Capacity of attempt `attempt` of a block-reserving pass: the estimate first;
@@ -525,7 +526,7 @@ int emit_join(gsj_context* c, JoinArgs<T>& a, uint64_t N, bool stamp, int model,
     unsigned long long* pairs = nullptr;
     unsigned long long used = 0, R = 0;
     for (int attempt = 0; attempt < 3; attempt++) {
-        cap = retry_cap(attempt, estimate, used, reserve_bound(R, warps, 64u));
+        cap = retry_cap(attempt, estimate, used, reserve_bound(R, warps, kScreenBlockSlack, 64u));
         GSJ_TRY(dev_get(c, c->pairs, cap ? cap : 1, &pairs));
         GSJ_TRY(reset());
         o.emit = true;
@@ -566,11 +567,10 @@ int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int mo
     o.cursor = cursor;
     o.shift = shift;
     o.rechecks = cursor + 1;  // the screen's exact count of undecided pairs
-    // the screen's consumer warps reserve blocks (a warp appends at most
-    // 32 x 16 undecided pairs at once; at most 64 warps per SM are resident);
-    // the tile join appends exactly
+    // the screen's consumer warps reserve blocks and fill them (at most 64 warps
+    // per SM are resident); the tile join appends exactly
     const uint64_t warps = (uint64_t)c->num_sms * 64u;
-    const uint64_t slack = screen ? warps * kScreenBlockSlack : 0u;
+    const uint64_t slack = screen ? warps * kScreenBlock : 0u;
     unsigned long long* cand = reinterpret_cast<unsigned long long*>(a.work_counter + 2);
     a.err_flag = a.work_counter + 1;
     ScreenConst sc = make_screen_const(a.n, a.thr);
@@ -586,26 +586,28 @@ int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int mo
     };
     GSJ_CUDA(c, cudaEventRecord(c->tev[2], st));
     if (screen) {
-        // centred BF16 rows and norms of all points, read by every candidate tile
+        // centred BF16 rows of all points, read by every candidate tile
         uint4* rows = nullptr;
-        float *norms = nullptr, *centre = nullptr;
+        uint32_t* qg = nullptr;
+        float* centre = nullptr;
         double* partial = nullptr;
-        GSJ_TRY(dev_get(c, c->srows, N * (sc.kpad / 8), &rows));
-        GSJ_TRY(dev_get(c, c->snorms, N, &norms));
+        GSJ_TRY(dev_get(c, c->srows, screen_rows_count(N, sc.kpad), &rows));
+        GSJ_TRY(dev_get(c, c->snorms, N, &qg));
         GSJ_TRY(dev_get(c, c->spartial, (size_t)kScreenPrepBlocks * a.n * 2, &partial));
         GSJ_TRY(dev_get(c, c->scentre, a.n, &centre));
         S.kernel_launches += 3;
-        GSJ_CUDA(c, launch_screen_prep(a.pts, (uint32_t)N, a.n, a.npad, sc.kpad, partial, centre, rows, norms, st));
+        GSJ_CUDA(c, launch_screen_prep(a.pts, (uint32_t)N, a.n, a.npad, sc, partial, centre, rows, qg, st));
         sc.rows = rows;
-        sc.norms = norms;
+        sc.qg = qg;
     }
     // ---- estimate of the exact pass's entries (pairs, or the screen's undecided pairs)
     if (learned && screen && !(c->model_unc_ratio > 0.0)) learned = false;  // no screened training join yet
     GSJ_CUDA(c, cudaEventRecord(c->tev[6], st));
-    double est = 0.0;
+    double est = 0.0, est_entries = 0.0;  // pairs, buffer entries (the screen's records hold one pair or more)
     if (learned) {
         GSJ_TRY(learned_estimate(c, &est));
         if (screen) est *= c->model_unc_ratio;
+        est_entries = est;
     } else if (!exact_size) {
         // sampled estimator: the exact pass over every kSampleStride-th item
         const uint32_t nsample = (ni + kSampleStride - 1) / kSampleStride;
@@ -614,24 +616,26 @@ int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int mo
         o.stride = kSampleStride;
         S.kernel_launches += 1;
         GSJ_CUDA(c, launch(nsample));
-        unsigned long long sampled = 0;
-        GSJ_TRY(d2h_small(c, &sampled, screen ? o.rechecks : cursor, 1));
+        unsigned long long sampled[2] = {0, 0};  // entries, and the screen's undecided pairs
+        GSJ_TRY(d2h_small(c, sampled, cursor, 2));
         uint32_t err = 0;
         GSJ_TRY(d2h_small(c, &err, a.err_flag, 1));
         if (err) return fail(c, GSJ_ERR_CUDA, "tile join: tensor-core wait timed out");
-        est = nsample ? (double)sampled * (double)ni / (double)nsample : 0.0;
+        est_entries = nsample ? (double)sampled[0] * (double)ni / (double)nsample : 0.0;
+        est = screen && nsample ? (double)sampled[1] * (double)ni / (double)nsample : est_entries;
     }
     GSJ_CUDA(c, cudaEventRecord(c->tev[7], st));
     S.estimate = (uint64_t)est;
-    const uint64_t estimate = exact_size ? 0u : (uint64_t)(est * 1.25) + N + (1u << 16) + slack;
+    const uint64_t estimate = exact_size ? 0u : (uint64_t)(est_entries * 1.25) + N + (1u << 16) + slack;
     uint64_t cap = estimate;
     // ---- full pass (repeated with a larger buffer if the buffer was short):
-    // the tile join's hits, or the screen's undecided pairs
+    // the tile join's hits, or the screen's records of undecided pairs
     unsigned long long *list = nullptr, *pairs = nullptr;
+    const uint64_t entry = screen ? 2u : 1u;  // 64-bit words per buffer entry
     unsigned long long U = 0, R = 0, nlist = 0, used = 0;
     for (int attempt = 0; attempt < 3; attempt++) {
-        cap = retry_cap(attempt, estimate, used, screen ? reserve_bound(U, warps, 512u) : U);
-        GSJ_TRY(dev_get(c, screen ? c->unc : c->pairs, cap ? cap : 1, &list));
+        cap = retry_cap(attempt, estimate, used, screen ? reserve_bound(U, warps, kScreenBlock, 1u) : U);
+        GSJ_TRY(dev_get(c, screen ? c->unc : c->pairs, (cap ? cap : 1) * entry, &list));
         GSJ_TRY(reset());
         o.emit = true;
         o.stride = 1;
@@ -639,7 +643,7 @@ int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int mo
         o.cap = cap;
         S.kernel_launches += 1;
         GSJ_CUDA(c, launch(ni));
-        // entries written (pairs), or reserved (undecided blocks)
+        // entries written (pairs), or reserved (records)
         GSJ_TRY(d2h_small(c, &used, cursor, 1));
         U = used;
         if (screen) GSJ_TRY(d2h_small(c, &U, o.rechecks, 1));
@@ -662,7 +666,7 @@ int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int mo
         ro.pairs = pairs;
         ro.cap = pcap;
         S.kernel_launches += 1;
-        GSJ_CUDA(c, launch_screen_recheck(a, list, nlist, ro, stamp, model, c->num_sms, st));
+        GSJ_CUDA(c, launch_screen_recheck(a, reinterpret_cast<const uint4*>(list), nlist, ro, stamp, model, c->num_sms, st));
         GSJ_TRY(d2h_small(c, &R, cursor, 1));
         if (R > pcap) return fail(c, GSJ_ERR_STATE, "screened join: more pairs than undecided candidates");
     } else {

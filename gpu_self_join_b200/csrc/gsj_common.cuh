@@ -125,4 +125,39 @@ __device__ __forceinline__ bool lookup_range(const JoinArgs<T>& a, uint64_t lin,
     return false;
 }
 
+// Slot range of a neighbour row: the cells x-1..x+1 of the grid row that offset
+// r (digit j of r is dim j+1's step + 1) leads to.  These cells are
+// consecutive in cell order (dim 0 is fastest), so the range is contiguous
+// whichever of them are non-empty.  With unicomp the own row (r's centre) adds
+// its dim-0 neighbours only when x is odd, every other row comes whole or not
+// at all (the highest moved dim is the same for its three cells).
+template <typename T, bool STAMP>
+__device__ __forceinline__ bool row_range(const JoinArgs<T>& a, uint32_t r, uint64_t own_lin, uint32_t lowmask,
+                                          uint32_t highmask, uint32_t oddmask, uint32_t& start, uint32_t& cnt) {
+    uint64_t lin;
+    if (!nb_offset<T, STAMP>(a, 3u * r + 1u, own_lin, lowmask, highmask, oddmask, lin)) return false;
+    const bool side = !STAMP || lin != own_lin || (oddmask & 1u);
+    const bool down = side && !(lowmask & 1u), up = side && !(highmask & 1u);
+    if (a.ds) {
+        start = a.ds[down ? lin - 1 : lin];
+        cnt = a.ds[(up ? lin + 1 : lin) + 1] - start;
+        return cnt != 0u;
+    }
+    uint32_t s = 0, c = 0;
+    start = cnt = 0u;
+    if (down && lookup_range(a, lin - 1, s, c)) {
+        start = s;
+        cnt = c;
+    }
+    if (lookup_range(a, lin, s, c)) {
+        if (!cnt) start = s;
+        cnt += c;
+    }
+    if (up && lookup_range(a, lin + 1, s, c)) {
+        if (!cnt) start = s;
+        cnt += c;
+    }
+    return cnt != 0u;
+}
+
 }  // namespace gsj

@@ -7,43 +7,55 @@
 // packed (query id, candidate id) key.  What changes is how a pair is decided:
 //
 //   1. Once per join (k_screen_rows), every point is centred on the data mean
-//      o and rounded to BF16, c^ = bf16(fl(c - o)), and stored with its norm
-//      as a row [c^, |c^|^2_hi, |c^|^2_lo] (slot order).  Candidate tiles are
-//      copied from these rows (cp.async, 16-byte chunks) into K-major
-//      shared-memory tiles (8 x 16-byte core matrices, no swizzle); the query
-//      tile holds [-2 q^, 1, 1], so the product carries the candidate norm.
+//      o and rounded to BF16, c^ = bf16(fl(c - o)), and stored as a row
+//      [c^, A_hi, A_lo, 1, 1, 0...] (K columns, a multiple of 16), with
+//          r = |(c - o) - c^|                       (its own rounding, bounded above)
+//          A <= |c^|^2 - 2 R0 r - 2 r^2 - c1 |c^|^2   (rounded down, two BF16 terms)
+//      and, for its role as a query, G >= R0^2 + 2 R0 r + 2 r^2 - |c^|^2 +
+//      c1 |c^|^2 + c0 R0^2 (rounded up, two BF16 terms).  The rows lie in
+//      groups of 8 consecutive slots, each group the 8 x 16-byte core matrices of
+//      a K-major shared-memory tile, so that any run of groups is one contiguous
+//      copy in global and in shared memory.
 //   2. One thread issues tcgen05.mma (kind::f16, BF16 x BF16 -> FP32, M = N =
-//      128, K = 16 per instruction) over the padded dimensions; the 128 x 128
-//      values |c^_j|^2 - 2 q^_i.c^_j accumulate in tensor memory (exact
-//      BF16 products; -2 q^ is exact in BF16).
+//      128, K = 16 per instruction) of the query tile [-2 q^, 1, 1, -G_hi, -G_lo]
+//      and a tile of 16 candidate groups: the accumulator is
+//          D_ij = A_j - 2 q^_i.c^_j - G_i.
 //   3. Every consumer thread reads its query's row (tcgen05.ld 32x32b) and
-//      rejects candidate j when that value exceeds
-//      G_i = (R0 + kE (|q^_i| + max_j |c^_j|))^2 + c1 (|q^_i|^2 + 2 max_j |c^_j|^2) - |q^_i|^2,
-//      the maximum over the 32 candidates of j's column group.
-//      The bound is proven, not tuned: R0^2 covers the rounding of the
-//      reference's own FP32 sum (at most 2n+8 roundings of non-negative
-//      terms), kE the BF16 rounding of both centred points and of the centring
-//      (|x - bf16(x)| <= 2^-8 |x|), c1 the FP32 accumulation (K + 32 steps of
-//      2^-20) and the two-term BF16 split of the norm (2^-16).  A pair within
-//      eps by the reference's arithmetic is therefore never rejected.
-//   4. Every pair not rejected is appended to a list of undecided pairs;
-//      k_screen_recheck recomputes each in the reference's exact FP32 order
-//      from the original coordinates (ILP/SHORTCIRCUIT model,
-//      kernel.cu:307-365) and keeps it iff s <= thr.
-// The emitted pair set is the plain path's, bit for bit.  Non-finite values
-// only make the test inconclusive, which sends the pair to the exact check.
+//      rejects candidate j when D_ij >= 0: one OR over the sign bits decides
+//      whether any of 32 candidates is left.  The bound is proven, not tuned:
+//      |c^ - q^| <= |c - q| + r_c + r_q, so a pair within eps by the reference's
+//      arithmetic (whose FP32 sum is covered by R0 >= sqrt(thr): at most 2n+8
+//      roundings of non-negative terms) has
+//          |c^ - q^|^2 <= (R0 + r_c + r_q)^2
+//                      <= R0^2 + 2 R0 (r_c + r_q) + 2 r_c^2 + 2 r_q^2,
+//      which is A_j - 2 q^.c^ - G_i <= -(c1 (|c^|^2 + |q^|^2) + c0 R0^2) in exact
+//      arithmetic, and c1, c0 exceed the FP32 accumulation error (K + 32 steps
+//      of 2^-20 of the summed magnitudes, a factor 8 above FP32 rounding), so
+//      D_ij < 0.  A point that is not finite (or beyond 1e15 from the centre)
+//      becomes a row with q^ = 0 and A, -G = -2^120: all its pairs stay undecided
+//      and no NaN can arise.
+//   4. The pairs not rejected are appended as records (query slot, first of 32
+//      candidate slots, 32-bit mask), one per query and 32 columns;
+//      k_screen_recheck recomputes each pair in the reference's exact FP32 order
+//      from the original coordinates (ILP/SHORTCIRCUIT model, kernel.cu:307-365)
+//      and keeps it iff s <= thr.
+// The emitted pair set is the plain path's, bit for bit.
 //
-// Synchronisation: warps 8-11 produce candidate tiles (slot search, cp.async of
-// the rows) and one of their threads issues the MMA, warps 0-7 consume;
-// candidate tiles rotate through kStages buffers and two accumulators
-// alternate, handed over by mbarriers only (staged: every producer thread's
-// slots and landed rows of a buffer; full: MMA commit + the issuer's release;
-// empty and free: the consumer arrivals), so the producer warps never wait for
-// one another.  Every wait is a bounded poll by one thread whose outcome is
-// shared before any warp-collective; on time-out the error flag is raised and
-// the CTA stops.  Tensor memory (2 x 128 columns) is allocated once
-// per CTA; the shared-memory request keeps at most 2 CTAs (512 columns) on an
-// SM; it is released before exit.
+// Candidates are walked in groups: the slot range of a neighbour row (the up to
+// three cells x-1..x+1 of one row of the grid, consecutive in cell order) is
+// widened to whole groups, and an 8-bit mask per group keeps the rows that
+// belong to the range; only undecided pairs look at it.
+//
+// Roles: warps 0-7 consume, warp 8 copies candidate tiles (a bulk copy per run of
+// consecutive groups; most tiles are one run), one thread of warp 9 issues the
+// MMAs.  Candidate tiles rotate through up to kMaxStages buffers and two
+// accumulators alternate, handed over by mbarriers (landed: a buffer's bytes have
+// arrived; drained: its MMA has read it; full / empty: an accumulator).  Every
+// wait is a bounded poll by one thread whose outcome is shared before any
+// warp-collective; on time-out the error flag is raised and the CTA stops.
+// Tensor memory (2 x 128 columns) is allocated once per CTA; the shared-memory
+// request keeps at most 2 CTAs (512 columns) on an SM; it is released before
+// exit.
 #include <algorithm>
 #include <cstdint>
 #include <cuda_bf16.h>
@@ -59,14 +71,25 @@ namespace {
 
 constexpr int kSQ = kScreenQ;        // queries per item = MMA M
 constexpr int kSC = 128;             // candidates per tile = MMA N
-constexpr int kSThreads = 384;      // warps 0-7 consume, warps 8-11 produce
-constexpr int kProd0 = 256;         // first producer thread
+constexpr uint32_t kGrp = 8;         // candidate slots per group (rows of a core matrix)
+constexpr uint32_t kTileGrps = kSC / kGrp;
+constexpr int kConsumers = 256;      // warps 0-7 consume
+constexpr int kCopyWarp = 8, kMmaWarp = 9;
+constexpr int kSThreads = 320;
 constexpr uint32_t kTmemCols = 128;  // FP32 accumulator columns (N)
-constexpr uint32_t kNone = 0xffffffffu;
 constexpr uint32_t kMinSmem = 80u * 1024u;  // at most 2 CTAs (2 x 256 TMEM columns) per SM
-constexpr uint32_t kWaitPolls = 1u << 20;
-constexpr uint32_t kBlk = (uint32_t)kScreenBlockSlack;  // undecided-pair entries a consumer warp reserves
-constexpr uint32_t kStages = 3;     // candidate tiles in flight (the accumulators alternate in 2)
+constexpr uint32_t kWaitHintNs = 20000u, kWaitPolls = 1u << 16;
+constexpr uint32_t kBlk = kScreenBlock;  // records a consumer warp reserves at a time
+constexpr uint32_t kMaxStages = 8;   // candidate tiles in flight (the accumulators alternate in 2)
+// Per-tile candidate metadata rotates through kMeta entries.  Tile g's entry is
+// rewritten for tile g + kMeta, whose buffer is free once the MMA of tile
+// g + kMeta - stages has run; that MMA waited for every consumer to have read
+// the accumulator two tiles earlier, and a consumer reads an accumulator only
+// after it is done with all earlier tiles.  So kMeta >= kMaxStages + 3 suffices.
+constexpr uint32_t kMeta = 16;
+constexpr uint32_t kMaxKpad = 144;   // 126 dimensions + 4 columns, padded to 16
+constexpr uint64_t kUnitsPerCta = 16, kMaxParts = 64;  // slicing of small launches
+constexpr float kFar = 1e30f;        // |c^|^2 above it: the point is screened by no bound
 
 // Instruction descriptor of tcgen05.mma kind::f16: FP32 accumulator (bit 4),
 // A and B BF16 (bits 7 and 10), both K-major, N >> 3 at bit 17, M >> 4 at bit 24.
@@ -109,16 +132,17 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
                  : "memory");
 }
 
-// try_wait suspends the thread in hardware until the phase completes or an
-// implementation-defined time passes; the loop bounds the total wait.
+// try_wait suspends the thread in hardware until the phase completes or the
+// hint (ns) passes, so that waiting warps leave the issue slots to the others;
+// the loop bounds the total wait (about a second).
 __device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
         "selp.b32 %0, 1, 0, p;\n\t}\n"
         : "=r"(ok)
-        : "r"(bar), "r"(parity)
+        : "r"(bar), "r"(parity), "r"(kWaitHintNs)
         : "memory");
     return ok != 0;
 }
@@ -129,12 +153,20 @@ __device__ __forceinline__ bool bar_wait_bounded(uint32_t bar, uint32_t parity) 
     return false;
 }
 
+// The whole warp waits; the outcome is the same for all lanes.
+__device__ __forceinline__ bool warp_wait_bounded(uint32_t bar, uint32_t parity) {
+    for (uint32_t it = 0; it < kWaitPolls; it++)
+        if (__all_sync(0xffffffffu, bar_try(bar, parity))) return true;
+    return false;
+}
+
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
-    uint32_t r[32];
+// 32 accumulator columns of the warp's 32 rows (row = lane); tmem_wait_ld
+// completes the loads.
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
         "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
@@ -143,9 +175,19 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
           "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
           "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
+}
+
+// The wait names every loaded register, so that no use of them can move above it.
+__device__ __forceinline__ void tmem_wait_ld(uint32_t* r) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]),
+                   "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]),
+                   "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]),
+                   "+r"(r[29])
+                 :
+                 : "memory");
+    asm volatile("" : "+r"(r[30]), "+r"(r[31])::"memory");
 }
 
 // The reference's squared distance in its exact order, one thread, stopping
@@ -178,7 +220,7 @@ __device__ float exact_sqdist(const float* __restrict__ q, const float* __restri
     }
 }
 
-// Same arithmetic, rows read as float4 blocks of 32 dimensions loaded before
+// Same arithmetic, rows read as float4 blocks of 16 dimensions loaded before
 // use (npad is a multiple of 4 here); the ILP model without SHORTCIRCUIT
 // walks its dimensions with stride ILP and keeps the scalar form.
 template <int MODEL>
@@ -189,10 +231,10 @@ __device__ float exact_sqdist4(const float* __restrict__ q, const float* __restr
     const float4* c4 = reinterpret_cast<const float4*>(c);
     float s = 0.f;
     uint32_t p = 0;
-    for (uint32_t l0 = 0; l0 < n; l0 += 32u) {
-        float4 qa[8], ca[8];
+    for (uint32_t l0 = 0; l0 < n; l0 += 16u) {
+        float4 qa[4], ca[4];
 #pragma unroll
-        for (int b = 0; b < 8; b++) {
+        for (int b = 0; b < 4; b++) {
             if (l0 + 4u * b < n) {
                 qa[b] = q4[(l0 >> 2) + b];
                 ca[b] = c4[(l0 >> 2) + b];
@@ -201,7 +243,7 @@ __device__ float exact_sqdist4(const float* __restrict__ q, const float* __restr
             }
         }
 #pragma unroll
-        for (int b = 0; b < 8; b++) {
+        for (int b = 0; b < 4; b++) {
             const float qv[4] = {qa[b].x, qa[b].y, qa[b].z, qa[b].w};
             const float cv[4] = {ca[b].x, ca[b].y, ca[b].z, ca[b].w};
 #pragma unroll
@@ -219,93 +261,106 @@ __device__ float exact_sqdist4(const float* __restrict__ q, const float* __restr
 }
 
 struct ScreenSmem {
-    uint32_t a, b, nbs, nbp, cslot, cwmax, qid, qinfo, misc, total;
+    uint32_t a, nbs, nbe, nbg, mbase, mmask, misc, b, total;
 };
 
-__host__ __device__ inline ScreenSmem screen_smem(uint32_t kpad, uint32_t noff) {
+// Byte sizes are rounded to 128 so that the tiles stay aligned; `stages`
+// candidate tiles follow at b.
+__host__ __device__ inline ScreenSmem screen_smem(uint32_t kpad, uint32_t nrow, uint32_t stages) {
     ScreenSmem t{};
     uint32_t o = 0;
     t.a = o;
     o += (uint32_t)kSQ * kpad * 2u;
-    t.b = o;  // kStages candidate tiles
-    o += kStages * (uint32_t)kSC * kpad * 2u;
-    t.nbs = o;
-    o += noff * 4u;
-    t.nbp = o;
-    o += (noff + 1u) * 4u;
+    t.nbs = o;  // per neighbour row: first slot, end slot, exclusive prefix of the groups
+    o += nrow * 4u;
+    t.nbe = o;
+    o += nrow * 4u;
+    t.nbg = o;
+    o += (nrow + 1u) * 4u;
+    o = (o + 15u) & ~15u;  // read as 16-byte vectors
+    t.mbase = o;  // [kMeta][16] first slot of each group of a tile
+    o += kMeta * kTileGrps * 4u;
+    t.mmask = o;  // [kMeta][16] bytes: rows of the group that are candidates
+    o += kMeta * kTileGrps;
     o = (o + 15u) & ~15u;
-    t.cslot = o;  // [kStages][kSC]
-    o += kStages * kSC * 4u;
-    t.cwmax = o;  // [kStages][8] per 32-candidate group: largest norm [0..3], its square root [4..7]
-    o += kStages * 8u * 4u;
-    t.qid = o;
-    o += kSQ * 4u;
-    o = (o + 15u) & ~15u;
-    t.qinfo = o;  // float4 per query: |q^|^2, R0 + kE |q^|, c1 |q^|^2, valid
-    o += kSQ * 16u;
-    t.misc = o;   // [0] item [1] failed [2] total [4] tmem [8..19] warp counts
-                  // [24..31] mbarriers full0 full1 empty0 empty1, [32..37] free0 free1 free2
-    o += 48u * 4u;
-    t.total = (o + 127u) & ~127u;
+    t.misc = o;   // [0] unit [1] failed [2] groups [3] candidates [4] tmem [8..17] warp counts
+                  // [20..] mbarriers: full 0 1, empty 0 1, landed 0..7, drained 0..7
+                  // [64..] undecided pairs and records of each consumer warp (64-bit)
+    o += 96u * 4u;
+    o = (o + 127u) & ~127u;
+    t.b = o;
+    o += stages * (uint32_t)kSC * kpad * 2u;
+    t.total = o;
     return t;
 }
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+__device__ __forceinline__ void bar_init(uint32_t bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
 
 __device__ __forceinline__ void bar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-// The CTA is warp-specialised: warps 8-11 produce (candidate slots, centred
-// BF16 candidate rows with the norm folded in, the MMA), warps 0-7 consume
-// (tensor-memory rows, the screen, the undecided-pair appends).  Candidate
-// tiles rotate through kStages buffers and two accumulators alternate;
-// mbarriers staged[b] (rows in place), full[s] (MMA done), empty[s]
-// (accumulator read) and free[b] (buffer read) hand them over.
+__device__ __forceinline__ void bar_arrive_tx(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+
+// Untiled bulk copy global -> this CTA's shared memory (16-byte aligned, whole
+// groups of rows), completing on `bar`.
+__device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+
+// A unit is a slice (one of `parts`) of the candidate tiles of an item (up to
+// 128 consecutive query slots of one cell): slices give small joins and the
+// sampling pass enough units for the whole chip and shorten the last wave.
 //
-// With the norm folded into the product (A row, the query = [-2 q^, 1, 1];
-// B row, the candidate = [c^, |c^|^2_hi, |c^|^2_lo]), the accumulator holds
-// |c^_j|^2 - 2 q^_i.c^_j directly and the screen is one comparison per pair.
-template <int MODEL, bool STAMP>
+// What bounds it: the consumers' dependent instructions.  At K = 32 the tensor
+// pipe needs 128 cycles for a tile; a tile takes about 600 cycles of an SM (0.21
+// of the tensor pipe), 16 consumer warps an SM issuing 0.47 instructions a cycle
+// and scheduler, half of them on the 32-column blocks that hold an undecided
+// pair.  A consumer warp reads 32 columns at a time: with 64 the registers spill
+// at 2 CTAs an SM (133 against 105 ms on the 18-D workload).  Measured (both
+// launches of a join): 18-D 5M points 270 -> 105 ms, 90-D 515k 117 -> 40 ms, 32-D
+// 45k 2.0 -> 0.64 ms, against four warps staging rows one by one with cp.async
+// and a compare per pair with a bound per 32 candidates (1,720 cycles a tile).
+template <bool STAMP>
 __global__ void __launch_bounds__(kSThreads, 2) k_tile_screen(const JoinArgs<float> a, const TileOut o,
-                                                              const ScreenConst sc, uint32_t noff, uint32_t nvisit) {
+                                                              const ScreenConst sc, uint32_t nrow, uint32_t stages,
+                                                              uint32_t parts, uint32_t nunits) {
     extern __shared__ __align__(1024) unsigned char ssm[];
-    const uint32_t n = a.n, npad = a.npad, k = a.g.k, kpad = sc.kpad;
-    const ScreenSmem L = screen_smem(kpad, noff);
+    const uint32_t n = a.n, npad = a.npad, k = a.g.k, kpad = sc.kpad, kch = kpad >> 3;
+    const ScreenSmem L = screen_smem(kpad, nrow, stages);
     unsigned char* A = ssm + L.a;
     uint32_t* nb_start = reinterpret_cast<uint32_t*>(ssm + L.nbs);
-    uint32_t* nb_pref = reinterpret_cast<uint32_t*>(ssm + L.nbp);
-    uint32_t* c_slot = reinterpret_cast<uint32_t*>(ssm + L.cslot);
-    float* cwmax = reinterpret_cast<float*>(ssm + L.cwmax);
-    uint32_t* q_id = reinterpret_cast<uint32_t*>(ssm + L.qid);
-    float4* qinfo = reinterpret_cast<float4*>(ssm + L.qinfo);
+    uint32_t* nb_end = reinterpret_cast<uint32_t*>(ssm + L.nbe);
+    uint32_t* nb_grp = reinterpret_cast<uint32_t*>(ssm + L.nbg);
+    uint32_t* m_base = reinterpret_cast<uint32_t*>(ssm + L.mbase);
+    unsigned char* m_mask = ssm + L.mmask;
     uint32_t* misc = reinterpret_cast<uint32_t*>(ssm + L.misc);
     const unsigned FULL = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned lt = lanemask_lt_s();
-    const uint32_t sbo = (kpad >> 3) * 128u;
-    const uint32_t a_addr = smem_u32(A);
-    const uint32_t full0 = smem_u32(misc + 24), full1 = smem_u32(misc + 26);
-    const uint32_t empty0 = smem_u32(misc + 28), empty1 = smem_u32(misc + 30);
-    const uint32_t free0 = smem_u32(misc + 32);  // free_b = free0 + 8 b
-    const uint32_t staged0 = smem_u32(misc + 38);  // staged_b = staged0 + 8 b
+    const uint32_t sbo = kch * 128u;                          // bytes of a group
+    const uint32_t stage_bytes = (uint32_t)kSC * kpad * 2u;
+    const uint32_t a_addr = smem_u32(A), b_addr = smem_u32(ssm + L.b);
+    const uint32_t full = smem_u32(misc + 20), empty = smem_u32(misc + 24);    // [2] each, 8 bytes apart
+    const uint32_t landed = smem_u32(misc + 28), drained = smem_u32(misc + 44);  // [stages] each
 
     // ---- set-up: mbarriers, tensor memory (two accumulators)
     if (tid == 0) {
         misc[1] = 0u;
-        // full[s]: the MMA's commit + the issuing thread's release of the tile's metadata
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(full0) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(full1) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 256;" ::"r"(empty0) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 256;" ::"r"(empty1) : "memory");
-        // free[b]: the consumers are done with stage b (candidate tile, slots, norm bound)
-        for (uint32_t b = 0; b < kStages; b++)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 256;" ::"r"(free0 + 8u * b) : "memory");
-        // staged[b]: the 128 producer threads' slots and rows of stage b are in place
-        for (uint32_t b = 0; b < kStages; b++)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 128;" ::"r"(staged0 + 8u * b) : "memory");
+        for (uint32_t s = 0; s < 2u; s++) {
+            bar_init(full + 8u * s, 2u);                  // the MMA's commit, the issuing thread
+            bar_init(empty + 8u * s, kConsumers / 32u);   // a thread of every consumer warp
+        }
+        for (uint32_t b = 0; b < stages; b++) {
+            bar_init(landed + 8u * b, 1u);   // the copying thread, and the bytes
+            bar_init(drained + 8u * b, 1u);  // the MMA's commit
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -318,25 +373,33 @@ __global__ void __launch_bounds__(kSThreads, 2) k_tile_screen(const JoinArgs<flo
     __syncthreads();
     fence_after();
     const uint32_t tmem = misc[4];
-    uint32_t tiles_done = 0;  // tiles of earlier items (the mbarrier phases)
+    // tiles of earlier units: tile g uses buffer g % stages, accumulator g % 2 and
+    // metadata entry g % kMeta, and its mbarriers' phases follow from g
+    uint32_t g0 = 0;
     unsigned long long cand_total = 0;
-    // consumer warps: the reserved block of undecided-pair entries and the count
-    unsigned long long blk_base = 0, und_count = 0;
+    // consumer warps: the reserved block of records; undecided pairs and records
+    // so far in shared memory
+    unsigned long long blk_base = 0;
     uint32_t blk_used = kBlk;
+    uint4* recs = reinterpret_cast<uint4*>(o.pairs);
+    unsigned long long* n_und = reinterpret_cast<unsigned long long*>(misc + 64) + warp;
+    unsigned long long* n_rec = n_und + kConsumers / 32;
+    if (tid < kConsumers && lane == 0) *n_und = *n_rec = 0ull;
 
     for (;;) {
         __syncthreads();
         if (tid == 0) misc[0] = atomicAdd(a.work_counter, 1u);
         __syncthreads();
-        const uint32_t vi = misc[0];
-        if (vi >= nvisit || misc[1]) break;
+        const uint32_t unit = misc[0];
+        if (unit >= nunits || misc[1]) break;
+        const uint32_t vi = unit / parts, part = unit - vi * parts;
         const uint2 wi = a.items[(size_t)vi * o.stride];
         const uint32_t cell = wi.x;
         const uint32_t cs0 = a.cell_start[cell], ce = a.cell_start[cell + 1];
         const uint32_t q0 = cs0 + wi.y * (uint32_t)kSQ;
         const uint32_t qn = min((uint32_t)kSQ, ce - q0);
 
-        // ---- neighbour cells in offset order (as the tile join)
+        // ---- neighbour rows in offset order (kernel.cu:180-303; stamploops.h)
         uint32_t own[kMaxK];
 #pragma unroll
         for (int j = 0; j < kMaxK; j++)
@@ -347,12 +410,11 @@ __global__ void __launch_bounds__(kSThreads, 2) k_tile_screen(const JoinArgs<flo
         uint32_t lowmask, highmask, oddmask;
         cell_masks(own, a.g, lowmask, highmask, oddmask);
         const uint64_t own_lin = a.cell_key[cell];
-        for (uint32_t base = 0; base < noff; base += kSThreads) {
-            const uint32_t off = base + tid;
-            uint64_t lin = 0;
-            const bool ok = off < noff && nb_offset<float, STAMP>(a, off, own_lin, lowmask, highmask, oddmask, lin);
+        for (uint32_t base = 0; base < nrow; base += kSThreads) {
+            const uint32_t r = base + (uint32_t)tid;
             uint32_t st = 0, cnt = 0;
-            const bool found = ok && lookup_range(a, lin, st, cnt);
+            const bool found =
+                r < nrow && row_range<float, STAMP>(a, r, own_lin, lowmask, highmask, oddmask, st, cnt);
             const unsigned m = __ballot_sync(FULL, found);
             if (lane == 0) misc[8 + warp] = __popc(m);
             __syncthreads();
@@ -366,252 +428,302 @@ __global__ void __launch_bounds__(kSThreads, 2) k_tile_screen(const JoinArgs<flo
             if (found) {
                 const uint32_t pos = nnb + before + __popc(m & lt);
                 nb_start[pos] = st;
-                nb_pref[pos] = cnt;
+                nb_end[pos] = st + cnt;
             }
             nnb += all;
             __syncthreads();
         }
-        if (warp == 0) {
-            uint32_t run = 0;
+        if (warp == kMmaWarp) {
+            // exclusive prefix of the groups, and the candidates of a query
+            uint32_t run = 0, cand = 0;
             for (uint32_t b0 = 0; b0 < nnb; b0 += 32) {
                 const uint32_t i = b0 + lane;
-                const uint32_t v = i < nnb ? nb_pref[i] : 0u;
+                uint32_t v = 0;
+                if (i < nnb) {
+                    const uint32_t s = nb_start[i], e = nb_end[i];
+                    v = (e + kGrp - 1u) / kGrp - s / kGrp;
+                    cand += e - s;
+                }
                 uint32_t x = v;
 #pragma unroll
                 for (int s = 1; s < 32; s <<= 1) {
                     const uint32_t y = __shfl_up_sync(FULL, x, s);
                     if (lane >= s) x += y;
                 }
-                if (i < nnb) nb_pref[i] = run + x - v;
+                if (i < nnb) nb_grp[i] = run + x - v;
                 run += __shfl_sync(FULL, x, 31);
             }
+            cand = __reduce_add_sync(FULL, cand);
             if (lane == 0) {
-                nb_pref[nnb] = run;
+                nb_grp[nnb] = run;
                 misc[2] = run;
+                misc[3] = cand;
             }
-        }
-        // ---- query tile [-2 q^, 1, 1] from the precomputed rows [q^, |q^|^2_hi, |q^|^2_lo]
-        const uint32_t kch = kpad >> 3;  // 16-byte chunks per row
-        if (tid < kSQ) {
-            const bool valid = (uint32_t)tid < qn;
-            q_id[tid] = valid ? a.ids[q0 + tid] : 0u;
-            const float nrm = valid ? sc.norms[q0 + tid] : 0.f;
-            qinfo[tid] = make_float4(nrm, __fmaf_ru(sc.ke, __fsqrt_ru(nrm), sc.r0), __fmul_ru(sc.c1, nrm),
-                                     valid ? 1.f : 0.f);
-        }
-        for (uint32_t e = tid; e < (uint32_t)kSQ * kch; e += kSThreads) {
-            const uint32_t r = e / kch, kc = e - r * kch;
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (r < qn) v = sc.rows[(size_t)(q0 + r) * kch + kc];
-            uint32_t w[4] = {v.x, v.y, v.z, v.w};
+        } else {
+            // ---- query tile [-2 q^, 1, 1, -G_hi, -G_lo] from the candidate rows; a row
+            // past qn is 0 with -G = 2^100: never undecided
+            const uint32_t nt = kSThreads - 32u;
+            for (uint32_t e = tid; e < (uint32_t)kSQ * kch; e += nt) {
+                const uint32_t kc = e / (uint32_t)kSQ, r = e - kc * (uint32_t)kSQ;
+                uint4 v = make_uint4(0u, 0u, 0u, 0u);
+                uint32_t g = 0x00007180u;  // BF16 (2^100, 0)
+                if (r < qn) {
+                    const uint32_t s = q0 + r;
+                    v = sc.rows[((size_t)(s / kGrp) * kch + kc) * kGrp + s % kGrp];
+                    g = sc.qg[s];
+                }
+                const uint16_t one = r < qn ? (uint16_t)0x3f80u : (uint16_t)0u;
+                uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-            for (int h = 0; h < 4; h++) {
-                __nv_bfloat162 b = *reinterpret_cast<__nv_bfloat162*>(&w[h]);
-                float2 f = __bfloat1622float2(b);
-                const uint32_t col = kc * 8u + 2u * (uint32_t)h;
-                f.x = col < n ? -2.f * f.x : (col < n + 2u && r < qn ? 1.f : 0.f);
-                f.y = col + 1u < n ? -2.f * f.y : (col + 1u < n + 2u && r < qn ? 1.f : 0.f);
-                b = __floats2bfloat162_rn(f.x, f.y);
-                w[h] = *reinterpret_cast<uint32_t*>(&b);
+                for (int h = 0; h < 4; h++) {
+                    uint32_t word = 0;
+#pragma unroll
+                    for (int x = 0; x < 2; x++) {
+                        const uint32_t col = kc * 8u + 2u * (uint32_t)h + (uint32_t)x;
+                        __nv_bfloat16_raw rb;
+                        rb.x = (uint16_t)(w[h] >> (16 * x));
+                        uint32_t bits;
+                        if (col < n) {
+                            // -2 q^ (exact)
+                            const __nv_bfloat16_raw d =
+                                __float2bfloat16_rn(-2.f * __bfloat162float(__nv_bfloat16(rb)));
+                            bits = d.x;
+                        } else if (col < n + 2u) {
+                            bits = one;
+                        } else if (col < n + 4u) {
+                            bits = col == n + 2u ? (g & 0xffffu) : (g >> 16);
+                        } else {
+                            bits = 0u;
+                        }
+                        word |= bits << (16 * x);
+                    }
+                    w[h] = word;
+                }
+                *reinterpret_cast<uint4*>(A + core_off(r, kc, kpad)) = make_uint4(w[0], w[1], w[2], w[3]);
             }
-            *reinterpret_cast<uint4*>(A + core_off(r, kc, kpad)) = make_uint4(w[0], w[1], w[2], w[3]);
         }
         fence_async_smem();
         __syncthreads();
-        const uint32_t total = misc[2];
-        const uint32_t T = (total + kSC - 1u) / kSC;
-        cand_total += (unsigned long long)total * qn;
+        const uint32_t groups = misc[2];
+        const uint32_t T = (groups + kTileGrps - 1u) / kTileGrps;
+        const uint32_t t0 = (uint32_t)((uint64_t)T * part / parts), t1 = (uint32_t)((uint64_t)T * (part + 1u) / parts);
+        if (part == 0u) cand_total += (unsigned long long)misc[3] * qn;
 
-        if (tid >= kProd0) {
-            // ================= producer warps: stage tile t + 1 (slots, cp.async of
-            // the rows) before publishing tile t (copies landed); one thread then
-            // issues tile t's MMA
-            const uint32_t pt = (uint32_t)tid - (uint32_t)kProd0;  // candidate row of the tile
-            uint32_t e = 0;  // neighbour range of this thread's current candidate (f grows by kSC per tile)
-            float wm_cur = 0.f, wm_next = 0.f;  // candidate norms of the last two prepared tiles
-            const uint32_t wbase = (uint32_t)(warp - 8) * 32u;  // this warp's first row of the tile
-            // stage tile t: this warp's 32 slots and rows (no barrier with the other
-            // producer warps: the stage is free once its consumers released it)
-            auto prepare = [&](uint32_t t) -> bool {
-                const uint32_t g = tiles_done + t, b = g % kStages;
-                if (g >= kStages) {
-                    bool ok = true;
-                    if (lane == 0) ok = bar_wait_bounded(free0 + 8u * b, ((g / kStages) - 1u) & 1u);
-                    if (!__shfl_sync(FULL, ok ? 1u : 0u, 0)) return false;
-                }
-                const uint32_t f = t * kSC + pt;
-                uint32_t slot = kNone;
-                wm_cur = wm_next;
-                wm_next = 0.f;
-                if (f < total) {
-                    while (nb_pref[e + 1] <= f) e++;
-                    slot = nb_start[e] + (f - nb_pref[e]);
-                    // |c^|^2 in FP32 bounds the folded hi + lo terms (reduced when the
-                    // tile is published, so that the load's latency is not waited for here)
-                    wm_next = sc.norms[slot];
-                }
-                c_slot[b * kSC + pt] = slot;
-                const uint32_t dst = smem_u32(ssm + L.b) + b * ((uint32_t)kSC * kpad * 2u);
-                if (kch <= 4u) {
-                    // short rows (up to 32 values): each thread copies its own row
-                    const bool valid = slot != kNone;
-                    const uint4* src = sc.rows + (size_t)(valid ? slot : 0u) * kch;
-                    for (uint32_t kc = 0; kc < kch; kc++)
-                        cp_async16(dst + core_off(pt, kc, kpad), src + kc, valid ? 16u : 0u);
-                } else {
-                    // longer rows: the warp's 32 rows, consecutive lanes on consecutive
-                    // chunks of a row
-                    for (uint32_t j = 0; j < kch; j++) {
-                        const uint32_t idx = j * 32u + (uint32_t)lane;
-                        const uint32_t r = idx / kch, kc = idx - r * kch;
-                        const uint32_t sl = __shfl_sync(FULL, slot, (int)r);
-                        const bool valid = sl != kNone;
-                        cp_async16(dst + core_off(wbase + r, kc, kpad),
-                                   sc.rows + (size_t)(valid ? sl : 0u) * kch + kc, valid ? 16u : 0u);
-                    }
-                }
-                asm volatile("cp.async.commit_group;" ::: "memory");
-                return true;
-            };
-            // tile t's rows landed (this thread's copies): publish slots, norm bound and rows
-            auto publish = [&](uint32_t t, bool next_pending) {
-                const uint32_t g = tiles_done + t, b = g % kStages;
-                float wm = next_pending ? wm_cur : wm_next;
-#pragma unroll
-                for (int sh = 16; sh > 0; sh >>= 1) wm = fmaxf(wm, __shfl_xor_sync(FULL, wm, sh));
-                if (lane == 0) {
-                    cwmax[b * 8u + (uint32_t)(warp - 8)] = wm;
-                    cwmax[b * 8u + 4u + (uint32_t)(warp - 8)] = __fsqrt_ru(wm);
-                }
-                if (next_pending) asm volatile("cp.async.wait_group 1;" ::: "memory");
-                else asm volatile("cp.async.wait_group 0;" ::: "memory");
-                fence_async_smem();
-                bar_arrive(staged0 + 8u * b);
-            };
-            // one thread: tile t staged by all producers and its accumulator free -> MMA
-            auto issue = [&](uint32_t t) -> bool {
-                const uint32_t g = tiles_done + t, b = g % kStages, s = g & 1u;
-                if (!bar_wait_bounded(staged0 + 8u * b, (g / kStages) & 1u)) return false;
-                if (g >= 2 && !bar_wait_bounded((s ? empty1 : empty0), ((g >> 1) - 1u) & 1u)) return false;
-                fence_after();
-                const uint32_t b_addr = smem_u32(ssm + L.b) + b * ((uint32_t)kSC * kpad * 2u);
-                for (uint32_t ks = 0; ks < (kpad >> 4); ks++)
-                    mma_bf16(tmem + s * kTmemCols, smem_desc(a_addr + ks * 256u, 128u, sbo),
-                             smem_desc(b_addr + ks * 256u, 128u, sbo), ks > 0 ? 1u : 0u);
-                mma_commit((s ? full1 : full0));
-                bar_arrive((s ? full1 : full0));
-                return true;
-            };
-            bool ok = T == 0 || prepare(0);
-            for (uint32_t t = 0; ok && t < T; t++) {
-                if (t + 1 < T) ok = prepare(t + 1);
-                if (!ok) break;
-                publish(t, t + 1 < T);
-                if (warp == 8) {
-                    bool r = true;
-                    if (lane == 0) r = issue(t);
-                    ok = __shfl_sync(FULL, r ? 1u : 0u, 0) != 0u;
+        if (warp == kCopyWarp) {
+            // ================= candidate tiles: lanes 0-15 own the groups of tile t,
+            // lanes 16-31 those of t + 1; a run of consecutive groups is one bulk copy
+            const uint32_t sub = (uint32_t)lane / kTileGrps, half = (uint32_t)lane % kTileGrps;
+            uint32_t e = 0;  // this lane's neighbour row (its group position grows by 32 per round)
+            {
+                uint32_t hi = nnb;
+                const uint32_t f = t0 * kTileGrps + (uint32_t)lane;
+                while (hi - e > 1u) {
+                    const uint32_t mid = (e + hi) / 2u;
+                    if (nb_grp[mid] <= f) e = mid;
+                    else hi = mid;
                 }
             }
-            asm volatile("cp.async.wait_all;" ::: "memory");
-            if (!ok) misc[1] = 1u;
+            uint32_t g = g0, b = g0 % stages, ph = (g0 / stages) & 1u;
+            bool ok = true;
+            for (uint32_t t = t0; ok && t < t1; t += 2u) {
+                const uint32_t f = t * kTileGrps + (uint32_t)lane;
+                const bool mine = f < groups;
+                uint32_t gid = 0;
+                unsigned char mask = 0;
+                if (mine) {
+                    while (nb_grp[e + 1] <= f) e++;
+                    const uint32_t s = nb_start[e], en = nb_end[e];
+                    gid = s / kGrp + (f - nb_grp[e]);
+                    const uint32_t b0 = gid * kGrp;
+                    const uint32_t lo = s > b0 ? s - b0 : 0u, hi = min(kGrp, en - b0);
+                    mask = (unsigned char)((0xffu << lo) & (0xffu >> (kGrp - hi)));
+                }
+                const uint32_t prev = __shfl_up_sync(FULL, gid, 1);
+                const bool head = mine && (half == 0u || gid != prev + 1u);
+                const unsigned heads = __ballot_sync(FULL, head);
+                for (uint32_t u = 0; u < 2u && t + u < t1; u++) {
+                    if (g >= stages) {
+                        ok = warp_wait_bounded(drained + 8u * b, ph ^ 1u);
+                        if (!ok) break;
+                    }
+                    const uint32_t ng = min(kTileGrps, groups - (t + u) * kTileGrps);
+                    const uint32_t bar = landed + 8u * b;
+                    if (sub == u) {
+                        m_base[(g % kMeta) * kTileGrps + half] = gid * kGrp;
+                        m_mask[(g % kMeta) * kTileGrps + half] = mask;
+                    }
+                    __syncwarp();
+                    if (lane == 0) bar_arrive_tx(bar, ng * sbo);
+                    __syncwarp();
+                    if (head && sub == u) {
+                        const unsigned after = (heads >> lane >> 1) & (0xffffu >> (half + 1u));
+                        const uint32_t len = after ? (uint32_t)__ffs(after) : ng - half;
+                        bulk_copy(b_addr + b * stage_bytes + half * sbo, sc.rows + (size_t)gid * kch * kGrp, len * sbo,
+                                  bar);
+                    }
+                    g++;
+                    if (++b == stages) {
+                        b = 0;
+                        ph ^= 1u;
+                    }
+                }
+            }
+            if (!ok) {
+                // give the copies in flight another bounded wait before the CTA stops
+                misc[1] = 1u;
+                for (uint32_t x = 0; x < stages && x < g; x++) {
+                    if (b == 0u) {
+                        b = stages;
+                        ph ^= 1u;
+                    }
+                    b--;
+                    warp_wait_bounded(landed + 8u * b, ph);
+                }
+            }
+        } else if (warp == kMmaWarp) {
+            // ================= one thread: a landed tile and a free accumulator -> MMA
+            if (lane == 0) {
+                bool ok = true;
+                uint32_t b = g0 % stages, ph = (g0 / stages) & 1u;
+                for (uint32_t t = t0, g = g0; t < t1; t++, g++) {
+                    // the first use of an accumulator waits for the phase before its first
+                    const uint32_t s = g & 1u;
+                    ok = bar_wait_bounded(landed + 8u * b, ph) &&
+                         bar_wait_bounded(empty + 8u * s, ((g >> 1) & 1u) ^ 1u);
+                    if (!ok) break;
+                    fence_after();
+                    const uint32_t bt = b_addr + b * stage_bytes;
+                    for (uint32_t ks = 0; ks < (kpad >> 4); ks++)
+                        mma_bf16(tmem + s * kTmemCols, smem_desc(a_addr + ks * 256u, 128u, sbo),
+                                 smem_desc(bt + ks * 256u, 128u, sbo), ks > 0 ? 1u : 0u);
+                    mma_commit(drained + 8u * b);
+                    mma_commit(full + 8u * s);
+                    bar_arrive(full + 8u * s);
+                    if (++b == stages) {
+                        b = 0;
+                        ph ^= 1u;
+                    }
+                }
+                if (!ok) misc[1] = 1u;
+            }
+            __syncwarp();
         } else {
             // ================= consumer warps: query row i = TMEM lane i; warps w and
             // w + 4 share lane quarter w % 4 and split the columns
             const uint32_t quarter = (uint32_t)warp & 3u, colbase = ((uint32_t)warp >> 2) * ((uint32_t)kSC / 2u);
-            const uint32_t i = quarter * 32u + (uint32_t)lane;
-            const float4 qi = qinfo[i];
-            const bool qvalid = qi.w != 0.f;
-            for (uint32_t t = 0; t < T; t++) {
-                const uint32_t g = tiles_done + t, s = g & 1u;
-                bool ok = true;
-                if (lane == 0) ok = bar_wait_bounded((s ? full1 : full0), (g >> 1) & 1u);
-                ok = __shfl_sync(FULL, ok ? 1u : 0u, 0) != 0u;
-                if (!ok) {
+            const uint32_t qslot = q0 + quarter * 32u + (uint32_t)lane;
+            const bool idle = quarter * 32u >= qn;  // no query in the warp's 32 rows
+            uint32_t und_count = 0, rec_count = 0;  // undecided pairs of the lane, records of the warp
+            for (uint32_t t = t0, g = g0; t < t1; t++, g++) {
+                const uint32_t s = g & 1u;
+                if (!warp_wait_bounded(full + 8u * s, (g >> 1) & 1u)) {
                     misc[1] = 1u;
                     break;
                 }
                 fence_after();
-                const uint32_t b = g % kStages;
-                const uint32_t nvalid = min((uint32_t)kSC, total - t * kSC);
-                // a warp whose 32 query rows are all empty still waits for every tile
-                // (its arrivals keep the phases of empty[] in order) but skips the work
-                const uint32_t col_end = (quarter * 32u < qn) ? colbase + (uint32_t)kSC / 2u : colbase;
-                for (uint32_t c32 = colbase; c32 < col_end; c32 += 32u) {
-                  // G_i from the group's largest candidate norm (an upper bound of each of
-                  // its 32 columns' bounds; the group's candidates are one producer warp's)
-                  const float cmax = cwmax[b * 8u + (c32 >> 5)], rcmax = cwmax[b * 8u + 4u + (c32 >> 5)];
-                  const float tt = __fmaf_ru(sc.ke, rcmax, qi.y);
-                  const float G =
-                      __fsub_ru(__fmaf_ru(tt, tt, __fadd_ru(qi.z, __fmul_ru(sc.c1, __fmul_ru(2.f, cmax)))), qi.x);
-                  float d32[32];
-                  tmem_ld32(tmem + s * kTmemCols + ((quarter * 32u) << 16) + c32, d32);
-                  // common case: every value of the 32 columns above G (NaN counts as undecided)
-                  bool all_out = true;
-#pragma unroll
-                  for (int jj = 0; jj < 32; jj++) all_out = all_out && (d32[jj] > G);
-                  if (__all_sync(FULL, !qvalid || all_out || c32 >= nvalid)) continue;
-                  for (uint32_t h16 = 0; h16 < 2u; h16++) {
-                    const uint32_t col0 = c32 + 16u * h16;
-                    unsigned und = 0;
-                    if (qvalid) {
-#pragma unroll
-                        for (int jj = 0; jj < 16; jj++) und |= (d32[16 * h16 + jj] > G) ? 0u : (1u << jj);
-                        if (col0 + 16u > nvalid) und &= (col0 >= nvalid) ? 0u : ((1u << (nvalid - col0)) - 1u);
-                    }
-                    if (!__any_sync(FULL, und != 0u)) continue;
-                    // the undecided pairs (query slot | cross << 31, candidate slot) go to
-                    // the exact check (k_screen_recheck), one atomic per warp and chunk
-                    const uint32_t nu = (uint32_t)__popc(und);
-                    uint32_t x = nu;
-#pragma unroll
-                    for (int sh = 1; sh < 32; sh <<= 1) {
-                        const uint32_t y = __shfl_up_sync(FULL, x, sh);
-                        if (lane >= sh) x += y;
-                    }
-                    const uint32_t wtotal = __shfl_sync(FULL, x, 31);
-                    und_count += wtotal;
-                    if (o.emit) {
-                        if (blk_used + wtotal > kBlk) {
-                            // pad the rest of the warp's block, reserve the next one
-                            for (uint32_t e2 = blk_used + (uint32_t)lane; e2 < kBlk; e2 += 32u)
-                                if (blk_base + e2 < o.cap) o.pairs[blk_base + e2] = kUndecidedPad;
-                            unsigned long long nb = 0;
-                            if (lane == 0) nb = atomicAdd(o.cursor, (unsigned long long)kBlk);
-                            blk_base = __shfl_sync(FULL, nb, 0);
-                            blk_used = 0;
-                        }
-                        unsigned long long p = blk_base + blk_used + (x - nu);
-                        blk_used += wtotal;
-                        const unsigned long long qword = (unsigned long long)(q0 + i);
-                        unsigned uu = und;
-                        while (uu) {
-                            const int bb = __ffs(uu) - 1;
-                            uu &= uu - 1u;
-                            const uint32_t sl = c_slot[b * kSC + col0 + (uint32_t)bb];
-                            const unsigned long long cr = (STAMP && (sl < cs0 || sl >= ce)) ? (1ull << 31) : 0ull;
-                            if (p < o.cap) o.pairs[p] = ((qword | cr) << 32) | sl;
-                            p++;
-                        }
-                    }
-                  }
+                const uint32_t ta = tmem + s * kTmemCols + ((quarter * 32u) << 16) + colbase;
+                if (idle) {
+                    fence_before();
+                    if (lane == 0) bar_arrive(empty + 8u * s);
+                    continue;
                 }
-                fence_before();
-                bar_arrive((s ? empty1 : empty0));
-                bar_arrive(free0 + 8u * b);
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    uint32_t v[32];
+                    tmem_ld32(ta + 32u * (uint32_t)h, v);
+                    tmem_wait_ld(v);
+                    if (h == 1) {  // the accumulator is read
+                        fence_before();
+                        __syncwarp();
+                        if (lane == 0) bar_arrive(empty + 8u * s);
+                    }
+                    // common case: every value of the 32 columns has its sign bit clear
+                    // (independent chains: one chain of dependent operations would take
+                    // several times the issue time)
+                    uint32_t x[4];
+#pragma unroll
+                    for (int c = 0; c < 4; c++) {
+                        x[c] = v[8 * c];
+#pragma unroll
+                        for (int j = 1; j < 8; j++) x[c] |= v[8 * c + j];
+                    }
+                    if (!__any_sync(FULL, (int)((x[0] | x[1]) | (x[2] | x[3])) < 0)) continue;
+                    const uint32_t mg = (g % kMeta) * kTileGrps + colbase / kGrp + 4u * (uint32_t)h;  // first group
+                    uint32_t und = 0;
+#pragma unroll
+                    for (int c = 0; c < 4; c++) {
+                        uint32_t y = 0;
+#pragma unroll
+                        for (int j = 7; j >= 0; j--) y = __funnelshift_l(v[8 * c + j], y, 1);
+                        und |= y << (8 * c);
+                    }
+                    und &= *reinterpret_cast<const uint32_t*>(m_mask + mg);
+                    und_count += (uint32_t)__popc(und);
+                    // a record per run of consecutive groups (nearly always all four)
+                    const uint4 gb = *reinterpret_cast<const uint4*>(m_base + mg);
+                    const uint32_t brk = (gb.y != gb.x + kGrp ? 1u : 0u) | (gb.z != gb.y + kGrp ? 2u : 0u) |
+                                         (gb.w != gb.z + kGrp ? 4u : 0u);
+                    for (uint32_t c0 = 0; c0 < 4u;) {
+                        // the run's groups [c0, c1), the slot gs of its first row
+                        const uint32_t cut = brk >> c0;
+                        const uint32_t c1 = cut ? c0 + (uint32_t)__ffs(cut) : 4u;
+                        const uint32_t gs = c0 == 0u ? gb.x : c0 == 1u ? gb.y : c0 == 2u ? gb.z : gb.w;
+                        const uint32_t col0 = kGrp * c0;
+                        const uint32_t mine = und & (0xffffffffu >> (32u - kGrp * c1)) & (0xffffffffu << col0);
+                        c0 = c1;
+                        const unsigned have = __ballot_sync(FULL, mine != 0u);
+                        if (!have) continue;
+                        const uint32_t cnt = (uint32_t)__popc(have);
+                        rec_count += cnt;
+                        if (!o.emit) continue;
+                        // the warp's block first, the rest in the next one
+                        unsigned long long next = 0;
+                        const bool over = blk_used + cnt > kBlk;
+                        if (over) {
+                            if (lane == 0) next = atomicAdd(o.cursor, (unsigned long long)kBlk);
+                            next = __shfl_sync(FULL, next, 0);
+                        }
+                        if (mine) {
+                            uint32_t cross = 0;
+                            if (STAMP) {
+                                // columns outside the query's cell [cs0, ce)
+                                const uint32_t lo = cs0 > gs ? min(32u, col0 + (cs0 - gs)) : col0;
+                                const uint32_t hi = ce > gs ? min(32u, col0 + (ce - gs)) : col0;
+                                const uint32_t below_hi = hi >= 32u ? 0xffffffffu : (1u << hi) - 1u;
+                                const uint32_t below_lo = lo >= 32u ? 0xffffffffu : (1u << lo) - 1u;
+                                cross = ~(below_hi & ~below_lo);
+                            }
+                            const uint32_t p = blk_used + (uint32_t)__popc(have & lt);
+                            const unsigned long long at = p < kBlk ? blk_base + p : next + (p - kBlk);
+                            // gs - col0: the slot of column 0 (modulo 2^32)
+                            if (at < o.cap) recs[at] = make_uint4(qslot, gs - col0, mine, cross);
+                        }
+                        blk_used += cnt;
+                        if (over) {
+                            blk_base = next;
+                            blk_used -= kBlk;
+                        }
+                    }
+                }
+            }
+            const uint32_t u0 = __reduce_add_sync(FULL, und_count & 0xffffu), u1 = __reduce_add_sync(FULL, und_count >> 16);
+            if (lane == 0) {
+                *n_und += u0 + ((unsigned long long)u1 << 16);
+                *n_rec += rec_count;
             }
         }
-        tiles_done += T;
+        g0 += t1 - t0;
     }
-    // ---- the consumer warps' last blocks and their exact undecided counts
-    if (tid < kProd0) {
+    // ---- the consumer warps' last blocks and their counts
+    if (tid < kConsumers) {
         if (o.emit && blk_used < kBlk)
             for (uint32_t e2 = blk_used + (uint32_t)lane; e2 < kBlk; e2 += 32u)
-                if (blk_base + e2 < o.cap) o.pairs[blk_base + e2] = kUndecidedPad;
-        if (lane == 0 && und_count) atomicAdd(o.rechecks, und_count);
+                if (blk_base + e2 < o.cap) recs[blk_base + e2] = make_uint4(0u, 0u, 0u, 0u);
+        if (lane == 0 && *n_und) atomicAdd(o.rechecks, *n_und);
+        if (lane == 0 && !o.emit && *n_rec) atomicAdd(o.cursor, *n_rec);
     }
-    // ---- tear-down: every MMA this CTA issued has been waited for (the last
-    // tiles by the epilogue), unless a wait timed out
+    // ---- tear-down: every copy and MMA of this CTA has been waited for by its
+    // consumers, unless a wait timed out
     if (misc[1] && tid == 0) *a.err_flag = 2u;
     fence_before();
     __syncthreads();
@@ -622,11 +734,15 @@ __global__ void __launch_bounds__(kSThreads, 2) k_tile_screen(const JoinArgs<flo
     if (tid == 0 && o.emit && cand_total) atomicAdd(a.cand_cnt, cand_total);
 }
 
-template <int MODEL, bool STAMP>
-cudaError_t launch_screen_one(const JoinArgs<float>& a, const TileOut& o, const ScreenConst& sc, uint32_t noff,
+template <bool STAMP>
+cudaError_t launch_screen_one(const JoinArgs<float>& a, const TileOut& o, const ScreenConst& sc, uint32_t nrow,
                               uint32_t nvisit, int num_sms, cudaStream_t st) {
-    auto kern = k_tile_screen<MODEL, STAMP>;
-    const ScreenSmem L = screen_smem(sc.kpad, noff);
+    auto kern = k_tile_screen<STAMP>;
+    // as many candidate tiles in flight as leave room for two CTAs on an SM
+    const uint32_t two = (228u * 1024u) / 2u - 1024u;
+    uint32_t stages = 2;
+    while (stages < kMaxStages && screen_smem(sc.kpad, nrow, stages + 1u).total <= two) stages++;
+    const ScreenSmem L = screen_smem(sc.kpad, nrow, stages);
     const uint32_t smem = L.total > kMinSmem ? L.total : kMinSmem;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -642,8 +758,13 @@ cudaError_t launch_screen_one(const JoinArgs<float>& a, const TileOut& o, const 
     if ((uint32_t)per_sm * 2u * kTmemCols > 512u) per_sm = (int)(512u / (2u * kTmemCols));
     if (a.shape_per_sm && (int)a.shape_per_sm < per_sm) per_sm = (int)a.shape_per_sm;
     uint64_t blocks = (uint64_t)num_sms * per_sm;
-    if (blocks > nvisit) blocks = nvisit ? nvisit : 1;
-    kern<<<(unsigned)blocks, kSThreads, smem, st>>>(a, o, sc, noff, nvisit);
+    // slices per item: 16 units per CTA, so that the last wave is short
+    uint64_t parts = (blocks * kUnitsPerCta + nvisit - 1u) / nvisit;
+    if (parts > kMaxParts) parts = kMaxParts;
+    const uint64_t units = (uint64_t)nvisit * parts;
+    if (units + blocks >= 0xffffffffull) return cudaErrorInvalidValue;
+    if (blocks > units) blocks = units;
+    kern<<<(unsigned)blocks, kSThreads, smem, st>>>(a, o, sc, nrow, stages, (uint32_t)parts, (uint32_t)units);
     return cudaGetLastError();
 }
 
@@ -651,132 +772,222 @@ cudaError_t launch_screen_one(const JoinArgs<float>& a, const TileOut& o, const 
 
 // The exact check of the pairs the screen could not reject: the reference's
 // arithmetic for the configured model (kernel.cu:307-365), s <= thr; a hit
-// appends (query id, candidate id), and with the cross flag (unicomp, the
-// candidate outside the query's cell) also the reverse pair.
+// appends (query id, candidate id), and with the record's cross bit (unicomp,
+// the candidate outside the query's cell) also the reverse pair.  A warp takes
+// 32 records, lists their pairs in shared memory and checks 32 pairs at a time,
+// so that records of one pair and of 32 keep the lanes equally busy.
 template <int MODEL, bool STAMP>
-__global__ void __launch_bounds__(256) k_screen_recheck(const float* __restrict__ pts, const uint32_t* __restrict__ ids,
+__global__ void __launch_bounds__(256, 4) k_screen_recheck(const float* __restrict__ pts, const uint32_t* __restrict__ ids,
                                                         uint32_t n, uint32_t npad, uint32_t ilp, float thr,
-                                                        uint32_t npoints, const unsigned long long* __restrict__ unc,
-                                                        unsigned long long nunc, const TileOut o) {
+                                                        uint32_t npoints, const uint4* __restrict__ recs,
+                                                        unsigned long long nrec, const TileOut o) {
+    __shared__ uint16_t list[8][1024];  // record lane << 5 | column
     const unsigned FULL = 0xffffffffu;
     const unsigned lt = lanemask_lt_s();
+    const uint32_t lane = threadIdx.x & 31u;
+    uint16_t* wl = list[threadIdx.x >> 5];
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < nunc; i0 += stride) {
-        const uint64_t e = i0 + threadIdx.x;
-        bool hit = false, cross = false;
-        uint32_t qs = 0, cs = 0;
-        const unsigned long long w = e < nunc ? unc[e] : kUndecidedPad;
-        const uint32_t qw = (uint32_t)(w >> 32);
-        if (w != kUndecidedPad && (qw & 0x7fffffffu) < npoints && (uint32_t)w < npoints) {
-            cs = (uint32_t)w;
-            qs = qw & 0x7fffffffu;
-            const float d = exact_sqdist4<MODEL>(pts + (size_t)qs * npad, pts + (size_t)cs * npad, n, ilp, thr);
-            hit = d <= thr;
-            cross = STAMP && hit && (qw >> 31) != 0u;
+    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); i0 < nrec; i0 += stride) {
+        const uint4 r = i0 + lane < nrec ? recs[i0 + lane] : make_uint4(0u, 0u, 0u, 0u);
+        const uint32_t cnt = (uint32_t)__popc(r.z);
+        uint32_t x = cnt;
+#pragma unroll
+        for (int s = 1; s < 32; s <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULL, x, s);
+            if (lane >= (uint32_t)s) x += y;
         }
-        const unsigned hb = __ballot_sync(FULL, hit), cb = __ballot_sync(FULL, cross);
-        if (hb == 0u) continue;
-        const uint32_t wtotal = (uint32_t)__popc(hb) + (uint32_t)__popc(cb);
-        unsigned long long base = 0;
-        if ((threadIdx.x & 31u) == 0u) base = atomicAdd(o.cursor, (unsigned long long)wtotal);
-        base = __shfl_sync(FULL, base, 0);
-        if (hit) {
-            unsigned long long p = base + (unsigned)__popc(hb & lt) + (unsigned)__popc(cb & lt);
-            const uint64_t qid = ids[qs], cid = ids[cs];
-            if (p < o.cap) o.pairs[p] = (qid << o.shift) | cid;
-            p++;
-            if (cross && p < o.cap) o.pairs[p] = (cid << o.shift) | qid;
+        const uint32_t total = __shfl_sync(FULL, x, 31);
+        uint32_t pos = x - cnt;
+        for (uint32_t m = r.z; m; m &= m - 1u) wl[pos++] = (uint16_t)((lane << 5) | ((uint32_t)__ffs(m) - 1u));
+        __syncwarp();
+        for (uint32_t b = 0; b < total; b += 32u) {
+            const bool valid = b + lane < total;
+            const uint32_t e = valid ? wl[b + lane] : 0u;
+            const uint32_t qs = __shfl_sync(FULL, r.x, (int)(e >> 5));
+            const uint32_t cs = __shfl_sync(FULL, r.y, (int)(e >> 5)) + (e & 31u);
+            const uint32_t crossm = STAMP ? __shfl_sync(FULL, r.w, (int)(e >> 5)) : 0u;
+            bool hit = false;
+            if (valid && qs < npoints && cs < npoints)
+                hit = exact_sqdist4<MODEL>(pts + (size_t)qs * npad, pts + (size_t)cs * npad, n, ilp, thr) <= thr;
+            const bool cross = STAMP && hit && ((crossm >> (e & 31u)) & 1u);
+            const unsigned hb = __ballot_sync(FULL, hit), cb = __ballot_sync(FULL, cross);
+            if (hb == 0u) continue;
+            const uint32_t wtotal = (uint32_t)__popc(hb) + (uint32_t)__popc(cb);
+            unsigned long long base = 0;
+            if (lane == 0u) base = atomicAdd(o.cursor, (unsigned long long)wtotal);
+            base = __shfl_sync(FULL, base, 0);
+            if (hit) {
+                unsigned long long p = base + (unsigned)__popc(hb & lt) + (unsigned)__popc(cb & lt);
+                const uint64_t qid = ids[qs], cid = ids[cs];
+                if (p < o.cap) o.pairs[p] = (qid << o.shift) | cid;
+                p++;
+                if (cross && p < o.cap) o.pairs[p] = (cid << o.shift) | qid;
+            }
         }
+        __syncwarp();
     }
 }
 
 template <int MODEL, bool STAMP>
-cudaError_t launch_recheck_one(const JoinArgs<float>& a, const unsigned long long* unc, unsigned long long nunc,
+cudaError_t launch_recheck_one(const JoinArgs<float>& a, const uint4* recs, unsigned long long nrec,
                                const TileOut& o, int num_sms, cudaStream_t st) {
-    uint64_t blocks = (nunc + 255) / 256;
+    uint64_t blocks = (nrec + 255) / 256;
     const uint64_t cap = (uint64_t)num_sms * 16;
     if (blocks > cap) blocks = cap;
     k_screen_recheck<MODEL, STAMP><<<(unsigned)blocks, 256, 0, st>>>(a.pts, a.ids, a.n, a.npad, a.ilp, a.thr,
-                                                                     a.n_points, unc, nunc, o);
+                                                                     a.n_points, recs, nrec, o);
     return cudaGetLastError();
 }
 
 // Per-block FP64 column sums and counts of the finite values over a fixed row
-// range (deterministic).  Non-finite coordinates are left out of the centre,
-// so that only their own rows (and pairs) become inconclusive for the screen.
-__global__ void k_col_partial(const float* __restrict__ pts, uint32_t N, uint32_t n, uint32_t npad,
-                              double* __restrict__ partial) {
+// range (deterministic): a thread keeps one column (the block's threads cover
+// whole rows, so a row is read by consecutive threads), the threads of a
+// column are added in order.  Non-finite coordinates are left out of the
+// centre, so that only their own rows (and pairs) become inconclusive for the
+// screen.
+constexpr uint32_t kColThreads = 512;
+
+__global__ void __launch_bounds__(kColThreads) k_col_partial(const float* __restrict__ pts, uint32_t N, uint32_t n,
+                                                             uint32_t npad, double* __restrict__ partial) {
+    __shared__ double s_acc[kColThreads], s_cnt[kColThreads];
+    const uint32_t rpi = kColThreads / npad;  // rows per iteration (npad <= kTileMaxN)
+    const uint32_t tr = threadIdx.x / npad, d = threadIdx.x - tr * npad;
     const uint32_t per = (N + gridDim.x - 1) / gridDim.x;
-    const uint32_t r0 = blockIdx.x * per, r1 = min(N, r0 + per);
-    for (uint32_t d = threadIdx.x; d < n; d += blockDim.x) {
-        double acc = 0.0, cnt = 0.0;
-        for (uint32_t r = r0; r < r1; r++) {
+    const uint32_t r0 = min(N, blockIdx.x * per), r1 = min(N, r0 + per);
+    double acc = 0.0, cnt = 0.0;
+    if (tr < rpi && d < n) {
+#pragma unroll 4
+        for (uint32_t r = r0 + tr; r < r1; r += rpi) {
             const float v = pts[(size_t)r * npad + d];
             if (isfinite(v)) {
                 acc += (double)v;
                 cnt += 1.0;
             }
         }
+    }
+    s_acc[threadIdx.x] = acc;
+    s_cnt[threadIdx.x] = cnt;
+    __syncthreads();
+    if (threadIdx.x < n) {
+        for (uint32_t t = 1; t < rpi; t++) {
+            acc += s_acc[t * npad + d];
+            cnt += s_cnt[t * npad + d];
+        }
         partial[((size_t)blockIdx.x * n + d) * 2] = acc;
         partial[((size_t)blockIdx.x * n + d) * 2 + 1] = cnt;
     }
 }
 
+// A warp per column: the blocks' sums, lane-strided, then a fixed tree.
 __global__ void k_col_mean(const double* __restrict__ partial, uint32_t nblocks, uint32_t n,
                            float* __restrict__ centre) {
-    for (uint32_t d = threadIdx.x; d < n; d += blockDim.x) {
-        double acc = 0.0, cnt = 0.0;
-        for (uint32_t b = 0; b < nblocks; b++) {
-            acc += partial[((size_t)b * n + d) * 2];
-            cnt += partial[((size_t)b * n + d) * 2 + 1];
-        }
-        const double m = cnt > 0.0 ? acc / cnt : 0.0;
-        centre[d] = isfinite(m) ? (float)m : 0.f;
+    const uint32_t d = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+    if (d >= n) return;
+    double acc = 0.0, cnt = 0.0;
+    for (uint32_t b = lane; b < nblocks; b += 32u) {
+        acc += partial[((size_t)b * n + d) * 2];
+        cnt += partial[((size_t)b * n + d) * 2 + 1];
     }
+    for (int s = 16; s > 0; s >>= 1) {
+        acc += __shfl_xor_sync(0xffffffffu, acc, s);
+        cnt += __shfl_xor_sync(0xffffffffu, cnt, s);
+    }
+    const double m = cnt > 0.0 ? acc / cnt : 0.0;
+    if (lane == 0) centre[d] = isfinite(m) ? (float)m : 0.f;
 }
 
-// Row s: x' = fl(x - centre), c^ = bf16(x'), |c^|^2 in FP32 (sequential
-// fused sum of the exact squares), split into two BF16 terms.
-__global__ void k_screen_rows(const float* __restrict__ pts, uint32_t N, uint32_t n, uint32_t npad, uint32_t kpad,
-                              const float* __restrict__ centre, uint4* __restrict__ rows, float* __restrict__ norms) {
-    const uint32_t kch = kpad >> 3;
-    for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < N; s += gridDim.x * blockDim.x) {
-        const float* x = pts + (size_t)s * npad;
-        float nrm = 0.f;
-        for (uint32_t kc = 0; kc < kch; kc++) {
-            uint32_t w[4];
+// Row of slot s (see the head of this file): x' = fl(x - centre), c^ =
+// bf16(x'), |c^|^2 between nlo and nhi, r bounded above by the exact residual
+// x' - c^ and 2^-23 of the row's length for the centring.
+__global__ void k_screen_rows(const float* __restrict__ pts, uint32_t N, uint32_t n, uint32_t npad,
+                              const ScreenConst sc, const float* __restrict__ centre, uint4* __restrict__ rows,
+                              uint32_t* __restrict__ qg) {
+    const uint32_t kch = sc.kpad >> 3;
+    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= (N + kGrp - 1u) / kGrp * kGrp) return;
+    uint4* row = rows + (size_t)(s / kGrp) * kch * kGrp + s % kGrp;  // chunk kc at row[kc * kGrp]
+    if (s >= N) {  // the last group's unused rows
+        for (uint32_t kc = 0; kc < kch; kc++) row[kc * kGrp] = make_uint4(0u, 0u, 0u, 0u);
+        return;
+    }
+    const float* x = pts + (size_t)s * npad;
+    float nlo = 0.f, nhi = 0.f, rsq = 0.f;
+    uint32_t w[4];
+    auto bits_of = [](__nv_bfloat16 b) { return (uint32_t)__bfloat16_as_ushort(b); };
+    const uint32_t full = n >> 3;  // chunks of coordinates alone
+    auto coord = [&](uint32_t l) -> uint32_t {
+        const float xp = __fsub_rn(x[l], centre[l]);
+        const __nv_bfloat16 b = __float2bfloat16_rn(xp);
+        const float f = __bfloat162float(b), e = __fsub_rn(xp, f);
+        nlo = __fmaf_rd(f, f, nlo);
+        nhi = __fmaf_ru(f, f, nhi);
+        rsq = __fmaf_ru(e, e, rsq);
+        return bits_of(b);
+    };
+    for (uint32_t kc = 0; kc < full; kc++) {
 #pragma unroll
-            for (int h = 0; h < 4; h++) {
-                const uint32_t l = kc * 8u + 2u * (uint32_t)h;
-                const float x0 = l < n ? __fsub_rn(x[l], centre[l]) : 0.f;
-                const float x1 = l + 1u < n ? __fsub_rn(x[l + 1u], centre[l + 1u]) : 0.f;
-                const __nv_bfloat162 b = __floats2bfloat162_rn(x0, x1);
-                const float2 f = __bfloat1622float2(b);
-                nrm = __fmaf_rn(f.x, f.x, nrm);
-                nrm = __fmaf_rn(f.y, f.y, nrm);
-                w[h] = *reinterpret_cast<const uint32_t*>(&b);
-            }
-            rows[(size_t)s * kch + kc] = make_uint4(w[0], w[1], w[2], w[3]);
+        for (int h = 0; h < 4; h++) {
+            const uint32_t lo = coord(kc * 8u + 2u * (uint32_t)h), hi = coord(kc * 8u + 2u * (uint32_t)h + 1u);
+            w[h] = lo | (hi << 16);
         }
-        // the norm terms go to columns n and n + 1
-        const __nv_bfloat16 hi = __float2bfloat16_rn(nrm);
-        const __nv_bfloat16 lo = __float2bfloat16_rn(__fsub_rn(nrm, __bfloat162float(hi)));
-        __nv_bfloat16* rb = reinterpret_cast<__nv_bfloat16*>(rows + (size_t)s * kch);
-        rb[n] = hi;
-        rb[n + 1u] = lo;
-        norms[s] = nrm;
+        row[kc * kGrp] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    // the remaining coordinates (fewer than 8), then A_hi, A_lo, 1, 1 and zeros
+    uint32_t tail[8];
+#pragma unroll
+    for (uint32_t i = 0; i < 8u; i++) tail[i] = full * 8u + i < n ? coord(full * 8u + i) : 0u;
+    const float len = __fsqrt_ru(nhi);
+    float r = __fsqrt_ru(rsq);
+    r = __fmaf_ru(0x1p-23f, __fadd_ru(len, r), r);
+    const float r2 = __fmul_ru(__fadd_ru(r, r), r), r0r = __fmul_ru(__fadd_ru(sc.r0, sc.r0), r);
+    const float acc = __fmul_ru(sc.c1, nhi), r0sq = __fmul_ru(sc.r0, sc.r0);
+    const bool far = !(nhi <= kFar) || !(rsq <= kFar);
+    uint32_t ahi, alo, ghi, glo;
+    if (far) {
+        ahi = ghi = 0xfb80u;  // BF16 -2^120
+        alo = glo = 0u;
+    } else {
+        const float A = __fsub_rd(__fsub_rd(__fsub_rd(nlo, r0r), r2), acc);
+        const __nv_bfloat16 h = __float2bfloat16_rn(A);
+        ahi = bits_of(h);
+        alo = bits_of(__float2bfloat16_rd(__fsub_rn(A, __bfloat162float(h))));
+        float G = __fadd_ru(__fadd_ru(__fadd_ru(r0sq, r0r), r2), acc);
+        G = __fsub_ru(__fmaf_ru(sc.c0, r0sq, G), nlo);
+        const __nv_bfloat16 gh = __float2bfloat16_rn(G);
+        const __nv_bfloat16 gl = __float2bfloat16_ru(__fsub_rn(G, __bfloat162float(gh)));
+        ghi = bits_of(gh) ^ 0x8000u;
+        glo = bits_of(gl) ^ 0x8000u;
+    }
+    qg[s] = ghi | (glo << 16);
+    if (far) {
+        for (uint32_t kc = 0; kc < full; kc++) row[kc * kGrp] = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int i = 0; i < 8; i++) tail[i] = 0u;
+    }
+    for (uint32_t kc = full; kc < kch; kc++) {
+        uint32_t c[8];
+#pragma unroll
+        for (uint32_t i = 0; i < 8u; i++) {
+            const uint32_t col = kc * 8u + i;
+            c[i] = col < n        ? tail[i]
+                   : col == n     ? ahi
+                   : col == n + 1 ? alo
+                   : col < n + 4u ? 0x3f80u
+                                  : 0u;
+        }
+        row[kc * kGrp] = make_uint4(c[0] | (c[1] << 16), c[2] | (c[3] << 16), c[4] | (c[5] << 16), c[6] | (c[7] << 16));
     }
 }
 
-cudaError_t launch_screen_prep(const float* pts, uint32_t N, uint32_t n, uint32_t npad, uint32_t kpad,
-                               double* partial, float* centre, uint4* rows, float* norms, cudaStream_t st) {
+uint64_t screen_rows_count(uint64_t N, uint32_t kpad) { return (N + kGrp - 1u) / kGrp * kGrp * (kpad / 8u); }
+
+cudaError_t launch_screen_prep(const float* pts, uint32_t N, uint32_t n, uint32_t npad, const ScreenConst& sc,
+                               double* partial, float* centre, uint4* rows, uint32_t* qg, cudaStream_t st) {
     if (N == 0) return cudaSuccess;
-    if (kpad < n + 2u || (kpad & 7u)) return cudaErrorInvalidValue;
-    k_col_partial<<<kScreenPrepBlocks, 128, 0, st>>>(pts, N, n, npad, partial);
-    k_col_mean<<<1, 128, 0, st>>>(partial, kScreenPrepBlocks, n, centre);
-    uint64_t blocks = ((uint64_t)N + 255) / 256;
-    if (blocks > 148u * 16u) blocks = 148u * 16u;
-    k_screen_rows<<<(unsigned)blocks, 256, 0, st>>>(pts, N, n, npad, kpad, centre, rows, norms);
+    if (sc.kpad < n + 4u || (sc.kpad & 15u) || npad > kTileMaxN) return cudaErrorInvalidValue;
+    k_col_partial<<<kScreenPrepBlocks, kColThreads, 0, st>>>(pts, N, n, npad, partial);
+    k_col_mean<<<(n + 7u) / 8u, 256, 0, st>>>(partial, kScreenPrepBlocks, n, centre);
+    k_screen_rows<<<(unsigned)(((uint64_t)N + 7u + 255u) / 256u), 256, 0, st>>>(pts, N, n, npad, sc, centre, rows, qg);
     return cudaGetLastError();
 }
 
@@ -788,53 +999,45 @@ bool screen_supported(uint32_t n, uint32_t npad, uint32_t k, int model, uint32_t
 
 ScreenConst make_screen_const(uint32_t n, float thr) {
     ScreenConst sc{};
-    sc.kpad = (n + 2u + 15u) & ~15u;
-    // R0 >= sqrt(thr / (1 - (2n + 8) 2^-24)), plus room for the FP32 evaluation of G
+    sc.kpad = (n + 4u + 15u) & ~15u;
+    // R0 >= sqrt(thr / (1 - (2n + 8) 2^-24)), plus room for the FP32 evaluation of A and G
     const double r0 = std::sqrt((double)thr) * (1.0 + (2.0 * n + 8.0) * 0x1p-24 + 0x1p-19);
     sc.r0 = std::nextafter((float)r0, INFINITY);
-    // BF16 rounding of a centred coordinate: |x - bf16(x)| <= 2^-8 |x|, plus
-    // the centring subtraction and the square root of the norm
-    sc.ke = 0x1p-8f * 1.0045f;
-    // FP32 accumulation (K + 32 steps of 2^-20) and the two-term split of the
-    // folded candidate norm (2^-16)
-    sc.c1 = (float)(sc.kpad + 48u) * 0x1p-20f;
+    // FP32 accumulation (K + 32 steps of 2^-20) of at most 2.1 (|q^|^2 + |c^|^2)
+    // + 1.1 R0^2 in magnitude: 2 |q^.c^| <= |q^|^2 + |c^|^2, and |A| and |G| are
+    // at most (1 + 2^-6)(|c^|^2 + 2^-8 R0^2) and (1 + 2^-6)(|q^|^2 + R0^2)
+    // because r <= 2^-8 (1 + 2^-7) |c^| for finite points
+    sc.c1 = 2.1f * (float)(sc.kpad + 32u) * 0x1p-20f;
+    sc.c0 = 1.1f * (float)(sc.kpad + 32u) * 0x1p-20f;
     return sc;
 }
 
-cudaError_t launch_screen_recheck(const JoinArgs<float>& a, const unsigned long long* unc, unsigned long long nunc,
+cudaError_t launch_screen_recheck(const JoinArgs<float>& a, const uint4* recs, unsigned long long nrec,
                                   const TileOut& o, bool stamp, int model, int num_sms, cudaStream_t st) {
-    if (nunc == 0) return cudaSuccess;
-    if ((a.npad & 3u) || !unc) return cudaErrorInvalidValue;
+    if (nrec == 0) return cudaSuccess;
+    if ((a.npad & 3u) || !recs) return cudaErrorInvalidValue;
     switch (model * 2 + (stamp ? 1 : 0)) {
-        case kSeq * 2: return launch_recheck_one<kSeq, false>(a, unc, nunc, o, num_sms, st);
-        case kSeq * 2 + 1: return launch_recheck_one<kSeq, true>(a, unc, nunc, o, num_sms, st);
-        case kIlp * 2: return launch_recheck_one<kIlp, false>(a, unc, nunc, o, num_sms, st);
-        case kIlp * 2 + 1: return launch_recheck_one<kIlp, true>(a, unc, nunc, o, num_sms, st);
-        case kIlpSc * 2: return launch_recheck_one<kIlpSc, false>(a, unc, nunc, o, num_sms, st);
-        case kIlpSc * 2 + 1: return launch_recheck_one<kIlpSc, true>(a, unc, nunc, o, num_sms, st);
+        case kSeq * 2: return launch_recheck_one<kSeq, false>(a, recs, nrec, o, num_sms, st);
+        case kSeq * 2 + 1: return launch_recheck_one<kSeq, true>(a, recs, nrec, o, num_sms, st);
+        case kIlp * 2: return launch_recheck_one<kIlp, false>(a, recs, nrec, o, num_sms, st);
+        case kIlp * 2 + 1: return launch_recheck_one<kIlp, true>(a, recs, nrec, o, num_sms, st);
+        case kIlpSc * 2: return launch_recheck_one<kIlpSc, false>(a, recs, nrec, o, num_sms, st);
+        case kIlpSc * 2 + 1: return launch_recheck_one<kIlpSc, true>(a, recs, nrec, o, num_sms, st);
         default: return cudaErrorInvalidValue;
     }
 }
 
 cudaError_t launch_tile_screen(const JoinArgs<float>& a, const TileOut& o, const ScreenConst& sc, bool stamp,
                                int model, uint32_t nvisit, int num_sms, cudaStream_t st) {
-    if (!screen_supported(a.n, a.npad, a.g.k, model, a.ilp, a.thr) || o.stride == 0 || sc.kpad < a.n + 2u ||
-        !sc.rows || !sc.norms ||
-        (sc.kpad & 15u) || sc.kpad > kTileMaxN)
+    if (!screen_supported(a.n, a.npad, a.g.k, model, a.ilp, a.thr) || o.stride == 0 || sc.kpad < a.n + 4u ||
+        !sc.rows || !sc.qg || (sc.kpad & 15u) || sc.kpad > kMaxKpad)
         return cudaErrorInvalidValue;
     if (nvisit == 0) return cudaSuccess;
     if ((uint64_t)(nvisit - 1) * o.stride >= a.num_items) return cudaErrorInvalidValue;
-    uint32_t noff = 1;
-    for (uint32_t j = 0; j < a.g.k; j++) noff *= 3u;
-    switch (model * 2 + (stamp ? 1 : 0)) {
-        case kSeq * 2: return launch_screen_one<kSeq, false>(a, o, sc, noff, nvisit, num_sms, st);
-        case kSeq * 2 + 1: return launch_screen_one<kSeq, true>(a, o, sc, noff, nvisit, num_sms, st);
-        case kIlp * 2: return launch_screen_one<kIlp, false>(a, o, sc, noff, nvisit, num_sms, st);
-        case kIlp * 2 + 1: return launch_screen_one<kIlp, true>(a, o, sc, noff, nvisit, num_sms, st);
-        case kIlpSc * 2: return launch_screen_one<kIlpSc, false>(a, o, sc, noff, nvisit, num_sms, st);
-        case kIlpSc * 2 + 1: return launch_screen_one<kIlpSc, true>(a, o, sc, noff, nvisit, num_sms, st);
-        default: return cudaErrorInvalidValue;
-    }
+    uint32_t nrow = 1;  // neighbour rows: 3^(k-1)
+    for (uint32_t j = 1; j < a.g.k; j++) nrow *= 3u;
+    return stamp ? launch_screen_one<true>(a, o, sc, nrow, nvisit, num_sms, st)
+                 : launch_screen_one<false>(a, o, sc, nrow, nvisit, num_sms, st);
 }
 
 }  // namespace gsj

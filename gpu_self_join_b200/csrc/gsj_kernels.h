@@ -126,32 +126,36 @@ cudaError_t launch_pairs_to_table(const unsigned long long* keys, uint64_t R, ui
 constexpr int kScreenQ = 128;         // queries per screened work item (MMA M)
 struct ScreenConst {
     float r0;             // >= sqrt(thr) with the reference sum's rounding room
-    float ke;             // BF16 rounding bound per unit norm
-    float c1;             // FP32 accumulation bound per unit squared norm
-    uint32_t kpad;        // dimensions + 2 padded to the MMA K step (16)
-    const uint4* rows;    // [N][kpad/8] centred BF16 rows [c^, |c^|^2_hi, |c^|^2_lo, 0...], slot order
-    const float* norms;   // [N] |c^|^2 (FP32 sum of the BF16 squares)
+    float c1, c0;         // FP32 accumulation bound per unit squared norm, per unit r0^2
+    uint32_t kpad;        // dimensions + 4 padded to the MMA K step (16)
+    const uint4* rows;    // [ceil(N/8)][kpad/8][8] BF16 rows in groups of 8 slots (gsj_join_screen.cu)
+    const uint32_t* qg;   // [N] the query side's (-G_hi, -G_lo), packed BF16
 };
-// Centred BF16 rows and norms of all points (slot order) for the screen:
-// centre = per-dimension mean of the finite values (deterministic two-level
-// FP64 sum); `partial` holds kScreenPrepBlocks x n x 2 doubles, `centre` n floats.
-constexpr uint32_t kScreenPrepBlocks = 256;
-cudaError_t launch_screen_prep(const float* pts, uint32_t N, uint32_t n, uint32_t npad, uint32_t kpad,
-                               double* partial, float* centre, uint4* rows, float* norms, cudaStream_t st);
+// BF16 rows and query terms of all points (slot order) for the screen: centre
+// = per-dimension mean of the finite values (deterministic two-level FP64
+// sum); `partial` holds kScreenPrepBlocks x n x 2 doubles, `centre` n floats,
+// `rows` screen_rows_count(N, kpad) uint4s.
+constexpr uint32_t kScreenPrepBlocks = 592;
+uint64_t screen_rows_count(uint64_t N, uint32_t kpad);
+cudaError_t launch_screen_prep(const float* pts, uint32_t N, uint32_t n, uint32_t npad, const ScreenConst& sc,
+                               double* partial, float* centre, uint4* rows, uint32_t* qg, cudaStream_t st);
 bool screen_supported(uint32_t n, uint32_t npad, uint32_t k, int model, uint32_t ilp, float thr);
 ScreenConst make_screen_const(uint32_t n, float thr);
-// Screen pass: the undecided pairs, packed as (query slot | cross << 31) << 32
-// | candidate slot, go to o.pairs in blocks of kScreenBlockSlack entries that
-// consumer warps reserve on o.cursor; a warp abandons its block when its next
-// chunk (up to 512 pairs) does not fit, padding the tail with kUndecidedPad,
-// so up to 511 entries of every block and most of each warp's last block can
-// stay unused; o.rechecks receives the exact number of undecided pairs.
+// Screen pass: the undecided pairs go to o.pairs as 16-byte records {query
+// slot, slot of column 0, mask of 32 columns, mask of the columns outside the
+// query's cell (unicomp)}, in blocks of kScreenBlock records that consumer warps
+// reserve on o.cursor and fill one after another, so that only a warp's last
+// block has unused records (mask 0); o.cap counts records; o.rechecks receives
+// the exact number of undecided pairs.  Without emission o.cursor receives the
+// number of records.
+constexpr uint32_t kScreenBlock = 256;
+// Keys of the warp join: blocks of kScreenBlockSlack entries, unused tails kUndecidedPad.
 constexpr unsigned long long kUndecidedPad = ~0ull;
 constexpr uint64_t kScreenBlockSlack = 1024;
 cudaError_t launch_tile_screen(const JoinArgs<float>& a, const TileOut& o, const ScreenConst& sc, bool stamp,
                                int model, uint32_t nvisit, int num_sms, cudaStream_t st);
 // Exact check of the undecided pairs; hits go to o as packed (query id, candidate id) keys.
-cudaError_t launch_screen_recheck(const JoinArgs<float>& a, const unsigned long long* unc, unsigned long long nunc,
+cudaError_t launch_screen_recheck(const JoinArgs<float>& a, const uint4* recs, unsigned long long nrec,
                                   const TileOut& o, bool stamp, int model, int num_sms, cudaStream_t st);
 
 // Brute-force neighbour counts over all N^2 pairs (the reference's algorithm
