@@ -172,10 +172,10 @@ struct gsj_context {
     cudaEvent_t ev[2] = {nullptr, nullptr};
     cudaEvent_t tev[8] = {};  // stage timing: index, count, fill (start/end), estimate start/end
     // device pool
-    Buf in, pts, ids, keys, keys2, vals, cell_key, cell_start, dense, dcnt, plan, plan_par, slot_cell, hkeys, hvals, order,
+    Buf in, pts, ids, keys, keys2, vals, cell_key, cell_start, dense, dcnt, plan, slot_cell, htab, order,
         sizes, nchunks,
         item_off, items, fwd, swords, counts, offsets, table, temp, scan_temp, misc, var, perm, minarr,
-        minmax_part, pairs, srows, snorms, spartial, scentre, unc, table2, nbtab, bitoff, hitbits, ptemp, sortv;
+        minmax_part, pairs, srows, snorms, spartial, scentre, unc, table2, nbtab, bitoff, hitbits, ptemp, sortv, heavy, gstart;
     PinnedBuf stage[2];
     PinnedBuf hmisc;
     // host-result pipeline: copy streams, per-segment events, pinned staging
@@ -479,7 +479,7 @@ int learned_estimate(gsj_context* c, double* est) {
 // the buffer; a short buffer is re-sized exactly and the pass repeated), then
 // the keys are sorted into the table.
 template <typename T>
-int emit_join(gsj_context* c, JoinArgs<T>& a, uint64_t N, bool stamp, int model, bool rows, bool exact_size,
+int emit_join(gsj_context* c, JoinArgs<T>& a, uint64_t N, bool stamp, int model, bool exact_size,
               bool learned, uint32_t* counts, uint64_t* offsets, unsigned long long* cursor, double t_join,
               double t_start) {
     constexpr uint32_t kSampleStride = 64;
@@ -494,12 +494,19 @@ int emit_join(gsj_context* c, JoinArgs<T>& a, uint64_t N, bool stamp, int model,
     o.shift = shift;
     unsigned long long* cand = reinterpret_cast<unsigned long long*>(a.work_counter + 2);
     // a warp appends at most 64 keys at once (32 hits and their reverse keys);
-    // at most 64 warps per SM are resident
-    const uint64_t warps = (uint64_t)c->num_sms * 64u;
+    // at most 64 warps per SM are resident, in each of the two launches of a pass
+    const uint64_t warps = (uint64_t)c->num_sms * 128u;
+    HeavyList heavy{};
+    GSJ_TRY(dev_get(c, c->heavy, kHeavyCap, &heavy.list));
+    heavy.cap = kHeavyCap;
+    heavy.count = reinterpret_cast<uint32_t*>(cursor + 2);
+    heavy.claim = heavy.count + 1;
+    int nl = 0;
     const uint64_t slack = warps * kScreenBlockSlack;
     auto reset = [&]() -> int {
         GSJ_CUDA(c, cudaMemsetAsync(a.work_counter, 0, 4 * sizeof(uint32_t), st));
-        GSJ_CUDA(c, cudaMemsetAsync(cursor, 0, 2 * sizeof(unsigned long long), st));
+        // the cursor and the key count, then the heavy list's counters
+        GSJ_CUDA(c, cudaMemsetAsync(cursor, 0, 3 * sizeof(unsigned long long), st));
         return GSJ_OK;
     };
     GSJ_CUDA(c, cudaEventRecord(c->tev[2], st));
@@ -513,8 +520,7 @@ int emit_join(gsj_context* c, JoinArgs<T>& a, uint64_t N, bool stamp, int model,
         GSJ_TRY(reset());
         o.emit = false;
         o.stride = kSampleStride;
-        S.kernel_launches += 1;
-        GSJ_CUDA(c, launch_join_emit<T>(a, o, nsample, model, stamp, rows, c->num_sms, st));
+        GSJ_CUDA(c, launch_join_emit<T>(a, o, heavy, nsample, model, stamp, c->num_sms, &nl, st));
         unsigned long long sampled = 0;
         GSJ_TRY(d2h_small(c, &sampled, o.rechecks, 1));
         est = nsample ? (double)sampled * (double)ni / (double)nsample : 0.0;
@@ -533,14 +539,14 @@ int emit_join(gsj_context* c, JoinArgs<T>& a, uint64_t N, bool stamp, int model,
         o.stride = 1;
         o.pairs = pairs;
         o.cap = cap;
-        S.kernel_launches += 1;
-        GSJ_CUDA(c, launch_join_emit<T>(a, o, ni, model, stamp, rows, c->num_sms, st));
+        GSJ_CUDA(c, launch_join_emit<T>(a, o, heavy, ni, model, stamp, c->num_sms, &nl, st));
         GSJ_TRY(d2h_small(c, &used, cursor, 1));
         GSJ_TRY(d2h_small(c, &R, o.rechecks, 1));
         if (used <= cap) break;
         if (attempt == 2) return fail(c, GSJ_ERR_STATE, "warp join: pair buffer short at its proven bound");
         c->stats.reruns++;
     }
+    S.kernel_launches += (uint64_t)nl;
     GSJ_CUDA(c, cudaEventRecord(c->tev[3], st));
     GSJ_TRY(pairs_to_csr(c, pairs, used, R, shift, N, counts, offsets, cand));
     S.join_path = GSJ_PATH_WARP;
@@ -1119,8 +1125,7 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     // cell id (cell L holds slots [ds[L], ds[L+1])), else a hash table of the
     // non-empty cells
     uint32_t *ds = nullptr, *dcnt = nullptr;
-    unsigned long long* hkeys = nullptr;
-    uint32_t* hvals = nullptr;
+    uint4* htab = nullptr;
     uint64_t hmask = 0;
     const uint64_t dense_limit = std::max<uint64_t>(1u << 24, 8ull * N);
     const bool dense = totalCells <= dense_limit && totalCells < (1ull << 30);
@@ -1132,33 +1137,29 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
         uint64_t hcap = 1024;
         while (hcap < 2ull * M) hcap <<= 1;
         hmask = hcap - 1;
-        GSJ_TRY(dev_get(c, c->hkeys, hcap, &hkeys));
-        GSJ_TRY(dev_get(c, c->hvals, hcap, &hvals));
-        GSJ_CUDA(c, cudaMemsetAsync(hkeys, 0xff, hcap * sizeof(unsigned long long), st));
+        GSJ_TRY(dev_get(c, c->htab, hcap, &htab));
+        GSJ_CUDA(c, cudaMemsetAsync(htab, 0xff, hcap * sizeof(uint4), st));
     }
     S.kernel_launches += 1;
-    GSJ_CUDA(c, launch_cell_tables(cell_key, cell_start, M, dcnt, hkeys, hvals, hmask, st));
+    GSJ_CUDA(c, launch_cell_tables(cell_key, cell_start, M, dcnt, g.ncells[0], htab, hmask, st));
     if (dense) {
         // the slot-prefix table: ds[L] = points in cells below L (ds[totalCells] = N)
         GSJ_TRY(dev_get(c, c->temp, scan_u32_u64_temp_bytes(totalCells), (unsigned char**)&temp));
         S.kernel_launches += 3;
         GSJ_CUDA(c, scan_u32_u32(dcnt, ds, totalCells, temp, st));
     }
-    // Dense low-dimensional grids use the row-range traversal driven by a
-    // per-cell plan of neighbour-row slot ranges.
-    const bool rows = dense && k <= 3;
+    // The ROWS path (dense low-dimensional grids) is driven by a per-cell plan of
+    // neighbour-row slot ranges.
+    const bool tpq = dense && k <= 3 && cfg.ilp == 0 && n <= 4 && !cfg.sort;
     uint2* plan = nullptr;
-    uint8_t* plan_par = nullptr;
-    if (rows) {
+    if (tpq) {
         const uint32_t nrows = k == 1 ? 1u : (k == 2 ? 3u : 9u);
         GSJ_TRY(dev_get(c, c->plan, (size_t)M * nrows, &plan));
-        GSJ_TRY(dev_get(c, c->plan_par, M, &plan_par));
         S.kernel_launches += 1;
-        GSJ_CUDA(c, launch_cell_plan(cell_key, M, g, ds, plan, plan_par, st));
+        GSJ_CUDA(c, launch_cell_plan(cell_key, M, g, ds, plan, st));
     }
     uint32_t* slot_cell = nullptr;
     uint64_t* bitoff = nullptr;
-    const bool tpq = rows && cfg.ilp == 0 && n <= 4 && !cfg.sort;
     if (tpq) {
         // slot -> cell, and the hit-mask layout: slot s's query owns words
         // [bitoff[s], bitoff[s+1]) of the count pass's bit masks
@@ -1213,12 +1214,33 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     // time, and the order in which queries run changes no result.
     uint32_t num_items = 0;
     uint2* items = nullptr;
+    // Query groups of the register form of the warp join: cells of few points are
+    // joined with their neighbours along dim 0, about 6 points a group, so that
+    // they share the enumeration of the neighbour rows and the candidate loads
+    // (up to 4 cells: 3 + 3 more cells of candidates are tested than needed).
+    uint32_t gspan = 1;
+    const uint32_t* gstart = cell_start;
+    if constexpr (std::is_same<T, float>::value) {
+        if (path_id == GSJ_PATH_WARP && join_reg_supported(n, npad, model, cfg.ilp))
+            gspan = (uint32_t)std::min<uint64_t>(4u, (6ull * M + N - 1u) / N);
+        if (gspan < 1u) gspan = 1u;
+    }
     if (tpq) {
         S.work_items = ((uint64_t)N + 31u) / 32u;
     } else {
         uint32_t *order = nullptr, *nchunks = nullptr, *item_off = nullptr;
         GSJ_TRY(dev_get(c, c->nchunks, M + 1, &nchunks));
         GSJ_TRY(dev_get(c, c->item_off, M + 1, &item_off));
+        if (gspan > 1u) {
+            uint32_t* gs = nullptr;
+            GSJ_TRY(dev_get(c, c->gstart, M + 1, &gs));
+            GSJ_TRY(dev_get(c, c->temp, scan_u32_u64_temp_bytes(M), (unsigned char**)&temp));
+            S.kernel_launches += 5;
+            GSJ_CUDA(c, launch_group_flags(cell_key, M, g.ncells[0], gspan, nchunks, st));
+            GSJ_CUDA(c, scan_u32_u32(nchunks, item_off, M, temp, st));
+            GSJ_CUDA(c, launch_group_starts_of(nchunks, item_off, cell_start, M, (uint32_t)N, gs, st));
+            gstart = gs;
+        }
         if (cfg.query_reorder) {
             uint32_t *sizes = nullptr, *sizes2 = nullptr, *iota = nullptr;
             GSJ_TRY(dev_get(c, c->sizes, 2 * (size_t)M, &sizes));
@@ -1228,7 +1250,7 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
             // stable descending sort by cell size (ties keep ascending cell order):
             // an ascending sort of the complemented sizes
             S.kernel_launches += 2;
-            GSJ_CUDA(c, launch_item_counts(cell_start, nullptr, M, qchunk, nchunks, sizes, st));
+            GSJ_CUDA(c, launch_item_counts(gstart, nullptr, M, qchunk, nchunks, sizes, st));
             GSJ_CUDA(c, launch_iota(iota, M, st));
             GSJ_TRY(dev_get(c, c->temp, radix_sort_temp_bytes(M), (unsigned char**)&temp));
             bool alt = false;
@@ -1240,10 +1262,10 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
                 GSJ_CUDA(c, cudaMemcpyAsync(order, iota, (size_t)M * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
             }
             S.kernel_launches += 1;
-            GSJ_CUDA(c, launch_item_counts(cell_start, order, M, qchunk, nchunks, nullptr, st));
+            GSJ_CUDA(c, launch_item_counts(gstart, order, M, qchunk, nchunks, nullptr, st));
         } else {
             S.kernel_launches += 1;
-            GSJ_CUDA(c, launch_item_counts(cell_start, nullptr, M, qchunk, nchunks, nullptr, st));
+            GSJ_CUDA(c, launch_item_counts(gstart, nullptr, M, qchunk, nchunks, nullptr, st));
         }
         GSJ_TRY(dev_get(c, c->temp, scan_u32_u64_temp_bytes(M), (unsigned char**)&temp));
         S.kernel_launches += 3;
@@ -1272,10 +1294,10 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     a.cell_key = cell_key;
     a.ds = ds;
     a.plan = plan;
-    a.plan_par = plan_par;
-    a.hkeys = reinterpret_cast<const uint64_t*>(hkeys);
-    a.hvals = hvals;
+    a.htab = htab;
     a.hmask = hmask;
+    a.gstart = gstart;
+    a.gspan = gspan;
     a.items = items;
     a.num_items = num_items;
     a.nbtab = d_nbtab;
@@ -1305,8 +1327,7 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     c->last.lookup.cell_start = cell_start;
     c->last.lookup.cell_key = cell_key;
     c->last.lookup.ds = ds;
-    c->last.lookup.hkeys = reinterpret_cast<const uint64_t*>(hkeys);
-    c->last.lookup.hvals = hvals;
+    c->last.lookup.htab = htab;
     c->last.lookup.hmask = hmask;
     c->last.lookup.g = g;
     c->last.lookup.n_points = (uint32_t)N;
@@ -1323,7 +1344,7 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     // Every other grid except the thread-per-query rows: one emit pass + pair sort.
     if (!tpq) {
         unsigned long long* cursor = reinterpret_cast<unsigned long long*>(ctr + 4);
-        return emit_join<T>(c, a, N, stamp, model, rows, exact_size, learned, counts, offsets, cursor, t_join,
+        return emit_join<T>(c, a, N, stamp, model, exact_size, learned, counts, offsets, cursor, t_join,
                             t_start);
     }
     // Dense low-dimensional grids (the ROWS path): the distance work is cheap
@@ -1500,13 +1521,12 @@ int gsj_destroy(gsj_context* c) {
     if (c->st) cudaStreamSynchronize(c->st);
     if (c->st2) cudaStreamSynchronize(c->st2);
     Buf* bufs[] = {&c->in,       &c->pts,   &c->ids,    &c->keys,      &c->keys2,   &c->vals,      &c->cell_key,
-                   &c->cell_start, &c->dense, &c->dcnt, &c->plan, &c->plan_par, &c->slot_cell, &c->hkeys,
-                   &c->hvals,
+                   &c->cell_start, &c->dense, &c->dcnt, &c->plan, &c->slot_cell, &c->htab,
                    &c->order,    &c->sizes,
                    &c->nchunks,  &c->item_off, &c->items, &c->fwd,     &c->swords,     &c->counts,    &c->offsets,
                    &c->table, &c->temp,   &c->scan_temp, &c->misc,    &c->var,       &c->perm,
                    &c->minarr,   &c->minmax_part, &c->pairs, &c->srows, &c->snorms,
-                   &c->spartial, &c->scentre, &c->unc, &c->table2, &c->nbtab, &c->bitoff, &c->hitbits, &c->ptemp, &c->sortv};
+                   &c->spartial, &c->scentre, &c->unc, &c->table2, &c->nbtab, &c->bitoff, &c->hitbits, &c->ptemp, &c->sortv, &c->heavy, &c->gstart};
     for (Buf* b : bufs)
         if (b->p) cudaFree(b->p);
     for (auto* pb : {&c->stage[0], &c->stage[1], &c->hmisc})

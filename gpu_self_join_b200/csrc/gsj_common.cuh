@@ -33,11 +33,13 @@ struct JoinArgs {
     const uint64_t* cell_key;     // [M]
     const uint32_t* ds;           // [totalCells+1] slot prefix over all linear ids (dense grids), or null
     const uint2* plan;            // [M][3^(k-1)] (slot start, count) of each neighbour row (dense, k <= 3)
-    const uint8_t* plan_par;      // [M] parities of the own cell coordinates (bit j = dim j)
-    const uint64_t* hkeys;        // [hcap] hash table keys (kEmptyKey = empty), or null
-    const uint32_t* hvals;        // [hcap] cell indices
+    const uint4* htab;            // [hcap] hash table of the grid rows that hold a cell {linear id of the row's
+                                  // cell 0 (lo, hi; kEmptyKey = empty), first cell, cells}, or null
     uint64_t hmask;               // hcap - 1
-    const uint2* items;           // [num_items] (cell, chunk)
+    const uint32_t* gstart;       // first slot of each query group (items' x; [group + 1] is its end): the cells,
+                                  // or runs of neighbouring cells of a grid row (gspan > 1)
+    uint32_t gspan;               // cells of a query group along dim 0 at most
+    const uint2* items;           // [num_items] (group, chunk)
     const uint4* nbtab;           // [3^k] neighbour offsets: linear-id delta (x lo, y hi), z = moved-down dims
                                   // | moved-up dims << 16, w = highest moved dim (0xff: none)
     uint32_t num_items;
@@ -101,62 +103,111 @@ __device__ __forceinline__ void cell_masks(const uint32_t (&own)[kMaxK], const G
         }
 }
 
-// Slot range of the cell with linear id `lin`: from the dense slot-prefix
-// table (ds[lin] .. ds[lin+1]) or through the hash table of non-empty cells.
+__device__ __forceinline__ uint64_t entry_key(const uint4& e) { return ((uint64_t)e.y << 32) | e.x; }
+
+// Cells of the grid row whose cell 0 has linear id `base`: indices [first,
+// first + n) of the sorted cell list (n = 0: none).  e: the table entry at the
+// row's own position.
 template <typename T>
-__device__ __forceinline__ bool lookup_range(const JoinArgs<T>& a, uint64_t lin, uint32_t& start, uint32_t& cnt) {
-    if (a.ds) {
-        start = a.ds[lin];
-        cnt = a.ds[lin + 1] - start;
-        return cnt != 0;
-    }
-    uint64_t h = mix64(lin) & a.hmask;
-    for (uint64_t p = 0; p <= a.hmask; p++) {
-        const uint64_t kk = a.hkeys[h];
-        if (kk == lin) {
-            const uint32_t c = a.hvals[h];
-            start = a.cell_start[c];
-            cnt = a.cell_start[c + 1] - start;
-            return true;
+__device__ __forceinline__ void row_entry(const JoinArgs<T>& a, uint64_t base, uint4 e, uint32_t& first, uint32_t& n) {
+    for (uint64_t p = 1; entry_key(e) != base; p++) {
+        if (entry_key(e) == kEmptyKey || p > a.hmask) {
+            n = 0u;
+            return;
         }
-        if (kk == kEmptyKey) return false;
-        h = (h + 1) & a.hmask;
+        e = a.htab[(mix64(base) + p) & a.hmask];
     }
-    return false;
+    first = e.z;
+    n = e.w;
 }
 
-// Slot range of a neighbour row: the cells x-1..x+1 of the grid row that offset
-// r (digit j of r is dim j+1's step + 1) leads to.  These cells are
-// consecutive in cell order (dim 0 is fastest), so the range is contiguous
-// whichever of them are non-empty.  With unicomp the own row (r's centre) adds
-// its dim-0 neighbours only when x is odd, every other row comes whole or not
-// at all (the highest moved dim is the same for its three cells).
-template <typename T, bool STAMP>
-__device__ __forceinline__ bool row_range(const JoinArgs<T>& a, uint32_t r, uint64_t own_lin, uint32_t lowmask,
-                                          uint32_t highmask, uint32_t oddmask, uint32_t& start, uint32_t& cnt) {
-    uint64_t lin;
-    if (!nb_offset<T, STAMP>(a, 3u * r + 1u, own_lin, lowmask, highmask, oddmask, lin)) return false;
-    const bool side = !STAMP || lin != own_lin || (oddmask & 1u);
-    const bool down = side && !(lowmask & 1u), up = side && !(highmask & 1u);
+// Slot range [start, start + cnt) of the cells xlo..xhi of the grid row whose
+// cell 0 has linear id `base`.  These cells are consecutive in cell order (dim
+// 0 is fastest), so the range is contiguous whichever of them are non-empty.
+// Dense grids read the slot-prefix table, the others the row's entry, its
+// cells' ids (a row of up to four cells at once, longer ones by bisection) and
+// their slots.  W: cand += points of every cell x times byte x - x0 of `weight`.
+template <typename T, bool W>
+__device__ __forceinline__ void row_slots(const JoinArgs<T>& a, uint64_t base, uint32_t xlo, uint32_t xhi,
+                                          uint32_t& start, uint32_t& cnt, uint32_t x0, uint64_t weight,
+                                          unsigned long long& cand) {
+    uint32_t lo = 0, hi = 0;  // the cells' indices (hashed grids)
     if (a.ds) {
-        start = a.ds[down ? lin - 1 : lin];
-        cnt = a.ds[(up ? lin + 1 : lin) + 1] - start;
-        return cnt != 0u;
+        start = a.ds[base + xlo];
+        cnt = a.ds[base + xhi + 1u] - start;
+    } else {
+        uint32_t first = 0, n = 0;
+        row_entry(a, base, a.htab[mix64(base) & a.hmask], first, n);
+        if (n > 4u) {
+            // the row's first cell at or past xlo
+            uint32_t l = first, h = first + n;
+            while (l < h) {
+                const uint32_t m = l + (h - l) / 2u;
+                if (a.cell_key[m] < base + xlo) l = m + 1u;
+                else h = m;
+            }
+            n -= l - first;
+            first = l;
+        }
+        uint64_t key[4];
+#pragma unroll
+        for (uint32_t i = 0; i < 4u; i++) key[i] = i < n ? a.cell_key[first + i] : kEmptyKey;
+        lo = hi = first;
+#pragma unroll
+        for (uint32_t i = 0; i < 4u; i++) {
+            lo += key[i] < base + xlo ? 1u : 0u;
+            hi += key[i] <= base + xhi ? 1u : 0u;
+        }
+        if (hi - first == 4u)
+            while (hi < first + n && a.cell_key[hi] <= base + xhi) hi++;
+        start = cnt = 0u;
+        if (hi > lo) {
+            start = a.cell_start[lo];
+            cnt = a.cell_start[hi] - start;
+        }
     }
-    uint32_t s = 0, c = 0;
-    start = cnt = 0u;
-    if (down && lookup_range(a, lin - 1, s, c)) {
-        start = s;
-        cnt = c;
+    if (W && cnt) {
+        uint32_t prev = start, x = xlo;
+        const uint32_t steps = a.ds ? xhi - xlo + 1u : hi - lo;
+        for (uint32_t i = 0; i < steps; i++) {
+            uint32_t next;
+            if (a.ds) {
+                x = xlo + i;
+                next = a.ds[base + x + 1u];
+            } else {
+                x = (uint32_t)(a.cell_key[lo + i] - base);
+                next = a.cell_start[lo + i + 1u];
+            }
+            cand += (unsigned long long)(next - prev) * (uint32_t)((weight >> (8u * (x - x0))) & 0xffu);
+            prev = next;
+        }
     }
-    if (lookup_range(a, lin, s, c)) {
-        if (!cnt) start = s;
-        cnt += c;
-    }
-    if (up && lookup_range(a, lin + 1, s, c)) {
-        if (!cnt) start = s;
-        cnt += c;
-    }
+}
+
+// Slot range of the cell with linear id `lin`.
+template <typename T>
+__device__ __forceinline__ bool lookup_range(const JoinArgs<T>& a, uint64_t lin, uint32_t& start, uint32_t& cnt) {
+    const uint32_t x = a.ds ? 0u : (uint32_t)(lin % a.g.ncells[0]);
+    unsigned long long cand = 0;
+    row_slots<T, false>(a, lin - x, x, x, start, cnt, 0u, 0u, cand);
+    return cnt != 0u;
+}
+
+// Slot range of a neighbour row of one cell: the cells x-1..x+1 of the grid row
+// that offset r (digit j of r is dim j+1's step + 1) leads to.  With unicomp
+// the own row (r's centre) adds its dim-0 neighbours only when x is odd, every
+// other row comes whole or not at all (the highest moved dim is the same for
+// its three cells).
+template <typename T, bool STAMP>
+__device__ __forceinline__ bool row_range(const JoinArgs<T>& a, bool valid, uint32_t r, uint64_t own_lin, uint32_t x,
+                                          uint32_t lowmask, uint32_t highmask, uint32_t oddmask, uint32_t& start,
+                                          uint32_t& cnt) {
+    uint64_t lin;
+    if (!valid || !nb_offset<T, STAMP>(a, 3u * r + 1u, own_lin, lowmask, highmask, oddmask, lin)) return false;
+    const bool side = !STAMP || lin != own_lin || (oddmask & 1u);
+    unsigned long long cand = 0;
+    row_slots<T, false>(a, lin - x, x - (side && !(lowmask & 1u) ? 1u : 0u), x + (side && !(highmask & 1u) ? 1u : 0u),
+                        start, cnt, 0u, 0u, cand);
     return cnt != 0u;
 }
 

@@ -241,30 +241,72 @@ __global__ void k_dense_counts(const uint64_t* __restrict__ cell_key, const uint
     if (c < M) dcnt[cell_key[c]] = cell_start[c + 1] - cell_start[c];
 }
 
-__global__ void k_hash_insert(const uint64_t* __restrict__ cell_key, uint32_t M, unsigned long long* hkeys,
-                              uint32_t* hvals, uint64_t hmask) {
+// Entries {linear id of the row's cell 0, first cell, cells} of the grid rows
+// that hold a cell; n0: cells of dim 0.  The first cell of a row finds the row's
+// end by a galloping search.
+__global__ void k_row_insert(const uint64_t* __restrict__ cell_key, uint32_t M, uint32_t n0, uint4* htab,
+                             uint64_t hmask) {
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= M) return;
     const unsigned long long key = cell_key[c];
-    uint64_t h = mix64(key) & hmask;
+    const unsigned long long base = key - key % n0;
+    if (c > 0u && cell_key[c - 1u] >= base) return;
+    // cells [c, lo) are in the row, hi (if below M) is not
+    uint32_t lo = c + 1u, hi = M;
+    for (uint32_t step = 1u; lo < M; step <<= 1) {
+        const uint32_t probe = step < M - lo ? lo + step - 1u : M - 1u;
+        if (cell_key[probe] - base >= n0) {
+            hi = probe;
+            break;
+        }
+        lo = probe + 1u;
+    }
+    while (lo < hi) {
+        const uint32_t m = lo + (hi - lo) / 2u;
+        if (cell_key[m] - base < n0) lo = m + 1u;
+        else hi = m;
+    }
+    const uint64_t h = mix64(base);
     for (uint64_t probe = 0; probe <= hmask; probe++) {
-        const unsigned long long prev = atomicCAS(&hkeys[h], (unsigned long long)kEmptyKey, key);
-        if (prev == kEmptyKey || prev == key) {
-            hvals[h] = c;
+        uint4* e = htab + ((h + probe) & hmask);
+        const unsigned long long prev =
+            atomicCAS(reinterpret_cast<unsigned long long*>(e), (unsigned long long)kEmptyKey, base);
+        if (prev == kEmptyKey) {
+            e->z = c;
+            e->w = lo - c;
             return;
         }
-        h = (h + 1) & hmask;
     }
+}
+
+// Query groups: runs of cells of one grid row within the same `span` cells of
+// dim 0 (aligned).  flags[c] = 1 where a group begins.
+__global__ void k_group_flags(const uint64_t* __restrict__ cell_key, uint32_t M, uint32_t n0, uint32_t span,
+                              uint32_t* __restrict__ flags) {
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= M) return;
+    const uint64_t key = cell_key[c];
+    const uint64_t first = key - (uint32_t)(key % n0) % span;  // the group's smallest possible id
+    flags[c] = (c == 0u || cell_key[c - 1u] < first) ? 1u : 0u;
+}
+
+// gstart[g] = first slot of group g, N from the last group's end on (gstart has M + 1 entries).
+__global__ void k_group_starts_of(const uint32_t* __restrict__ flags, const uint32_t* __restrict__ pos,
+                                  const uint32_t* __restrict__ cell_start, uint32_t M, uint32_t N,
+                                  uint32_t* __restrict__ gstart) {
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c > M) return;
+    if (c < M && flags[c]) gstart[pos[c]] = cell_start[c];
+    if (c >= pos[M]) gstart[c] = N;
 }
 
 // Cell plan of dense low-dimensional grids (k <= 3): for every non-empty
 // cell and each of its 3^(k-1) neighbour rows, the slot range of the row's
 // cells x-1..x+1, clipped to the grid (kernel.cu:180-188 clamp the same way).
 // These cells have consecutive linear ids (dim 0 is fastest), so the range is
-// [ds[row + xlo], ds[row + xhi + 1]).  par holds the parity bit of each own
-// coordinate for the unicomp traversal.
+// [ds[row + xlo], ds[row + xhi + 1]).
 __global__ void k_cell_plan(const uint64_t* __restrict__ cell_key, uint32_t M, GridGeom g,
-                            const uint32_t* __restrict__ ds, uint2* __restrict__ plan, uint8_t* __restrict__ par) {
+                            const uint32_t* __restrict__ ds, uint2* __restrict__ plan) {
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= M) return;
     const uint32_t k = g.k;
@@ -289,7 +331,6 @@ __global__ void k_cell_plan(const uint64_t* __restrict__ cell_key, uint32_t M, G
         }
         plan[(size_t)c * nrows + r] = e;
     }
-    par[c] = (uint8_t)((o0 & 1u) | ((o1 & 1u) << 1) | ((o2 & 1u) << 2));
 }
 
 // ------------------------------------------------------------ work items
@@ -361,15 +402,27 @@ cudaError_t launch_gather_points(const T* in, uint64_t N, uint32_t n, uint32_t n
 
 
 cudaError_t launch_cell_tables(const uint64_t* cell_key, const uint32_t* cell_start, uint32_t M, uint32_t* dcnt,
-                               unsigned long long* hkeys, uint32_t* hvals, uint64_t hmask, cudaStream_t st) {
+                               uint32_t n0, uint4* htab, uint64_t hmask, cudaStream_t st) {
     if (dcnt) k_dense_counts<<<blocks_for(M, 256), 256, 0, st>>>(cell_key, cell_start, M, dcnt);
-    if (hkeys) k_hash_insert<<<blocks_for(M, 256), 256, 0, st>>>(cell_key, M, hkeys, hvals, hmask);
+    if (htab) k_row_insert<<<blocks_for(M, 256), 256, 0, st>>>(cell_key, M, n0, htab, hmask);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_group_flags(const uint64_t* cell_key, uint32_t M, uint32_t n0, uint32_t span, uint32_t* flags,
+                               cudaStream_t st) {
+    k_group_flags<<<blocks_for(M, 256), 256, 0, st>>>(cell_key, M, n0, span, flags);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_group_starts_of(const uint32_t* flags, const uint32_t* pos, const uint32_t* cell_start, uint32_t M,
+                                   uint32_t N, uint32_t* gstart, cudaStream_t st) {
+    k_group_starts_of<<<blocks_for((uint64_t)M + 1u, 256), 256, 0, st>>>(flags, pos, cell_start, M, N, gstart);
     return cudaGetLastError();
 }
 
 cudaError_t launch_cell_plan(const uint64_t* cell_key, uint32_t M, const GridGeom& g, const uint32_t* ds,
-                             uint2* plan, uint8_t* par, cudaStream_t st) {
-    k_cell_plan<<<blocks_for(M, 256), 256, 0, st>>>(cell_key, M, g, ds, plan, par);
+                             uint2* plan, cudaStream_t st) {
+    k_cell_plan<<<blocks_for(M, 256), 256, 0, st>>>(cell_key, M, g, ds, plan);
     return cudaGetLastError();
 }
 

@@ -5,22 +5,27 @@
 // thread per query point, repeats the neighbour-cell search (2 binary searches
 // per cell) for every query, and appends every hit with a global atomicAdd.
 // Here one warp owns a work item: up to 32 consecutive query slots of one
-// non-empty cell.  The warp
-//   1. enumerates the cell's 3^k neighbour offsets once, lanes in parallel,
-//      resolving each through the dense cell table or the hash table, and
-//      compacts the non-empty ones (ballot) into a per-warp list in shared
-//      memory - with STAMP only the unicomp half-space of stamploops.h;
+// non-empty cell, or of a few neighbouring cells of a grid row.  The warp
+//   1. enumerates the item's 3^(k-1) neighbour rows once, lanes in parallel (the
+//      cells of a row next to the item's are one contiguous slot range,
+//      row_slots), and compacts the non-empty ones (ballot) into a per-warp list in shared memory -
+//      with STAMP only the unicomp half-space of stamploops.h;
 //   2. stages the queries in shared memory;
 //   3. walks the concatenated candidate slots 32 at a time, one candidate per
-//      lane (rows are contiguous in the cell-sorted layout), and tests every
-//      query against the 32 candidates with the reference's exact arithmetic
-//      (s <= thr is sqrt(s) <= eps, see gsj_threshold_*).
+//      lane, and tests every query against the 32 candidates with the
+//      reference's exact arithmetic (s <= thr is sqrt(s) <= eps, see
+//      gsj_threshold_*).
 // Every hit becomes a packed (query id, candidate id) key appended to the pair
-// buffer (emit_keys), with STAMP also the reverse key of a hit in another cell
-// (the reference emits (q,c) twice there, kernel.cu:367-375); the buffer is
-// sorted into the neighbour table afterwards (the reference's pair buffers +
-// sort_by_key, GPU.cu:863-980).  One traversal per join; a sampling run over
-// every stride-th item sizes the buffer first.
+// buffer, with STAMP also the reverse key of a hit in another cell (the
+// reference emits (q,c) twice there, kernel.cu:367-375); the buffer becomes the
+// neighbour table afterwards (the reference's pair buffers + sort_by_key,
+// GPU.cu:863-980).  One traversal per join; a sampling run over every stride-th
+// item sizes the buffer first.
+//
+// Two kernels: k_join_reg for float rows of up to 16 values (candidate rows in
+// registers, hits through a per-warp queue, heavy items cut into slices), k_join
+// for the rest (double, longer rows, ILP chains that a register form would have
+// to reorder).
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -119,20 +124,118 @@ __device__ __forceinline__ uint32_t cand_slot(const uint32_t* nb_start, const ui
     return f < total ? nb_start[my] + (f - pf) : 0u;
 }
 
-// 4 CTAs of 8 warps per SM for float data (at most 64 registers a thread; the
-// 6-D register path spills 36 bytes): on the 6-D mixture the emit stage went
-// from 38.7 to 34.7 ms against 3 CTAs at 80 registers, the candidate-row loads
-// being latency-bound.
-template <typename T, int NT, int MODEL, int POL, bool STAMP, bool ROWS>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_join(const JoinArgs<T> a, uint32_t nb_cap, uint32_t noff,
-                                              const TileOut o, uint32_t nvisit) {
+// The queries of an item: slots [q0, q0 + qn) of one grid row, in the cells
+// xa..xb of it.
+struct ItemCells {
+    uint64_t base;             // linear id of the row's cell 0
+    uint32_t xa, xb;
+    uint32_t low, high, odd;   // edge and parity masks of the own coordinates (bit 0: cell xa's)
+};
+
+template <typename T>
+__device__ __forceinline__ ItemCells item_cells(const JoinArgs<T>& a, uint32_t q0, uint32_t qn) {
+    // cell coordinates with the formula the keys were built with (main.cu:744, kernel.cu:184)
+    uint32_t own[kMaxK];
+    ItemCells c;
+    c.base = 0;
+#pragma unroll
+    for (int j = 0; j < kMaxK; j++) {
+        own[j] = (j < (int)a.g.k) ? FP<T>::to_uint_rz(FP<T>::div(FP<T>::sub(a.pts[(size_t)q0 * a.npad + j], a.minv[j]),
+                                                                 a.eps))
+                                  : 0u;
+        if (j > 0 && j < (int)a.g.k) c.base += (uint64_t)own[j] * a.g.mult[j];
+    }
+    cell_masks(own, a.g, c.low, c.high, c.odd);
+    c.xa = own[0];
+    c.xb = a.gspan > 1u ? FP<T>::to_uint_rz(FP<T>::div(FP<T>::sub(a.pts[(size_t)(q0 + qn - 1u) * a.npad], a.minv[0]),
+                                                       a.eps))
+                        : c.xa;
+    return c;
+}
+
+// The neighbour rows of an item (kernel.cu:180-303; stamploops.h for STAMP) as
+// slot ranges in nb_start and the exclusive prefix of their sizes in nb_pref
+// (nb_pref[rows] = total): the cells xa-1..xb+1 of every row.  With xa < xb a
+// candidate may lie two or more cells from a query; the caller tells them apart.
+// own: slot range of the own row (set for the whole warp).  SEG: cand += the
+// lane's rows' candidates by the reference's rule, nq[i] = queries in cell x0 + i
+// packed in bytes (at most 4 cells); else the caller counts total x qn.  Returns
+// the number of rows; the whole warp calls.
+template <typename T, bool STAMP, bool SEG>
+__device__ __forceinline__ uint32_t enumerate_rows(const JoinArgs<T>& a, const ItemCells& ic, uint32_t nrow,
+                                                   uint32_t* nb_start, uint32_t* nb_pref, int lane, unsigned lt,
+                                                   uint32_t& total, uint2& own, uint32_t nq, unsigned long long& cand) {
+    const unsigned FULL = 0xffffffffu;
+    const uint32_t rc = nrow / 2u;  // the own row
+    // dims 1.. decide which rows are visited; bit 0 of the masks plays no part there
+    const uint64_t own_lin = ic.base + ic.xa;
+    const uint32_t n0 = a.g.ncells[0];
+    const uint32_t xlo0 = ic.xa - (ic.xa > 0u ? 1u : 0u), xhi0 = min(ic.xb + 1u, n0 - 1u);
+    const bool one = ic.xa == ic.xb;
+    // candidates of the cell x0 - 1 + d (byte d): queries of the cells within one
+    // step; with unicomp only the odd cells look at their own row's neighbours
+    const uint32_t x0 = ic.xa;
+    uint64_t w_all = 0, w_own = 0;
+    if (SEG) {
+#pragma unroll
+        for (uint32_t d = 0; d < 6u; d++) {
+            uint32_t wa = 0, wo = 0;
+#pragma unroll
+            for (uint32_t i = 0; i < 4u; i++) {
+                const uint32_t q = (nq >> (8u * i)) & 0xffu;
+                if (i + 2u >= d && i <= d) {  // |x0 + i - (x0 - 1 + d)| <= 1
+                    wa += q;
+                    if (i + 1u == d || ((x0 + i) & 1u)) wo += q;
+                }
+            }
+            w_all |= (uint64_t)wa << (8u * d);
+            w_own |= (uint64_t)(STAMP ? wo : wa) << (8u * d);
+        }
+    }
+    uint32_t nnb = 0, run = 0;
+    uint2 mine = make_uint2(0u, 0u);
+    for (uint32_t b0 = 0; b0 < nrow; b0 += 32) {
+        const uint32_t r = b0 + (uint32_t)lane;
+        uint64_t lin;
+        uint32_t st = 0, v = 0;
+        if (r < nrow && nb_offset<T, STAMP>(a, 3u * r + 1u, own_lin, ic.low, ic.high, ic.odd, lin)) {
+            const bool self = STAMP && one && r == rc && !(ic.xa & 1u);
+            row_slots<T, SEG>(a, lin - ic.xa, self ? ic.xa : xlo0, self ? ic.xa : xhi0, st, v, x0 - 1u,
+                              r == rc ? w_own : w_all, cand);
+        }
+        if (r == rc) mine = make_uint2(st, st + v);
+        const unsigned m = __ballot_sync(FULL, v != 0u);
+        uint32_t x = v;
+#pragma unroll
+        for (int s = 1; s < 32; s <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULL, x, s);
+            if (lane >= s) x += y;
+        }
+        if (v) {
+            const uint32_t pos = nnb + (uint32_t)__popc(m & lt);
+            nb_start[pos] = st;
+            nb_pref[pos] = run + x - v;
+        }
+        nnb += (uint32_t)__popc(m);
+        run += __shfl_sync(FULL, x, 31);
+    }
+    if (lane == 0) nb_pref[nnb] = run;
+    total = run;
+    own.x = __shfl_sync(FULL, mine.x, (int)(rc & 31u));
+    own.y = __shfl_sync(FULL, mine.y, (int)(rc & 31u));
+    return nnb;
+}
+
+template <typename T, int NT, int MODEL, int POL, bool STAMP>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_join(const JoinArgs<T> a, uint32_t nrow,
+                                                                       const TileOut o, uint32_t nvisit) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr bool GENERIC = (NT == 0);
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const uint32_t npad = a.npad;
-    const WarpSmem L = warp_smem_layout(npad, sizeof(T), nb_cap, GENERIC);
+    const WarpSmem L = warp_smem_layout(npad, sizeof(T), nrow, GENERIC);
     unsigned char* wb = smem_raw + (size_t)warp * L.total;
     T* q_s = reinterpret_cast<T*>(wb + L.q_off);
     uint32_t* qid_s = reinterpret_cast<uint32_t*>(wb + L.qid_off);
@@ -140,7 +243,6 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_join(const Join
     uint32_t* nb_pref = reinterpret_cast<uint32_t*>(wb + L.nbp_off);
     T* cand_s = reinterpret_cast<T*>(wb + L.cand_off);
     const unsigned lt = lanemask_lt();
-    const uint32_t k = a.g.k;
     unsigned long long cand_total = 0;
     unsigned long long blk_base = 0, emitted = 0;
     uint32_t blk_used = kEmitBlk;
@@ -159,85 +261,13 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_join(const Join
         if (item >= nvisit) break;
         if (lane == 0) claim = atomicAdd(a.work_counter, 1u);
         const uint2 wi = a.items[(size_t)item * o.stride];
-        const uint32_t cell = wi.x;
-        const uint32_t cs = a.cell_start[cell], ce = a.cell_start[cell + 1];
+        const uint32_t cs = a.gstart[wi.x], ce = a.gstart[wi.x + 1];  // a cell (gspan is 1)
         const uint32_t q0 = cs + wi.y * kQChunk;
         const uint32_t qn = min((uint32_t)kQChunk, ce - q0);
-
-        uint32_t nnb = 0;
-        if constexpr (ROWS) {
-            // ---- dense grid, k <= 3: the cell plan holds, per neighbour row, the
-            // slot range of cells x-1..x+1 (one contiguous range, see
-            // k_cell_plan) and the parities of the own coordinates.
-            const uint32_t nrows = k == 1 ? 1u : (k == 2 ? 3u : 9u);
-            uint2 e = make_uint2(0u, 0u);
-            if ((uint32_t)lane < nrows) e = a.plan[(size_t)cell * nrows + lane];
-            if (STAMP) {
-                // stamploops.h: own row -> its dim-0 neighbours only when x is odd;
-                // another row -> all three cells when the own coordinate of its
-                // highest differing dim is odd
-                const uint32_t par = a.plan_par[cell];
-                const int d1 = k >= 2 ? (int)(lane % 3) - 1 : 0;
-                const int d2 = k >= 3 ? (int)(lane / 3) - 1 : 0;
-                if (d1 == 0 && d2 == 0) {
-                    if (!(par & 1u)) e = make_uint2(cs, ce - cs);
-                } else if (!((par >> (d2 != 0 ? 2 : 1)) & 1u)) {
-                    e.y = 0u;
-                }
-            }
-            const bool found = (uint32_t)lane < nrows && e.y != 0u;
-            const unsigned m = __ballot_sync(FULL, found);
-            if (found) {
-                const uint32_t pos = __popc(m & lt);
-                nb_start[pos] = e.x;
-                nb_pref[pos] = e.y;
-            }
-            nnb = __popc(m);
-        } else {
-            // ---- own cell coordinates, from the first query of the cell with the
-            // formula the keys were built with (main.cu:744, kernel.cu:184)
-            uint32_t own[kMaxK];
-#pragma unroll
-            for (int j = 0; j < kMaxK; j++)
-                own[j] = (j < (int)k) ? FP<T>::to_uint_rz(FP<T>::div(FP<T>::sub(a.pts[(size_t)cs * npad + j], a.minv[j]),
-                                                                       a.eps))
-                                      : 0u;
-            // ---- neighbour cells (kernel.cu:180-303; stamploops.h for STAMP)
-            uint32_t lowmask, highmask, oddmask;
-            cell_masks(own, a.g, lowmask, highmask, oddmask);
-            const uint64_t own_lin = a.cell_key[cell];
-            for (uint32_t base = 0; base < noff; base += 32) {
-                const uint32_t o = base + lane;
-                uint64_t lin = 0;
-                const bool ok = o < noff && nb_offset<T, STAMP>(a, o, own_lin, lowmask, highmask, oddmask, lin);
-                uint32_t st = 0, cnt = 0;
-                const bool found = ok && lookup_range(a, lin, st, cnt);
-                const unsigned m = __ballot_sync(FULL, found);
-                if (found) {
-                    const uint32_t pos = nnb + __popc(m & lt);
-                    nb_start[pos] = st;
-                    nb_pref[pos] = cnt;
-                }
-                nnb += __popc(m);
-            }
-        }
-        __syncwarp();
-        // exclusive prefix of candidate counts over the list
-        uint32_t run = 0;
-        for (uint32_t base = 0; base < nnb; base += 32) {
-            const uint32_t i = base + lane;
-            const uint32_t v = i < nnb ? nb_pref[i] : 0u;
-            uint32_t x = v;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(FULL, x, o);
-                if (lane >= o) x += y;
-            }
-            if (i < nnb) nb_pref[i] = run + x - v;
-            run += __shfl_sync(FULL, x, 31);
-        }
-        const uint32_t total = run;
-        if (lane == 0) nb_pref[nnb] = total;
+        uint32_t total;
+        uint2 own;
+        const uint32_t nnb = enumerate_rows<T, STAMP, false>(a, item_cells(a, q0, qn), nrow, nb_start, nb_pref, lane, lt,
+                                                             total, own, 0u, cand_total);
 
         // ---- queries
         for (uint32_t e = lane; e < qn * npad; e += 32) q_s[e] = a.pts[(size_t)q0 * npad + e];
@@ -336,95 +366,438 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_join(const Join
     if (lane == 0 && emitted) atomicAdd(o.rechecks, emitted);
 }
 
+// ------------------------------------------------------------------ register form
+// Float rows of up to NP <= 16 values.  Each lane keeps G candidate rows in
+// registers, so a query costs NP/4 broadcast reads and 2 NP arithmetic
+// instructions per 32 candidates, and one vote per 32 G candidates when
+// nothing is within eps.  Columns from n to NP are zero in every row: a
+// zero difference leaves every running sum unchanged bit for bit, so NP need not
+// be n.  Lanes without a candidate hold NaN coordinates, which are within
+// no threshold.
+//
+// Bound by instruction issue (0.71 of the slots on the 6-D mixture) and by the
+// latency of the enumeration.  Measured, both launches of a join and the
+// sampling pass: 6-D 5M points 40.8 -> 17.1 ms, 8-D 142k points (ILP 8 with
+// SHORTCIRCUIT, formerly through shared memory) 16.8 -> 2.2 ms.  What did not
+// help: 16-byte entries for single cells hashed next to their row neighbours (33
+// ms, the table no longer fits the L2 and its probe chains diverge); two rows'
+// lookups in flight a lane with the hit's cell check inline (17.8 + 6.4 ms, the
+// code outgrows the instruction cache).
+//
+// How the terms are summed (gsj_dist.cuh, float):
+//   kSumSeq    s = fma(d, d, s) (ILP 0 and 1)
+//   kSumFirst  ILP >= n with either ILP model: one square per register, the
+//              registers added in order: s = d0^2, s += d_l^2
+//   kSumMask   SHORTCIRCUIT with 1 < ILP < n: the first dim of every ILP block is
+//              fused into s, the others are squared and added
+enum RegSum : int { kSumSeq = 0, kSumFirst = 1, kSumMask = 2 };
+
+template <int NP, int SUM>
+__device__ __forceinline__ float reg_sqdist(const float (&q)[NP], const float (&c)[NP], uint32_t fused) {
+    float s = 0.f;
+#pragma unroll
+    for (int l = 0; l < NP; l++) {
+        const float d = __fsub_rn(c[l], q[l]);
+        if (SUM == kSumSeq || l == 0) s = __fmaf_rn(d, d, s);
+        else if (SUM == kSumFirst) s = __fadd_rn(s, __fmul_rn(d, d));
+        else s = ((fused >> l) & 1u) ? __fmaf_rn(d, d, s) : __fadd_rn(s, __fmul_rn(d, d));
+    }
+    return s;
+}
+
+template <int NP>
+__device__ __forceinline__ void reg_load(const float* __restrict__ p, float (&r)[NP]) {
+#pragma unroll
+    for (int l = 0; l < NP; l += 4) {
+        if (l + 4 <= NP) {
+            const float4 v = *reinterpret_cast<const float4*>(p + l);
+            r[l] = v.x;
+            r[l + 1] = v.y;
+            r[l + 2] = v.z;
+            r[l + 3] = v.w;
+        } else {  // NP = 6: rows are padded to 8
+            const float2 v = *reinterpret_cast<const float2*>(p + l);
+            r[l] = v.x;
+            r[l + 1] = v.y;
+        }
+    }
+}
+
+// Entries of the per-warp hit queue: up to 31 left over and the hits of a query
+// among 32 G candidates.
+constexpr uint32_t kMaxTiles = 4;
+constexpr uint32_t kHitQueue = 32u + 32u * kMaxTiles;
+
+struct RegSmem {
+    uint32_t q, nbs, nbp, hits, total;
+};
+
+__host__ __device__ inline RegSmem reg_smem(uint32_t np4, uint32_t nrow) {
+    RegSmem t{};
+    uint32_t o = 0;
+    t.q = o;
+    o += 32u * np4 * 4u;
+    t.hits = o;
+    o += kHitQueue * 8u;
+    t.nbs = o;
+    o += nrow * 4u;
+    t.nbp = o;
+    o += (nrow + 1u) * 4u;
+    t.total = align16(o);
+    return t;
+}
+
+// Work of one unit in (query, 32 G candidates) steps: an item of more than twice
+// that goes to the heavy list in slices.  A step is about 60 instructions, so a
+// unit is some 100 us of a warp: long against the enumeration that every slice
+// repeats (about 10 us), short against a join.  (142k points in 8-D, 32 queries
+// an item in the dense cells: the longest items held the launch for two thirds
+// of its time, 22 % of the warps active on average.)
+constexpr uint32_t kUnitSteps = 512;
+
+// SEG: items are up to 32 queries of up to gspan (at most 4) neighbouring cells
+// of a grid row, which share the enumeration and the candidate loads; a hit is
+// then checked for its cells' distance.  (Cells of 2 points and 130 non-empty
+// neighbour rows each, as on a 5M-point 6-D mixture, spend more on enumerating
+// than on distances.)
+template <int NP, int SUM, int G, bool STAMP, bool SLICES, bool SEG>
+__global__ void __launch_bounds__(256, 4) k_join_reg(const JoinArgs<float> a, uint32_t nrow, const TileOut o,
+                                                     const HeavyList heavy, uint32_t nvisit) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr uint32_t NP4 = (NP + 3) / 4 * 4;
+    static_assert(G <= (int)kMaxTiles, "hit queue");
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const RegSmem L = reg_smem(NP4, nrow);
+    unsigned char* wb = smem_raw + (size_t)(threadIdx.x >> 5) * L.total;
+    float* q_s = reinterpret_cast<float*>(wb + L.q);
+    uint2* hits = reinterpret_cast<uint2*>(wb + L.hits);  // (query slot | flag << 31, candidate slot)
+    uint32_t* nb_start = reinterpret_cast<uint32_t*>(wb + L.nbs);
+    uint32_t* nb_pref = reinterpret_cast<uint32_t*>(wb + L.nbp);
+    const unsigned lt = lanemask_lt();
+    unsigned long long cand_total = 0;
+    unsigned long long blk_base = 0, emitted = 0;
+    uint32_t blk_used = kEmitBlk, nq = 0;  // nq: entries in the hit queue
+    uint32_t fused = 0;                    // kSumMask: dims fused into the sum
+    if (SUM == kSumMask)
+        for (uint32_t l = 0; l < NP; l += a.ilp) fused |= 1u << l;
+
+    // The last `cnt` (at most 32) entries of the queue become keys, a full warp of
+    // them at a time.  The flag of an entry: the candidate lies outside the query's
+    // cell (unicomp, one cell an item), or in its grid row (SEG).
+    auto flush = [&](uint32_t cnt) {
+        __syncwarp();
+        bool v = (uint32_t)lane < cnt;
+        const uint2 e = v ? hits[nq - cnt + (uint32_t)lane] : make_uint2(0u, 0u);
+        const uint32_t qs = e.x & 0x7fffffffu;
+        bool cr = STAMP && (e.x >> 31) != 0u;
+        if (SEG) {
+            // cells more than one step apart are no candidates; with unicomp the own
+            // row's neighbours are those of the odd cells
+            const uint32_t xq = FP<float>::to_uint_rz(
+                FP<float>::div(FP<float>::sub(a.pts[(size_t)qs * NP4], a.minv[0]), a.eps));
+            const uint32_t xc = FP<float>::to_uint_rz(
+                FP<float>::div(FP<float>::sub(a.pts[(size_t)e.y * NP4], a.minv[0]), a.eps));
+            const bool row = (e.x >> 31) != 0u;
+            v = v && xc + 1u - xq <= 2u && !(STAMP && row && xc != xq && !(xq & 1u));
+            cr = STAMP && v && !(row && xc == xq);
+        }
+        const unsigned b = __ballot_sync(FULL, v), cb = __ballot_sync(FULL, cr);
+        const uint64_t qid = v && o.emit ? a.ids[qs] : 0u, cid = v && o.emit ? a.ids[e.y] : 0u;
+        emit_keys(o, blk_base, blk_used, emitted, v, cr, b, cb, lt, lane, qid, cid);
+        nq -= cnt;
+        __syncwarp();
+    };
+
+    const uint32_t nunits = SLICES ? min(*heavy.count, heavy.cap) : nvisit;
+    uint32_t* counter = SLICES ? heavy.claim : a.work_counter;
+    // one claim at a time, the next one in flight while an item is processed (see k_join)
+    uint32_t claim = 0;
+    if (lane == 0) claim = atomicAdd(counter, 1u);
+    for (;;) {
+        const uint32_t unit = __shfl_sync(FULL, claim, 0);
+        if (unit >= nunits) break;
+        if (lane == 0) claim = atomicAdd(counter, 1u);
+        uint32_t visit = unit, slice = 0;
+        if (SLICES) {
+            const uint2 h = heavy.list[unit];
+            visit = h.x;
+            slice = h.y;
+            if (visit >= nvisit) continue;  // an entry of an item that found the list full
+        }
+        const uint2 wi = a.items[(size_t)visit * o.stride];
+        const uint32_t cs = a.gstart[wi.x], ce = a.gstart[wi.x + 1];
+        const uint32_t q0 = cs + wi.y * kQChunk;
+        const uint32_t qn = min((uint32_t)kQChunk, ce - q0);
+        const ItemCells ic = item_cells(a, q0, qn);
+        uint32_t nqx = 0;  // queries of each of the item's cells (bytes)
+        if (SEG) {
+            const uint32_t x = FP<float>::to_uint_rz(FP<float>::div(
+                FP<float>::sub(a.pts[(size_t)(q0 + min((uint32_t)lane, qn - 1u)) * NP4], a.minv[0]), a.eps));
+#pragma unroll
+            for (uint32_t i = 0; i < 4u; i++)
+                nqx |= (uint32_t)__popc(__ballot_sync(FULL, lane < qn && x == ic.xa + i)) << (8u * i);
+        }
+        uint32_t total;
+        uint2 own;
+        unsigned long long cand = 0;
+        const uint32_t nnb =
+            enumerate_rows<float, STAMP, SEG>(a, ic, nrow, nb_start, nb_pref, lane, lt, total, own, nqx, cand);
+        uint32_t g_lo = 0, g_hi = (total + 32u * G - 1u) / (32u * G);  // candidate groups of this unit
+        const uint32_t per = (kUnitSteps + qn - 1u) / qn;              // groups of a slice
+        if (SLICES) {
+            g_lo = slice * per;
+            g_hi = min(g_hi, g_lo + per);
+        } else {
+            cand_total += SEG ? cand : lane == 0 ? (unsigned long long)total * qn : 0ull;
+            if (g_hi > 2u * per) {
+                const uint32_t ns = (g_hi + per - 1u) / per;
+                uint32_t at = 0;
+                if (lane == 0) at = atomicAdd(heavy.count, ns);
+                at = __shfl_sync(FULL, at, 0);
+                const bool fits = at < heavy.cap && ns <= heavy.cap - at;
+                for (uint32_t i = (uint32_t)lane; i < ns; i += 32u)
+                    if (at < heavy.cap && i < heavy.cap - at)
+                        heavy.list[at + i] = make_uint2(fits ? visit : 0xffffffffu, i);
+                if (fits) continue;
+            }
+        }
+        // ---- queries
+        __syncwarp();
+        {
+            const float4* src = reinterpret_cast<const float4*>(a.pts + (size_t)q0 * NP4);
+            for (uint32_t e = lane; e < qn * (NP4 / 4u); e += 32) reinterpret_cast<float4*>(q_s)[e] = src[e];
+        }
+        __syncwarp();
+
+        uint32_t ent = 0;  // the neighbour row of the group's first candidate
+        if (SLICES && g_lo) {
+            uint32_t hi = nnb;
+            while (hi - ent > 1u) {
+                const uint32_t mid = (ent + hi) / 2u;
+                if (nb_pref[mid] <= g_lo * 32u * G) ent = mid;
+                else hi = mid;
+            }
+        }
+        for (uint32_t g = g_lo; g < g_hi; g++) {
+            float cx[G][NP];
+            uint32_t slot[G];
+#pragma unroll
+            for (int t = 0; t < G; t++) {
+                const uint32_t f0 = (g * G + (uint32_t)t) * 32u;
+                slot[t] = 0u;
+                if (f0 < total) slot[t] = cand_slot(nb_start, nb_pref, nnb, ent, f0, lane, total);
+                reg_load<NP>(a.pts + (size_t)slot[t] * NP4, cx[t]);
+                if (f0 + (uint32_t)lane >= total) cx[t][0] = __int_as_float(0x7fffffff);
+            }
+            for (uint32_t j = 0; j < qn; j++) {
+                float q[NP];
+                reg_load<NP>(q_s + (size_t)j * NP4, q);
+                float s[G];
+                bool any = false;
+#pragma unroll
+                for (int t = 0; t < G; t++) {
+                    s[t] = reg_sqdist<NP, SUM>(q, cx[t], fused);
+                    any = any || s[t] <= a.thr;
+                }
+                if (!__any_sync(FULL, any)) continue;
+#pragma unroll
+                for (int t = 0; t < G; t++) {
+                    const bool hit = s[t] <= a.thr;
+                    const unsigned b = __ballot_sync(FULL, hit);
+                    bool flag = false;
+                    if (SEG) flag = slot[t] >= own.x && slot[t] < own.y;
+                    else if (STAMP) flag = slot[t] < cs || slot[t] >= ce;
+                    if (hit)
+                        hits[nq + (uint32_t)__popc(b & lt)] =
+                            make_uint2((q0 + j) | (flag ? 0x80000000u : 0u), slot[t]);
+                    nq += (uint32_t)__popc(b);
+                }
+                while (nq >= 32u) flush(32u);
+            }
+        }
+    }
+    if (nq) flush(nq);
+    if (!SLICES && o.emit) {
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1) cand_total += __shfl_xor_sync(FULL, cand_total, s);
+        if (lane == 0 && cand_total) atomicAdd(a.cand_cnt, cand_total);
+    }
+    if (o.emit && blk_used < kEmitBlk)
+        for (uint32_t e = blk_used + (uint32_t)lane; e < kEmitBlk; e += 32u)
+            if (blk_base + e < o.cap) o.pairs[blk_base + e] = kUndecidedPad;
+    if (lane == 0 && emitted) atomicAdd(o.rechecks, emitted);
+}
+
 // ------------------------------------------------------------------ launch
-template <typename T, int NT, int MODEL, int POL, bool STAMP, bool ROWS>
-static cudaError_t launch_one(const JoinArgs<T>& a, uint32_t nb_cap, uint32_t noff, const TileOut& o,
-                              uint32_t nvisit, int num_sms, cudaStream_t st) {
-    auto kern = k_join<T, NT, MODEL, POL, STAMP, ROWS>;
-    const WarpSmem L = warp_smem_layout(a.npad, sizeof(T), nb_cap, NT == 0);
+// Grid and shared memory of a warp-per-unit kernel (`per_warp` bytes a warp).
+static cudaError_t warp_grid(const void* kern, uint32_t per_warp, const uint32_t shape_warps, uint32_t shape_per_sm,
+                             uint32_t nvisit, int num_sms, int& threads, size_t& smem, uint64_t& blocks) {
     const uint32_t max_smem = 200u * 1024u;
-    int warps = (int)(max_smem / L.total);
+    int warps = (int)(max_smem / per_warp);
     if (warps > 8) warps = 8;
-    if (a.shape_warps && (int)a.shape_warps < warps) warps = (int)a.shape_warps;
+    if (shape_warps && (int)shape_warps < warps) warps = (int)shape_warps;
     if (warps < 1) return cudaErrorInvalidValue;
-    const int threads = warps * 32;
-    const size_t smem = (size_t)warps * L.total;
+    threads = warps * 32;
+    smem = (size_t)warps * per_warp;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    // the whole unified L1/shared array as shared memory, so that the CTAs the
-    // occupancy calculation counts on are resident together
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return e;
     int per_sm = 0;
-    e = blocks_per_sm((const void*)kern, threads, smem, &per_sm);
+    e = blocks_per_sm(kern, threads, smem, &per_sm);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) per_sm = 1;
-    if (a.shape_per_sm && (int)a.shape_per_sm < per_sm) per_sm = (int)a.shape_per_sm;
+    if (shape_per_sm && (int)shape_per_sm < per_sm) per_sm = (int)shape_per_sm;
+    // as much of the unified array as those CTAs need; the rest caches candidate
+    // rows, which consecutive items (cells of one grid row) share
+    const size_t need = (size_t)per_sm * (smem + 1024u);
+    int pct = (int)((need * 100u + 228u * 1024u - 1u) / (228u * 1024u));
+    if (pct > 100) pct = 100;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
+    if (e != cudaSuccess) return e;
     const uint64_t needed = ((uint64_t)nvisit + warps - 1) / warps;
-    uint64_t blocks = (uint64_t)num_sms * per_sm;
+    blocks = (uint64_t)num_sms * per_sm;
     if (blocks > needed) blocks = needed ? needed : 1;
     // every warp claims once past the last item: the counter must not wrap
-    const uint64_t total_warps = blocks * (uint64_t)warps;
-    if ((uint64_t)nvisit + total_warps >= 0xffffffffull) return cudaErrorInvalidValue;
-    kern<<<(unsigned)blocks, threads, smem, st>>>(a, nb_cap, noff, o, nvisit);
+    if ((uint64_t)nvisit + blocks * (uint64_t)warps >= 0xffffffffull) return cudaErrorInvalidValue;
+    return cudaSuccess;
+}
+
+template <typename T, int NT, int MODEL, int POL, bool STAMP>
+static cudaError_t launch_one(const JoinArgs<T>& a, uint32_t nrow, const TileOut& o, uint32_t nvisit, int num_sms,
+                              int* launches, cudaStream_t st) {
+    auto kern = k_join<T, NT, MODEL, POL, STAMP>;
+    const WarpSmem L = warp_smem_layout(a.npad, sizeof(T), nrow, NT == 0);
+    int threads = 0;
+    size_t smem = 0;
+    uint64_t blocks = 0;
+    const cudaError_t e = warp_grid((const void*)kern, L.total, a.shape_warps, a.shape_per_sm, nvisit, num_sms,
+                                    threads, smem, blocks);
+    if (e != cudaSuccess) return e;
+    kern<<<(unsigned)blocks, threads, smem, st>>>(a, nrow, o, nvisit);
+    *launches += 1;
     return cudaGetLastError();
 }
 
+template <int NP, int SUM, int G, bool STAMP, bool SEG>
+static cudaError_t launch_reg(const JoinArgs<float>& a, uint32_t nrow, const TileOut& o, const HeavyList& heavy,
+                              uint32_t nvisit, int num_sms, int* launches, cudaStream_t st) {
+    auto k1 = k_join_reg<NP, SUM, G, STAMP, false, SEG>;
+    auto k2 = k_join_reg<NP, SUM, G, STAMP, true, SEG>;
+    const RegSmem L = reg_smem((NP + 3) / 4 * 4, nrow);
+    int threads = 0;
+    size_t smem = 0;
+    uint64_t blocks = 0;
+    cudaError_t e = warp_grid((const void*)k1, L.total, a.shape_warps, a.shape_per_sm, nvisit, num_sms, threads, smem,
+                              blocks);
+    if (e != cudaSuccess) return e;
+    k1<<<(unsigned)blocks, threads, smem, st>>>(a, nrow, o, heavy, nvisit);
+    // the slices of the heavy items, whose number only the device knows
+    e = warp_grid((const void*)k2, L.total, a.shape_warps, a.shape_per_sm, kHeavyCap, num_sms, threads, smem, blocks);
+    if (e != cudaSuccess) return e;
+    k2<<<(unsigned)blocks, threads, smem, st>>>(a, nrow, o, heavy, nvisit);
+    *launches += 2;
+    return cudaGetLastError();
+}
+
+bool join_reg_supported(uint32_t n, uint32_t npad, int model, uint32_t ilp) {
+    if (n > 16 || npad != npad_for(n, 4u) || npad < 4u || (npad & 3u)) return false;
+    // ILP chains of several dims take the shared-memory form
+    return model == kSeq || model == kIlpSc || ilp <= 1u || ilp >= n;
+}
+
+// The register form's dispatch: false when the join takes k_join.
+template <bool STAMP>
+static bool try_reg(const JoinArgs<float>& a, int model, uint32_t nrow, const TileOut& o, const HeavyList& heavy,
+                    uint32_t nvisit, int num_sms, int* launches, cudaStream_t st, cudaError_t* e) {
+    if (!join_reg_supported(a.n, a.npad, model, a.ilp)) return false;
+    const bool seq = model == kSeq || a.ilp <= 1u;
+    const bool first = !seq && a.ilp >= a.n;
+#define GSJ_REG(NP, SUM, G)                                                                            \
+    do {                                                                                               \
+        *e = a.gspan > 1u                                                                              \
+                 ? launch_reg<NP, SUM, G, STAMP, true>(a, nrow, o, heavy, nvisit, num_sms, launches, st)    \
+                 : launch_reg<NP, SUM, G, STAMP, false>(a, nrow, o, heavy, nvisit, num_sms, launches, st);  \
+        return true;                                                                                   \
+    } while (0)
+    if (seq) {
+        if (a.n == 6) GSJ_REG(6, kSumSeq, 4);
+        if (a.npad == 4) GSJ_REG(4, kSumSeq, 4);
+        if (a.npad == 8) GSJ_REG(8, kSumSeq, 4);
+        if (a.npad == 12) GSJ_REG(12, kSumSeq, 2);
+        GSJ_REG(16, kSumSeq, 2);
+    }
+    if (first) {
+        if (a.npad == 4) GSJ_REG(4, kSumFirst, 4);
+        if (a.npad == 8) GSJ_REG(8, kSumFirst, 4);
+        if (a.npad == 12) GSJ_REG(12, kSumFirst, 2);
+        GSJ_REG(16, kSumFirst, 2);
+    }
+    if (a.npad == 4) GSJ_REG(4, kSumMask, 4);
+    if (a.npad == 8) GSJ_REG(8, kSumMask, 4);
+    if (a.npad == 12) GSJ_REG(12, kSumMask, 2);
+    GSJ_REG(16, kSumMask, 2);
+#undef GSJ_REG
+}
+
 template <typename T, int MODEL, int POL, bool STAMP>
-static cudaError_t dispatch_nt(const JoinArgs<T>& a, bool rows, uint32_t nb_cap, uint32_t noff, const TileOut& o,
-                               uint32_t nvisit, int num_sms, cudaStream_t st) {
-    if (rows) {
-        // low-dimensional dense grids (k <= 3): registers for n <= 4
-        if (MODEL == kSeq && a.npad == npad_for(a.n, sizeof(T))) {
+static cudaError_t dispatch_nt(const JoinArgs<T>& a, uint32_t nrow, const TileOut& o, uint32_t nvisit, int num_sms,
+                               int* launches, cudaStream_t st) {
+    if constexpr (MODEL == kSeq) {
+        if (a.npad == npad_for(a.n, sizeof(T))) {
             switch (a.n) {
-                case 1: return launch_one<T, 1, MODEL, POL, STAMP, true>(a, nb_cap, noff, o, nvisit, num_sms, st);
-                case 2: return launch_one<T, 2, MODEL, POL, STAMP, true>(a, nb_cap, noff, o, nvisit, num_sms, st);
-                case 3: return launch_one<T, 3, MODEL, POL, STAMP, true>(a, nb_cap, noff, o, nvisit, num_sms, st);
-                case 4: return launch_one<T, 4, MODEL, POL, STAMP, true>(a, nb_cap, noff, o, nvisit, num_sms, st);
+                case 1: return launch_one<T, 1, MODEL, POL, STAMP>(a, nrow, o, nvisit, num_sms, launches, st);
+                case 2: return launch_one<T, 2, MODEL, POL, STAMP>(a, nrow, o, nvisit, num_sms, launches, st);
                 default: break;
             }
+            if constexpr (sizeof(T) == 8) {
+                switch (a.n) {
+                    case 3: return launch_one<T, 3, MODEL, POL, STAMP>(a, nrow, o, nvisit, num_sms, launches, st);
+                    case 4: return launch_one<T, 4, MODEL, POL, STAMP>(a, nrow, o, nvisit, num_sms, launches, st);
+                    case 6: return launch_one<T, 6, MODEL, POL, STAMP>(a, nrow, o, nvisit, num_sms, launches, st);
+                    case 8: return launch_one<T, 8, MODEL, POL, STAMP>(a, nrow, o, nvisit, num_sms, launches, st);
+                    default: break;
+                }
+            }
         }
-        return launch_one<T, 0, MODEL, POL, STAMP, true>(a, nb_cap, noff, o, nvisit, num_sms, st);
     }
-    if (MODEL == kSeq && a.npad == npad_for(a.n, sizeof(T))) {
-        switch (a.n) {
-            case 6: return launch_one<T, 6, MODEL, POL, STAMP, false>(a, nb_cap, noff, o, nvisit, num_sms, st);
-            case 8: return launch_one<T, 8, MODEL, POL, STAMP, false>(a, nb_cap, noff, o, nvisit, num_sms, st);
-            default: break;
-        }
-    }
-    return launch_one<T, 0, MODEL, POL, STAMP, false>(a, nb_cap, noff, o, nvisit, num_sms, st);
+    return launch_one<T, 0, MODEL, POL, STAMP>(a, nrow, o, nvisit, num_sms, launches, st);
 }
 
 template <typename T, bool STAMP>
-static cudaError_t dispatch_model(const JoinArgs<T>& a, int model, bool rows, uint32_t nb_cap, uint32_t noff,
-                                  const TileOut& o, uint32_t nvisit, int num_sms, cudaStream_t st) {
+static cudaError_t dispatch_model(const JoinArgs<T>& a, int model, uint32_t nrow, const TileOut& o,
+                                  const HeavyList& heavy, uint32_t nvisit, int num_sms, int* launches,
+                                  cudaStream_t st) {
     constexpr int P = sizeof(T) == 8 ? kPolF64 : kPolF32;
+    if constexpr (sizeof(T) == 4) {
+        cudaError_t e = cudaSuccess;
+        if (try_reg<STAMP>(a, model, nrow, o, heavy, nvisit, num_sms, launches, st, &e)) return e;
+    }
     switch (model) {
-        case kSeq: return dispatch_nt<T, kSeq, P, STAMP>(a, rows, nb_cap, noff, o, nvisit, num_sms, st);
-        case kIlp: return dispatch_nt<T, kIlp, P, STAMP>(a, rows, nb_cap, noff, o, nvisit, num_sms, st);
-        case kIlpSc: return dispatch_nt<T, kIlpSc, P, STAMP>(a, rows, nb_cap, noff, o, nvisit, num_sms, st);
+        case kSeq: return dispatch_nt<T, kSeq, P, STAMP>(a, nrow, o, nvisit, num_sms, launches, st);
+        case kIlp: return dispatch_nt<T, kIlp, P, STAMP>(a, nrow, o, nvisit, num_sms, launches, st);
+        case kIlpSc: return dispatch_nt<T, kIlpSc, P, STAMP>(a, nrow, o, nvisit, num_sms, launches, st);
         default: return cudaErrorInvalidValue;
     }
 }
 
 template <typename T>
-cudaError_t launch_join_emit(const JoinArgs<T>& a, const TileOut& o, uint32_t nvisit, int model, bool stamp, bool rows,
-                             int num_sms, cudaStream_t st) {
-    uint32_t noff = 1;
-    for (uint32_t j = 0; j < a.g.k; j++) noff *= 3u;
-    if (rows && (a.g.k > 3 || !a.ds)) return cudaErrorInvalidValue;
-    if (o.stride == 0) return cudaErrorInvalidValue;
+cudaError_t launch_join_emit(const JoinArgs<T>& a, const TileOut& o, const HeavyList& heavy, uint32_t nvisit,
+                             int model, bool stamp, int num_sms, int* launches, cudaStream_t st) {
+    uint32_t nrow = 1;  // neighbour rows: 3^(k-1)
+    for (uint32_t j = 1; j < a.g.k; j++) nrow *= 3u;
+    if (o.stride == 0 || !heavy.list || heavy.cap != kHeavyCap || !a.gstart || a.gspan < 1u || a.gspan > 4u)
+        return cudaErrorInvalidValue;
+    if (a.gspan > 1u && (sizeof(T) != 4 || !join_reg_supported(a.n, a.npad, model, a.ilp)))
+        return cudaErrorInvalidValue;
     if (nvisit == 0) return cudaSuccess;
     if ((uint64_t)(nvisit - 1) * o.stride >= a.num_items) return cudaErrorInvalidValue;
-    const uint32_t nb_cap = rows ? 32u : noff;
-    return stamp ? dispatch_model<T, true>(a, model, rows, nb_cap, noff, o, nvisit, num_sms, st)
-                 : dispatch_model<T, false>(a, model, rows, nb_cap, noff, o, nvisit, num_sms, st);
+    return stamp ? dispatch_model<T, true>(a, model, nrow, o, heavy, nvisit, num_sms, launches, st)
+                 : dispatch_model<T, false>(a, model, nrow, o, heavy, nvisit, num_sms, launches, st);
 }
 
-template cudaError_t launch_join_emit<float>(const JoinArgs<float>&, const TileOut&, uint32_t, int, bool, bool, int,
-                                             cudaStream_t);
-template cudaError_t launch_join_emit<double>(const JoinArgs<double>&, const TileOut&, uint32_t, int, bool, bool, int,
-                                              cudaStream_t);
+template cudaError_t launch_join_emit<float>(const JoinArgs<float>&, const TileOut&, const HeavyList&, uint32_t, int,
+                                             bool, int, int*, cudaStream_t);
+template cudaError_t launch_join_emit<double>(const JoinArgs<double>&, const TileOut&, const HeavyList&, uint32_t, int,
+                                              bool, int, int*, cudaStream_t);
 
 }  // namespace gsj

@@ -414,7 +414,7 @@ __global__ void __launch_bounds__(kSThreads, 2) k_tile_screen(const JoinArgs<flo
             const uint32_t r = base + (uint32_t)tid;
             uint32_t st = 0, cnt = 0;
             const bool found =
-                r < nrow && row_range<float, STAMP>(a, r, own_lin, lowmask, highmask, oddmask, st, cnt);
+                row_range<float, STAMP>(a, r < nrow, r, own_lin, own[0], lowmask, highmask, oddmask, st, cnt);
             const unsigned m = __ballot_sync(FULL, found);
             if (lane == 0) misc[8 + warp] = __popc(m);
             __syncthreads();

@@ -4,7 +4,7 @@
 // traversal (kernelNDGridIndexGlobal / evaluateCell / evalPoint,
 // kernel.cu:132-480) and its pair buffers + sort (GPU.cu:863-980).  A CTA owns
 // a work item: up to kTileQ = 64 consecutive query slots of one cell.  It
-//   1. enumerates the cell's 3^k neighbour offsets once (threads in parallel,
+//   1. enumerates the cell's 3^(k-1) neighbour rows once (threads in parallel,
 //      dense slot-prefix table or hash table, unicomp half-space with STAMP)
 //      and compacts the non-empty ones in offset order;
 //   2. keeps the 64 queries in shared memory, dimension-major;
@@ -50,7 +50,7 @@ struct TileSmem {
     uint32_t qs, cs, nbs, nbp, cslot, cid, qid, misc, total;
 };
 
-__host__ __device__ inline TileSmem tile_smem(uint32_t npad, uint32_t noff) {
+__host__ __device__ inline TileSmem tile_smem(uint32_t npad, uint32_t nrow) {
     TileSmem t{};
     uint32_t o = 0;
     t.qs = o;
@@ -58,9 +58,9 @@ __host__ __device__ inline TileSmem tile_smem(uint32_t npad, uint32_t noff) {
     t.cs = o;
     o += npad * kTC * 4u;
     t.nbs = o;
-    o += noff * 4u;
+    o += nrow * 4u;
     t.nbp = o;
-    o += (noff + 1u) * 4u;
+    o += (nrow + 1u) * 4u;
     t.cslot = o;
     o += kTC * 4u;
     t.cid = o;
@@ -145,11 +145,11 @@ __device__ __forceinline__ void tile_dists(const float* __restrict__ qs, const f
 }
 
 template <int MODEL, bool STAMP>
-__global__ void __launch_bounds__(kThreads) k_tile_join(const JoinArgs<float> a, const TileOut o, uint32_t noff,
+__global__ void __launch_bounds__(kThreads) k_tile_join(const JoinArgs<float> a, const TileOut o, uint32_t nrow,
                                                         uint32_t nvisit) {
     extern __shared__ __align__(16) unsigned char tsm[];
     const uint32_t n = a.n, npad = a.npad, k = a.g.k;
-    const TileSmem L = tile_smem(npad, noff);
+    const TileSmem L = tile_smem(npad, nrow);
     float* qs = reinterpret_cast<float*>(tsm + L.qs);
     float* cs = reinterpret_cast<float*>(tsm + L.cs);
     uint32_t* nb_start = reinterpret_cast<uint32_t*>(tsm + L.nbs);
@@ -183,17 +183,16 @@ __global__ void __launch_bounds__(kThreads) k_tile_join(const JoinArgs<float> a,
             own[j] = (j < (int)k) ? FP<float>::to_uint_rz(FP<float>::div(
                                         FP<float>::sub(a.pts[(size_t)cs0 * npad + j], a.minv[j]), a.eps))
                                   : 0u;
-        // ---- neighbour cells in offset order (kernel.cu:180-303; stamploops.h)
+        // ---- neighbour rows in offset order (kernel.cu:180-303; stamploops.h)
         uint32_t nnb = 0;
         uint32_t lowmask, highmask, oddmask;
         cell_masks(own, a.g, lowmask, highmask, oddmask);
         const uint64_t own_lin = a.cell_key[cell];
-        for (uint32_t base = 0; base < noff; base += kThreads) {
-            const uint32_t off = base + tid;
-            uint64_t lin = 0;
-            const bool ok = off < noff && nb_offset<float, STAMP>(a, off, own_lin, lowmask, highmask, oddmask, lin);
+        for (uint32_t base = 0; base < nrow; base += kThreads) {
+            const uint32_t r = base + (uint32_t)tid;
             uint32_t st = 0, cnt = 0;
-            const bool found = ok && lookup_range(a, lin, st, cnt);
+            const bool found =
+                row_range<float, STAMP>(a, r < nrow, r, own_lin, own[0], lowmask, highmask, oddmask, st, cnt);
             const unsigned m = __ballot_sync(FULL, found);
             if (lane == 0) misc[4 + warp] = __popc(m);
             __syncthreads();
@@ -337,10 +336,10 @@ __global__ void __launch_bounds__(kThreads) k_tile_join(const JoinArgs<float> a,
 }
 
 template <int MODEL, bool STAMP>
-cudaError_t launch_tile_one(const JoinArgs<float>& a, const TileOut& o, uint32_t noff, uint32_t nvisit, int num_sms,
+cudaError_t launch_tile_one(const JoinArgs<float>& a, const TileOut& o, uint32_t nrow, uint32_t nvisit, int num_sms,
                             cudaStream_t st) {
     auto kern = k_tile_join<MODEL, STAMP>;
-    const TileSmem L = tile_smem(a.npad, noff);
+    const TileSmem L = tile_smem(a.npad, nrow);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total);
     if (e != cudaSuccess) return e;
     // the whole unified L1/shared array as shared memory, so that the CTAs the
@@ -354,7 +353,7 @@ cudaError_t launch_tile_one(const JoinArgs<float>& a, const TileOut& o, uint32_t
     if (a.shape_per_sm && (int)a.shape_per_sm < per_sm) per_sm = (int)a.shape_per_sm;
     uint64_t blocks = (uint64_t)num_sms * per_sm;
     if (blocks > nvisit) blocks = nvisit ? nvisit : 1;
-    kern<<<(unsigned)blocks, kThreads, L.total, st>>>(a, o, noff, nvisit);
+    kern<<<(unsigned)blocks, kThreads, L.total, st>>>(a, o, nrow, nvisit);
     return cudaGetLastError();
 }
 
@@ -389,15 +388,15 @@ cudaError_t launch_tile_join(const JoinArgs<float>& a, const TileOut& o, bool st
     if (!tile_supported(a.n, a.npad, a.g.k, model, a.ilp) || o.stride == 0) return cudaErrorInvalidValue;
     if (nvisit == 0) return cudaSuccess;
     if ((uint64_t)(nvisit - 1) * o.stride >= a.num_items) return cudaErrorInvalidValue;
-    uint32_t noff = 1;
-    for (uint32_t j = 0; j < a.g.k; j++) noff *= 3u;
+    uint32_t nrow = 1;  // neighbour rows: 3^(k-1)
+    for (uint32_t j = 1; j < a.g.k; j++) nrow *= 3u;
     switch (model * 2 + (stamp ? 1 : 0)) {
-        case kSeq * 2: return launch_tile_one<kSeq, false>(a, o, noff, nvisit, num_sms, st);
-        case kSeq * 2 + 1: return launch_tile_one<kSeq, true>(a, o, noff, nvisit, num_sms, st);
-        case kIlp * 2: return launch_tile_one<kIlp, false>(a, o, noff, nvisit, num_sms, st);
-        case kIlp * 2 + 1: return launch_tile_one<kIlp, true>(a, o, noff, nvisit, num_sms, st);
-        case kIlpSc * 2: return launch_tile_one<kIlpSc, false>(a, o, noff, nvisit, num_sms, st);
-        case kIlpSc * 2 + 1: return launch_tile_one<kIlpSc, true>(a, o, noff, nvisit, num_sms, st);
+        case kSeq * 2: return launch_tile_one<kSeq, false>(a, o, nrow, nvisit, num_sms, st);
+        case kSeq * 2 + 1: return launch_tile_one<kSeq, true>(a, o, nrow, nvisit, num_sms, st);
+        case kIlp * 2: return launch_tile_one<kIlp, false>(a, o, nrow, nvisit, num_sms, st);
+        case kIlp * 2 + 1: return launch_tile_one<kIlp, true>(a, o, nrow, nvisit, num_sms, st);
+        case kIlpSc * 2: return launch_tile_one<kIlpSc, false>(a, o, nrow, nvisit, num_sms, st);
+        case kIlpSc * 2 + 1: return launch_tile_one<kIlpSc, true>(a, o, nrow, nvisit, num_sms, st);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -32,11 +32,19 @@ template <typename T>
 cudaError_t launch_gather_points(const T* in, uint64_t N, uint32_t n, uint32_t npad, const uint32_t* perm,
                                  const uint32_t* ids, T* pts, cudaStream_t st);
 // Either the dense per-linear-id point counts (dcnt[key] = size, to be
-// scanned into the slot-prefix table) or the hash table of the non-empty cells.
+// scanned into the slot-prefix table) or the hash table of the grid rows that
+// hold a cell (n0: the grid's cells in dim 0).
 cudaError_t launch_cell_tables(const uint64_t* cell_key, const uint32_t* cell_start, uint32_t M, uint32_t* dcnt,
-                               unsigned long long* hkeys, uint32_t* hvals, uint64_t hmask, cudaStream_t st);
+                               uint32_t n0, uint4* htab, uint64_t hmask, cudaStream_t st);
 cudaError_t launch_cell_plan(const uint64_t* cell_key, uint32_t M, const GridGeom& g, const uint32_t* ds,
-                             uint2* plan, uint8_t* par, cudaStream_t st);
+                             uint2* plan, cudaStream_t st);
+// Query groups of up to `span` neighbouring cells of a grid row: flags[M] marks
+// their first cells, and with pos = the exclusive scan of flags (M + 1
+// entries) gstart[M + 1] receives their first slots (N past the last group).
+cudaError_t launch_group_flags(const uint64_t* cell_key, uint32_t M, uint32_t n0, uint32_t span, uint32_t* flags,
+                               cudaStream_t st);
+cudaError_t launch_group_starts_of(const uint32_t* flags, const uint32_t* pos, const uint32_t* cell_start, uint32_t M,
+                                   uint32_t N, uint32_t* gstart, cudaStream_t st);
 cudaError_t launch_item_counts(const uint32_t* cell_start, const uint32_t* order, uint32_t M, uint32_t qchunk,
                                uint32_t* nchunks, uint32_t* sizes, cudaStream_t st);
 cudaError_t launch_make_items(const uint32_t* order, const uint32_t* nchunks, const uint32_t* item_off,
@@ -46,13 +54,24 @@ cudaError_t launch_iota(uint32_t* out, uint32_t M, cudaStream_t st);
 // The warp-per-item join: appends packed pair keys into `o` (its rechecks
 // counter receives the exact number of keys; with o.emit false only that
 // count is taken) and visits items 0, o.stride, ..., (nvisit - 1) * o.stride.
-// `model` is one of Model; `stamp` selects the unicomp traversal; `rows` the
-// dense low-dimensional specialisation (k <= 3, a.ds set).  The launcher picks
-// the specialisation.
+// `model` is one of Model; `stamp` selects the unicomp traversal.  heavy.count
+// and heavy.claim must be zero.  The launcher picks the specialisation.
 struct TileOut;
+// Slices of the items that are too long for one warp: found by the first launch,
+// processed by a second one.
+struct HeavyList {
+    uint2* list;      // [cap] (visit, slice)
+    uint32_t* count;  // slices found (may exceed cap; those entries are dropped)
+    uint32_t* claim;  // the second launch's work counter
+    uint32_t cap;
+};
+constexpr uint32_t kHeavyCap = 1u << 20;
+// Whether the join of float rows runs in registers (query groups of several
+// cells need that form).
+bool join_reg_supported(uint32_t n, uint32_t npad, int model, uint32_t ilp);
 template <typename T>
-cudaError_t launch_join_emit(const JoinArgs<T>& a, const TileOut& o, uint32_t nvisit, int model, bool stamp, bool rows,
-                             int num_sms, cudaStream_t st);
+cudaError_t launch_join_emit(const JoinArgs<T>& a, const TileOut& o, const HeavyList& heavy, uint32_t nvisit,
+                             int model, bool stamp, int num_sms, int* launches, cudaStream_t st);
 
 // ROWS path: dense low-dimensional grids (k <= 3, n <= 4), full neighbourhood.
 // slot_cell[s] = cell of slot s; with swords non-null also the bit-mask words

@@ -250,21 +250,36 @@ __global__ void __launch_bounds__(kTT) k_model_grad(const float* __restrict__ X,
     if (tid == 0) *loss = se_all / (float)n;
 }
 
-// Network output for one feature row (weights in shared memory).
-__device__ float mlp_out(const float* __restrict__ w, const float* x) {
+// Network output for one feature row (weights in shared memory, 16-byte
+// aligned: one broadcast read per four multiply-adds; the hidden layer stays in
+// registers).
+__device__ __forceinline__ float mlp_out(const float* __restrict__ w, const float (&x)[kF]) {
     float h1[kH1];
-#pragma unroll 4
+#pragma unroll
     for (int j = 0; j < kH1; j++) {
         float acc = w[kOffB1 + j];
 #pragma unroll
-        for (int f = 0; f < kF; f++) acc = fmaf(w[j * kF + f], x[f], acc);
+        for (int f = 0; f < kF; f += 4) {
+            const float4 v = *reinterpret_cast<const float4*>(w + j * kF + f);
+            acc = fmaf(v.x, x[f], acc);
+            acc = fmaf(v.y, x[f + 1], acc);
+            acc = fmaf(v.z, x[f + 2], acc);
+            acc = fmaf(v.w, x[f + 3], acc);
+        }
         h1[j] = relu(acc);
     }
     float o = w[kOffB3];
+#pragma unroll 2
     for (int j = 0; j < kH2; j++) {
         float acc = w[kOffB2 + j];
-#pragma unroll 8
-        for (int i = 0; i < kH1; i++) acc = fmaf(w[kOffW2 + j * kH1 + i], h1[i], acc);
+#pragma unroll
+        for (int i = 0; i < kH1; i += 4) {
+            const float4 v = *reinterpret_cast<const float4*>(w + kOffW2 + j * kH1 + i);
+            acc = fmaf(v.x, h1[i], acc);
+            acc = fmaf(v.y, h1[i + 1], acc);
+            acc = fmaf(v.z, h1[i + 2], acc);
+            acc = fmaf(v.w, h1[i + 3], acc);
+        }
         o = fmaf(w[kOffW3 + j], relu(acc), o);
     }
     return o;
@@ -276,7 +291,7 @@ __global__ void __launch_bounds__(256) k_model_predict(const float* __restrict__
                                                        const float* __restrict__ W, float* __restrict__ out,
                                                        const uint32_t* __restrict__ cell_start, float nmax,
                                                        double* __restrict__ est) {
-    __shared__ float w[kModelWeights];
+    __shared__ __align__(16) float w[kModelWeights];
     __shared__ double red[8];
     for (int i = threadIdx.x; i < kModelWeights; i += blockDim.x) w[i] = W[i];
     __syncthreads();
@@ -285,7 +300,13 @@ __global__ void __launch_bounds__(256) k_model_predict(const float* __restrict__
     if (c < m) {
         float x[kF];
 #pragma unroll
-        for (int f = 0; f < kF; f++) x[f] = X[(size_t)c * kF + f];
+        for (int f = 0; f < kF; f += 4) {
+            const float4 v = *reinterpret_cast<const float4*>(X + (size_t)c * kF + f);
+            x[f] = v.x;
+            x[f + 1] = v.y;
+            x[f + 2] = v.z;
+            x[f + 3] = v.w;
+        }
         const float o = mlp_out(w, x);
         if (out) out[c] = o;
         if (cell_start) {
