@@ -682,7 +682,7 @@ int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int mo
     GSJ_CUDA(c, cudaEventRecord(c->tev[3], st));
     GSJ_TRY(pairs_to_csr(c, pairs, R, R, shift, N, counts, offsets, cand));
     S.screen_rechecks = screen ? U : 0;
-    S.join_path = screen ? GSJ_PATH_SCREEN : GSJ_PATH_TILE;
+    S.join_path = a.n >= kScreenPathDims && screen ? GSJ_PATH_SCREEN : GSJ_PATH_TILE;
     S.ms_join = now_ms() - t_join;
     S.ms_total = now_ms() - t_start;
     return GSJ_OK;
@@ -1177,8 +1177,10 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     // High-dimensional float data with populated cells (at least 8 points per
     // non-empty cell on average) takes the tile join; everything else the
     // warp-per-item passes.
-    // From 16 dimensions on, the tile join screens pairs with BF16 dot
-    // products on the tensor cores (GSJ_FLAG_PLAIN turns the screen off).
+    // The tile join screens pairs with BF16 dot products on the tensor cores
+    // (GSJ_FLAG_PLAIN turns the screen off): a tile of 128 x 128 pairs takes about
+    // 600 cycles of an SM at any n up to 28, the FP32 form 2,000 at n = 5 and
+    // 3,000 and more from 8 on.
     const int model = model_of(cfg);
     bool tile = false, screen = false;
     if constexpr (std::is_same<T, float>::value) {
@@ -1191,9 +1193,9 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     // (path, dim, density), else the launchers' defaults
     const uint32_t path_id = cfg.sort ? GSJ_PATH_SORT
                              : tpq    ? GSJ_PATH_ROWS
-                             : screen ? GSJ_PATH_SCREEN
-                             : tile   ? GSJ_PATH_TILE
-                                      : GSJ_PATH_WARP;
+                             : screen && n >= kScreenPathDims ? GSJ_PATH_SCREEN
+                             : tile                           ? GSJ_PATH_TILE
+                                                              : GSJ_PATH_WARP;
     uint32_t dlog = 0;
     while (dlog < 31 && (N / std::max<uint32_t>(M, 1u)) >> (dlog + 1)) dlog++;
     S.density_log2 = dlog;
@@ -1840,7 +1842,7 @@ int gsj_model_train(gsj_context* c, uint32_t steps, float* loss) {
     GSJ_TRY(d2h_small(c, &l, d_loss + 2, 1));
     if (loss) *loss = l;
     c->model_trained = steps > 0 || c->model_trained;
-    if (c->stats.join_path == GSJ_PATH_SCREEN && c->stats.total_pairs)
+    if (c->stats.screen_rechecks && c->stats.total_pairs)
         c->model_unc_ratio = (double)c->stats.screen_rechecks / (double)c->stats.total_pairs;
     return GSJ_OK;
 }

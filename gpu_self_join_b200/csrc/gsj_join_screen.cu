@@ -992,9 +992,9 @@ cudaError_t launch_screen_prep(const float* pts, uint32_t N, uint32_t n, uint32_
 }
 
 bool screen_supported(uint32_t n, uint32_t npad, uint32_t k, int model, uint32_t ilp, float thr) {
-    // n + 2 columns: the dimensions and the folded candidate norm
-    return tile_supported(n, npad, k, model, ilp) && n >= 16 && n + 2u <= kTileMaxN && thr >= 1e-30f &&
-           thr <= 1e30f;
+    // n + 4 columns: the dimensions, the candidate's and the query's bound terms
+    return tile_supported(n, npad, k, model, ilp) && ((n + 4u + 15u) & ~15u) <= kMaxKpad && n + 2u <= kTileMaxN &&
+           thr >= 1e-30f && thr <= 1e30f;
 }
 
 ScreenConst make_screen_const(uint32_t n, float thr) {

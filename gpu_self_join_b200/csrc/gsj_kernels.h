@@ -143,6 +143,7 @@ cudaError_t launch_pairs_to_table(const unsigned long long* keys, uint64_t R, ui
 // Tensor-core screened tile join (gsj_join_screen.cu): BF16 tcgen05 dot
 // products with a proven rejection bound, exact FP32 check of the rest.
 constexpr int kScreenQ = 128;         // queries per screened work item (MMA M)
+constexpr uint32_t kScreenPathDims = 16;  // a screened join reports GSJ_PATH_SCREEN from here on, GSJ_PATH_TILE below
 struct ScreenConst {
     float r0;             // >= sqrt(thr) with the reference sum's rounding room
     float c1, c0;         // FP32 accumulation bound per unit squared norm, per unit r0^2

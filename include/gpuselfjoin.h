@@ -120,8 +120,9 @@ typedef struct gsj_stats {
     double dev_ms_fill;       /* fill pass (other paths: pair sort + table)     */
     uint64_t kernel_launches; /* launches of this library's own kernels         */
     uint64_t join_path;       /* GSJ_PATH_* taken by the last join              */
-    uint64_t screen_rechecks; /* GSJ_PATH_SCREEN: pairs the BF16 screen could not
-                                 reject, evaluated exactly (0 on other paths)   */
+    uint64_t screen_rechecks; /* GSJ_PATH_TILE, GSJ_PATH_SCREEN: pairs the BF16 screen
+                                 could not reject, evaluated exactly (0 when the
+                                 join was not screened)                        */
     uint64_t reruns;          /* passes repeated because a buffer sized from the
                                  estimate was short (the output is unchanged)  */
     uint64_t batches;         /* result batches of gsj_join_host (1 otherwise)  */
@@ -137,7 +138,9 @@ typedef struct gsj_stats {
 #define GSJ_PATH_WARP 0u  /* warp per (cell, 32 queries): pair keys + on-device sort */
 #define GSJ_PATH_ROWS 1u  /* dense k <= 3, n <= 4: thread-per-query count + fill   */
 #define GSJ_PATH_TILE 2u  /* float, 5 <= n <= 128, k <= 6, >= 8 points per cell:
-                             64 x 64 register tiles, pair buffer, on-device sort */
+                             screened below 16 dimensions like GSJ_PATH_SCREEN, with
+                             GSJ_FLAG_PLAIN (or above 126) 64 x 64 register tiles
+                             of the exact arithmetic                          */
 #define GSJ_PATH_SCREEN 3u /* float, 16 <= n <= 128, k <= 6, >= 8 points per cell:
                              BF16 tcgen05 screen with a proven bound, exact FP32
                              check of the rest, pair buffer, on-device sort   */

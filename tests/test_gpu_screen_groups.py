@@ -34,3 +34,16 @@ def test_screen_far_and_tight_points(oracle, n):
     pts[2000:2300] = pts[2000] + np.float32(0.01) * np.random.default_rng(1).standard_normal((300, n)).astype(np.float32)
     st = assert_same(oracle, pts, 3.0, indexed_dims=6, stamp=False)
     assert st["join_path"] == 3
+
+
+@pytest.mark.parametrize("stamp", [False, True])
+@pytest.mark.parametrize("n,k,ilp,sc", [(5, 5, 0, False), (6, 2, 8, True), (8, 3, 8, True), (11, 6, 4, False),
+                                        (12, 6, 0, False), (13, 6, 8, False), (15, 1, 2, True)])
+def test_low_dimensional_screen(oracle, n, k, ilp, sc, stamp):
+    """Below 16 dimensions (one MMA step of 16 columns up to n = 12) the tile
+    join is screened too and still reports GSJ_PATH_TILE; plain turns it off."""
+    pts = tile_points(n, 6003, 3.0, 700 + n)
+    st = assert_same(oracle, pts, 3.0, indexed_dims=k, ilp=ilp, shortcircuit=sc, stamp=stamp)
+    assert st["join_path"] == 2 and st["screen_rechecks"] > 0
+    st = assert_same(oracle, pts, 3.0, indexed_dims=k, ilp=ilp, shortcircuit=sc, stamp=stamp, plain=True)
+    assert st["join_path"] == 2 and st["screen_rechecks"] == 0
