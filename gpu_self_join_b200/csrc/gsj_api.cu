@@ -172,7 +172,7 @@ struct gsj_context {
     cudaEvent_t ev[2] = {nullptr, nullptr};
     cudaEvent_t tev[8] = {};  // stage timing: index, count, fill (start/end), estimate start/end
     // device pool
-    Buf in, pts, ids, keys, keys2, vals, cell_key, cell_start, dense, dcnt, plan, slot_cell, htab, order,
+    Buf in, pts, ids, keys, keys2, vals, cell_key, cell_start, dense, plan, slot_cell, htab, order,
         sizes, nchunks,
         item_off, items, fwd, swords, counts, offsets, table, temp, scan_temp, misc, var, perm, minarr,
         minmax_part, pairs, srows, snorms, spartial, scentre, unc, table2, nbtab, bitoff, hitbits, ptemp, sortv, heavy, gstart;
@@ -838,20 +838,16 @@ int rows_to_host(gsj_context* c, JoinArgs<T>& a, const gsj_config& cfg, uint64_t
 // pass, list offsets, fill pass writing every list in candidate order.
 template <typename T>
 int sort_join(gsj_context* c, JoinArgs<T>& a, uint64_t N, int model, uint32_t* counts, uint64_t* offsets,
-              const uint32_t* cell_start, uint32_t M, double t_join, double t_start) {
+              const uint32_t* slot_cell, double t_join, double t_start) {
     gsj_stats& S = c->stats;
     cudaStream_t st = c->st;
-    uint32_t* slot_cell = nullptr;
-    GSJ_TRY(dev_get(c, c->slot_cell, N, &slot_cell));
-    S.kernel_launches += 1;
-    GSJ_CUDA(c, launch_slot_cell(cell_start, M, nullptr, 0, slot_cell, nullptr, st));
     GSJ_CUDA(c, cudaEventRecord(c->tev[2], st));
     S.kernel_launches += 1;
     GSJ_CUDA(c, launch_sort_join<T>(a, slot_cell, counts, model, false, c->num_sms, st));
     GSJ_CUDA(c, cudaEventRecord(c->tev[3], st));
     void* stemp = nullptr;
     GSJ_TRY(dev_get(c, c->scan_temp, scan_u32_u64_temp_bytes(N), (unsigned char**)&stemp));
-    S.kernel_launches += 3;
+    S.kernel_launches += (uint64_t)scan_launches(N);
     GSJ_CUDA(c, scan_u32_u64(counts, offsets, N, stemp, st));
     uint64_t R = 0;
     GSJ_TRY(d2h_small(c, &R, offsets + N, 1));
@@ -1064,17 +1060,27 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
         std::swap(vals, ids);
     }
 
-    // ---- runs of equal keys = non-empty cells: cell_key[M], cell_start[M+1]
+    // cell lookup: on dense grids a slot-prefix table over every linear cell id,
+    // else a hash table of the grid rows that hold a cell
+    const uint64_t dense_limit = std::max<uint64_t>(1u << 24, 8ull * N);
+    const bool dense = totalCells <= dense_limit && totalCells < (1ull << 30);
+    const bool tpq = dense && k <= 3 && cfg.ilp == 0 && n <= 4 && !cfg.sort;
+
+    // ---- runs of equal keys = non-empty cells: cell_key[M], cell_start[M+1], and
+    // each slot's cell for the paths with a thread or warp per query
+    uint32_t* slot_cell = nullptr;
+    if (tpq || cfg.sort) GSJ_TRY(dev_get(c, c->slot_cell, N, &slot_cell));
     uint64_t* cell_key = nullptr;
     uint32_t* cell_start = nullptr;
     GSJ_TRY(dev_get(c, c->cell_key, N, &cell_key));
     GSJ_TRY(dev_get(c, c->cell_start, N + 1, &cell_start));
-    S.kernel_launches += 5;
+    nl = 0;
     if (key32)
-        GSJ_CUDA(c, run_length<uint32_t>(reinterpret_cast<const uint32_t*>(keys2), N, cell_key, cell_start, d_nruns,
-                                         temp, st));
+        GSJ_CUDA(c, run_length<uint32_t>(reinterpret_cast<const uint32_t*>(keys2), N, cell_key, cell_start, slot_cell,
+                                         d_nruns, temp, &nl, st));
     else
-        GSJ_CUDA(c, run_length<uint64_t>(keys2, N, cell_key, cell_start, d_nruns, temp, st));
+        GSJ_CUDA(c, run_length<uint64_t>(keys2, N, cell_key, cell_start, slot_cell, d_nruns, temp, &nl, st));
+    S.kernel_launches += (uint64_t)nl;
     uint32_t runs[2] = {0, 0};
     GSJ_TRY(d2h_small(c, runs, d_nruns, 2));
     if (runs[1])
@@ -1121,36 +1127,24 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     S.kernel_launches += 1;
     GSJ_CUDA(c, launch_gather_points<T>(d_in, N, n, npad, d_perm, ids, pts, st));
 
-    // ---- cell lookup: on dense grids a slot-prefix table over every linear
-    // cell id (cell L holds slots [ds[L], ds[L+1])), else a hash table of the
-    // non-empty cells
-    uint32_t *ds = nullptr, *dcnt = nullptr;
+    // ---- cell lookup
+    uint32_t* ds = nullptr;
     uint4* htab = nullptr;
     uint64_t hmask = 0;
-    const uint64_t dense_limit = std::max<uint64_t>(1u << 24, 8ull * N);
-    const bool dense = totalCells <= dense_limit && totalCells < (1ull << 30);
+    S.kernel_launches += 1;
     if (dense) {
         GSJ_TRY(dev_get(c, c->dense, totalCells + 1, &ds));
-        GSJ_TRY(dev_get(c, c->dcnt, totalCells + 1, &dcnt));
-        GSJ_CUDA(c, cudaMemsetAsync(dcnt, 0, (totalCells + 1) * sizeof(uint32_t), st));
+        GSJ_CUDA(c, launch_dense_slots(cell_key, cell_start, M, totalCells, ds, st));
     } else {
         uint64_t hcap = 1024;
         while (hcap < 2ull * M) hcap <<= 1;
         hmask = hcap - 1;
         GSJ_TRY(dev_get(c, c->htab, hcap, &htab));
         GSJ_CUDA(c, cudaMemsetAsync(htab, 0xff, hcap * sizeof(uint4), st));
-    }
-    S.kernel_launches += 1;
-    GSJ_CUDA(c, launch_cell_tables(cell_key, cell_start, M, dcnt, g.ncells[0], htab, hmask, st));
-    if (dense) {
-        // the slot-prefix table: ds[L] = points in cells below L (ds[totalCells] = N)
-        GSJ_TRY(dev_get(c, c->temp, scan_u32_u64_temp_bytes(totalCells), (unsigned char**)&temp));
-        S.kernel_launches += 3;
-        GSJ_CUDA(c, scan_u32_u32(dcnt, ds, totalCells, temp, st));
+        GSJ_CUDA(c, launch_row_table(cell_key, M, g.ncells[0], htab, hmask, st));
     }
     // The ROWS path (dense low-dimensional grids) is driven by a per-cell plan of
     // neighbour-row slot ranges.
-    const bool tpq = dense && k <= 3 && cfg.ilp == 0 && n <= 4 && !cfg.sort;
     uint2* plan = nullptr;
     if (tpq) {
         const uint32_t nrows = k == 1 ? 1u : (k == 2 ? 3u : 9u);
@@ -1158,18 +1152,16 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
         S.kernel_launches += 1;
         GSJ_CUDA(c, launch_cell_plan(cell_key, M, g, ds, plan, st));
     }
-    uint32_t* slot_cell = nullptr;
     uint64_t* bitoff = nullptr;
     if (tpq) {
-        // slot -> cell, and the hit-mask layout: slot s's query owns words
-        // [bitoff[s], bitoff[s+1]) of the count pass's bit masks
+        // the hit-mask layout: slot s's query owns words [bitoff[s], bitoff[s+1]) of
+        // the count pass's bit masks
         uint32_t* swords = nullptr;
         const uint32_t nrows = k == 1 ? 1u : (k == 2 ? 3u : 9u);
-        GSJ_TRY(dev_get(c, c->slot_cell, N, &slot_cell));
         GSJ_TRY(dev_get(c, c->swords, N, &swords));
         GSJ_TRY(dev_get(c, c->bitoff, N + 1, &bitoff));
         GSJ_TRY(dev_get(c, c->scan_temp, scan_u32_u64_temp_bytes(N), (unsigned char**)&temp));
-        S.kernel_launches += 4;
+        S.kernel_launches += 1 + (uint64_t)scan_launches(N);
         GSJ_CUDA(c, launch_slot_cell(cell_start, M, plan, nrows, slot_cell, swords, st));
         GSJ_CUDA(c, scan_u32_u64(swords, bitoff, N, temp, st));
     }
@@ -1237,7 +1229,7 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
             uint32_t* gs = nullptr;
             GSJ_TRY(dev_get(c, c->gstart, M + 1, &gs));
             GSJ_TRY(dev_get(c, c->temp, scan_u32_u64_temp_bytes(M), (unsigned char**)&temp));
-            S.kernel_launches += 5;
+            S.kernel_launches += 2 + (uint64_t)scan_launches(M);
             GSJ_CUDA(c, launch_group_flags(cell_key, M, g.ncells[0], gspan, nchunks, st));
             GSJ_CUDA(c, scan_u32_u32(nchunks, item_off, M, temp, st));
             GSJ_CUDA(c, launch_group_starts_of(nchunks, item_off, cell_start, M, (uint32_t)N, gs, st));
@@ -1270,7 +1262,7 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
             GSJ_CUDA(c, launch_item_counts(gstart, nullptr, M, qchunk, nchunks, nullptr, st));
         }
         GSJ_TRY(dev_get(c, c->temp, scan_u32_u64_temp_bytes(M), (unsigned char**)&temp));
-        S.kernel_launches += 3;
+        S.kernel_launches += (uint64_t)scan_launches(M);
         GSJ_CUDA(c, scan_u32_u32(nchunks, item_off, M, temp, st));
         GSJ_TRY(d2h_small(c, &num_items, item_off + M, 1));
         S.work_items = num_items;
@@ -1335,7 +1327,7 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     c->last.lookup.n_points = (uint32_t)N;
     c->last.lookup.ids = ids;
     const bool learned = !exact_size && cfg.estimator == GSJ_EST_LEARNED && c->model_trained;
-    if (cfg.sort) return sort_join<T>(c, a, N, model, counts, offsets, cell_start, M, t_join, t_start);
+    if (cfg.sort) return sort_join<T>(c, a, N, model, counts, offsets, slot_cell, t_join, t_start);
     if constexpr (std::is_same<T, float>::value) {
         if (tile) {
             unsigned long long* cursor = reinterpret_cast<unsigned long long*>(ctr + 4);
@@ -1367,7 +1359,7 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     // ---- list offsets (counts are by point id)
     void* stemp = nullptr;
     GSJ_TRY(dev_get(c, c->scan_temp, scan_u32_u64_temp_bytes(N), (unsigned char**)&stemp));
-    S.kernel_launches += 3;
+    S.kernel_launches += (uint64_t)scan_launches(N);
     GSJ_CUDA(c, scan_u32_u64(counts, offsets, N, stemp, st));
     uint64_t R = 0;
     GSJ_TRY(d2h_small(c, &R, offsets + N, 1));
@@ -1523,7 +1515,7 @@ int gsj_destroy(gsj_context* c) {
     if (c->st) cudaStreamSynchronize(c->st);
     if (c->st2) cudaStreamSynchronize(c->st2);
     Buf* bufs[] = {&c->in,       &c->pts,   &c->ids,    &c->keys,      &c->keys2,   &c->vals,      &c->cell_key,
-                   &c->cell_start, &c->dense, &c->dcnt, &c->plan, &c->slot_cell, &c->htab,
+                   &c->cell_start, &c->dense, &c->plan, &c->slot_cell, &c->htab,
                    &c->order,    &c->sizes,
                    &c->nchunks,  &c->item_off, &c->items, &c->fwd,     &c->swords,     &c->counts,    &c->offsets,
                    &c->table, &c->temp,   &c->scan_temp, &c->misc,    &c->var,       &c->perm,

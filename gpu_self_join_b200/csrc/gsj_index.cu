@@ -14,6 +14,7 @@
 #include "gsj_common.cuh"
 #include "gsj_fp.cuh"
 #include "gsj_kernels.h"
+#include "gsj_scan.cuh"
 
 namespace gsj {
 
@@ -233,12 +234,72 @@ __global__ void k_gather_rows(const T* __restrict__ in, uint64_t N, uint32_t n, 
 }
 
 // ------------------------------------------------------------ cell lookup
-// Points per linear cell id (zero elsewhere); its exclusive scan is the
-// slot-prefix table ds: cell L holds slots [ds[L], ds[L+1]).
-__global__ void k_dense_counts(const uint64_t* __restrict__ cell_key, const uint32_t* __restrict__ cell_start,
-                               uint32_t M, uint32_t* __restrict__ dcnt) {
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < M) dcnt[cell_key[c]] = cell_start[c + 1] - cell_start[c];
+// First index of sorted keys[0 .. M) at or past `v`, found by a warp: 32 probes
+// cut the range to a 33rd at a time.
+__device__ __forceinline__ uint32_t warp_lower_bound(const uint64_t* __restrict__ keys, uint32_t M, uint64_t v) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t lo = 0, hi = M;
+    while (lo < hi) {
+        const uint32_t step = (hi - lo) / 33u + 1u;
+        const uint32_t at = (uint32_t)min((uint64_t)hi - 1u, (uint64_t)lo + (uint64_t)(lane + 1u) * step - 1u);
+        const uint32_t below = (uint32_t)__popc(__ballot_sync(0xffffffffu, keys[at] < v));  // a prefix of the lanes
+        // keys[probe of lane below - 1] < v <= keys[probe of lane below]
+        const uint64_t nlo = below ? min((uint64_t)hi, (uint64_t)lo + (uint64_t)below * step) : lo;
+        const uint64_t nhi = below < 32u ? min((uint64_t)hi - 1u, (uint64_t)lo + (uint64_t)(below + 1u) * step - 1u) : hi;
+        lo = (uint32_t)nlo;
+        hi = (uint32_t)(nhi < nlo ? nlo : nhi);
+    }
+    return lo;
+}
+
+// Slot-prefix table of a dense grid: ds[L] = points in cells below L, for L in
+// [0, total] (cell L holds slots [ds[L], ds[L+1])).  A block owns kScanTile
+// linear ids: it finds its cells in the sorted list, marks their places, and
+// the rank of every place leads to the first slot of the next cell.  (Before:
+// a cleared count array, a scatter of the cells' sizes and a scan of the
+// whole grid, three more passes over it.)
+__global__ void __launch_bounds__(kScanThreads) k_dense_slots(const uint64_t* __restrict__ cell_key,
+                                                              const uint32_t* __restrict__ cell_start, uint32_t M,
+                                                              uint64_t total, uint32_t* __restrict__ ds) {
+    __shared__ uint32_t mark[kScanTile / 32];
+    __shared__ uint32_t starts[kScanTile + 1];
+    __shared__ uint32_t range[2];
+    const uint64_t l0 = blockIdx.x * kScanTile;
+    if (threadIdx.x < kScanTile / 32) mark[threadIdx.x] = 0u;
+    if (threadIdx.x < 64u) {
+        const uint32_t w = threadIdx.x >> 5;
+        const uint32_t r = warp_lower_bound(cell_key, M, l0 + w * kScanTile);
+        if ((threadIdx.x & 31u) == 0u) range[w] = r;
+    }
+    __syncthreads();
+    const uint32_t c0 = range[0], n = range[1] - c0;
+    for (uint32_t i = threadIdx.x; i <= n; i += kScanThreads) {
+        starts[i] = cell_start[c0 + i];
+        if (i < n) {
+            const uint32_t at = (uint32_t)(cell_key[c0 + i] - l0);
+            atomicOr(&mark[at >> 5], 1u << (at & 31u));
+        }
+    }
+    __syncthreads();
+    const uint32_t bits = (mark[threadIdx.x >> 1] >> (16u * (threadIdx.x & 1u))) & 0xffffu;
+    unsigned long long tot;
+    uint32_t rank = (uint32_t)block_excl_scan<kScanThreads>((unsigned long long)__popc(bits), &tot);
+    const uint64_t e0 = l0 + (uint64_t)threadIdx.x * kScanItems;
+    uint32_t o[kScanItems];
+#pragma unroll
+    for (int i = 0; i < kScanItems; i++) {
+        o[i] = starts[rank];
+        rank += (bits >> i) & 1u;
+    }
+    if (e0 + kScanItems <= total + 1u) {
+        uint4* p = reinterpret_cast<uint4*>(ds + e0);
+#pragma unroll
+        for (int q = 0; q < kScanItems / 4; q++) p[q] = make_uint4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < kScanItems; i++)
+            if (e0 + (uint64_t)i <= total) ds[e0 + i] = o[i];
+    }
 }
 
 // Entries {linear id of the row's cell 0, first cell, cells} of the grid rows
@@ -401,10 +462,17 @@ cudaError_t launch_gather_points(const T* in, uint64_t N, uint32_t n, uint32_t n
 }
 
 
-cudaError_t launch_cell_tables(const uint64_t* cell_key, const uint32_t* cell_start, uint32_t M, uint32_t* dcnt,
-                               uint32_t n0, uint4* htab, uint64_t hmask, cudaStream_t st) {
-    if (dcnt) k_dense_counts<<<blocks_for(M, 256), 256, 0, st>>>(cell_key, cell_start, M, dcnt);
-    if (htab) k_row_insert<<<blocks_for(M, 256), 256, 0, st>>>(cell_key, M, n0, htab, hmask);
+cudaError_t launch_dense_slots(const uint64_t* cell_key, const uint32_t* cell_start, uint32_t M, uint64_t total,
+                               uint32_t* ds, cudaStream_t st) {
+    if (reinterpret_cast<uintptr_t>(ds) & 15u) return cudaErrorInvalidValue;
+    k_dense_slots<<<(unsigned)((total + 1u + kScanTile - 1u) / kScanTile), kScanThreads, 0, st>>>(cell_key, cell_start,
+                                                                                                  M, total, ds);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_row_table(const uint64_t* cell_key, uint32_t M, uint32_t n0, uint4* htab, uint64_t hmask,
+                             cudaStream_t st) {
+    k_row_insert<<<blocks_for(M, 256), 256, 0, st>>>(cell_key, M, n0, htab, hmask);
     return cudaGetLastError();
 }
 

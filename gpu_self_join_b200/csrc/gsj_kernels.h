@@ -31,11 +31,13 @@ cudaError_t launch_cell_keys(const T* in, uint64_t N, uint32_t n, const uint32_t
 template <typename T>
 cudaError_t launch_gather_points(const T* in, uint64_t N, uint32_t n, uint32_t npad, const uint32_t* perm,
                                  const uint32_t* ids, T* pts, cudaStream_t st);
-// Either the dense per-linear-id point counts (dcnt[key] = size, to be
-// scanned into the slot-prefix table) or the hash table of the grid rows that
-// hold a cell (n0: the grid's cells in dim 0).
-cudaError_t launch_cell_tables(const uint64_t* cell_key, const uint32_t* cell_start, uint32_t M, uint32_t* dcnt,
-                               uint32_t n0, uint4* htab, uint64_t hmask, cudaStream_t st);
+// Dense grids: the slot-prefix table ds[0 .. total] (16-byte aligned).  The
+// others: the hash table of the grid rows that hold a cell (n0: the grid's
+// cells in dim 0; all entries empty).
+cudaError_t launch_dense_slots(const uint64_t* cell_key, const uint32_t* cell_start, uint32_t M, uint64_t total,
+                               uint32_t* ds, cudaStream_t st);
+cudaError_t launch_row_table(const uint64_t* cell_key, uint32_t M, uint32_t n0, uint4* htab, uint64_t hmask,
+                             cudaStream_t st);
 cudaError_t launch_cell_plan(const uint64_t* cell_key, uint32_t M, const GridGeom& g, const uint32_t* ds,
                              uint2* plan, cudaStream_t st);
 // Query groups of up to `span` neighbouring cells of a grid row: flags[M] marks

@@ -383,7 +383,7 @@ cudaError_t place_pairs(const unsigned long long* keys, uint64_t nkeys, uint32_t
     e = scan_u32_u64(counts, offsets, nlists, temp, st);
     if (e != cudaSuccess) return e;
     if (nkeys) k_pair_place<<<g, 256, 0, st>>>(keys, nkeys, shift, offsets, cursor, table, cap, err);
-    if (launches) *launches += 5;
+    if (launches) *launches += (nkeys ? 2 : 0) + scan_launches(nlists);
     return cudaGetLastError();
 }
 

@@ -4,8 +4,10 @@
 // stitching (GPU.cu:863-980, kernel.cu:79-105, GPU.cu:1143-1214): with exact
 // per-point counts the table is laid out by one scan.
 //
-// Three phases over tiles of kScanTile elements: tile sums, a single-block
-// scan of the tile sums, and the tile-local scans with the tile prefix added.
+// Over tiles of kScanTile elements: one launch for one tile; up to kDirectTiles
+// tiles a launch of tile sums and one of tile-local scans, each block adding up
+// the sums before its tile; beyond that a single-block scan of the tile sums
+// between the two.
 // Thread t of a tile owns its elements [16 t, 16 t + 16): four 16-byte loads
 // when the arrays are 16-byte aligned, one block-wide scan of the 256 thread
 // sums, then 16 sequential outputs per thread.
@@ -19,63 +21,12 @@
 
 #include "../../include/gpuselfjoin.h"
 #include "gsj_kernels.h"
+#include "gsj_scan.cuh"
 #include "gsj_scan.h"
 
 namespace gsj {
 
-constexpr int kScanThreads = 256;
-constexpr int kScanItems = 16;
-constexpr uint64_t kScanTile = (uint64_t)kScanThreads * kScanItems;
 constexpr int kTileSumThreads = 1024;  // the single block scanning the tile sums
-
-__device__ __forceinline__ unsigned long long warp_incl_scan(unsigned long long x, int lane) {
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    return x;
-}
-
-// Block-wide exclusive scan of one value per thread (THREADS threads);
-// returns the exclusive prefix and writes the block total to *total.
-template <int THREADS>
-__device__ __forceinline__ unsigned long long block_excl_scan(unsigned long long v, unsigned long long* total) {
-    __shared__ unsigned long long wsum[THREADS / 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned long long inc = warp_incl_scan(v, lane);
-    if (lane == 31) wsum[warp] = inc;
-    __syncthreads();
-    if (warp == 0) {
-        unsigned long long w = lane < THREADS / 32 ? wsum[lane] : 0ull;
-        w = warp_incl_scan(w, lane);
-        if (lane < THREADS / 32) wsum[lane] = w;
-    }
-    __syncthreads();
-    const unsigned long long before = warp ? wsum[warp - 1] : 0ull;
-    *total = wsum[THREADS / 32 - 1];
-    __syncthreads();
-    return before + inc - v;
-}
-
-// Elements [e0, e0 + kScanItems) (zero past n); vec: in is 16-byte aligned.
-__device__ __forceinline__ void load_items(const uint32_t* __restrict__ in, uint64_t e0, uint64_t n, bool vec,
-                                           uint32_t (&v)[kScanItems]) {
-    if (vec && e0 + kScanItems <= n) {
-        const uint4* p = reinterpret_cast<const uint4*>(in + e0);
-#pragma unroll
-        for (int q = 0; q < kScanItems / 4; q++) {
-            const uint4 x = p[q];
-            v[4 * q] = x.x;
-            v[4 * q + 1] = x.y;
-            v[4 * q + 2] = x.z;
-            v[4 * q + 3] = x.w;
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < kScanItems; i++) v[i] = e0 + (uint64_t)i < n ? in[e0 + i] : 0u;
-    }
-}
 
 __global__ void __launch_bounds__(kScanThreads) k_tile_sums(const uint32_t* __restrict__ in, uint64_t n, bool vec,
                                                             unsigned long long* __restrict__ tsum) {
@@ -115,19 +66,21 @@ __global__ void __launch_bounds__(kTileSumThreads) k_scan_tile_sums(unsigned lon
 // OutT is uint64_t (list offsets) or uint32_t (slot offsets, digit offsets:
 // the caller guarantees that the total fits).  vin / vout: in / out are
 // 16-byte aligned (a thread's 16 elements are then 4 aligned vectors in and
-// 4 or 8 out).
+// 4 or 8 out).  scanned: tsum holds the exclusive prefix of the tile sums, else
+// the tile sums themselves (not read with one tile).
 template <typename OutT>
 __global__ void __launch_bounds__(kScanThreads) k_tile_scan(const uint32_t* __restrict__ in, uint64_t n, bool vin,
-                                                            const unsigned long long* __restrict__ tsum,
-                                                            uint64_t ntiles, OutT* __restrict__ out, bool vout) {
+                                                            const unsigned long long* __restrict__ tsum, bool scanned,
+                                                            OutT* __restrict__ out, bool vout) {
     const uint64_t e0 = blockIdx.x * kScanTile + (uint64_t)threadIdx.x * kScanItems;
     uint32_t v[kScanItems];
     load_items(in, e0, n, vin, v);
+    const unsigned long long before = scanned ? tsum[blockIdx.x] : tile_prefix(tsum, blockIdx.x);
     unsigned long long s = 0;
 #pragma unroll
     for (int i = 0; i < kScanItems; i++) s += v[i];
     unsigned long long tot;
-    unsigned long long pre = tsum[blockIdx.x] + block_excl_scan<kScanThreads>(s, &tot);
+    unsigned long long pre = before + block_excl_scan<kScanThreads>(s, &tot);
     OutT o[kScanItems];
 #pragma unroll
     for (int i = 0; i < kScanItems; i++) {
@@ -149,7 +102,12 @@ __global__ void __launch_bounds__(kScanThreads) k_tile_scan(const uint32_t* __re
         for (int i = 0; i < kScanItems; i++)
             if (e0 + (uint64_t)i < n) out[e0 + i] = o[i];
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) out[n] = (OutT)tsum[ntiles];
+    if (blockIdx.x == gridDim.x - 1u && threadIdx.x == 0) out[n] = (OutT)(before + tot);
+}
+
+cudaError_t scan_tile_sums(unsigned long long* tsum, uint64_t ntiles, cudaStream_t st) {
+    k_scan_tile_sums<<<1, kTileSumThreads, 0, st>>>(tsum, ntiles);
+    return cudaGetLastError();
 }
 
 size_t scan_u32_u64_temp_bytes(uint64_t n) { return ((n + kScanTile - 1) / kScanTile + 1) * sizeof(unsigned long long); }
@@ -161,10 +119,19 @@ static cudaError_t scan_any(const uint32_t* in, OutT* out, uint64_t n, void* tem
     if (ntiles == 0) return cudaMemsetAsync(out, 0, sizeof(OutT), st);
     const bool vin = (reinterpret_cast<uintptr_t>(in) & 15u) == 0;
     const bool vout = (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
-    k_tile_sums<<<(unsigned)ntiles, kScanThreads, 0, st>>>(in, n, vin, tsum);
-    k_scan_tile_sums<<<1, kTileSumThreads, 0, st>>>(tsum, ntiles);
-    k_tile_scan<OutT><<<(unsigned)ntiles, kScanThreads, 0, st>>>(in, n, vin, tsum, ntiles, out, vout);
+    const bool scanned = ntiles > kDirectTiles;
+    if (ntiles > 1) k_tile_sums<<<(unsigned)ntiles, kScanThreads, 0, st>>>(in, n, vin, tsum);
+    if (scanned) {
+        const cudaError_t e = scan_tile_sums(tsum, ntiles, st);
+        if (e != cudaSuccess) return e;
+    }
+    k_tile_scan<OutT><<<(unsigned)ntiles, kScanThreads, 0, st>>>(in, n, vin, tsum, scanned, out, vout);
     return cudaGetLastError();
+}
+
+int scan_launches(uint64_t n) {
+    const uint64_t ntiles = (n + kScanTile - 1) / kScanTile;
+    return ntiles <= 1 ? (int)ntiles : ntiles <= kDirectTiles ? 2 : 3;
 }
 
 cudaError_t scan_u32_u64(const uint32_t* in, uint64_t* out, uint64_t n, void* temp, cudaStream_t st) {

@@ -12,4 +12,7 @@ cudaError_t scan_u32_u64(const uint32_t* in, uint64_t* out, uint64_t n, void* te
 // The same with 32-bit outputs (the caller guarantees that the total fits);
 // temp as for scan_u32_u64.
 cudaError_t scan_u32_u32(const uint32_t* in, uint32_t* out, uint64_t n, void* temp, cudaStream_t st);
+// Kernel launches of one scan of n elements.
+int scan_launches(uint64_t n);
+
 }  // namespace gsj

@@ -11,7 +11,9 @@
 // reduce-then-scan over tiles of kSortTile keys:
 //   k_radix_hist     per-tile digit counts, written digit-major
 //   scan_u32_u32     exclusive scan of the counts: the global offset of each
-//                    (digit, tile) run
+//                    (digit, tile) run; with few tiles (kFewTiles) every block
+//                    of the scatter derives its offsets from the counts
+//                    itself, and with one tile the counts are its own
 //   k_radix_scatter  the tile is ranked stably in shared memory (per-warp
 //                    match_any groups, in index order), then written out in
 //                    sorted order, so each digit's run of the tile is stored
@@ -21,6 +23,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "gsj_scan.cuh"
 #include "gsj_scan.h"
 #include "gsj_sort.h"
 
@@ -34,6 +37,10 @@ constexpr int kSortItems = 8;                           // keys per thread
 constexpr int kSortTile = kSortThreads * kSortItems;    // keys per tile
 constexpr int kWarpKeys = kSortTile / kSortWarps;       // keys per warp (8 rounds of 32)
 constexpr int kMaxBins = 512;  // digits of 8 or 9 bits
+// Tiles up to which a block of the scatter reads all the tiles' digit counts (64
+// x 512 words at most, 1 to 2 us) instead of two more launches per pass (a scan
+// of a few thousand counts takes 5 us and its gaps): up to 131,072 keys.
+constexpr uint64_t kFewTiles = 64;
 static_assert(kMaxBins % kSortThreads == 0, "whole digits per thread in the tile prefix");
 
 __device__ __forceinline__ unsigned lanemask_lt_s() {
@@ -74,7 +81,8 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_scatter(const K* __restr
                                                                 const uint32_t* __restrict__ vin,
                                                                 K* __restrict__ kout, uint32_t* __restrict__ vout,
                                                                 uint64_t n, int shift,
-                                                                const uint32_t* __restrict__ offs, uint32_t ntiles) {
+                                                                const uint32_t* __restrict__ hist, bool scanned,
+                                                                uint32_t ntiles) {
     extern __shared__ __align__(16) unsigned char sort_smem[];
     K* skeys = reinterpret_cast<K*>(sort_smem);
     uint32_t* svals = reinterpret_cast<uint32_t*>(sort_smem + sizeof(K) * kSortTile);
@@ -142,11 +150,47 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_scatter(const K* __restr
         for (int w = 0; w < kSortWarps; w++)
             if (w < warp) before += wsum[w];
         uint32_t ex = before + x - p;
+        // global offset of each digit's run of this tile: from the scanned counts, or
+        // the digit's start over all tiles plus its counts in the tiles before
+        uint32_t run[DPT];
+        if (scanned) {
+#pragma unroll
+            for (int dd = 0; dd < DPT; dd++) run[dd] = hist[(uint64_t)(d0 + dd) * ntiles + blockIdx.x];
+        } else if (ntiles == 1u) {
+            uint32_t e1 = ex;
+#pragma unroll
+            for (int dd = 0; dd < DPT; dd++) {
+                run[dd] = e1;
+                e1 += pd[dd];
+            }
+        } else {
+            uint32_t all[DPT], sum = 0;
+#pragma unroll
+            for (int dd = 0; dd < DPT; dd++) {
+                const uint32_t* h = hist + (uint64_t)(d0 + dd) * ntiles;
+                uint32_t here = 0, t_all = 0;
+                for (uint32_t t = 0; t < ntiles; t++) {
+                    const uint32_t c = h[t];
+                    here += t < blockIdx.x ? c : 0u;
+                    t_all += c;
+                }
+                run[dd] = here;
+                all[dd] = t_all;
+                sum += t_all;
+            }
+            unsigned long long tot;
+            uint32_t start = (uint32_t)block_excl_scan<kSortThreads>(sum, &tot);
+#pragma unroll
+            for (int dd = 0; dd < DPT; dd++) {
+                run[dd] += start;
+                start += all[dd];
+            }
+        }
 #pragma unroll
         for (int dd = 0; dd < DPT; dd++) {
             const int d = d0 + dd;
             tile_off[d] = ex;
-            gbase[d] = offs[(uint64_t)d * ntiles + blockIdx.x] - ex;  // modulo 2^32, re-added below
+            gbase[d] = run[dd] - ex;  // modulo 2^32, re-added below
             ex += pd[dd];
         }
     }
@@ -171,22 +215,91 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_scatter(const K* __restr
     }
 }
 
+// Runs of equal keys: a run begins where a key differs from the one before it.
+// Run heads among elements [e0, e0 + kScanItems), bit i for e0 + i, with the
+// keys in key[]; vec: keys is 16-byte aligned.
 template <typename K>
-__global__ void k_run_flags(const K* __restrict__ keys, uint64_t n, uint32_t* __restrict__ flags) {
-    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i < n) flags[i] = (i == 0 || keys[i] != keys[i - 1]) ? 1u : 0u;
+__device__ __forceinline__ uint32_t run_heads(const K* __restrict__ keys, uint64_t e0, uint64_t n, bool vec,
+                                              K (&key)[kScanItems]) {
+    if (vec && e0 + kScanItems <= n) {
+        const uint4* p = reinterpret_cast<const uint4*>(keys + e0);
+#pragma unroll
+        for (int q = 0; q < kScanItems * (int)sizeof(K) / 16; q++) {
+            const uint4 x = p[q];
+            if constexpr (sizeof(K) == 4) {
+                key[4 * q] = x.x;
+                key[4 * q + 1] = x.y;
+                key[4 * q + 2] = x.z;
+                key[4 * q + 3] = x.w;
+            } else {
+                key[2 * q] = ((K)x.y << 32) | x.x;
+                key[2 * q + 1] = ((K)x.w << 32) | x.z;
+            }
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < kScanItems; i++) key[i] = e0 + (uint64_t)i < n ? keys[e0 + i] : K(0);
+    }
+    uint32_t heads = 0;
+    if (e0 < n) heads = e0 == 0 || keys[e0 - 1] != key[0] ? 1u : 0u;
+#pragma unroll
+    for (int i = 1; i < kScanItems; i++) heads |= (e0 + (uint64_t)i < n && key[i] != key[i - 1] ? 1u : 0u) << i;
+    return heads;
 }
 
 template <typename K>
-__global__ void k_run_compact(const K* __restrict__ keys, uint64_t n, const uint32_t* __restrict__ flags,
-                              const uint32_t* __restrict__ pos, uint64_t* __restrict__ run_key,
-                              uint32_t* __restrict__ run_start) {
-    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i < n && flags[i]) {
-        run_key[pos[i]] = (uint64_t)keys[i];
-        run_start[pos[i]] = (uint32_t)i;
+__global__ void __launch_bounds__(kScanThreads) k_run_sums(const K* __restrict__ keys, uint64_t n, bool vec,
+                                                           unsigned long long* __restrict__ tsum) {
+    const uint64_t e0 = blockIdx.x * kScanTile + (uint64_t)threadIdx.x * kScanItems;
+    K key[kScanItems];
+    const uint32_t heads = run_heads(keys, e0, n, vec, key);
+    unsigned long long tot;
+    block_excl_scan<kScanThreads>((unsigned long long)__popc(heads), &tot);
+    if (threadIdx.x == 0) tsum[blockIdx.x] = tot;
+}
+
+// run_key, run_start and (optionally) elem_run[i] = run of element i, in one pass
+// over the keys once the tiles' run counts are known (see k_tile_scan for
+// `scanned`).
+template <typename K>
+__global__ void __launch_bounds__(kScanThreads) k_run_write(const K* __restrict__ keys, uint64_t n, bool vec,
+                                                            const unsigned long long* __restrict__ tsum, bool scanned,
+                                                            uint64_t* __restrict__ run_key,
+                                                            uint32_t* __restrict__ run_start,
+                                                            uint32_t* __restrict__ elem_run, bool vout,
+                                                            uint32_t* __restrict__ nruns) {
+    const uint64_t e0 = blockIdx.x * kScanTile + (uint64_t)threadIdx.x * kScanItems;
+    K key[kScanItems];
+    const uint32_t heads = run_heads(keys, e0, n, vec, key);
+    const unsigned long long before = scanned ? tsum[blockIdx.x] : tile_prefix(tsum, blockIdx.x);
+    unsigned long long tot;
+    uint32_t run = (uint32_t)(before + block_excl_scan<kScanThreads>((unsigned long long)__popc(heads), &tot));
+    uint32_t er[kScanItems];
+#pragma unroll
+    for (int i = 0; i < kScanItems; i++) {
+        if ((heads >> i) & 1u) {
+            run_key[run] = (uint64_t)key[i];
+            run_start[run] = (uint32_t)(e0 + (uint64_t)i);
+            run++;
+        }
+        er[i] = run - 1u;
     }
-    if (i == 0) run_start[pos[n]] = (uint32_t)n;
+    if (elem_run) {
+        if (vout && e0 + kScanItems <= n) {
+            uint4* p = reinterpret_cast<uint4*>(elem_run + e0);
+#pragma unroll
+            for (int q = 0; q < kScanItems / 4; q++)
+                p[q] = make_uint4(er[4 * q], er[4 * q + 1], er[4 * q + 2], er[4 * q + 3]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < kScanItems; i++)
+                if (e0 + (uint64_t)i < n) elem_run[e0 + i] = er[i];
+        }
+    }
+    if (blockIdx.x == gridDim.x - 1u && threadIdx.x == 0) {
+        run_start[before + tot] = (uint32_t)n;
+        *nruns = (uint32_t)(before + tot);
+    }
 }
 
 inline unsigned blocks_for(uint64_t n, unsigned t) { return (unsigned)((n + t - 1) / t); }
@@ -211,7 +324,7 @@ cudaError_t radix_sort(K* keys, K* keys_alt, uint32_t* vals, uint32_t* vals_alt,
     const uint64_t nt = tiles_of(n);
     const size_t hist_bytes = (size_t)kMaxBins * nt * sizeof(uint32_t);
     uint32_t* hist = static_cast<uint32_t*>(temp);
-    uint32_t* offs = reinterpret_cast<uint32_t*>(static_cast<unsigned char*>(temp) + hist_bytes);
+    uint32_t* scan = reinterpret_cast<uint32_t*>(static_cast<unsigned char*>(temp) + hist_bytes);
     void* stemp = static_cast<unsigned char*>(temp) + (2 * hist_bytes + sizeof(uint32_t) + 255) / 256 * 256;
     const size_t smem = sizeof(K) * kSortTile + (vals ? sizeof(uint32_t) * kSortTile : 0);
     cudaError_t e;
@@ -232,20 +345,30 @@ cudaError_t radix_sort(K* keys, K* keys_alt, uint32_t* vals, uint32_t* vals_alt,
     for (int pass = 0; pass < passes; pass++) {
         const bool wide = pass < nine;
         const uint32_t bins = wide ? 512u : 256u;
-        if (wide) k_radix_hist<K, 512><<<(unsigned)nt, kSortThreads, 0, st>>>(ki, n, shift, hist, (uint32_t)nt);
-        else k_radix_hist<K, 256><<<(unsigned)nt, kSortThreads, 0, st>>>(ki, n, shift, hist, (uint32_t)nt);
-        e = scan_u32_u32(hist, offs, (uint64_t)bins * nt, stemp, st);
-        if (e != cudaSuccess) return e;
+        const bool scanned = nt > kFewTiles;
+        const uint32_t* offs = hist;
+        int nl = 1;
+        if (nt > 1) {
+            if (wide) k_radix_hist<K, 512><<<(unsigned)nt, kSortThreads, 0, st>>>(ki, n, shift, hist, (uint32_t)nt);
+            else k_radix_hist<K, 256><<<(unsigned)nt, kSortThreads, 0, st>>>(ki, n, shift, hist, (uint32_t)nt);
+            nl++;
+        }
+        if (scanned) {
+            e = scan_u32_u32(hist, scan, (uint64_t)bins * nt, stemp, st);
+            if (e != cudaSuccess) return e;
+            nl += scan_launches((uint64_t)bins * nt);
+            offs = scan;
+        }
         if (wide) {
-            if (vals) k_radix_scatter<K, true, 512><<<(unsigned)nt, kSortThreads, smem, st>>>(ki, vi, ko, vo, n, shift, offs, (uint32_t)nt);
-            else k_radix_scatter<K, false, 512><<<(unsigned)nt, kSortThreads, smem, st>>>(ki, nullptr, ko, nullptr, n, shift, offs, (uint32_t)nt);
+            if (vals) k_radix_scatter<K, true, 512><<<(unsigned)nt, kSortThreads, smem, st>>>(ki, vi, ko, vo, n, shift, offs, scanned, (uint32_t)nt);
+            else k_radix_scatter<K, false, 512><<<(unsigned)nt, kSortThreads, smem, st>>>(ki, nullptr, ko, nullptr, n, shift, offs, scanned, (uint32_t)nt);
         } else {
-            if (vals) k_radix_scatter<K, true, 256><<<(unsigned)nt, kSortThreads, smem, st>>>(ki, vi, ko, vo, n, shift, offs, (uint32_t)nt);
-            else k_radix_scatter<K, false, 256><<<(unsigned)nt, kSortThreads, smem, st>>>(ki, nullptr, ko, nullptr, n, shift, offs, (uint32_t)nt);
+            if (vals) k_radix_scatter<K, true, 256><<<(unsigned)nt, kSortThreads, smem, st>>>(ki, vi, ko, vo, n, shift, offs, scanned, (uint32_t)nt);
+            else k_radix_scatter<K, false, 256><<<(unsigned)nt, kSortThreads, smem, st>>>(ki, nullptr, ko, nullptr, n, shift, offs, scanned, (uint32_t)nt);
         }
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
-        if (launches) *launches += 5;
+        if (launches) *launches += nl;
         shift += wide ? 9 : 8;
         K* tk = ki;
         ki = ko;
@@ -264,35 +387,31 @@ template cudaError_t radix_sort<uint32_t>(uint32_t*, uint32_t*, uint32_t*, uint3
 template cudaError_t radix_sort<uint64_t>(uint64_t*, uint64_t*, uint32_t*, uint32_t*, uint64_t, int, int, void*,
                                           bool*, int*, cudaStream_t);
 
-// flags[n + 1], then pos[n + 1] from the next 16-byte boundary (the scan moves
-// whole 16-byte vectors only between aligned arrays), then the scan's scratch.
-static uint64_t runs_pos_offset(uint64_t n) { return (n + 1 + 3) & ~3ull; }
-
-static size_t runs_arrays_bytes(uint64_t n) {
-    return ((runs_pos_offset(n) + n + 1) * sizeof(uint32_t) + 255) / 256 * 256;
-}
-
-size_t runs_temp_bytes(uint64_t n) { return runs_arrays_bytes(n) + scan_u32_u64_temp_bytes(n) + 256; }
+size_t runs_temp_bytes(uint64_t n) { return scan_u32_u64_temp_bytes(n); }
 
 template <typename K>
-cudaError_t run_length(const K* keys, uint64_t n, uint64_t* run_key, uint32_t* run_start, uint32_t* d_nruns,
-                       void* temp, cudaStream_t st) {
+cudaError_t run_length(const K* keys, uint64_t n, uint64_t* run_key, uint32_t* run_start, uint32_t* elem_run,
+                       uint32_t* d_nruns, void* temp, int* launches, cudaStream_t st) {
     if (n == 0) return cudaMemsetAsync(d_nruns, 0, sizeof(uint32_t), st);
-    uint32_t* flags = static_cast<uint32_t*>(temp);
-    uint32_t* pos = flags + runs_pos_offset(n);
-    void* stemp = static_cast<unsigned char*>(temp) + runs_arrays_bytes(n);
-    k_run_flags<K><<<blocks_for(n, 256), 256, 0, st>>>(keys, n, flags);
-    cudaError_t e = scan_u32_u32(flags, pos, n, stemp, st);
-    if (e != cudaSuccess) return e;
-    k_run_compact<K><<<blocks_for(n, 256), 256, 0, st>>>(keys, n, flags, pos, run_key, run_start);
-    e = cudaMemcpyAsync(d_nruns, pos + n, sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);
-    if (e != cudaSuccess) return e;
+    unsigned long long* tsum = static_cast<unsigned long long*>(temp);
+    const uint64_t nt = (n + kScanTile - 1) / kScanTile;
+    const bool scanned = nt > kDirectTiles;
+    const bool vec = (reinterpret_cast<uintptr_t>(keys) & 15u) == 0;
+    const bool vout = (reinterpret_cast<uintptr_t>(elem_run) & 15u) == 0;
+    if (nt > 1) k_run_sums<K><<<(unsigned)nt, kScanThreads, 0, st>>>(keys, n, vec, tsum);
+    if (scanned) {
+        const cudaError_t e = scan_tile_sums(tsum, nt, st);
+        if (e != cudaSuccess) return e;
+    }
+    k_run_write<K><<<(unsigned)nt, kScanThreads, 0, st>>>(keys, n, vec, tsum, scanned, run_key, run_start, elem_run,
+                                                          vout, d_nruns);
+    if (launches) *launches += scan_launches(n);
     return cudaGetLastError();
 }
 
-template cudaError_t run_length<uint32_t>(const uint32_t*, uint64_t, uint64_t*, uint32_t*, uint32_t*, void*,
-                                          cudaStream_t);
-template cudaError_t run_length<uint64_t>(const uint64_t*, uint64_t, uint64_t*, uint32_t*, uint32_t*, void*,
-                                          cudaStream_t);
+template cudaError_t run_length<uint32_t>(const uint32_t*, uint64_t, uint64_t*, uint32_t*, uint32_t*, uint32_t*, void*,
+                                          int*, cudaStream_t);
+template cudaError_t run_length<uint64_t>(const uint64_t*, uint64_t, uint64_t*, uint32_t*, uint32_t*, uint32_t*, void*,
+                                          int*, cudaStream_t);
 
 }  // namespace gsj

@@ -23,9 +23,10 @@ size_t runs_temp_bytes(uint64_t n);
 
 // Runs of equal keys in a sorted array: run_key[r] (as uint64), run_start[r]
 // for r < M and run_start[M] = n, with M written to *d_nruns (device).
-// run_key and run_start need n and n + 1 entries.
+// run_key and run_start need n and n + 1 entries; elem_run (optional, n
+// entries) receives each element's run.
 template <typename K>
-cudaError_t run_length(const K* keys, uint64_t n, uint64_t* run_key, uint32_t* run_start, uint32_t* d_nruns,
-                       void* temp, cudaStream_t st);
+cudaError_t run_length(const K* keys, uint64_t n, uint64_t* run_key, uint32_t* run_start, uint32_t* elem_run,
+                       uint32_t* d_nruns, void* temp, int* launches, cudaStream_t st);
 
 }  // namespace gsj
