@@ -174,8 +174,8 @@ struct gsj_context {
     // device pool
     Buf in, pts, ids, keys, keys2, vals, cell_key, cell_start, dense, plan, slot_cell, htab, order,
         sizes, nchunks,
-        item_off, items, fwd, swords, counts, offsets, table, temp, scan_temp, misc, var, perm, minarr,
-        minmax_part, pairs, srows, snorms, spartial, scentre, unc, table2, nbtab, bitoff, hitbits, ptemp, sortv, heavy, gstart;
+        item_off, items, cursor, counts, offsets, table, temp, scan_temp, misc, var, perm, minarr,
+        minmax_part, pairs, srows, snorms, spartial, scentre, unc, table2, nbtab, ptemp, sortv, heavy, gstart;
     PinnedBuf stage[2];
     PinnedBuf hmisc;
     // host-result pipeline: copy streams, per-segment events, pinned staging
@@ -417,7 +417,7 @@ int pairs_to_csr(gsj_context* c, unsigned long long* pairs, uint64_t nkeys, uint
     GSJ_CUDA(c, cudaEventRecord(c->tev[4], st));
     uint32_t *table = nullptr, *cursor = nullptr;
     GSJ_TRY(dev_get(c, c->table, R ? R : 1, &table));
-    GSJ_TRY(dev_get(c, c->fwd, N, &cursor));
+    GSJ_TRY(dev_get(c, c->cursor, N, &cursor));
     void* temp = nullptr;
     GSJ_TRY(dev_get(c, c->ptemp, place_temp_bytes(N), (unsigned char**)&temp));
     uint32_t* d_err = reinterpret_cast<uint32_t*>(c->misc.p) + 4 * kMaxK + 20;
@@ -712,8 +712,7 @@ int ensure_copy_streams(gsj_context* c, int nseg) {
 // has a known place in the host table.
 template <typename T>
 int rows_to_host(gsj_context* c, JoinArgs<T>& a, const gsj_config& cfg, uint64_t N, uint64_t R,
-                 const uint32_t* slot_cell, const uint64_t* bitoff, const uint32_t* hitbits, const uint32_t* counts,
-                 const uint64_t* offsets, const HostOut& ho) {
+                 const uint32_t* slot_cell, const uint32_t* counts, const uint64_t* offsets, const HostOut& ho) {
     gsj_stats& S = c->stats;
     cudaStream_t st = c->st;
     uint32_t* ctr = a.work_counter;
@@ -814,8 +813,7 @@ int rows_to_host(gsj_context* c, JoinArgs<T>& a, const gsj_config& cfg, uint64_t
         a.table = seg;
         GSJ_CUDA(c, cudaMemsetAsync(ctr, 0, sizeof(uint32_t), st));
         S.kernel_launches += 1;
-        GSJ_CUDA(c, launch_rows_fill<T>(a, slot_cell, bitoff, hitbits, qslots + h_gs[b], h_gs[b + 1] - h_gs[b],
-                                        h_bo[b], c->num_sms, st));
+        GSJ_CUDA(c, launch_rows_fill<T>(a, slot_cell, qslots + h_gs[b], h_gs[b + 1] - h_gs[b], h_bo[b], c->num_sms, st));
         GSJ_CUDA(c, cudaEventRecord(c->seg_filled[sg], st));
         const uint64_t rb = h_bo[b + 1] - h_bo[b];
         GSJ_CUDA(c, cudaStreamWaitEvent(c->cst[sg], c->seg_filled[sg], 0));
@@ -1152,20 +1150,6 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
         S.kernel_launches += 1;
         GSJ_CUDA(c, launch_cell_plan(cell_key, M, g, ds, plan, st));
     }
-    uint64_t* bitoff = nullptr;
-    if (tpq) {
-        // the hit-mask layout: slot s's query owns words [bitoff[s], bitoff[s+1]) of
-        // the count pass's bit masks
-        uint32_t* swords = nullptr;
-        const uint32_t nrows = k == 1 ? 1u : (k == 2 ? 3u : 9u);
-        GSJ_TRY(dev_get(c, c->swords, N, &swords));
-        GSJ_TRY(dev_get(c, c->bitoff, N + 1, &bitoff));
-        GSJ_TRY(dev_get(c, c->scan_temp, scan_u32_u64_temp_bytes(N), (unsigned char**)&temp));
-        S.kernel_launches += 1 + (uint64_t)scan_launches(N);
-        GSJ_CUDA(c, launch_slot_cell(cell_start, M, plan, nrows, slot_cell, swords, st));
-        GSJ_CUDA(c, scan_u32_u64(swords, bitoff, N, temp, st));
-    }
-
     // High-dimensional float data with populated cells (at least 8 points per
     // non-empty cell on average) takes the tile join; everything else the
     // warp-per-item passes.
@@ -1275,9 +1259,7 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     const double t_join = now_ms();
     S.ms_index = t_join - t_index;
 
-    // ---- join arguments (every path); per-slot list lengths of the ROWS path
-    uint32_t* fwd = nullptr;
-    if (tpq) GSJ_TRY(dev_get(c, c->fwd, N, &fwd));
+    // ---- join arguments (every path)
     uint32_t* ctr = reinterpret_cast<uint32_t*>(d_mm + 2 * kMaxK) + 2;  // work counter
     unsigned long long* cand = reinterpret_cast<unsigned long long*>(reinterpret_cast<uint32_t*>(d_mm + 2 * kMaxK) + 4);
     GSJ_CUDA(c, cudaMemsetAsync(ctr, 0, 4 * sizeof(uint32_t), st));
@@ -1299,12 +1281,12 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     a.n = n;
     a.npad = npad;
     a.n_points = (uint32_t)N;
+    a.num_cells = M;
     a.ilp = cfg.ilp;
     a.g = g;
     a.thr = threshold_of<T>(eps);
     a.eps = eps;
     for (uint32_t j = 0; j < k; j++) a.minv[j] = minArr[j];
-    a.fwd_cnt = fwd;
     a.cand_cnt = cand;
     a.shape_threads = shape.threads;
     a.shape_warps = shape.warps;
@@ -1341,19 +1323,11 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
         return emit_join<T>(c, a, N, stamp, model, exact_size, learned, counts, offsets, cursor, t_join,
                             t_start);
     }
-    // Dense low-dimensional grids (the ROWS path): the distance work is cheap
-    // and the cells too small for per-cell warp work, so one thread per query
-    // evaluates its full neighbourhood once, recording the decisions as a bit
-    // mask; the fill pass replays the masks into the table.
-    uint32_t* hitbits = nullptr;
-    {
-        uint64_t nwords = 0;
-        GSJ_TRY(d2h_small(c, &nwords, bitoff + N, 1));
-        GSJ_TRY(dev_get(c, c->hitbits, nwords ? nwords : 1, &hitbits));
-    }
+    // Dense low-dimensional grids (the ROWS path): the distance work is cheap, so
+    // a count pass gives every list its place and a fill pass repeats the tests.
     GSJ_CUDA(c, cudaEventRecord(c->tev[2], st));
     S.kernel_launches += 1;
-    GSJ_CUDA(c, launch_rows_count<T>(a, slot_cell, bitoff, hitbits, counts, c->num_sms, st));
+    GSJ_CUDA(c, launch_rows_count<T>(a, slot_cell, counts, c->num_sms, st));
     GSJ_CUDA(c, cudaEventRecord(c->tev[3], st));
 
     // ---- list offsets (counts are by point id)
@@ -1378,7 +1352,7 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
         }
         gsj_config pcfg = cfg;
         if (shape.streams) pcfg.streams = shape.streams;
-        GSJ_TRY(rows_to_host<T>(c, a, pcfg, N, R, slot_cell, bitoff, hitbits, counts, offsets, *ho));
+        GSJ_TRY(rows_to_host<T>(c, a, pcfg, N, R, slot_cell, counts, offsets, *ho));
         {
             float ms = 0;
             GSJ_CUDA(c, cudaEventElapsedTime(&ms, c->tev[0], c->tev[1]));
@@ -1408,7 +1382,7 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     a.err_flag = ctr + 1;  // zeroed with the counters before the count pass
     GSJ_CUDA(c, cudaEventRecord(c->tev[4], st));
     S.kernel_launches += 1;
-    GSJ_CUDA(c, launch_rows_fill<T>(a, slot_cell, bitoff, hitbits, nullptr, (uint32_t)N, 0, c->num_sms, st));
+    GSJ_CUDA(c, launch_rows_fill<T>(a, slot_cell, nullptr, (uint32_t)N, 0, c->num_sms, st));
     GSJ_CUDA(c, cudaEventRecord(c->tev[5], st));
     GSJ_CUDA(c, cudaStreamSynchronize(st));
     {
@@ -1517,10 +1491,10 @@ int gsj_destroy(gsj_context* c) {
     Buf* bufs[] = {&c->in,       &c->pts,   &c->ids,    &c->keys,      &c->keys2,   &c->vals,      &c->cell_key,
                    &c->cell_start, &c->dense, &c->plan, &c->slot_cell, &c->htab,
                    &c->order,    &c->sizes,
-                   &c->nchunks,  &c->item_off, &c->items, &c->fwd,     &c->swords,     &c->counts,    &c->offsets,
+                   &c->nchunks,  &c->item_off, &c->items, &c->cursor,  &c->counts,    &c->offsets,
                    &c->table, &c->temp,   &c->scan_temp, &c->misc,    &c->var,       &c->perm,
                    &c->minarr,   &c->minmax_part, &c->pairs, &c->srows, &c->snorms,
-                   &c->spartial, &c->scentre, &c->unc, &c->table2, &c->nbtab, &c->bitoff, &c->hitbits, &c->ptemp, &c->sortv, &c->heavy, &c->gstart};
+                   &c->spartial, &c->scentre, &c->unc, &c->table2, &c->nbtab, &c->ptemp, &c->sortv, &c->heavy, &c->gstart};
     for (Buf* b : bufs)
         if (b->p) cudaFree(b->p);
     for (auto* pb : {&c->stage[0], &c->stage[1], &c->hmisc})

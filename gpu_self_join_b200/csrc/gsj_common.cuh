@@ -46,12 +46,11 @@ struct JoinArgs {
     uint32_t* work_counter;       // dynamic work distribution
     uint32_t n, npad, ilp;
     uint32_t n_points;            // N
+    uint32_t num_cells;           // non-empty cells
     GridGeom g;
     T thr;                        // s <= thr  <=>  sqrt(s) <= eps
     T eps;                        // epsilon in T (cell formula)
     T minv[kMaxK];                // minArr (grid origin per indexed dim)
-    // counts (ROWS path; the other paths add to cand_cnt only)
-    uint32_t* fwd_cnt;            // [N] list length by slot
     unsigned long long* cand_cnt; // candidate evaluations
     // fill pass (ROWS path)
     const uint64_t* offsets;      // [N+1] by original id

@@ -7,22 +7,28 @@
 // neighbourhood of kernel.cu:292-302, taken in a fixed order: candidate f of
 // query s is the f-th slot of the concatenated ranges.
 //
-//   k_rows_count  one thread per query slot (the slots of a warp are
-//                 consecutive in cell order, so lanes of one cell walk the same
-//                 ranges: broadcast loads).  It evaluates every candidate in the
-//                 reference's arithmetic and records the decisions as a bit
-//                 mask (bit f of the query's words), the list length by slot and
-//                 by point id.
-//   k_rows_fill   a warp per 32 consecutive query slots, two queries at a time
-//                 (one per half-warp).  A half-warp replays its query's bit mask
-//                 - no second distance pass - one mask word per step: lane l
-//                 takes bits 2l and 2l + 1, loads the ids of those candidates
-//                 whose bit is set, and stores them at the query's next free list
-//                 positions, so each word's hits are written by the half's lanes
-//                 to consecutive places of the point-id-ordered table.
-// Both kernels claim their 32-slot chunks dynamically (one atomic per warp,
-// the next claim issued before the current chunk is processed), since chunk
-// costs vary with the local density by orders of magnitude.
+// k_rows_join takes 32 consecutive query slots a warp (a few cells) and cell by
+// cell puts 128 candidates of the cell in the lanes' registers, coordinates and
+// ids, four a lane; every query of the cell is then tested against 32 candidates
+// at a time, a vote giving the hits.  The count pass adds up the votes; the fill
+// pass, which runs once the lists have their places, repeats the tests and lets
+// the lanes with a hit store their ids to consecutive list places.
+//
+// Repeating the test (4 instructions in 2-D) costs less than keeping its result:
+// the earlier form had the count pass record every decision as a bit (a thread
+// per query, 60 % of the lanes active, since neighbouring queries have candidate
+// rows of different lengths) and the fill pass replay the bits of two queries a
+// warp step, loading each hit's id on its own; the masks also needed a per-slot
+// layout (a pass over the cells and a scan), 0.5 GB of traffic and a host
+// read-back of their size between the index and the join.  Bound by instruction
+// issue (0.77 of the slots in the fill).  Measured, count + fill (and the mask
+// layout before): 2-D 20M points 1.28 + 3.00 + 0.23 -> 0.93 + 2.80 ms; 3-D
+// double 250k 0.120 + 0.126 -> 0.080 + 0.101 ms.  Four CTAs an SM (64 registers)
+// for float: 2-D 20M 3.03 / 2.80 / 3.01 / 2.80 ms with 3 / 4 / 5 / 6; double
+// spills there (3-D 250k 0.101 / 0.114 with 2 / 4).
+// The chunks are claimed dynamically (one atomic per warp, the next claim
+// issued before the current chunk is processed), since chunk costs vary with the
+// local density by orders of magnitude.
 #include <cstdint>
 #include <cuda_runtime.h>
 #include <type_traits>
@@ -74,9 +80,162 @@ __device__ __forceinline__ void load_row(const T* __restrict__ p, T (&r)[NT]) {
     }
 }
 
+template <typename T>
+__device__ __forceinline__ T quiet_nan();
+template <>
+__device__ __forceinline__ float quiet_nan<float>() {
+    return __int_as_float(0x7fffffff);
+}
+template <>
+__device__ __forceinline__ double quiet_nan<double>() {
+    return __longlong_as_double(0x7fffffffffffffffll);
+}
+
+// Where a query's list goes: read back with one 16-byte broadcast.
+struct alignas(16) FillList {
+    unsigned long long dst;
+    uint32_t len, pad;
+};
+
+// Queries: the slots qslots[0 .. nq) (slots 0 .. nq-1 when qslots is null).
+// Count pass: counts_by_id[id] = list length.  Fill pass: the list of point id i
+// goes to a.table[offsets[i] - base]; a list that would leave the table or
+// differ from its counted length raises *err_flag and is not written past it.
+template <typename T, int NT, int NR, int POL, bool FILL>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_rows_join(const JoinArgs<T> a, const uint32_t* __restrict__ slot_cell,
+                                                   uint32_t* __restrict__ counts_by_id,
+                                                   const uint32_t* __restrict__ qslots, uint32_t nq, uint64_t base) {
+    constexpr int G = 4;                             // candidates a lane holds
+    static_assert(G == 4, "the tile counts below");
+    __shared__ T sq[8][32 * NT];                     // the chunk's query rows (blockDim.x <= 256)
+    __shared__ FillList slist[FILL ? 8 : 1][32];
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned lt;
+    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
+    const uint32_t npad = a.npad;
+    const T thr = a.thr;
+    unsigned long long cand = 0;
+    uint32_t cur = __shfl_sync(FULL, claim32(a.work_counter, lane), 0);
+    while (cur < nq) {
+        const uint32_t nxt = claim32(a.work_counter, lane);  // in flight while this chunk runs
+        const uint32_t nv = min(32u, nq - cur);
+        const bool valid = (uint32_t)lane < nv;
+        const uint32_t s = valid ? (qslots ? qslots[cur + (uint32_t)lane] : cur + (uint32_t)lane) : 0u;
+        const uint32_t id = a.ids[s];
+        const uint32_t cell = valid ? slot_cell[s] : 0xffffffffu;
+        T own[NT];
+        load_row<T, NT>(a.pts + (size_t)s * npad, own);
+        uint32_t len = 0;
+        uint2 e[NR <= 3 ? NR : 1];
+        if (NR <= 3) {
+#pragma unroll
+            for (int r = 0; r < (NR <= 3 ? NR : 1); r++)
+                e[r] = valid ? a.plan[(size_t)cell * NR + r] : make_uint2(0u, 0u);
+        }
+        __syncwarp();  // the previous chunk's reads of the staging are done
+#pragma unroll
+        for (int l = 0; l < NT; l++) sq[warp][lane * NT + l] = own[l];
+        if (FILL) {
+            unsigned long long dst = 0;
+            if (valid) {
+                dst = a.offsets[id] - base;
+                len = (uint32_t)(a.offsets[id + 1] - a.offsets[id]);
+                if (dst + len > a.table_cap) {
+                    *a.err_flag = 1u;
+                    len = 0u;
+                }
+            }
+            slist[warp][lane] = FillList{dst, len, 0u};
+        }
+        __syncwarp();
+        const uint32_t prev = __shfl_up_sync(FULL, cell, 1);
+        unsigned heads = __ballot_sync(FULL, valid && (lane == 0 || cell != prev));
+        uint32_t run = 0;  // hits of this lane's query so far
+        while (heads) {
+            // queries [j0, j1) of one cell
+            const uint32_t j0 = (uint32_t)__ffs(heads) - 1u;
+            heads &= heads - 1u;
+            const uint32_t j1 = heads ? (uint32_t)__ffs(heads) - 1u : nv;
+            // candidate f is slot f + adj[r] of the last row r with pre[r] <= f
+            uint32_t adj[NR], pre[NR], total = 0;
+            uint2 er = make_uint2(0u, 0u);
+            if (NR > 3) {
+                const uint32_t c = __shfl_sync(FULL, cell, (int)j0);
+                if (lane < NR) er = a.plan[(size_t)c * NR + lane];
+            }
+#pragma unroll
+            for (int r = 0; r < NR; r++) {
+                const uint32_t st = __shfl_sync(FULL, NR <= 3 ? e[NR <= 3 ? r : 0].x : er.x, NR <= 3 ? (int)j0 : r);
+                const uint32_t n = __shfl_sync(FULL, NR <= 3 ? e[NR <= 3 ? r : 0].y : er.y, NR <= 3 ? (int)j0 : r);
+                pre[r] = total;
+                adj[r] = st - total;
+                total += n;
+            }
+            if (!FILL) cand += (unsigned long long)total * (j1 - j0);
+            for (uint32_t f0 = 0; f0 < total; f0 += 32u * G) {
+                T cx[G][NT];
+                uint32_t cid[G];
+#pragma unroll
+                for (int t = 0; t < G; t++) {
+                    const uint32_t f = f0 + 32u * (uint32_t)t + (uint32_t)lane;
+                    uint32_t d = adj[0];
+#pragma unroll
+                    for (int r = 1; r < NR; r++)
+                        if (f >= pre[r]) d = adj[r];
+                    const bool in = f < total;
+                    if (f0 + 32u * (uint32_t)t < total) {
+                        const uint32_t slot = in ? f + d : s;
+                        load_row<T, NT>(a.pts + (size_t)slot * npad, cx[t]);
+                        if (FILL) cid[t] = a.ids[slot];
+                        if (!in) cx[t][0] = quiet_nan<T>();  // within no threshold
+                    }
+                }
+                // the cell's queries against the group's W tiles of 32 candidates
+                auto test = [&](auto tiles) {
+                    constexpr int W = decltype(tiles)::value;
+                    for (uint32_t j = j0; j < j1; j++) {
+                        T q[NT];
+#pragma unroll
+                        for (int l = 0; l < NT; l++) q[l] = sq[warp][j * NT + l];
+                        uint32_t rj = f0 ? __shfl_sync(FULL, run, (int)j) : 0u;
+                        FillList fl{};
+                        if (FILL) fl = slist[FILL ? warp : 0][j];
+                        uint32_t* list = FILL ? a.table + fl.dst : nullptr;
+#pragma unroll
+                        for (int t = 0; t < W; t++) {
+                            const bool hit = sqdist_seq_reg<T, NT, POL>(q, cx[t]) <= thr;
+                            const unsigned b = __ballot_sync(FULL, hit);
+                            if (FILL) {
+                                const uint32_t pos = rj + (uint32_t)__popc(b & lt);
+                                if (hit && pos < fl.len) list[pos] = cid[t];
+                            }
+                            rj += (uint32_t)__popc(b);
+                        }
+                        if ((uint32_t)lane == j) run = rj;
+                    }
+                };
+                const uint32_t left = total - f0;
+                if (left > 96u) test(std::integral_constant<int, 4>{});
+                else if (left > 64u) test(std::integral_constant<int, 3>{});
+                else if (left > 32u) test(std::integral_constant<int, 2>{});
+                else test(std::integral_constant<int, 1>{});
+            }
+        }
+        if (FILL) {
+            if (valid && run != len) *a.err_flag = 1u;
+        } else if (valid) {
+            counts_by_id[id] = run;
+        }
+        cur = __shfl_sync(FULL, nxt, 0);
+    }
+    if (!FILL && lane == 0 && cand) atomicAdd(a.cand_cnt, cand);
+}
+
+// Count pass with a thread per query: the slots of a warp are consecutive in
+// cell order, so lanes of one cell walk the same ranges (broadcast loads).
 template <typename T, int NT, int NR, int POL>
 __global__ void __launch_bounds__(256) k_rows_count(const JoinArgs<T> a, const uint32_t* __restrict__ slot_cell,
-                                                    const uint64_t* __restrict__ bitoff, uint32_t* __restrict__ bits,
                                                     uint32_t* __restrict__ counts_by_id) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -92,40 +251,20 @@ __global__ void __launch_bounds__(256) k_rows_count(const JoinArgs<T> a, const u
             const uint32_t cell = slot_cell[s];
             T q[NT];
             load_row<T, NT>(a.pts + (size_t)s * npad, q);
-            uint64_t wp = bitoff[s];
-            uint32_t cnt = 0, word = 0, b = 0;  // b: next bit of the current mask word
+            uint32_t cnt = 0;
 #pragma unroll
             for (int r = 0; r < NR; r++) {
                 const uint2 e = a.plan[(size_t)cell * NR + r];
                 const T* cp = a.pts + (size_t)e.x * npad;
-                uint32_t left = e.y;
-                cand += left;
-                while (left) {
-                    // candidates up to the end of the current mask word
-                    const uint32_t m = min(left, 32u - b);
+                cand += e.y;
 #pragma unroll 4
-                    for (uint32_t u = 0; u < m; u++) {
-                        T cr[NT];
-                        load_row<T, NT>(cp, cr);
-                        cp += npad;
-                        const T d2 = sqdist_seq_reg<T, NT, POL>(q, cr);
-                        word |= (d2 <= thr ? 1u : 0u) << (b + u);
-                    }
-                    b += m;
-                    left -= m;
-                    if (b == 32u) {
-                        bits[wp++] = word;
-                        cnt += (uint32_t)__popc(word);
-                        word = 0u;
-                        b = 0u;
-                    }
+                for (uint32_t u = 0; u < e.y; u++) {
+                    T cr[NT];
+                    load_row<T, NT>(cp, cr);
+                    cp += npad;
+                    cnt += sqdist_seq_reg<T, NT, POL>(q, cr) <= thr ? 1u : 0u;
                 }
             }
-            if (b) {
-                bits[wp] = word;
-                cnt += (uint32_t)__popc(word);
-            }
-            a.fwd_cnt[s] = cnt;
             counts_by_id[a.ids[s]] = cnt;
         }
         cur = __shfl_sync(FULL, nxt, 0);
@@ -135,94 +274,6 @@ __global__ void __launch_bounds__(256) k_rows_count(const JoinArgs<T> a, const u
     if (lane == 0 && cand) atomicAdd(a.cand_cnt, cand);
 }
 
-// Queries: the slots qslots[0 .. nq) (all slots 0 .. nq-1 when qslots is
-// null); the list of point id i goes to a.table[offsets[i] - base].
-// Per-query parameters of the fill, staged in shared memory by the lane that
-// loaded them and read back by the whole warp (one broadcast per 16 bytes).
-template <int NR>
-struct alignas(16) FillQuery {
-    unsigned long long dst;  // list place in the table (relative to the batch base)
-    unsigned long long bo;   // first mask word
-    uint32_t cnt, nw;        // list length, mask words
-    uint32_t lo[NR];         // first slot of each candidate row
-    uint32_t pre[NR];        // candidates before each row
-};
-
-template <int NR>
-__global__ void __launch_bounds__(256) k_rows_fill(const JoinArgs<float> a, const uint32_t* __restrict__ slot_cell,
-                                                   const uint64_t* __restrict__ bitoff,
-                                                   const uint32_t* __restrict__ bits,
-                                                   const uint32_t* __restrict__ qslots, uint32_t nq, uint64_t base) {
-    __shared__ FillQuery<NR> qp[8][32];  // blockDim.x <= 256
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    FillQuery<NR>* wq = qp[threadIdx.x >> 5];
-    uint32_t cur = __shfl_sync(FULL, claim32(a.work_counter, lane), 0);
-    while (cur < nq) {
-        const uint32_t nxt = claim32(a.work_counter, lane);
-        const uint32_t j = cur + (uint32_t)lane;
-        const uint32_t nv = min(32u, nq - cur);
-        // lane j: query j's list length, mask words, list place and candidate rows
-        FillQuery<NR> f{};
-        if (j < nq) {
-            const uint32_t s = qslots ? qslots[j] : j;
-            f.cnt = a.fwd_cnt[s];
-            f.bo = bitoff[s];
-            f.nw = (uint32_t)(bitoff[s + 1] - f.bo);
-            f.dst = a.offsets[a.ids[s]] - base;
-            if (f.dst + f.cnt > a.table_cap) {
-                *a.err_flag = 1u;
-                f.cnt = 0u;
-            }
-            const uint32_t cell = slot_cell[s];
-            uint32_t p = 0;
-#pragma unroll
-            for (int r = 0; r < NR; r++) {
-                const uint2 e = a.plan[(size_t)cell * NR + r];
-                f.lo[r] = e.x;
-                f.pre[r] = p;
-                p += e.y;
-            }
-        }
-        __syncwarp();  // the previous chunk's reads of wq are done
-        wq[lane] = f;
-        __syncwarp();
-        // two queries at a time, one per half-warp: lane l of a half takes bits
-        // 2l and 2l + 1 of each of its query's mask words
-        const uint32_t h = (uint32_t)lane >> 4, hl = (uint32_t)lane & 15u;
-        for (uint32_t qi = 0; qi < nv; qi += 2u) {
-            const FillQuery<NR> q = wq[qi + h];  // entries past nv are zero (no words)
-            const uint32_t qnw = q.cnt ? q.nw : 0u;
-            uint32_t* list = a.table + q.dst;
-            const uint32_t* qb = bits + q.bo;
-            const uint32_t nwmax = max(__shfl_sync(FULL, qnw, 0), __shfl_sync(FULL, qnw, 16));
-            uint32_t run = 0;  // entries of this half's list written so far
-            for (uint32_t t0 = 0; t0 < nwmax; t0 += 16u) {
-                const uint32_t myw = (t0 + hl < qnw) ? qb[t0 + hl] : 0u;
-                const uint32_t tn = min(16u, nwmax - t0);
-                for (uint32_t tt = 0; tt < tn; tt++) {
-                    const uint32_t w = __shfl_sync(FULL, myw, (int)(h * 16u + tt));
-                    if (__ballot_sync(FULL, w != 0u) == 0u) continue;
-#pragma unroll
-                    for (uint32_t bs = 0; bs < 2u; bs++) {
-                        const uint32_t bit = 2u * hl + bs;
-                        if ((w >> bit) & 1u) {
-                            const uint32_t f = (t0 + tt) * 32u + bit;
-                            uint32_t st = q.lo[0] + f;
-#pragma unroll
-                            for (int r = 1; r < NR; r++)
-                                if (f >= q.pre[r]) st = q.lo[r] + (f - q.pre[r]);
-                            list[run + (uint32_t)__popc(w & ((1u << bit) - 1u))] = a.ids[st];
-                        }
-                    }
-                    run += (uint32_t)__popc(w);
-                }
-            }
-        }
-        cur = __shfl_sync(FULL, nxt, 0);
-    }
-}
-
 // Resident CTAs of a kernel, for persistent grids.
 static int resident_blocks(const void* kern, int threads, size_t smem, int num_sms) {
     int per_sm = 0;
@@ -230,94 +281,76 @@ static int resident_blocks(const void* kern, int threads, size_t smem, int num_s
     return num_sms * per_sm;
 }
 
-template <typename T, int NT, int NR>
-static cudaError_t launch_count_nt(const JoinArgs<T>& a, const uint32_t* slot_cell, const uint64_t* bitoff,
-                                   uint32_t* bits, uint32_t* counts_by_id, int num_sms, cudaStream_t st) {
+template <typename T, int NT, int NR, bool FILL>
+static cudaError_t launch_rows(const JoinArgs<T>& a, const uint32_t* slot_cell, uint32_t* counts_by_id,
+                               const uint32_t* qslots, uint32_t nq, uint64_t base, int num_sms, cudaStream_t st) {
     constexpr int POL = sizeof(T) == 8 ? kPolF64 : kPolF32;
-    auto kern = k_rows_count<T, NT, NR, POL>;
     const int threads = a.shape_threads ? (int)a.shape_threads : 256;
+    if constexpr (!FILL) {
+        // Sparse cells leave the lanes of k_rows_join's cells half empty and pay its
+        // set-up for few queries; from about 7 points a cell on (5 in double) the
+        // cell form is faster.  Count pass, cell form against thread per query: 2-D
+        // 20M at 3.1 points a cell 1.76 / 0.93 ms, 3-D 2M at 7.3 0.349 / 0.357,
+        // 3-D 250k double at 7.0 0.082 / 0.113, 3-D 2M with 2 dims indexed at 175
+        // 1.46 / 1.68.
+        if (a.n_points < (sizeof(T) == 8 ? 5u : 7u) * (uint64_t)a.num_cells) {
+            auto kern = k_rows_count<T, NT, NR, POL>;
+            uint64_t blocks = (uint64_t)resident_blocks((const void*)kern, threads, 0, num_sms);
+            const uint64_t needed = ((uint64_t)nq + threads - 1) / threads;
+            if (blocks > needed) blocks = needed ? needed : 1;
+            kern<<<(unsigned)blocks, threads, 0, st>>>(a, slot_cell, counts_by_id);
+            return cudaGetLastError();
+        }
+    }
+    auto kern = k_rows_join<T, NT, NR, POL, FILL>;
     uint64_t blocks = (uint64_t)resident_blocks((const void*)kern, threads, 0, num_sms);
-    const uint64_t needed = ((uint64_t)a.n_points + threads - 1) / threads;
+    const uint64_t needed = ((uint64_t)nq + threads - 1) / threads;
     if (blocks > needed) blocks = needed ? needed : 1;
-    kern<<<(unsigned)blocks, threads, 0, st>>>(a, slot_cell, bitoff, bits, counts_by_id);
+    kern<<<(unsigned)blocks, threads, 0, st>>>(a, slot_cell, counts_by_id, qslots, nq, base);
     return cudaGetLastError();
 }
 
-template <typename T, int NR>
-static cudaError_t count_nr(const JoinArgs<T>& a, const uint32_t* slot_cell, const uint64_t* bitoff, uint32_t* bits,
-                            uint32_t* counts_by_id, int num_sms, cudaStream_t st) {
+template <typename T, int NR, bool FILL>
+static cudaError_t rows_nr(const JoinArgs<T>& a, const uint32_t* slot_cell, uint32_t* counts_by_id,
+                           const uint32_t* qslots, uint32_t nq, uint64_t base, int num_sms, cudaStream_t st) {
     switch (a.n) {
-        case 1: return launch_count_nt<T, 1, NR>(a, slot_cell, bitoff, bits, counts_by_id, num_sms, st);
-        case 2: return launch_count_nt<T, 2, NR>(a, slot_cell, bitoff, bits, counts_by_id, num_sms, st);
-        case 3: return launch_count_nt<T, 3, NR>(a, slot_cell, bitoff, bits, counts_by_id, num_sms, st);
-        case 4: return launch_count_nt<T, 4, NR>(a, slot_cell, bitoff, bits, counts_by_id, num_sms, st);
+        case 1: return launch_rows<T, 1, NR, FILL>(a, slot_cell, counts_by_id, qslots, nq, base, num_sms, st);
+        case 2: return launch_rows<T, 2, NR, FILL>(a, slot_cell, counts_by_id, qslots, nq, base, num_sms, st);
+        case 3: return launch_rows<T, 3, NR, FILL>(a, slot_cell, counts_by_id, qslots, nq, base, num_sms, st);
+        case 4: return launch_rows<T, 4, NR, FILL>(a, slot_cell, counts_by_id, qslots, nq, base, num_sms, st);
         default: return cudaErrorInvalidValue;
     }
 }
 
-template <typename T>
-bool tpq_supported(const JoinArgs<T>& a) {
-    return a.n >= 1 && a.n <= 4 && a.ilp == 0 && a.g.k <= 3 && a.plan != nullptr;
-}
-
-template <typename T>
-cudaError_t launch_rows_count(const JoinArgs<T>& a, const uint32_t* slot_cell, const uint64_t* bitoff, uint32_t* bits,
-                              uint32_t* counts_by_id, int num_sms, cudaStream_t st) {
-    if (!tpq_supported(a)) return cudaErrorInvalidValue;
-    if (a.g.k == 1) return count_nr<T, 1>(a, slot_cell, bitoff, bits, counts_by_id, num_sms, st);
-    if (a.g.k == 2) return count_nr<T, 3>(a, slot_cell, bitoff, bits, counts_by_id, num_sms, st);
-    return count_nr<T, 9>(a, slot_cell, bitoff, bits, counts_by_id, num_sms, st);
-}
-
-template <int NR>
-static cudaError_t fill_nr(const JoinArgs<float>& a, const uint32_t* slot_cell, const uint64_t* bitoff,
-                           const uint32_t* bits, const uint32_t* qslots, uint32_t nq, uint64_t base, int num_sms,
-                           cudaStream_t st) {
+template <typename T, bool FILL>
+static cudaError_t rows_any(const JoinArgs<T>& a, const uint32_t* slot_cell, uint32_t* counts_by_id,
+                            const uint32_t* qslots, uint32_t nq, uint64_t base, int num_sms, cudaStream_t st) {
+    if (a.n < 1 || a.n > 4 || a.ilp != 0 || a.g.k > 3 || !a.plan) return cudaErrorInvalidValue;
     if (nq == 0) return cudaSuccess;
-    auto kern = k_rows_fill<NR>;
-    const int threads = a.shape_threads ? (int)a.shape_threads : 256;
-    uint64_t blocks = (uint64_t)resident_blocks((const void*)kern, threads, 0, num_sms);
-    const uint64_t needed = ((uint64_t)nq + threads - 1) / threads;
-    if (blocks > needed) blocks = needed ? needed : 1;
-    kern<<<(unsigned)blocks, threads, 0, st>>>(a, slot_cell, bitoff, bits, qslots, nq, base);
-    return cudaGetLastError();
+    if (a.g.k == 1) return rows_nr<T, 1, FILL>(a, slot_cell, counts_by_id, qslots, nq, base, num_sms, st);
+    if (a.g.k == 2) return rows_nr<T, 3, FILL>(a, slot_cell, counts_by_id, qslots, nq, base, num_sms, st);
+    return rows_nr<T, 9, FILL>(a, slot_cell, counts_by_id, qslots, nq, base, num_sms, st);
 }
 
-// The fill pass reads no coordinates: the table, offsets, ids and plan are
-// independent of the coordinate type, so both precisions share one kernel
-// (JoinArgs<float> view of the same buffers).
 template <typename T>
-cudaError_t launch_rows_fill(const JoinArgs<T>& a, const uint32_t* slot_cell, const uint64_t* bitoff,
-                             const uint32_t* bits, const uint32_t* qslots, uint32_t nq, uint64_t base, int num_sms,
-                             cudaStream_t st) {
-    if (!tpq_supported(a)) return cudaErrorInvalidValue;
-    JoinArgs<float> f{};
-    f.ids = a.ids;
-    f.plan = a.plan;
-    f.work_counter = a.work_counter;
-    f.n_points = a.n_points;
-    f.fwd_cnt = a.fwd_cnt;
-    f.offsets = a.offsets;
-    f.table = a.table;
-    f.table_cap = a.table_cap;
-    f.err_flag = a.err_flag;
-    f.shape_threads = a.shape_threads;
-    if (a.g.k == 1) return fill_nr<1>(f, slot_cell, bitoff, bits, qslots, nq, base, num_sms, st);
-    if (a.g.k == 2) return fill_nr<3>(f, slot_cell, bitoff, bits, qslots, nq, base, num_sms, st);
-    return fill_nr<9>(f, slot_cell, bitoff, bits, qslots, nq, base, num_sms, st);
+cudaError_t launch_rows_count(const JoinArgs<T>& a, const uint32_t* slot_cell, uint32_t* counts_by_id, int num_sms,
+                              cudaStream_t st) {
+    return rows_any<T, false>(a, slot_cell, counts_by_id, nullptr, a.n_points, 0, num_sms, st);
 }
 
-template bool tpq_supported<float>(const JoinArgs<float>&);
-template bool tpq_supported<double>(const JoinArgs<double>&);
-template cudaError_t launch_rows_count<float>(const JoinArgs<float>&, const uint32_t*, const uint64_t*, uint32_t*,
-                                              uint32_t*, int, cudaStream_t);
-template cudaError_t launch_rows_count<double>(const JoinArgs<double>&, const uint32_t*, const uint64_t*, uint32_t*,
-                                               uint32_t*, int, cudaStream_t);
-template cudaError_t launch_rows_fill<float>(const JoinArgs<float>&, const uint32_t*, const uint64_t*,
-                                             const uint32_t*, const uint32_t*, uint32_t, uint64_t, int, cudaStream_t);
-template cudaError_t launch_rows_fill<double>(const JoinArgs<double>&, const uint32_t*, const uint64_t*,
-                                              const uint32_t*, const uint32_t*, uint32_t, uint64_t, int,
-                                              cudaStream_t);
+template <typename T>
+cudaError_t launch_rows_fill(const JoinArgs<T>& a, const uint32_t* slot_cell, const uint32_t* qslots, uint32_t nq,
+                             uint64_t base, int num_sms, cudaStream_t st) {
+    return rows_any<T, true>(a, slot_cell, nullptr, qslots, nq, base, num_sms, st);
+}
+
+template cudaError_t launch_rows_count<float>(const JoinArgs<float>&, const uint32_t*, uint32_t*, int, cudaStream_t);
+template cudaError_t launch_rows_count<double>(const JoinArgs<double>&, const uint32_t*, uint32_t*, int,
+                                               cudaStream_t);
+template cudaError_t launch_rows_fill<float>(const JoinArgs<float>&, const uint32_t*, const uint32_t*, uint32_t,
+                                             uint64_t, int, cudaStream_t);
+template cudaError_t launch_rows_fill<double>(const JoinArgs<double>&, const uint32_t*, const uint32_t*, uint32_t,
+                                              uint64_t, int, cudaStream_t);
 
 // ---------------------------------------------------------------- result batches
 // Batch b of the host-result pipeline holds the point ids [bound[b],
@@ -408,28 +441,6 @@ cudaError_t launch_max_u32(const uint32_t* in, uint64_t n, uint32_t* out, cudaSt
     uint64_t blocks = (n + 255) / 256;
     if (blocks > 1184) blocks = 1184;
     k_max_u32<<<(unsigned)(blocks ? blocks : 1), 256, 0, st>>>(in, n, out);
-    return cudaGetLastError();
-}
-
-// Slot -> cell map and the bit-mask words of each slot's query: every query
-// of cell c has the same candidates, ceil(sum of its plan rows / 32) words.
-__global__ void k_slot_cell(const uint32_t* __restrict__ cell_start, uint32_t M, const uint2* __restrict__ plan,
-                            uint32_t nrows, uint32_t* __restrict__ slot_cell, uint32_t* __restrict__ swords) {
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= M) return;
-    uint64_t tot = 0;
-    if (swords)
-        for (uint32_t r = 0; r < nrows; r++) tot += plan[(size_t)c * nrows + r].y;
-    const uint32_t w = (uint32_t)((tot + 31u) / 32u);
-    for (uint32_t s = cell_start[c]; s < cell_start[c + 1]; s++) {
-        slot_cell[s] = c;
-        if (swords) swords[s] = w;
-    }
-}
-
-cudaError_t launch_slot_cell(const uint32_t* cell_start, uint32_t M, const uint2* plan, uint32_t nrows,
-                             uint32_t* slot_cell, uint32_t* swords, cudaStream_t st) {
-    k_slot_cell<<<(M + 255) / 256, 256, 0, st>>>(cell_start, M, plan, nrows, slot_cell, swords);
     return cudaGetLastError();
 }
 

@@ -76,25 +76,18 @@ cudaError_t launch_join_emit(const JoinArgs<T>& a, const TileOut& o, const Heavy
                              int model, bool stamp, int num_sms, int* launches, cudaStream_t st);
 
 // ROWS path: dense low-dimensional grids (k <= 3, n <= 4), full neighbourhood.
-// slot_cell[s] = cell of slot s; with swords non-null also the bit-mask words
-// of slot s's query (ceil(candidates / 32); plan rows nrows per cell).
-cudaError_t launch_slot_cell(const uint32_t* cell_start, uint32_t M, const uint2* plan, uint32_t nrows,
-                             uint32_t* slot_cell, uint32_t* swords, cudaStream_t st);
+// slot_cell[s] = cell of slot s; a.plan holds 3^(k-1) rows a cell.
+// Count pass (a.work_counter zeroed): counts_by_id[ids[s]] = list length.
 template <typename T>
-bool tpq_supported(const JoinArgs<T>& a);
-// Count pass (a.work_counter zeroed): a.fwd_cnt[s] and counts_by_id[ids[s]]
-// receive the list lengths, bits[bitoff[s] ...] the query's hit mask.
-template <typename T>
-cudaError_t launch_rows_count(const JoinArgs<T>& a, const uint32_t* slot_cell, const uint64_t* bitoff, uint32_t* bits,
-                              uint32_t* counts_by_id, int num_sms, cudaStream_t st);
+cudaError_t launch_rows_count(const JoinArgs<T>& a, const uint32_t* slot_cell, uint32_t* counts_by_id, int num_sms,
+                              cudaStream_t st);
 // Fill pass (a.work_counter zeroed, a.offsets/table/table_cap/err_flag set):
-// replays the hit masks of the queries at slots qslots[0 .. nq) (slots
-// 0 .. nq-1 when qslots is null) into the point-id-ordered table; the list of
-// point id i lands at a.table[offsets[i] - base].
+// the lists of the queries at slots qslots[0 .. nq) (slots 0 .. nq-1 when
+// qslots is null) into the point-id-ordered table; the list of point id i lands
+// at a.table[offsets[i] - base].
 template <typename T>
-cudaError_t launch_rows_fill(const JoinArgs<T>& a, const uint32_t* slot_cell, const uint64_t* bitoff,
-                             const uint32_t* bits, const uint32_t* qslots, uint32_t nq, uint64_t base, int num_sms,
-                             cudaStream_t st);
+cudaError_t launch_rows_fill(const JoinArgs<T>& a, const uint32_t* slot_cell, const uint32_t* qslots, uint32_t nq,
+                             uint64_t base, int num_sms, cudaStream_t st);
 // Result batches by point-id range: bound[0..nb] (ids) and boff[0..nb] (their
 // table offsets), each batch's lists at most `step` + the longest list
 // entries; per-slot batch keys (with the slot index as value, for a stable
