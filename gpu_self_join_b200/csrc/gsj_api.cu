@@ -174,7 +174,7 @@ struct gsj_context {
     // device pool
     Buf in, pts, ids, keys, keys2, vals, cell_key, cell_start, dense, plan, slot_cell, htab, order,
         sizes, nchunks,
-        item_off, items, cursor, counts, offsets, table, temp, scan_temp, misc, var, perm, minarr,
+        item_off, items, cursor, counts, offsets, table, temp, scan_temp, misc, var, perm,
         minmax_part, pairs, srows, snorms, spartial, scentre, unc, table2, nbtab, ptemp, sortv, heavy, gstart;
     PinnedBuf stage[2];
     PinnedBuf hmisc;
@@ -339,10 +339,69 @@ int h2d_copy(gsj_context* c, void* dst, const void* src, size_t bytes) {
     return GSJ_OK;
 }
 
+// Scalars read back together: the copies go to the context's pinned block, one
+// wait covers them all, and only then are the destinations written (a pageable
+// destination would cost a staged copy and a wait each).
+constexpr size_t kPinnedScalars = 64u << 10;
+
+class Readback {
+public:
+    explicit Readback(gsj_context* c) : c_(c) {}
+    template <typename X>
+    int add(X* dst, const X* src, size_t count) {
+        const size_t bytes = count * sizeof(X), at = (used_ + 15u) & ~size_t(15);
+        if (n_ == kMax || at + bytes > kPinnedScalars) return fail(c_, GSJ_ERR_STATE, "readback block full");
+        GSJ_CUDA(c_, cudaMemcpyAsync(static_cast<char*>(c_->hmisc.p) + at, src, bytes, cudaMemcpyDeviceToHost, c_->st));
+        item_[n_++] = {dst, at, bytes};
+        used_ = at + bytes;
+        return GSJ_OK;
+    }
+    int wait() {
+        GSJ_CUDA(c_, cudaStreamSynchronize(c_->st));
+        for (int i = 0; i < n_; i++)
+            std::memcpy(item_[i].dst, static_cast<const char*>(c_->hmisc.p) + item_[i].at, item_[i].bytes);
+        n_ = 0;
+        used_ = 0;
+        return GSJ_OK;
+    }
+
+private:
+    static constexpr int kMax = 8;
+    struct Item {
+        void* dst;
+        size_t at, bytes;
+    } item_[kMax];
+    gsj_context* c_;
+    int n_ = 0;
+    size_t used_ = 0;
+};
+
 template <typename X>
 int d2h_small(gsj_context* c, X* dst, const X* src, size_t count) {
+    if (count * sizeof(X) <= kPinnedScalars) {
+        Readback rb(c);
+        GSJ_TRY(rb.add(dst, src, count));
+        return rb.wait();
+    }
     GSJ_CUDA(c, cudaMemcpyAsync(dst, src, count * sizeof(X), cudaMemcpyDeviceToHost, c->st));
     GSJ_CUDA(c, cudaStreamSynchronize(c->st));
+    return GSJ_OK;
+}
+
+// Device times of the last join's stages (their events have completed).
+int stage_times(gsj_context* c, bool estimate) {
+    gsj_stats& S = c->stats;
+    float ms = 0;
+    GSJ_CUDA(c, cudaEventElapsedTime(&ms, c->tev[0], c->tev[1]));
+    S.dev_ms_index = ms;
+    GSJ_CUDA(c, cudaEventElapsedTime(&ms, c->tev[2], c->tev[3]));
+    S.dev_ms_count = ms;
+    GSJ_CUDA(c, cudaEventElapsedTime(&ms, c->tev[4], c->tev[5]));
+    S.dev_ms_fill = ms;
+    if (estimate) {
+        GSJ_CUDA(c, cudaEventElapsedTime(&ms, c->tev[6], c->tev[7]));
+        S.dev_ms_estimate = ms;
+    }
     return GSJ_OK;
 }
 
@@ -382,26 +441,30 @@ int validate(gsj_context* c, const gsj_config& cfg, uint64_t N) {
 // ------------------------------------------------------------------ lists ascending
 // Sorts every list of the table ascending (ids below N): a warp per list up
 // to 256 entries, a CTA bitonic network up to 4096, CTA radix passes with a
-// scratch copy of the table above.
-int sort_table_lists(gsj_context* c, uint32_t* table, const uint64_t* offsets, uint64_t N, uint64_t R) {
-    gsj_stats& S = c->stats;
-    cudaStream_t st = c->st;
+// scratch copy of the table above.  The numbers of long lists are queued on `rb`
+// (nlong); the caller waits and calls sort_very_long.
+int sort_table_lists(gsj_context* c, uint32_t* table, const uint64_t* offsets, uint64_t N, Readback& rb,
+                     uint32_t (&nlong)[2]) {
     int nl = 0;
     void* temp = nullptr;
     GSJ_TRY(dev_get(c, c->ptemp, place_temp_bytes(N), (unsigned char**)&temp));
-    uint32_t* d_nlong = reinterpret_cast<uint32_t*>(c->misc.p) + 4 * kMaxK + 24;
-    uint32_t nlong = 0, nvery = 0;
-    GSJ_CUDA(c, sort_short_lists<uint64_t>(table, offsets, (uint32_t)N, 1u, temp, d_nlong, &nlong, &nvery,
-                                           c->num_sms, &nl, st));
-    if (nlong) {
-        uint32_t* scratch = nullptr;
-        if (nvery) GSJ_TRY(dev_get(c, c->table2, R, &scratch));
-        uint32_t id_bits = 1;
-        while (id_bits < 32 && ((N - 1) >> id_bits)) id_bits++;
-        GSJ_CUDA(c, sort_long_lists<uint64_t>(table, scratch, offsets, temp, nlong, nvery, id_bits, c->num_sms, &nl,
-                                              st));
-    }
-    S.kernel_launches += (uint64_t)nl;
+    uint32_t* d_nlong = reinterpret_cast<uint32_t*>(c->misc.p) + 4 * kMaxK + 24;  // zeroed with the other scalars
+    GSJ_CUDA(c, sort_lists<uint64_t>(table, offsets, (uint32_t)N, temp, d_nlong, c->num_sms, &nl, c->st));
+    c->stats.kernel_launches += (uint64_t)nl;
+    return rb.add(nlong, d_nlong, 2);
+}
+
+int sort_very_long(gsj_context* c, uint32_t* table, const uint64_t* offsets, uint64_t N, uint64_t R,
+                   const uint32_t (&nlong)[2]) {
+    if (nlong[1] == 0) return GSJ_OK;
+    int nl = 0;
+    uint32_t* scratch = nullptr;
+    GSJ_TRY(dev_get(c, c->table2, R, &scratch));
+    uint32_t id_bits = 1;
+    while (id_bits < 32 && ((N - 1) >> id_bits)) id_bits++;
+    GSJ_CUDA(c, sort_very_long_lists<uint64_t>(table, scratch, offsets, c->ptemp.p, nlong[0], nlong[1], id_bits,
+                                               c->num_sms, &nl, c->st));
+    c->stats.kernel_launches += (uint64_t)nl;
     return GSJ_OK;
 }
 
@@ -420,33 +483,29 @@ int pairs_to_csr(gsj_context* c, unsigned long long* pairs, uint64_t nkeys, uint
     GSJ_TRY(dev_get(c, c->cursor, N, &cursor));
     void* temp = nullptr;
     GSJ_TRY(dev_get(c, c->ptemp, place_temp_bytes(N), (unsigned char**)&temp));
-    uint32_t* d_err = reinterpret_cast<uint32_t*>(c->misc.p) + 4 * kMaxK + 20;
-    GSJ_CUDA(c, cudaMemsetAsync(d_err, 0, sizeof(uint32_t), st));
+    uint32_t* d_err = reinterpret_cast<uint32_t*>(c->misc.p) + 4 * kMaxK + 20;  // zeroed with the other scalars
     int nl = 0;
     GSJ_CUDA(c, place_pairs(pairs, nkeys, shift, (uint32_t)N, counts, offsets, table, R, cursor, d_err, temp,
                             c->num_sms, &nl, st));
     S.kernel_launches += (uint64_t)nl;
-    GSJ_TRY(sort_table_lists(c, table, offsets, N, R));
-    GSJ_CUDA(c, cudaEventRecord(c->tev[5], st));
     uint64_t total = 0;
-    GSJ_TRY(d2h_small(c, &total, offsets + N, 1));
-    if (total != R) return fail(c, GSJ_ERR_STATE, "list lengths disagree with the pair count");
-    uint32_t err = 0;
-    GSJ_TRY(d2h_small(c, &err, d_err, 1));
-    if (err) return fail(c, GSJ_ERR_STATE, "pair placement left a list (internal error)");
+    uint32_t err = 0, nlong[2] = {0, 0};
     unsigned long long ncand = 0;
-    GSJ_TRY(d2h_small(c, &ncand, cand, 1));
-    {
-        float ms = 0;
-        GSJ_CUDA(c, cudaEventElapsedTime(&ms, c->tev[0], c->tev[1]));
-        S.dev_ms_index = ms;
-        GSJ_CUDA(c, cudaEventElapsedTime(&ms, c->tev[2], c->tev[3]));
-        S.dev_ms_count = ms;
-        GSJ_CUDA(c, cudaEventElapsedTime(&ms, c->tev[4], c->tev[5]));
-        S.dev_ms_fill = ms;
-        GSJ_CUDA(c, cudaEventElapsedTime(&ms, c->tev[6], c->tev[7]));
-        S.dev_ms_estimate = ms;
+    Readback rb(c);
+    GSJ_TRY(sort_table_lists(c, table, offsets, N, rb, nlong));
+    GSJ_CUDA(c, cudaEventRecord(c->tev[5], st));
+    GSJ_TRY(rb.add(&total, offsets + N, 1));
+    GSJ_TRY(rb.add(&err, d_err, 1));
+    GSJ_TRY(rb.add(&ncand, cand, 1));
+    GSJ_TRY(rb.wait());
+    if (total != R) return fail(c, GSJ_ERR_STATE, "list lengths disagree with the pair count");
+    if (err) return fail(c, GSJ_ERR_STATE, "pair placement left a list (internal error)");
+    if (nlong[1]) {
+        GSJ_TRY(sort_very_long(c, table, offsets, N, R, nlong));
+        GSJ_CUDA(c, cudaEventRecord(c->tev[5], st));
+        GSJ_CUDA(c, cudaStreamSynchronize(st));
     }
+    GSJ_TRY(stage_times(c, true));
     S.candidates = ncand;
     S.total_pairs = R;
     c->R = R;
@@ -540,8 +599,10 @@ int emit_join(gsj_context* c, JoinArgs<T>& a, uint64_t N, bool stamp, int model,
         o.pairs = pairs;
         o.cap = cap;
         GSJ_CUDA(c, launch_join_emit<T>(a, o, heavy, ni, model, stamp, c->num_sms, &nl, st));
-        GSJ_TRY(d2h_small(c, &used, cursor, 1));
-        GSJ_TRY(d2h_small(c, &R, o.rechecks, 1));
+        unsigned long long got[2] = {0, 0};  // entries reserved, keys
+        GSJ_TRY(d2h_small(c, got, cursor, 2));
+        used = got[0];
+        R = got[1];
         if (used <= cap) break;
         if (attempt == 2) return fail(c, GSJ_ERR_STATE, "warp join: pair buffer short at its proven bound");
         c->stats.reruns++;
@@ -623,9 +684,11 @@ int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int mo
         S.kernel_launches += 1;
         GSJ_CUDA(c, launch(nsample));
         unsigned long long sampled[2] = {0, 0};  // entries, and the screen's undecided pairs
-        GSJ_TRY(d2h_small(c, sampled, cursor, 2));
         uint32_t err = 0;
-        GSJ_TRY(d2h_small(c, &err, a.err_flag, 1));
+        Readback rb(c);
+        GSJ_TRY(rb.add(sampled, cursor, 2));
+        GSJ_TRY(rb.add(&err, a.err_flag, 1));
+        GSJ_TRY(rb.wait());
         if (err) return fail(c, GSJ_ERR_CUDA, "tile join: tensor-core wait timed out");
         est_entries = nsample ? (double)sampled[0] * (double)ni / (double)nsample : 0.0;
         est = screen && nsample ? (double)sampled[1] * (double)ni / (double)nsample : est_entries;
@@ -650,11 +713,14 @@ int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int mo
         S.kernel_launches += 1;
         GSJ_CUDA(c, launch(ni));
         // entries written (pairs), or reserved (records)
-        GSJ_TRY(d2h_small(c, &used, cursor, 1));
-        U = used;
-        if (screen) GSJ_TRY(d2h_small(c, &U, o.rechecks, 1));
+        unsigned long long got[2] = {0, 0};
         uint32_t err = 0;
-        GSJ_TRY(d2h_small(c, &err, a.err_flag, 1));
+        Readback rb(c);
+        GSJ_TRY(rb.add(got, cursor, 2));
+        GSJ_TRY(rb.add(&err, a.err_flag, 1));
+        GSJ_TRY(rb.wait());
+        used = got[0];
+        U = screen ? got[1] : used;
         if (err) return fail(c, GSJ_ERR_CUDA, "tile join: tensor-core wait timed out");
         if (used <= cap) {
             nlist = used;
@@ -859,21 +925,14 @@ int sort_join(gsj_context* c, JoinArgs<T>& a, uint64_t N, int model, uint32_t* c
     S.kernel_launches += 1;
     GSJ_CUDA(c, launch_sort_join<T>(a, slot_cell, counts, model, true, c->num_sms, st));
     GSJ_CUDA(c, cudaEventRecord(c->tev[5], st));
-    GSJ_CUDA(c, cudaStreamSynchronize(st));
     uint32_t err = 0;
-    GSJ_TRY(d2h_small(c, &err, a.err_flag, 1));
-    if (err) return fail(c, GSJ_ERR_STATE, "SORT fill pass disagreed with its count pass (internal error)");
     unsigned long long ncand = 0;
-    GSJ_TRY(d2h_small(c, &ncand, a.cand_cnt, 1));
-    {
-        float ms = 0;
-        GSJ_CUDA(c, cudaEventElapsedTime(&ms, c->tev[0], c->tev[1]));
-        S.dev_ms_index = ms;
-        GSJ_CUDA(c, cudaEventElapsedTime(&ms, c->tev[2], c->tev[3]));
-        S.dev_ms_count = ms;
-        GSJ_CUDA(c, cudaEventElapsedTime(&ms, c->tev[4], c->tev[5]));
-        S.dev_ms_fill = ms;
-    }
+    Readback rb(c);
+    GSJ_TRY(rb.add(&err, a.err_flag, 1));
+    GSJ_TRY(rb.add(&ncand, a.cand_cnt, 1));
+    GSJ_TRY(rb.wait());
+    if (err) return fail(c, GSJ_ERR_STATE, "SORT fill pass disagreed with its count pass (internal error)");
+    GSJ_TRY(stage_times(c, false));
     S.candidates = ncand;
     S.total_pairs = R;
     S.join_path = GSJ_PATH_SORT;
@@ -948,15 +1007,18 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
         std::sort(dv.begin(), dv.end(), compareByDimVariance<T>);
         for (uint32_t j = 0; j < n; j++) perm[j] = dv[j].dim;
     }
-    uint32_t* d_perm = nullptr;
-    GSJ_TRY(dev_get(c, c->perm, n, &d_perm));
-    GSJ_CUDA(c, cudaMemcpyAsync(d_perm, perm.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+    uint32_t* d_perm = nullptr;  // null: the columns keep their order
+    if (cfg.reorder) {
+        GSJ_TRY(dev_get(c, c->perm, n, &d_perm));
+        GSJ_CUDA(c, cudaMemcpyAsync(d_perm, perm.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+    }
 
     // ---- grid extents (main.cu:891-948)
     const uint32_t nparts = (uint32_t)std::min<uint64_t>((N + 255) / 256, (uint64_t)c->num_sms * 4);
     T *d_part = nullptr, *d_mm = nullptr;
     GSJ_TRY(dev_get(c, c->minmax_part, (size_t)nparts * 2 * k, &d_part));
     GSJ_TRY(dev_get(c, c->misc, kMiscWords, &d_mm));
+    GSJ_CUDA(c, cudaMemsetAsync(d_mm, 0, kMiscWords * sizeof(uint32_t), st));  // every counter and flag of the join
     S.kernel_launches += 2;
     GSJ_CUDA(c, launch_minmax<T>(d_in, N, n, k, d_perm, d_part, nparts, d_mm, st));
     std::vector<T> mm(2 * k);
@@ -989,33 +1051,8 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
         totalCells = (j == 0) ? g.ncells[0] : totalCells * g.ncells[j];
     }
     S.total_cells = totalCells;
-    // neighbour offsets in the kernels' order (digit j of o is dim j's step + 1):
-    // linear-id delta, moved-down / moved-up dims, highest moved dim
-    uint4* d_nbtab = nullptr;
-    {
-        uint32_t noff = 1;
-        for (uint32_t j = 0; j < k; j++) noff *= 3u;
-        std::vector<uint4> tab(noff);
-        for (uint32_t o = 0; o < noff; o++) {
-            long long delta = 0;
-            uint32_t down = 0, up = 0, hd = 0xffu, t = o;
-            for (uint32_t j = 0; j < k; j++) {
-                const int dl = (int)(t % 3u) - 1;
-                t /= 3u;
-                delta += (long long)dl * (long long)g.mult[j];
-                if (dl < 0) down |= 1u << j;
-                if (dl > 0) up |= 1u << j;
-                if (dl != 0) hd = j;
-            }
-            const uint64_t d = (uint64_t)delta;
-            tab[o] = make_uint4((uint32_t)d, (uint32_t)(d >> 32), down | (up << 16), hd);
-        }
-        GSJ_TRY(dev_get(c, c->nbtab, noff, &d_nbtab));
-        GSJ_CUDA(c, cudaMemcpyAsync(d_nbtab, tab.data(), noff * sizeof(uint4), cudaMemcpyHostToDevice, st));
-    }
-    T* d_min = nullptr;
-    GSJ_TRY(dev_get(c, c->minarr, k, &d_min));
-    GSJ_CUDA(c, cudaMemcpyAsync(d_min, minArr.data(), k * sizeof(T), cudaMemcpyHostToDevice, st));
+    MinVals<T> minv{};
+    for (uint32_t j = 0; j < k; j++) minv.v[j] = minArr[j];
 
     // ---- cell keys + radix sort (subsystem (a)): points ordered by cell, ties
     // by point id (a stable sort of keys generated in point-id order).  (A
@@ -1038,15 +1075,14 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     // the number of non-empty cells (word 0) and the out-of-range flag of the
     // cell keys (word 1)
     uint32_t* d_nruns = reinterpret_cast<uint32_t*>(d_mm + 2 * kMaxK);
-    GSJ_CUDA(c, cudaMemsetAsync(d_nruns, 0, 2 * sizeof(uint32_t), st));
     S.kernel_launches += 1;
     if (key32) {
         uint32_t* k32 = reinterpret_cast<uint32_t*>(keys);
         uint32_t* k32b = reinterpret_cast<uint32_t*>(keys2);
-        GSJ_CUDA(c, (launch_cell_keys<T, uint32_t>(d_in, N, n, d_perm, g, d_min, eps, k32, vals, d_nruns + 1, st)));
+        GSJ_CUDA(c, (launch_cell_keys<T, uint32_t>(d_in, N, n, d_perm, g, minv, eps, k32, vals, d_nruns + 1, st)));
         GSJ_CUDA(c, radix_sort<uint32_t>(k32, k32b, vals, ids, N, 0, bits, temp, &in_alt, &nl, st));
     } else {
-        GSJ_CUDA(c, (launch_cell_keys<T, uint64_t>(d_in, N, n, d_perm, g, d_min, eps, keys, vals, d_nruns + 1, st)));
+        GSJ_CUDA(c, (launch_cell_keys<T, uint64_t>(d_in, N, n, d_perm, g, minv, eps, keys, vals, d_nruns + 1, st)));
         GSJ_CUDA(c, radix_sort<uint64_t>(keys, keys2, vals, ids, N, 0, bits, temp, &in_alt, &nl, st));
     }
     S.kernel_launches += (uint64_t)nl;
@@ -1142,8 +1178,16 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
         GSJ_CUDA(c, launch_row_table(cell_key, M, g.ncells[0], htab, hmask, st));
     }
     // The ROWS path (dense low-dimensional grids) is driven by a per-cell plan of
-    // neighbour-row slot ranges.
+    // neighbour-row slot ranges, the others by the table of neighbour offsets.
     uint2* plan = nullptr;
+    uint4* d_nbtab = nullptr;
+    if (!tpq) {
+        uint32_t noff = 1;
+        for (uint32_t j = 0; j < k; j++) noff *= 3u;
+        GSJ_TRY(dev_get(c, c->nbtab, noff, &d_nbtab));
+        S.kernel_launches += 1;
+        GSJ_CUDA(c, launch_neighbour_table(g, noff, d_nbtab, st));
+    }
     if (tpq) {
         const uint32_t nrows = k == 1 ? 1u : (k == 2 ? 3u : 9u);
         GSJ_TRY(dev_get(c, c->plan, (size_t)M * nrows, &plan));
@@ -1255,14 +1299,12 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
         GSJ_CUDA(c, launch_make_items(order, nchunks, item_off, M, items, st));
     }
     GSJ_CUDA(c, cudaEventRecord(c->tev[1], st));
-    GSJ_CUDA(c, cudaStreamSynchronize(st));
     const double t_join = now_ms();
     S.ms_index = t_join - t_index;
 
     // ---- join arguments (every path)
     uint32_t* ctr = reinterpret_cast<uint32_t*>(d_mm + 2 * kMaxK) + 2;  // work counter
     unsigned long long* cand = reinterpret_cast<unsigned long long*>(reinterpret_cast<uint32_t*>(d_mm + 2 * kMaxK) + 4);
-    GSJ_CUDA(c, cudaMemsetAsync(ctr, 0, 4 * sizeof(uint32_t), st));
     JoinArgs<T> a{};
     a.pts = pts;
     a.ids = ids;
@@ -1336,9 +1378,11 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     S.kernel_launches += (uint64_t)scan_launches(N);
     GSJ_CUDA(c, scan_u32_u64(counts, offsets, N, stemp, st));
     uint64_t R = 0;
-    GSJ_TRY(d2h_small(c, &R, offsets + N, 1));
     unsigned long long ncand = 0;
-    GSJ_TRY(d2h_small(c, &ncand, cand, 1));
+    Readback rb(c);
+    GSJ_TRY(rb.add(&R, offsets + N, 1));
+    GSJ_TRY(rb.add(&ncand, cand, 1));
+    GSJ_TRY(rb.wait());
     S.candidates = ncand;
 
     // ---- fill pass: into the device table, or in batches to the host
@@ -1353,15 +1397,7 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
         gsj_config pcfg = cfg;
         if (shape.streams) pcfg.streams = shape.streams;
         GSJ_TRY(rows_to_host<T>(c, a, pcfg, N, R, slot_cell, counts, offsets, *ho));
-        {
-            float ms = 0;
-            GSJ_CUDA(c, cudaEventElapsedTime(&ms, c->tev[0], c->tev[1]));
-            S.dev_ms_index = ms;
-            GSJ_CUDA(c, cudaEventElapsedTime(&ms, c->tev[2], c->tev[3]));
-            S.dev_ms_count = ms;
-            GSJ_CUDA(c, cudaEventElapsedTime(&ms, c->tev[4], c->tev[5]));
-            S.dev_ms_fill = ms;
-        }
+        GSJ_TRY(stage_times(c, false));
         uint32_t errflag = 0;
         GSJ_TRY(d2h_small(c, &errflag, ctr + 1, 1));
         if (errflag) return fail(c, GSJ_ERR_STATE, "fill pass: a list would leave its segment (internal error)");
@@ -1384,24 +1420,18 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     S.kernel_launches += 1;
     GSJ_CUDA(c, launch_rows_fill<T>(a, slot_cell, nullptr, (uint32_t)N, 0, c->num_sms, st));
     GSJ_CUDA(c, cudaEventRecord(c->tev[5], st));
-    GSJ_CUDA(c, cudaStreamSynchronize(st));
-    {
-        float ms = 0;
-        GSJ_CUDA(c, cudaEventElapsedTime(&ms, c->tev[0], c->tev[1]));
-        S.dev_ms_index = ms;
-        GSJ_CUDA(c, cudaEventElapsedTime(&ms, c->tev[2], c->tev[3]));
-        S.dev_ms_count = ms;
-        GSJ_CUDA(c, cudaEventElapsedTime(&ms, c->tev[4], c->tev[5]));
-        S.dev_ms_fill = ms;
-    }
-    uint32_t errflag = 0;
-    GSJ_TRY(d2h_small(c, &errflag, ctr + 1, 1));
+    uint32_t errflag = 0, nlong[2] = {0, 0};
+    // every list ascending
+    const bool sorted = (cfg.flags & GSJ_FLAG_SORT_LISTS) && R > 1;
+    if (sorted) GSJ_TRY(sort_table_lists(c, table, offsets, N, rb, nlong));
+    GSJ_TRY(rb.add(&errflag, ctr + 1, 1));
+    GSJ_TRY(rb.wait());
     if (errflag) return fail(c, GSJ_ERR_STATE, "fill pass: a list would leave the table (internal error)");
-    if ((cfg.flags & GSJ_FLAG_SORT_LISTS) && R > 1) {
-        // every list ascending
-        GSJ_TRY(sort_table_lists(c, table, offsets, N, R));
+    if (nlong[1]) {
+        GSJ_TRY(sort_very_long(c, table, offsets, N, R, nlong));
         GSJ_CUDA(c, cudaStreamSynchronize(st));
     }
+    GSJ_TRY(stage_times(c, false));
     S.ms_join = now_ms() - t_join;
     S.total_pairs = R;
     S.join_path = GSJ_PATH_ROWS;
@@ -1479,6 +1509,7 @@ int gsj_create(gsj_context** out, int device) {
     GSJ_CUDA(c, cudaEventCreateWithFlags(&c->ev[0], cudaEventDisableTiming));
     GSJ_CUDA(c, cudaEventCreateWithFlags(&c->ev[1], cudaEventDisableTiming));
     for (auto& e : c->tev) GSJ_CUDA(c, cudaEventCreate(&e));
+    GSJ_TRY(pinned_get(c, c->hmisc, kPinnedScalars));
     *out = c;
     return GSJ_OK;
 }
@@ -1493,7 +1524,7 @@ int gsj_destroy(gsj_context* c) {
                    &c->order,    &c->sizes,
                    &c->nchunks,  &c->item_off, &c->items, &c->cursor,  &c->counts,    &c->offsets,
                    &c->table, &c->temp,   &c->scan_temp, &c->misc,    &c->var,       &c->perm,
-                   &c->minarr,   &c->minmax_part, &c->pairs, &c->srows, &c->snorms,
+                   &c->minmax_part, &c->pairs, &c->srows, &c->snorms,
                    &c->spartial, &c->scentre, &c->unc, &c->table2, &c->nbtab, &c->ptemp, &c->sortv, &c->heavy, &c->gstart};
     for (Buf* b : bufs)
         if (b->p) cudaFree(b->p);

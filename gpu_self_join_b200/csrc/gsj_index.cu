@@ -74,7 +74,7 @@ __global__ void k_minmax_partial(const T* __restrict__ in, uint64_t N, uint32_t 
 #pragma unroll
     for (int j = 0; j < kMaxK; j++)
         if (j < (int)k) {
-            col[j] = perm[j];
+            col[j] = perm ? perm[j] : (uint32_t)j;
             mn[j] = mx[j] = in[col[j]];
         }
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -168,14 +168,14 @@ __global__ void k_minmax_final(const T* __restrict__ part, uint32_t nparts, uint
 template <typename T>
 __device__ __forceinline__ uint64_t cell_key_of(const T* __restrict__ in, uint64_t i, uint32_t n,
                                                 const uint32_t* __restrict__ perm, const GridGeom& g,
-                                                const T* __restrict__ minArr, T eps, uint32_t* bad) {
+                                                const MinVals<T>& minArr, T eps, uint32_t* bad) {
     uint64_t key = 0;
     bool out = false;
 #pragma unroll
     for (int j = 0; j < kMaxK; j++)
         if (j < (int)g.k) {
-            const T x = in[i * n + perm[j]];
-            const uint32_t c = FP<T>::to_uint_rz(FP<T>::div(FP<T>::sub(x, minArr[j]), eps));
+            const T x = in[i * n + (perm ? perm[j] : (uint32_t)j)];
+            const uint32_t c = FP<T>::to_uint_rz(FP<T>::div(FP<T>::sub(x, minArr.v[j]), eps));
             out |= c >= g.ncells[j];
             key += (uint64_t)c * g.mult[j];
         }
@@ -188,7 +188,7 @@ __device__ __forceinline__ uint64_t cell_key_of(const T* __restrict__ in, uint64
 
 template <typename T, typename K>
 __global__ void k_cell_keys(const T* __restrict__ in, uint64_t N, uint32_t n, const uint32_t* __restrict__ perm,
-                            GridGeom g, const T* __restrict__ minArr, T eps,
+                            GridGeom g, MinVals<T> minArr, T eps,
                             K* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t* __restrict__ bad) {
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (i >= N) return;
@@ -205,7 +205,7 @@ __global__ void k_gather_points(const T* __restrict__ in, uint64_t N, uint32_t n
     if (e >= N * npad) return;
     const uint64_t s = e / npad;
     const uint32_t j = (uint32_t)(e - s * npad);
-    pts[e] = j < n ? in[(uint64_t)ids[s] * n + perm[j]] : T(0);
+    pts[e] = j < n ? in[(uint64_t)ids[s] * n + (perm ? perm[j] : j)] : T(0);
 }
 
 // The same for rows of npad = NP <= 4 entries: a thread per point, one id
@@ -218,7 +218,7 @@ __global__ void k_gather_rows(const T* __restrict__ in, uint64_t N, uint32_t n, 
     const T* src = in + (uint64_t)ids[s] * n;
     T v[NP];
 #pragma unroll
-    for (int j = 0; j < NP; j++) v[j] = (uint32_t)j < n ? src[perm[j]] : T(0);
+    for (int j = 0; j < NP; j++) v[j] = (uint32_t)j < n ? src[perm ? perm[j] : (uint32_t)j] : T(0);
     T* dst = pts + s * NP;
     if constexpr (std::is_same<T, float>::value && NP == 2) {
         *reinterpret_cast<float2*>(dst) = make_float2(v[0], v[1]);
@@ -416,6 +416,29 @@ __global__ void k_make_items(const uint32_t* __restrict__ order, const uint32_t*
     for (uint32_t q = 0; q < nc; q++) items[off + q] = make_uint2(c, q);
 }
 
+// Neighbour offsets in the kernels' order (digit j of o is dim j's step + 1):
+// linear-id delta (x lo, y hi), moved-down dims | moved-up dims << 16, highest
+// moved dim (0xff: none).
+__global__ void k_neighbour_table(GridGeom g, uint32_t noff, uint4* __restrict__ tab) {
+    const uint32_t o = blockIdx.x * blockDim.x + threadIdx.x;
+    if (o >= noff) return;
+    uint64_t delta = 0;
+    uint32_t down = 0, up = 0, hd = 0xffu, t = o;
+    for (uint32_t j = 0; j < g.k; j++) {
+        const uint32_t d = t % 3u;
+        t /= 3u;
+        if (d == 0u) {
+            delta -= g.mult[j];
+            down |= 1u << j;
+        } else if (d == 2u) {
+            delta += g.mult[j];
+            up |= 1u << j;
+        }
+        if (d != 1u) hd = j;
+    }
+    tab[o] = make_uint4((uint32_t)delta, (uint32_t)(delta >> 32), down | (up << 16), hd);
+}
+
 __global__ void k_iota(uint32_t* __restrict__ out, uint32_t M) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < M) out[i] = i;
@@ -446,7 +469,8 @@ cudaError_t launch_minmax(const T* in, uint64_t N, uint32_t n, uint32_t k, const
 
 template <typename T, typename K>
 cudaError_t launch_cell_keys(const T* in, uint64_t N, uint32_t n, const uint32_t* perm, const GridGeom& g,
-                             const T* minArr, T eps, K* keys, uint32_t* vals, uint32_t* bad, cudaStream_t st) {
+                             const MinVals<T>& minArr, T eps, K* keys, uint32_t* vals, uint32_t* bad,
+                             cudaStream_t st) {
     k_cell_keys<T, K><<<blocks_for(N, 256), 256, 0, st>>>(in, N, n, perm, g, minArr, eps, keys, vals, bad);
     return cudaGetLastError();
 }
@@ -506,6 +530,11 @@ cudaError_t launch_make_items(const uint32_t* order, const uint32_t* nchunks, co
     return cudaGetLastError();
 }
 
+cudaError_t launch_neighbour_table(const GridGeom& g, uint32_t noff, uint4* tab, cudaStream_t st) {
+    k_neighbour_table<<<blocks_for(noff, 256), 256, 0, st>>>(g, noff, tab);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_iota(uint32_t* out, uint32_t M, cudaStream_t st) {
     k_iota<<<blocks_for(M, 256), 256, 0, st>>>(out, M);
     return cudaGetLastError();
@@ -517,10 +546,10 @@ cudaError_t launch_iota(uint32_t* out, uint32_t M, cudaStream_t st) {
     template cudaError_t launch_minmax<T>(const T*, uint64_t, uint32_t, uint32_t, const uint32_t*, T*,     \
                                           uint32_t, T*, cudaStream_t);                                     \
     template cudaError_t launch_cell_keys<T, uint64_t>(const T*, uint64_t, uint32_t, const uint32_t*,      \
-                                                       const GridGeom&, const T*, T, uint64_t*, uint32_t*, \
+                                                       const GridGeom&, const MinVals<T>&, T, uint64_t*, uint32_t*, \
                                                        uint32_t*, cudaStream_t);                           \
     template cudaError_t launch_cell_keys<T, uint32_t>(const T*, uint64_t, uint32_t, const uint32_t*,      \
-                                                       const GridGeom&, const T*, T, uint32_t*, uint32_t*, \
+                                                       const GridGeom&, const MinVals<T>&, T, uint32_t*, uint32_t*, \
                                                        uint32_t*, cudaStream_t);                           \
     template cudaError_t launch_gather_points<T>(const T*, uint64_t, uint32_t, uint32_t, const uint32_t*,  \
                                                  const uint32_t*, T*, cudaStream_t);

@@ -22,12 +22,19 @@ cudaError_t launch_variance(const T* in, uint64_t N, uint32_t n, T denom, T* var
 template <typename T>
 cudaError_t launch_minmax(const T* in, uint64_t N, uint32_t n, uint32_t k, const uint32_t* perm, T* part,
                           uint32_t nparts, T* out, cudaStream_t st);
+// Grid origin per indexed dim, passed to kernels by value.
+template <typename T>
+struct MinVals {
+    T v[kMaxK];
+};
+// `perm` (column of each dim) may be null where columns keep their order.
 // Cell key per point (K = uint32_t when the grid has fewer than 2^32 cells)
 // and the point ids 0..N-1.  *bad (zeroed by the caller) is raised when a
 // point's cell index reaches its dimension's extent.
 template <typename T, typename K>
 cudaError_t launch_cell_keys(const T* in, uint64_t N, uint32_t n, const uint32_t* perm, const GridGeom& g,
-                             const T* minArr, T eps, K* keys, uint32_t* vals, uint32_t* bad, cudaStream_t st);
+                             const MinVals<T>& minArr, T eps, K* keys, uint32_t* vals, uint32_t* bad,
+                             cudaStream_t st);
 template <typename T>
 cudaError_t launch_gather_points(const T* in, uint64_t N, uint32_t n, uint32_t npad, const uint32_t* perm,
                                  const uint32_t* ids, T* pts, cudaStream_t st);
@@ -51,6 +58,8 @@ cudaError_t launch_item_counts(const uint32_t* cell_start, const uint32_t* order
                                uint32_t* nchunks, uint32_t* sizes, cudaStream_t st);
 cudaError_t launch_make_items(const uint32_t* order, const uint32_t* nchunks, const uint32_t* item_off,
                               uint32_t M, uint2* items, cudaStream_t st);
+// The 3^k neighbour offsets (JoinArgs::nbtab).
+cudaError_t launch_neighbour_table(const GridGeom& g, uint32_t noff, uint4* tab, cudaStream_t st);
 cudaError_t launch_iota(uint32_t* out, uint32_t M, cudaStream_t st);
 
 // The warp-per-item join: appends packed pair keys into `o` (its rechecks

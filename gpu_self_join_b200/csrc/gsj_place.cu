@@ -223,8 +223,9 @@ template <typename OffT>
 __global__ void __launch_bounds__(kCtaSortThreads) k_list_sort_cta(uint32_t* __restrict__ table,
                                                                    const OffT* __restrict__ offsets,
                                                                    const uint32_t* __restrict__ long_lists,
-                                                                   uint32_t nlong) {
+                                                                   const uint32_t* __restrict__ d_nlong) {
     __shared__ uint32_t sb[2][kCtaSortMax];
+    const uint32_t nlong = *d_nlong;
     int buf = 0;
     for (uint32_t li = blockIdx.x; li < nlong; li += gridDim.x) {
         const uint32_t l = long_lists[li];
@@ -321,55 +322,37 @@ size_t place_temp_bytes(uint64_t nlists) {
 }
 
 template <typename OffT>
-cudaError_t sort_short_lists(uint32_t* table, const OffT* offsets, uint32_t nlists, uint32_t min_len, void* temp,
-                             uint32_t* d_nlong, uint32_t* h_nlong, uint32_t* h_nvery, int num_sms, int* launches,
-                             cudaStream_t st) {
-    *h_nlong = *h_nvery = 0;
+cudaError_t sort_lists(uint32_t* table, const OffT* offsets, uint32_t nlists, void* temp, uint32_t* d_nlong,
+                       int num_sms, int* launches, cudaStream_t st) {
     if (nlists == 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(d_nlong, 0, 2 * sizeof(uint32_t), st);
-    if (e != cudaSuccess) return e;
+    uint32_t* ll = static_cast<uint32_t*>(temp);
     const unsigned g = grid_for((uint64_t)nlists, 256, (uint64_t)num_sms * 64);
-    k_list_sort_short<OffT><<<g, 256, 0, st>>>(table, offsets, nlists, min_len, static_cast<uint32_t*>(temp), d_nlong);
-    if (launches) *launches += 1;
-    uint32_t h[2];
-    e = cudaMemcpyAsync(h, d_nlong, sizeof(h), cudaMemcpyDeviceToHost, st);
-    if (e != cudaSuccess) return e;
-    e = cudaStreamSynchronize(st);
-    *h_nlong = h[0];
-    *h_nvery = h[1];
-    return e;
-}
-
-template <typename OffT>
-cudaError_t sort_long_lists(uint32_t* table, uint32_t* scratch, const OffT* offsets, const void* temp,
-                            uint32_t nlong, uint32_t nvery, uint32_t id_bits, int num_sms, int* launches,
-                            cudaStream_t st) {
-    if (nlong == 0) return cudaSuccess;
-    const uint32_t* ll = static_cast<const uint32_t*>(temp);
-    if (nlong > nvery) {
-        k_list_sort_cta<OffT><<<grid_for(nlong - nvery, 1, (uint64_t)num_sms * 6), kCtaSortThreads, 0, st>>>(
-            table, offsets, ll, nlong);
-        if (launches) *launches += 1;
-    }
-    if (nvery) {
-        if (!scratch) return cudaErrorInvalidValue;
-        int passes = (int)((id_bits + 7u) / 8u);
-        passes += passes & 1;  // even: the sorted list ends in the table
-        k_list_sort_block<OffT><<<grid_for(nvery, 1, (uint64_t)num_sms * 8), kBlockSortThreads, 0, st>>>(
-            table, scratch, offsets, ll, nlong, passes);
-        if (launches) *launches += 1;
-    }
+    k_list_sort_short<OffT><<<g, 256, 0, st>>>(table, offsets, nlists, 1u, ll, d_nlong);
+    // the longer lists' number stays on the device: a CTA that finds none ends at once
+    k_list_sort_cta<OffT><<<grid_for(nlists, 1, (uint64_t)num_sms * 6), kCtaSortThreads, 0, st>>>(table, offsets, ll,
+                                                                                                 d_nlong);
+    if (launches) *launches += 2;
     return cudaGetLastError();
 }
 
-template cudaError_t sort_short_lists<uint64_t>(uint32_t*, const uint64_t*, uint32_t, uint32_t, void*, uint32_t*,
-                                                uint32_t*, uint32_t*, int, int*, cudaStream_t);
-template cudaError_t sort_short_lists<uint32_t>(uint32_t*, const uint32_t*, uint32_t, uint32_t, void*, uint32_t*,
-                                                uint32_t*, uint32_t*, int, int*, cudaStream_t);
-template cudaError_t sort_long_lists<uint64_t>(uint32_t*, uint32_t*, const uint64_t*, const void*, uint32_t,
-                                               uint32_t, uint32_t, int, int*, cudaStream_t);
-template cudaError_t sort_long_lists<uint32_t>(uint32_t*, uint32_t*, const uint32_t*, const void*, uint32_t,
-                                               uint32_t, uint32_t, int, int*, cudaStream_t);
+template <typename OffT>
+cudaError_t sort_very_long_lists(uint32_t* table, uint32_t* scratch, const OffT* offsets, const void* temp,
+                                 uint32_t nlong, uint32_t nvery, uint32_t id_bits, int num_sms, int* launches,
+                                 cudaStream_t st) {
+    if (nvery == 0) return cudaSuccess;
+    if (!scratch) return cudaErrorInvalidValue;
+    int passes = (int)((id_bits + 7u) / 8u);
+    passes += passes & 1;  // even: the sorted list ends in the table
+    k_list_sort_block<OffT><<<grid_for(nvery, 1, (uint64_t)num_sms * 8), kBlockSortThreads, 0, st>>>(
+        table, scratch, offsets, static_cast<const uint32_t*>(temp), nlong, passes);
+    if (launches) *launches += 1;
+    return cudaGetLastError();
+}
+
+template cudaError_t sort_lists<uint64_t>(uint32_t*, const uint64_t*, uint32_t, void*, uint32_t*, int, int*,
+                                          cudaStream_t);
+template cudaError_t sort_very_long_lists<uint64_t>(uint32_t*, uint32_t*, const uint64_t*, const void*, uint32_t,
+                                                    uint32_t, uint32_t, int, int*, cudaStream_t);
 
 cudaError_t place_pairs(const unsigned long long* keys, uint64_t nkeys, uint32_t shift, uint32_t nlists,
                         uint32_t* counts, uint64_t* offsets, uint32_t* table, uint64_t cap, uint32_t* cursor,

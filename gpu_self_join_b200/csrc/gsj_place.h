@@ -20,22 +20,20 @@ cudaError_t place_pairs(const unsigned long long* keys, uint64_t nkeys, uint32_t
                         uint32_t* counts, uint64_t* offsets, uint32_t* table, uint64_t cap, uint32_t* cursor,
                         uint32_t* err, void* temp, int num_sms, int* launches, cudaStream_t st);
 
-// Sorts every list of min_len+1 .. 256 entries ascending (a warp per list;
-// shorter lists are left as they are) and gathers the indices of the longer
-// lists into temp: *h_nlong receives their number, *h_nvery the number above
-// 4096 entries (synchronises the stream).  List l is table[offsets[l] ..
-// offsets[l+1]) (OffT = uint64_t or uint32_t).  d_nlong: two device words.
+// Sorts every list of up to 4096 entries ascending (a warp per list up to 256
+// entries, a CTA above) and gathers the indices of the lists above 256 into
+// temp.  List l is table[offsets[l] .. offsets[l+1]).  d_nlong: two device
+// words, zeroed by the caller, which receive the number of lists above 256 and
+// above 4096 entries.
 template <typename OffT>
-cudaError_t sort_short_lists(uint32_t* table, const OffT* offsets, uint32_t nlists, uint32_t min_len, void* temp,
-                             uint32_t* d_nlong, uint32_t* h_nlong, uint32_t* h_nvery, int num_sms, int* launches,
-                             cudaStream_t st);
-// Sorts the lists gathered by sort_short_lists (ids below 2^id_bits): a CTA
-// bitonic network up to 4096 entries; above that LSD radix passes using the
-// same ranges of `scratch` (as large as the table; needed only when nvery > 0)
-// as a second buffer.
+cudaError_t sort_lists(uint32_t* table, const OffT* offsets, uint32_t nlists, void* temp, uint32_t* d_nlong,
+                       int num_sms, int* launches, cudaStream_t st);
+// Sorts the gathered lists above 4096 entries (ids below 2^id_bits): LSD radix
+// passes using the same ranges of `scratch` (as large as the table) as a second
+// buffer.
 template <typename OffT>
-cudaError_t sort_long_lists(uint32_t* table, uint32_t* scratch, const OffT* offsets, const void* temp,
-                            uint32_t nlong, uint32_t nvery, uint32_t id_bits, int num_sms, int* launches,
-                            cudaStream_t st);
+cudaError_t sort_very_long_lists(uint32_t* table, uint32_t* scratch, const OffT* offsets, const void* temp,
+                                 uint32_t nlong, uint32_t nvery, uint32_t id_bits, int num_sms, int* launches,
+                                 cudaStream_t st);
 
 }  // namespace gsj

@@ -328,11 +328,7 @@ cudaError_t radix_sort(K* keys, K* keys_alt, uint32_t* vals, uint32_t* vals_alt,
     void* stemp = static_cast<unsigned char*>(temp) + (2 * hist_bytes + sizeof(uint32_t) + 255) / 256 * 256;
     const size_t smem = sizeof(K) * kSortTile + (vals ? sizeof(uint32_t) * kSortTile : 0);
     cudaError_t e;
-    for (const void* f : {(const void*)k_radix_scatter<K, true, 256>, (const void*)k_radix_scatter<K, false, 256>,
-                          (const void*)k_radix_scatter<K, true, 512>, (const void*)k_radix_scatter<K, false, 512>}) {
-        e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    // 24 KiB at most: no opt-in needed
     // digits of 8 bits, or of 9 where that saves a pass (25 key bits: 9 + 8 + 8)
     const int B = end_bit - begin_bit;
     const int p8 = (B + 7) / 8, p9 = (B + 8) / 9;
