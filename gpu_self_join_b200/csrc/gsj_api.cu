@@ -175,7 +175,7 @@ struct gsj_context {
     Buf in, pts, ids, keys, keys2, vals, cell_key, cell_start, dense, plan, slot_cell, htab, order,
         sizes, nchunks,
         item_off, items, cursor, counts, offsets, table, temp, scan_temp, misc, var, perm,
-        minmax_part, pairs, srows, snorms, spartial, scentre, unc, table2, nbtab, ptemp, sortv, heavy, gstart;
+        minmax_part, pairs, srows, snorms, spartial, scentre, unc, table2, nbtab, ptemp, sortv, heavy;
     PinnedBuf stage[2];
     PinnedBuf hmisc;
     // host-result pipeline: copy streams, per-segment events, pinned staging
@@ -516,19 +516,25 @@ int pairs_to_csr(gsj_context* c, unsigned long long* pairs, uint64_t nkeys, uint
 // ------------------------------------------------------------------ learned estimate
 // Pairs the exact pass of the last indexed join will produce, predicted by the
 // context's model from the per-cell features (requires model_trained).
+constexpr uint32_t kEstimateCells = 1u << 19;
+
 int learned_estimate(gsj_context* c, double* est) {
     cudaStream_t st = c->st;
-    const uint32_t M = c->last.M;
+    // every stride-th cell, weighted by points: half a million cells give the total
+    // to a few percent, against a buffer margin of a quarter
+    const uint32_t M = c->last.M, stride = std::max<uint32_t>(1u, M / kEstimateCells), rows = (M + stride - 1) / stride;
     float* X = nullptr;
-    GSJ_TRY(dev_get(c, c->mx, (size_t)M * kModelFeatures, &X));
+    GSJ_TRY(dev_get(c, c->mx, (size_t)rows * kModelFeatures, &X));
     double* d_est = nullptr;
     GSJ_TRY(dev_get(c, c->mtmp, 4, &d_est));
-    GSJ_CUDA(c, cudaMemsetAsync(d_est, 0, sizeof(double), st));
+    GSJ_CUDA(c, cudaMemsetAsync(d_est, 0, 2 * sizeof(double), st));
     c->stats.kernel_launches += 2;
-    GSJ_CUDA(c, model_features(c->last.lookup, M, c->last.log2_eps, c->last.n, X, st));
-    GSJ_CUDA(c, model_predict(X, M, static_cast<const float*>(c->mw.p), nullptr, c->last.lookup.cell_start,
+    GSJ_CUDA(c, model_features(c->last.lookup, rows, stride, c->last.log2_eps, c->last.n, X, st));
+    GSJ_CUDA(c, model_predict(X, rows, static_cast<const float*>(c->mw.p), nullptr, c->last.lookup.cell_start, stride,
                               (float)c->last.lookup.n_points, d_est, st));
-    GSJ_TRY(d2h_small(c, est, d_est, 1));
+    double got[2] = {0.0, 0.0};
+    GSJ_TRY(d2h_small(c, got, d_est, 2));
+    *est = got[1] > 0.0 ? got[0] * ((double)c->last.lookup.n_points / got[1]) : 0.0;
     return GSJ_OK;
 }
 
@@ -570,7 +576,7 @@ int emit_join(gsj_context* c, JoinArgs<T>& a, uint64_t N, bool stamp, int model,
     };
     GSJ_CUDA(c, cudaEventRecord(c->tev[2], st));
     GSJ_CUDA(c, cudaEventRecord(c->tev[6], st));
-    double est = 0.0;
+    double est = 0.0, est_cand = 0.0;
     if (learned) {
         GSJ_TRY(learned_estimate(c, &est));
     } else if (!exact_size) {
@@ -579,11 +585,17 @@ int emit_join(gsj_context* c, JoinArgs<T>& a, uint64_t N, bool stamp, int model,
         GSJ_TRY(reset());
         o.emit = false;
         o.stride = kSampleStride;
+        heavy.unit = 32u;  // few items: short units
         GSJ_CUDA(c, launch_join_emit<T>(a, o, heavy, nsample, model, stamp, c->num_sms, &nl, st));
-        unsigned long long sampled = 0;
-        GSJ_TRY(d2h_small(c, &sampled, o.rechecks, 1));
+        unsigned long long sampled = 0, sampled_cand = 0;
+        Readback rb(c);
+        GSJ_TRY(rb.add(&sampled, o.rechecks, 1));
+        GSJ_TRY(rb.add(&sampled_cand, cand, 1));
+        GSJ_TRY(rb.wait());
         est = nsample ? (double)sampled * (double)ni / (double)nsample : 0.0;
+        est_cand = nsample ? (double)sampled_cand * (double)ni / (double)nsample : 0.0;
     }
+    heavy.unit = join_unit_steps(est_cand, c->num_sms);
     GSJ_CUDA(c, cudaEventRecord(c->tev[7], st));
     S.estimate = (uint64_t)est;
     const uint64_t estimate = exact_size ? 0u : (uint64_t)(est * 1.25) + N + (1u << 16) + slack;
@@ -1236,33 +1248,12 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     // time, and the order in which queries run changes no result.
     uint32_t num_items = 0;
     uint2* items = nullptr;
-    // Query groups of the register form of the warp join: cells of few points are
-    // joined with their neighbours along dim 0, about 6 points a group, so that
-    // they share the enumeration of the neighbour rows and the candidate loads
-    // (up to 4 cells: 3 + 3 more cells of candidates are tested than needed).
-    uint32_t gspan = 1;
-    const uint32_t* gstart = cell_start;
-    if constexpr (std::is_same<T, float>::value) {
-        if (path_id == GSJ_PATH_WARP && join_reg_supported(n, npad, model, cfg.ilp))
-            gspan = (uint32_t)std::min<uint64_t>(4u, (6ull * M + N - 1u) / N);
-        if (gspan < 1u) gspan = 1u;
-    }
     if (tpq) {
         S.work_items = ((uint64_t)N + 31u) / 32u;
     } else {
         uint32_t *order = nullptr, *nchunks = nullptr, *item_off = nullptr;
         GSJ_TRY(dev_get(c, c->nchunks, M + 1, &nchunks));
         GSJ_TRY(dev_get(c, c->item_off, M + 1, &item_off));
-        if (gspan > 1u) {
-            uint32_t* gs = nullptr;
-            GSJ_TRY(dev_get(c, c->gstart, M + 1, &gs));
-            GSJ_TRY(dev_get(c, c->temp, scan_u32_u64_temp_bytes(M), (unsigned char**)&temp));
-            S.kernel_launches += 2 + (uint64_t)scan_launches(M);
-            GSJ_CUDA(c, launch_group_flags(cell_key, M, g.ncells[0], gspan, nchunks, st));
-            GSJ_CUDA(c, scan_u32_u32(nchunks, item_off, M, temp, st));
-            GSJ_CUDA(c, launch_group_starts_of(nchunks, item_off, cell_start, M, (uint32_t)N, gs, st));
-            gstart = gs;
-        }
         if (cfg.query_reorder) {
             uint32_t *sizes = nullptr, *sizes2 = nullptr, *iota = nullptr;
             GSJ_TRY(dev_get(c, c->sizes, 2 * (size_t)M, &sizes));
@@ -1272,7 +1263,7 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
             // stable descending sort by cell size (ties keep ascending cell order):
             // an ascending sort of the complemented sizes
             S.kernel_launches += 2;
-            GSJ_CUDA(c, launch_item_counts(gstart, nullptr, M, qchunk, nchunks, sizes, st));
+            GSJ_CUDA(c, launch_item_counts(cell_start, nullptr, M, qchunk, nchunks, sizes, st));
             GSJ_CUDA(c, launch_iota(iota, M, st));
             GSJ_TRY(dev_get(c, c->temp, radix_sort_temp_bytes(M), (unsigned char**)&temp));
             bool alt = false;
@@ -1284,10 +1275,10 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
                 GSJ_CUDA(c, cudaMemcpyAsync(order, iota, (size_t)M * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
             }
             S.kernel_launches += 1;
-            GSJ_CUDA(c, launch_item_counts(gstart, order, M, qchunk, nchunks, nullptr, st));
+            GSJ_CUDA(c, launch_item_counts(cell_start, order, M, qchunk, nchunks, nullptr, st));
         } else {
             S.kernel_launches += 1;
-            GSJ_CUDA(c, launch_item_counts(gstart, nullptr, M, qchunk, nchunks, nullptr, st));
+            GSJ_CUDA(c, launch_item_counts(cell_start, nullptr, M, qchunk, nchunks, nullptr, st));
         }
         GSJ_TRY(dev_get(c, c->temp, scan_u32_u64_temp_bytes(M), (unsigned char**)&temp));
         S.kernel_launches += (uint64_t)scan_launches(M);
@@ -1314,8 +1305,6 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     a.plan = plan;
     a.htab = htab;
     a.hmask = hmask;
-    a.gstart = gstart;
-    a.gspan = gspan;
     a.items = items;
     a.num_items = num_items;
     a.nbtab = d_nbtab;
@@ -1525,7 +1514,7 @@ int gsj_destroy(gsj_context* c) {
                    &c->nchunks,  &c->item_off, &c->items, &c->cursor,  &c->counts,    &c->offsets,
                    &c->table, &c->temp,   &c->scan_temp, &c->misc,    &c->var,       &c->perm,
                    &c->minmax_part, &c->pairs, &c->srows, &c->snorms,
-                   &c->spartial, &c->scentre, &c->unc, &c->table2, &c->nbtab, &c->ptemp, &c->sortv, &c->heavy, &c->gstart};
+                   &c->spartial, &c->scentre, &c->unc, &c->table2, &c->nbtab, &c->ptemp, &c->sortv, &c->heavy};
     for (Buf* b : bufs)
         if (b->p) cudaFree(b->p);
     for (auto* pb : {&c->stage[0], &c->stage[1], &c->hmisc})
@@ -1802,7 +1791,7 @@ static int model_dataset(gsj_context* c, uint32_t* M_out) {
     float *X = nullptr, *Y = nullptr;
     GSJ_TRY(dev_get(c, c->mx, (size_t)M * kModelFeatures, &X));
     GSJ_TRY(dev_get(c, c->my, M, &Y));
-    GSJ_CUDA(c, model_features(c->last.lookup, M, c->last.log2_eps, c->last.n, X, c->st));
+    GSJ_CUDA(c, model_features(c->last.lookup, M, 1u, c->last.log2_eps, c->last.n, X, c->st));
     GSJ_CUDA(c, model_targets(c->last.lookup.cell_start, c->last.lookup.ids, static_cast<const uint32_t*>(c->counts.p),
                               M, Y, c->st));
     *M_out = M;
@@ -1896,7 +1885,7 @@ int gsj_model_predict(gsj_context* c, const float* features, uint32_t n, float* 
     GSJ_TRY(model_ensure(c));
     float *X = nullptr, *Y = nullptr;
     GSJ_TRY(model_upload(c, features, nullptr, n, &X, &Y));
-    GSJ_CUDA(c, model_predict(X, n, static_cast<const float*>(c->mw.p), Y, nullptr, 0.f, nullptr, c->st));
+    GSJ_CUDA(c, model_predict(X, n, static_cast<const float*>(c->mw.p), Y, nullptr, 1u, 0.f, nullptr, c->st));
     return d2h_small(c, out, Y, n);
 }
 

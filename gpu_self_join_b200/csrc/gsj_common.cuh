@@ -36,10 +36,7 @@ struct JoinArgs {
     const uint4* htab;            // [hcap] hash table of the grid rows that hold a cell {linear id of the row's
                                   // cell 0 (lo, hi; kEmptyKey = empty), first cell, cells}, or null
     uint64_t hmask;               // hcap - 1
-    const uint32_t* gstart;       // first slot of each query group (items' x; [group + 1] is its end): the cells,
-                                  // or runs of neighbouring cells of a grid row (gspan > 1)
-    uint32_t gspan;               // cells of a query group along dim 0 at most
-    const uint2* items;           // [num_items] (group, chunk)
+    const uint2* items;           // [num_items] (cell, chunk)
     const uint4* nbtab;           // [3^k] neighbour offsets: linear-id delta (x lo, y hi), z = moved-down dims
                                   // | moved-up dims << 16, w = highest moved dim (0xff: none)
     uint32_t num_items;
@@ -120,93 +117,112 @@ __device__ __forceinline__ void row_entry(const JoinArgs<T>& a, uint64_t base, u
     n = e.w;
 }
 
-// Slot range [start, start + cnt) of the cells xlo..xhi of the grid row whose
-// cell 0 has linear id `base`.  These cells are consecutive in cell order (dim
-// 0 is fastest), so the range is contiguous whichever of them are non-empty.
-// Dense grids read the slot-prefix table, the others the row's entry, its
-// cells' ids (a row of up to four cells at once, longer ones by bisection) and
-// their slots.  W: cand += points of every cell x times byte x - x0 of `weight`.
-template <typename T, bool W>
-__device__ __forceinline__ void row_slots(const JoinArgs<T>& a, uint64_t base, uint32_t xlo, uint32_t xhi,
-                                          uint32_t& start, uint32_t& cnt, uint32_t x0, uint64_t weight,
-                                          unsigned long long& cand) {
-    uint32_t lo = 0, hi = 0;  // the cells' indices (hashed grids)
+// Slot range [start, start + cnt) of the cells xlo..xhi (at most three) of the
+// grid row whose cell 0 has linear id `base`.  These cells are consecutive in
+// cell order (dim 0 is fastest), so the range is contiguous whichever of them
+// are non-empty.
+//
+// row_probe issues the first loads of a row, so that a thread can have the next
+// row's in flight: on dense grids the slot-prefix table's entries, which are all
+// it takes, else the row's table entry.  row_slots finishes: a hashed row needs
+// one more step, its cells' ids and slots together (rows of more than four
+// cells are bisected first).
+struct RowProbe {
+    bool ok;
+    uint64_t base;
+    uint32_t xlo, xhi;
+    uint4 e;  // the row's entry, or (dense) first slot of cell xlo and of cell xhi + 1
+};
+
+template <typename T>
+__device__ __forceinline__ void row_probe(const JoinArgs<T>& a, bool ok, uint64_t base, uint32_t xlo, uint32_t xhi,
+                                          RowProbe& p) {
+    p.ok = ok;
+    p.base = base;
+    p.xlo = xlo;
+    p.xhi = xhi;
+    if (!ok) return;
     if (a.ds) {
-        start = a.ds[base + xlo];
-        cnt = a.ds[base + xhi + 1u] - start;
+        p.e.x = a.ds[base + xlo];
+        p.e.y = a.ds[base + xhi + 1u];
     } else {
-        uint32_t first = 0, n = 0;
-        row_entry(a, base, a.htab[mix64(base) & a.hmask], first, n);
-        if (n > 4u) {
-            // the row's first cell at or past xlo
-            uint32_t l = first, h = first + n;
-            while (l < h) {
-                const uint32_t m = l + (h - l) / 2u;
-                if (a.cell_key[m] < base + xlo) l = m + 1u;
-                else h = m;
-            }
-            n -= l - first;
-            first = l;
-        }
-        uint64_t key[4];
-#pragma unroll
-        for (uint32_t i = 0; i < 4u; i++) key[i] = i < n ? a.cell_key[first + i] : kEmptyKey;
-        lo = hi = first;
-#pragma unroll
-        for (uint32_t i = 0; i < 4u; i++) {
-            lo += key[i] < base + xlo ? 1u : 0u;
-            hi += key[i] <= base + xhi ? 1u : 0u;
-        }
-        if (hi - first == 4u)
-            while (hi < first + n && a.cell_key[hi] <= base + xhi) hi++;
-        start = cnt = 0u;
-        if (hi > lo) {
-            start = a.cell_start[lo];
-            cnt = a.cell_start[hi] - start;
-        }
+        p.e = a.htab[mix64(base) & a.hmask];
     }
-    if (W && cnt) {
-        uint32_t prev = start, x = xlo;
-        const uint32_t steps = a.ds ? xhi - xlo + 1u : hi - lo;
-        for (uint32_t i = 0; i < steps; i++) {
-            uint32_t next;
-            if (a.ds) {
-                x = xlo + i;
-                next = a.ds[base + x + 1u];
-            } else {
-                x = (uint32_t)(a.cell_key[lo + i] - base);
-                next = a.cell_start[lo + i + 1u];
-            }
-            cand += (unsigned long long)(next - prev) * (uint32_t)((weight >> (8u * (x - x0))) & 0xffu);
-            prev = next;
-        }
+}
+
+template <typename T>
+__device__ __forceinline__ void row_slots(const JoinArgs<T>& a, const RowProbe& p, uint32_t& start, uint32_t& cnt) {
+    start = cnt = 0u;
+    if (!p.ok) return;
+    if (a.ds) {
+        start = p.e.x;
+        cnt = p.e.y - start;
+        return;
     }
+    const uint64_t klo = p.base + p.xlo, khi = p.base + p.xhi;
+    uint32_t first = 0, n = 0;
+    row_entry(a, p.base, p.e, first, n);
+    if (n > 4u) {
+        // the row's first cell at or past xlo; at most three cells follow up to xhi
+        uint32_t l = first, h = first + n;
+        while (l < h) {
+            const uint32_t m = l + (h - l) / 2u;
+            if (a.cell_key[m] < klo) l = m + 1u;
+            else h = m;
+        }
+        n -= l - first;
+        first = l;
+    }
+    if (n == 0u) return;
+    uint64_t key[4];
+    uint32_t slot[5];
+#pragma unroll
+    for (uint32_t i = 0; i < 4u; i++) key[i] = i < n ? a.cell_key[first + i] : kEmptyKey;
+#pragma unroll
+    for (uint32_t i = 0; i < 5u; i++) slot[i] = a.cell_start[first + min(i, n)];
+    uint32_t end = 0;
+    start = 0xffffffffu;
+#pragma unroll
+    for (uint32_t i = 0; i < 4u; i++)
+        if (key[i] >= klo && key[i] <= khi) {
+            start = min(start, slot[i]);
+            end = slot[i + 1u];
+        }
+    if (end) cnt = end - start;
 }
 
 // Slot range of the cell with linear id `lin`.
 template <typename T>
 __device__ __forceinline__ bool lookup_range(const JoinArgs<T>& a, uint64_t lin, uint32_t& start, uint32_t& cnt) {
     const uint32_t x = a.ds ? 0u : (uint32_t)(lin % a.g.ncells[0]);
-    unsigned long long cand = 0;
-    row_slots<T, false>(a, lin - x, x, x, start, cnt, 0u, 0u, cand);
+    RowProbe p;
+    row_probe(a, true, lin - x, x, x, p);
+    row_slots(a, p, start, cnt);
     return cnt != 0u;
 }
 
-// Slot range of a neighbour row of one cell: the cells x-1..x+1 of the grid row
-// that offset r (digit j of r is dim j+1's step + 1) leads to.  With unicomp
-// the own row (r's centre) adds its dim-0 neighbours only when x is odd, every
-// other row comes whole or not at all (the highest moved dim is the same for
-// its three cells).
+// A neighbour row of the cell with linear id own_lin and dim-0 coordinate x: the
+// cells x-1..x+1 of the grid row that offset r (digit j of r is dim j+1's step +
+// 1) leads to.  With unicomp the own row (r's centre) adds its dim-0 neighbours
+// only when x is odd, every other row comes whole or not at all (the highest
+// moved dim is the same for its three cells).
+template <typename T, bool STAMP>
+__device__ __forceinline__ void neighbour_row(const JoinArgs<T>& a, bool valid, uint32_t r, uint64_t own_lin,
+                                              uint32_t x, uint32_t lowmask, uint32_t highmask, uint32_t oddmask,
+                                              RowProbe& p) {
+    uint64_t lin = 0;
+    const bool ok = valid && nb_offset<T, STAMP>(a, 3u * r + 1u, own_lin, lowmask, highmask, oddmask, lin);
+    const bool side = !STAMP || lin != own_lin || (oddmask & 1u);
+    row_probe(a, ok, lin - x, x - (side && !(lowmask & 1u) ? 1u : 0u), x + (side && !(highmask & 1u) ? 1u : 0u), p);
+}
+
 template <typename T, bool STAMP>
 __device__ __forceinline__ bool row_range(const JoinArgs<T>& a, bool valid, uint32_t r, uint64_t own_lin, uint32_t x,
                                           uint32_t lowmask, uint32_t highmask, uint32_t oddmask, uint32_t& start,
                                           uint32_t& cnt) {
-    uint64_t lin;
-    if (!valid || !nb_offset<T, STAMP>(a, 3u * r + 1u, own_lin, lowmask, highmask, oddmask, lin)) return false;
-    const bool side = !STAMP || lin != own_lin || (oddmask & 1u);
-    unsigned long long cand = 0;
-    row_slots<T, false>(a, lin - x, x - (side && !(lowmask & 1u) ? 1u : 0u), x + (side && !(highmask & 1u) ? 1u : 0u),
-                        start, cnt, 0u, 0u, cand);
+    RowProbe p;
+    neighbour_row<T, STAMP>(a, valid, r, own_lin, x, lowmask, highmask, oddmask, p);
+    row_slots(a, p, start, cnt);
     return cnt != 0u;
 }
 

@@ -340,27 +340,6 @@ __global__ void k_row_insert(const uint64_t* __restrict__ cell_key, uint32_t M, 
     }
 }
 
-// Query groups: runs of cells of one grid row within the same `span` cells of
-// dim 0 (aligned).  flags[c] = 1 where a group begins.
-__global__ void k_group_flags(const uint64_t* __restrict__ cell_key, uint32_t M, uint32_t n0, uint32_t span,
-                              uint32_t* __restrict__ flags) {
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= M) return;
-    const uint64_t key = cell_key[c];
-    const uint64_t first = key - (uint32_t)(key % n0) % span;  // the group's smallest possible id
-    flags[c] = (c == 0u || cell_key[c - 1u] < first) ? 1u : 0u;
-}
-
-// gstart[g] = first slot of group g, N from the last group's end on (gstart has M + 1 entries).
-__global__ void k_group_starts_of(const uint32_t* __restrict__ flags, const uint32_t* __restrict__ pos,
-                                  const uint32_t* __restrict__ cell_start, uint32_t M, uint32_t N,
-                                  uint32_t* __restrict__ gstart) {
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c > M) return;
-    if (c < M && flags[c]) gstart[pos[c]] = cell_start[c];
-    if (c >= pos[M]) gstart[c] = N;
-}
-
 // Cell plan of dense low-dimensional grids (k <= 3): for every non-empty
 // cell and each of its 3^(k-1) neighbour rows, the slot range of the row's
 // cells x-1..x+1, clipped to the grid (kernel.cu:180-188 clamp the same way).
@@ -497,18 +476,6 @@ cudaError_t launch_dense_slots(const uint64_t* cell_key, const uint32_t* cell_st
 cudaError_t launch_row_table(const uint64_t* cell_key, uint32_t M, uint32_t n0, uint4* htab, uint64_t hmask,
                              cudaStream_t st) {
     k_row_insert<<<blocks_for(M, 256), 256, 0, st>>>(cell_key, M, n0, htab, hmask);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_group_flags(const uint64_t* cell_key, uint32_t M, uint32_t n0, uint32_t span, uint32_t* flags,
-                               cudaStream_t st) {
-    k_group_flags<<<blocks_for(M, 256), 256, 0, st>>>(cell_key, M, n0, span, flags);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_group_starts_of(const uint32_t* flags, const uint32_t* pos, const uint32_t* cell_start, uint32_t M,
-                                   uint32_t N, uint32_t* gstart, cudaStream_t st) {
-    k_group_starts_of<<<blocks_for((uint64_t)M + 1u, 256), 256, 0, st>>>(flags, pos, cell_start, M, N, gstart);
     return cudaGetLastError();
 }
 

@@ -5,10 +5,10 @@
 // thread per query point, repeats the neighbour-cell search (2 binary searches
 // per cell) for every query, and appends every hit with a global atomicAdd.
 // Here one warp owns a work item: up to 32 consecutive query slots of one
-// non-empty cell, or of a few neighbouring cells of a grid row.  The warp
-//   1. enumerates the item's 3^(k-1) neighbour rows once, lanes in parallel (the
-//      cells of a row next to the item's are one contiguous slot range,
-//      row_slots), and compacts the non-empty ones (ballot) into a per-warp list in shared memory -
+// non-empty cell.  The warp
+//   1. enumerates the cell's 3^(k-1) neighbour rows once, lanes in parallel (a
+//      row's up to three cells are one contiguous slot range, row_slots), and
+//      compacts the non-empty ones (ballot) into a per-warp list in shared memory -
 //      with STAMP only the unicomp half-space of stamploops.h;
 //   2. stages the queries in shared memory;
 //   3. walks the concatenated candidate slots 32 at a time, one candidate per
@@ -26,6 +26,7 @@
 // registers, hits through a per-warp queue, heavy items cut into slices), k_join
 // for the rest (double, longer rows, ILP chains that a register form would have
 // to reorder).
+#include <algorithm>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -124,86 +125,37 @@ __device__ __forceinline__ uint32_t cand_slot(const uint32_t* nb_start, const ui
     return f < total ? nb_start[my] + (f - pf) : 0u;
 }
 
-// The queries of an item: slots [q0, q0 + qn) of one grid row, in the cells
-// xa..xb of it.
-struct ItemCells {
-    uint64_t base;             // linear id of the row's cell 0
-    uint32_t xa, xb;
-    uint32_t low, high, odd;   // edge and parity masks of the own coordinates (bit 0: cell xa's)
-};
-
-template <typename T>
-__device__ __forceinline__ ItemCells item_cells(const JoinArgs<T>& a, uint32_t q0, uint32_t qn) {
-    // cell coordinates with the formula the keys were built with (main.cu:744, kernel.cu:184)
+// The neighbour rows of `cell` (first slot cs; kernel.cu:180-303; stamploops.h
+// for STAMP) as slot ranges in nb_start and the exclusive prefix of their sizes
+// in nb_pref (nb_pref[rows] = total).  Returns the number of rows; the whole
+// warp calls.
+template <typename T, bool STAMP>
+__device__ __forceinline__ uint32_t enumerate_rows(const JoinArgs<T>& a, uint32_t cell, uint32_t cs, uint32_t nrow,
+                                                   uint32_t* nb_start, uint32_t* nb_pref, int lane, unsigned lt,
+                                                   uint32_t& total) {
+    const unsigned FULL = 0xffffffffu;
+    // own cell coordinates, from the first query of the cell with the formula the
+    // keys were built with (main.cu:744, kernel.cu:184)
     uint32_t own[kMaxK];
-    ItemCells c;
-    c.base = 0;
 #pragma unroll
-    for (int j = 0; j < kMaxK; j++) {
-        own[j] = (j < (int)a.g.k) ? FP<T>::to_uint_rz(FP<T>::div(FP<T>::sub(a.pts[(size_t)q0 * a.npad + j], a.minv[j]),
+    for (int j = 0; j < kMaxK; j++)
+        own[j] = (j < (int)a.g.k) ? FP<T>::to_uint_rz(FP<T>::div(FP<T>::sub(a.pts[(size_t)cs * a.npad + j], a.minv[j]),
                                                                  a.eps))
                                   : 0u;
-        if (j > 0 && j < (int)a.g.k) c.base += (uint64_t)own[j] * a.g.mult[j];
-    }
-    cell_masks(own, a.g, c.low, c.high, c.odd);
-    c.xa = own[0];
-    c.xb = a.gspan > 1u ? FP<T>::to_uint_rz(FP<T>::div(FP<T>::sub(a.pts[(size_t)(q0 + qn - 1u) * a.npad], a.minv[0]),
-                                                       a.eps))
-                        : c.xa;
-    return c;
-}
-
-// The neighbour rows of an item (kernel.cu:180-303; stamploops.h for STAMP) as
-// slot ranges in nb_start and the exclusive prefix of their sizes in nb_pref
-// (nb_pref[rows] = total): the cells xa-1..xb+1 of every row.  With xa < xb a
-// candidate may lie two or more cells from a query; the caller tells them apart.
-// own: slot range of the own row (set for the whole warp).  SEG: cand += the
-// lane's rows' candidates by the reference's rule, nq[i] = queries in cell x0 + i
-// packed in bytes (at most 4 cells); else the caller counts total x qn.  Returns
-// the number of rows; the whole warp calls.
-template <typename T, bool STAMP, bool SEG>
-__device__ __forceinline__ uint32_t enumerate_rows(const JoinArgs<T>& a, const ItemCells& ic, uint32_t nrow,
-                                                   uint32_t* nb_start, uint32_t* nb_pref, int lane, unsigned lt,
-                                                   uint32_t& total, uint2& own, uint32_t nq, unsigned long long& cand) {
-    const unsigned FULL = 0xffffffffu;
-    const uint32_t rc = nrow / 2u;  // the own row
-    // dims 1.. decide which rows are visited; bit 0 of the masks plays no part there
-    const uint64_t own_lin = ic.base + ic.xa;
-    const uint32_t n0 = a.g.ncells[0];
-    const uint32_t xlo0 = ic.xa - (ic.xa > 0u ? 1u : 0u), xhi0 = min(ic.xb + 1u, n0 - 1u);
-    const bool one = ic.xa == ic.xb;
-    // candidates of the cell x0 - 1 + d (byte d): queries of the cells within one
-    // step; with unicomp only the odd cells look at their own row's neighbours
-    const uint32_t x0 = ic.xa;
-    uint64_t w_all = 0, w_own = 0;
-    if (SEG) {
-#pragma unroll
-        for (uint32_t d = 0; d < 6u; d++) {
-            uint32_t wa = 0, wo = 0;
-#pragma unroll
-            for (uint32_t i = 0; i < 4u; i++) {
-                const uint32_t q = (nq >> (8u * i)) & 0xffu;
-                if (i + 2u >= d && i <= d) {  // |x0 + i - (x0 - 1 + d)| <= 1
-                    wa += q;
-                    if (i + 1u == d || ((x0 + i) & 1u)) wo += q;
-                }
-            }
-            w_all |= (uint64_t)wa << (8u * d);
-            w_own |= (uint64_t)(STAMP ? wo : wa) << (8u * d);
-        }
-    }
+    uint32_t lowmask, highmask, oddmask;
+    cell_masks(own, a.g, lowmask, highmask, oddmask);
+    const uint64_t own_lin = a.cell_key[cell];
     uint32_t nnb = 0, run = 0;
-    uint2 mine = make_uint2(0u, 0u);
+    // the next round's first loads are in flight while a round is finished
+    RowProbe next;
+    neighbour_row<T, STAMP>(a, (uint32_t)lane < nrow, (uint32_t)lane, own_lin, own[0], lowmask, highmask, oddmask,
+                            next);
     for (uint32_t b0 = 0; b0 < nrow; b0 += 32) {
-        const uint32_t r = b0 + (uint32_t)lane;
-        uint64_t lin;
-        uint32_t st = 0, v = 0;
-        if (r < nrow && nb_offset<T, STAMP>(a, 3u * r + 1u, own_lin, ic.low, ic.high, ic.odd, lin)) {
-            const bool self = STAMP && one && r == rc && !(ic.xa & 1u);
-            row_slots<T, SEG>(a, lin - ic.xa, self ? ic.xa : xlo0, self ? ic.xa : xhi0, st, v, x0 - 1u,
-                              r == rc ? w_own : w_all, cand);
-        }
-        if (r == rc) mine = make_uint2(st, st + v);
+        const uint32_t r = b0 + 32u + (uint32_t)lane;
+        const RowProbe cur = next;
+        neighbour_row<T, STAMP>(a, r < nrow, r, own_lin, own[0], lowmask, highmask, oddmask, next);
+        uint32_t st, v;
+        row_slots(a, cur, st, v);
         const unsigned m = __ballot_sync(FULL, v != 0u);
         uint32_t x = v;
 #pragma unroll
@@ -221,8 +173,6 @@ __device__ __forceinline__ uint32_t enumerate_rows(const JoinArgs<T>& a, const I
     }
     if (lane == 0) nb_pref[nnb] = run;
     total = run;
-    own.x = __shfl_sync(FULL, mine.x, (int)(rc & 31u));
-    own.y = __shfl_sync(FULL, mine.y, (int)(rc & 31u));
     return nnb;
 }
 
@@ -261,13 +211,11 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_join(const Join
         if (item >= nvisit) break;
         if (lane == 0) claim = atomicAdd(a.work_counter, 1u);
         const uint2 wi = a.items[(size_t)item * o.stride];
-        const uint32_t cs = a.gstart[wi.x], ce = a.gstart[wi.x + 1];  // a cell (gspan is 1)
+        const uint32_t cs = a.cell_start[wi.x], ce = a.cell_start[wi.x + 1];
         const uint32_t q0 = cs + wi.y * kQChunk;
         const uint32_t qn = min((uint32_t)kQChunk, ce - q0);
         uint32_t total;
-        uint2 own;
-        const uint32_t nnb = enumerate_rows<T, STAMP, false>(a, item_cells(a, q0, qn), nrow, nb_start, nb_pref, lane, lt,
-                                                             total, own, 0u, cand_total);
+        const uint32_t nnb = enumerate_rows<T, STAMP>(a, wi.x, cs, nrow, nb_start, nb_pref, lane, lt, total);
 
         // ---- queries
         for (uint32_t e = lane; e < qn * npad; e += 32) q_s[e] = a.pts[(size_t)q0 * npad + e];
@@ -359,7 +307,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_join(const Join
         }
         __syncwarp();
     }
-    if (lane == 0 && cand_total && o.emit) atomicAdd(a.cand_cnt, cand_total);
+    if (lane == 0 && cand_total) atomicAdd(a.cand_cnt, cand_total);
     if (o.emit && blk_used < kEmitBlk)
         for (uint32_t e = blk_used + (uint32_t)lane; e < kEmitBlk; e += 32u)
             if (blk_base + e < o.cap) o.pairs[blk_base + e] = kUndecidedPad;
@@ -377,12 +325,14 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_join(const Join
 //
 // Bound by instruction issue (0.71 of the slots on the 6-D mixture) and by the
 // latency of the enumeration.  Measured, both launches of a join and the
-// sampling pass: 6-D 5M points 40.8 -> 17.1 ms, 8-D 142k points (ILP 8 with
-// SHORTCIRCUIT, formerly through shared memory) 16.8 -> 2.2 ms.  What did not
+// sampling pass: 6-D 5M points 40.8 -> 17.4 ms, 8-D 142k points (ILP 8 with
+// SHORTCIRCUIT, formerly through shared memory) 16.8 -> 1.4 ms.  What did not
 // help: 16-byte entries for single cells hashed next to their row neighbours (33
 // ms, the table no longer fits the L2 and its probe chains diverge); two rows'
-// lookups in flight a lane with the hit's cell check inline (17.8 + 6.4 ms, the
-// code outgrows the instruction cache).
+// lookups in flight with all their steps unrolled (the code outgrows the
+// instruction cache); items of 2 to 4 neighbouring cells of a grid row (17.1 ms at
+// 5M, 5 to 10 % slower on the smaller ones: what the shared enumeration saves
+// goes into candidates of cells two steps away).
 //
 // How the terms are summed (gsj_dist.cuh, float):
 //   kSumSeq    s = fma(d, d, s) (ILP 0 and 1)
@@ -447,20 +397,12 @@ __host__ __device__ inline RegSmem reg_smem(uint32_t np4, uint32_t nrow) {
     return t;
 }
 
-// Work of one unit in (query, 32 G candidates) steps: an item of more than twice
-// that goes to the heavy list in slices.  A step is about 60 instructions, so a
-// unit is some 100 us of a warp: long against the enumeration that every slice
-// repeats (about 10 us), short against a join.  (142k points in 8-D, 32 queries
-// an item in the dense cells: the longest items held the launch for two thirds
-// of its time, 22 % of the warps active on average.)
-constexpr uint32_t kUnitSteps = 512;
-
-// SEG: items are up to 32 queries of up to gspan (at most 4) neighbouring cells
-// of a grid row, which share the enumeration and the candidate loads; a hit is
-// then checked for its cells' distance.  (Cells of 2 points and 130 non-empty
-// neighbour rows each, as on a 5M-point 6-D mixture, spend more on enumerating
-// than on distances.)
-template <int NP, int SUM, int G, bool STAMP, bool SLICES, bool SEG>
+// A unit is heavy.unit steps of (query, 32 G candidates); an item of more than
+// twice that goes to the heavy list in slices.  A step is about 60 instructions.
+// Short units balance a small join (142k points in 8-D, 32 queries an item in the
+// dense cells: unsliced, the longest items held the launch for two thirds of its
+// time), long ones repeat the enumeration less often: see join_unit_steps.
+template <int NP, int SUM, int G, bool STAMP, bool SLICES>
 __global__ void __launch_bounds__(256, 4) k_join_reg(const JoinArgs<float> a, uint32_t nrow, const TileOut o,
                                                      const HeavyList heavy, uint32_t nvisit) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -471,7 +413,7 @@ __global__ void __launch_bounds__(256, 4) k_join_reg(const JoinArgs<float> a, ui
     const RegSmem L = reg_smem(NP4, nrow);
     unsigned char* wb = smem_raw + (size_t)(threadIdx.x >> 5) * L.total;
     float* q_s = reinterpret_cast<float*>(wb + L.q);
-    uint2* hits = reinterpret_cast<uint2*>(wb + L.hits);  // (query slot | flag << 31, candidate slot)
+    uint2* hits = reinterpret_cast<uint2*>(wb + L.hits);  // (query slot | cross << 31, candidate slot)
     uint32_t* nb_start = reinterpret_cast<uint32_t*>(wb + L.nbs);
     uint32_t* nb_pref = reinterpret_cast<uint32_t*>(wb + L.nbp);
     const unsigned lt = lanemask_lt();
@@ -483,27 +425,14 @@ __global__ void __launch_bounds__(256, 4) k_join_reg(const JoinArgs<float> a, ui
         for (uint32_t l = 0; l < NP; l += a.ilp) fused |= 1u << l;
 
     // The last `cnt` (at most 32) entries of the queue become keys, a full warp of
-    // them at a time.  The flag of an entry: the candidate lies outside the query's
-    // cell (unicomp, one cell an item), or in its grid row (SEG).
+    // them at a time.
     auto flush = [&](uint32_t cnt) {
         __syncwarp();
-        bool v = (uint32_t)lane < cnt;
+        const bool v = (uint32_t)lane < cnt;
         const uint2 e = v ? hits[nq - cnt + (uint32_t)lane] : make_uint2(0u, 0u);
-        const uint32_t qs = e.x & 0x7fffffffu;
-        bool cr = STAMP && (e.x >> 31) != 0u;
-        if (SEG) {
-            // cells more than one step apart are no candidates; with unicomp the own
-            // row's neighbours are those of the odd cells
-            const uint32_t xq = FP<float>::to_uint_rz(
-                FP<float>::div(FP<float>::sub(a.pts[(size_t)qs * NP4], a.minv[0]), a.eps));
-            const uint32_t xc = FP<float>::to_uint_rz(
-                FP<float>::div(FP<float>::sub(a.pts[(size_t)e.y * NP4], a.minv[0]), a.eps));
-            const bool row = (e.x >> 31) != 0u;
-            v = v && xc + 1u - xq <= 2u && !(STAMP && row && xc != xq && !(xq & 1u));
-            cr = STAMP && v && !(row && xc == xq);
-        }
+        const bool cr = STAMP && (e.x >> 31) != 0u;
         const unsigned b = __ballot_sync(FULL, v), cb = __ballot_sync(FULL, cr);
-        const uint64_t qid = v && o.emit ? a.ids[qs] : 0u, cid = v && o.emit ? a.ids[e.y] : 0u;
+        const uint64_t qid = v && o.emit ? a.ids[e.x & 0x7fffffffu] : 0u, cid = v && o.emit ? a.ids[e.y] : 0u;
         emit_keys(o, blk_base, blk_used, emitted, v, cr, b, cb, lt, lane, qid, cid);
         nq -= cnt;
         __syncwarp();
@@ -526,30 +455,18 @@ __global__ void __launch_bounds__(256, 4) k_join_reg(const JoinArgs<float> a, ui
             if (visit >= nvisit) continue;  // an entry of an item that found the list full
         }
         const uint2 wi = a.items[(size_t)visit * o.stride];
-        const uint32_t cs = a.gstart[wi.x], ce = a.gstart[wi.x + 1];
+        const uint32_t cs = a.cell_start[wi.x], ce = a.cell_start[wi.x + 1];
         const uint32_t q0 = cs + wi.y * kQChunk;
         const uint32_t qn = min((uint32_t)kQChunk, ce - q0);
-        const ItemCells ic = item_cells(a, q0, qn);
-        uint32_t nqx = 0;  // queries of each of the item's cells (bytes)
-        if (SEG) {
-            const uint32_t x = FP<float>::to_uint_rz(FP<float>::div(
-                FP<float>::sub(a.pts[(size_t)(q0 + min((uint32_t)lane, qn - 1u)) * NP4], a.minv[0]), a.eps));
-#pragma unroll
-            for (uint32_t i = 0; i < 4u; i++)
-                nqx |= (uint32_t)__popc(__ballot_sync(FULL, lane < qn && x == ic.xa + i)) << (8u * i);
-        }
         uint32_t total;
-        uint2 own;
-        unsigned long long cand = 0;
-        const uint32_t nnb =
-            enumerate_rows<float, STAMP, SEG>(a, ic, nrow, nb_start, nb_pref, lane, lt, total, own, nqx, cand);
+        const uint32_t nnb = enumerate_rows<float, STAMP>(a, wi.x, cs, nrow, nb_start, nb_pref, lane, lt, total);
         uint32_t g_lo = 0, g_hi = (total + 32u * G - 1u) / (32u * G);  // candidate groups of this unit
-        const uint32_t per = (kUnitSteps + qn - 1u) / qn;              // groups of a slice
+        const uint32_t per = (heavy.unit + qn - 1u) / qn;              // groups of a slice
         if (SLICES) {
             g_lo = slice * per;
             g_hi = min(g_hi, g_lo + per);
         } else {
-            cand_total += SEG ? cand : lane == 0 ? (unsigned long long)total * qn : 0ull;
+            cand_total += (unsigned long long)total * qn;
             if (g_hi > 2u * per) {
                 const uint32_t ns = (g_hi + per - 1u) / per;
                 uint32_t at = 0;
@@ -605,12 +522,11 @@ __global__ void __launch_bounds__(256, 4) k_join_reg(const JoinArgs<float> a, ui
                 for (int t = 0; t < G; t++) {
                     const bool hit = s[t] <= a.thr;
                     const unsigned b = __ballot_sync(FULL, hit);
-                    bool flag = false;
-                    if (SEG) flag = slot[t] >= own.x && slot[t] < own.y;
-                    else if (STAMP) flag = slot[t] < cs || slot[t] >= ce;
+                    // outside the own cell: the reverse pair too
+                    const bool cross = STAMP && (slot[t] < cs || slot[t] >= ce);
                     if (hit)
                         hits[nq + (uint32_t)__popc(b & lt)] =
-                            make_uint2((q0 + j) | (flag ? 0x80000000u : 0u), slot[t]);
+                            make_uint2((q0 + j) | (cross ? 0x80000000u : 0u), slot[t]);
                     nq += (uint32_t)__popc(b);
                 }
                 while (nq >= 32u) flush(32u);
@@ -618,11 +534,7 @@ __global__ void __launch_bounds__(256, 4) k_join_reg(const JoinArgs<float> a, ui
         }
     }
     if (nq) flush(nq);
-    if (!SLICES && o.emit) {
-#pragma unroll
-        for (int s = 16; s > 0; s >>= 1) cand_total += __shfl_xor_sync(FULL, cand_total, s);
-        if (lane == 0 && cand_total) atomicAdd(a.cand_cnt, cand_total);
-    }
+    if (!SLICES && lane == 0 && cand_total) atomicAdd(a.cand_cnt, cand_total);
     if (o.emit && blk_used < kEmitBlk)
         for (uint32_t e = blk_used + (uint32_t)lane; e < kEmitBlk; e += 32u)
             if (blk_base + e < o.cap) o.pairs[blk_base + e] = kUndecidedPad;
@@ -678,11 +590,11 @@ static cudaError_t launch_one(const JoinArgs<T>& a, uint32_t nrow, const TileOut
     return cudaGetLastError();
 }
 
-template <int NP, int SUM, int G, bool STAMP, bool SEG>
+template <int NP, int SUM, int G, bool STAMP>
 static cudaError_t launch_reg(const JoinArgs<float>& a, uint32_t nrow, const TileOut& o, const HeavyList& heavy,
                               uint32_t nvisit, int num_sms, int* launches, cudaStream_t st) {
-    auto k1 = k_join_reg<NP, SUM, G, STAMP, false, SEG>;
-    auto k2 = k_join_reg<NP, SUM, G, STAMP, true, SEG>;
+    auto k1 = k_join_reg<NP, SUM, G, STAMP, false>;
+    auto k2 = k_join_reg<NP, SUM, G, STAMP, true>;
     const RegSmem L = reg_smem((NP + 3) / 4 * 4, nrow);
     int threads = 0;
     size_t smem = 0;
@@ -699,24 +611,27 @@ static cudaError_t launch_reg(const JoinArgs<float>& a, uint32_t nrow, const Til
     return cudaGetLastError();
 }
 
-bool join_reg_supported(uint32_t n, uint32_t npad, int model, uint32_t ilp) {
-    if (n > 16 || npad != npad_for(n, 4u) || npad < 4u || (npad & 3u)) return false;
-    // ILP chains of several dims take the shared-memory form
-    return model == kSeq || model == kIlpSc || ilp <= 1u || ilp >= n;
+// Steps of a unit for a join of about `cand` candidate evaluations (0: unknown):
+// some 32 units a resident warp.  Emit stage at 32 / 64 / 128 / 256 steps: 6-D
+// 200k 0.73 / 0.84 / 0.89 / 1.10 ms, 8-D 142k 1.44 / 1.42 / 1.46 / 1.50, 8-D
+// 280k 5.91 / 5.35 / 5.27 / 5.19, 6-D 5M 22.8 / 19.4 / 17.8 / 17.4.
+uint32_t join_unit_steps(double cand, int num_sms) {
+    if (cand <= 0.0) return 128u;
+    const double per_warp = cand / 128.0 / ((double)num_sms * 32.0);
+    return (uint32_t)std::min(256.0, std::max(32.0, per_warp / 32.0));
 }
 
 // The register form's dispatch: false when the join takes k_join.
 template <bool STAMP>
 static bool try_reg(const JoinArgs<float>& a, int model, uint32_t nrow, const TileOut& o, const HeavyList& heavy,
                     uint32_t nvisit, int num_sms, int* launches, cudaStream_t st, cudaError_t* e) {
-    if (!join_reg_supported(a.n, a.npad, model, a.ilp)) return false;
+    if (a.n > 16 || a.npad != npad_for(a.n, 4u) || a.npad < 4u || (a.npad & 3u)) return false;
     const bool seq = model == kSeq || a.ilp <= 1u;
     const bool first = !seq && a.ilp >= a.n;
+    if (!seq && !first && model != kIlpSc) return false;  // ILP chains of several dims
 #define GSJ_REG(NP, SUM, G)                                                                            \
     do {                                                                                               \
-        *e = a.gspan > 1u                                                                              \
-                 ? launch_reg<NP, SUM, G, STAMP, true>(a, nrow, o, heavy, nvisit, num_sms, launches, st)    \
-                 : launch_reg<NP, SUM, G, STAMP, false>(a, nrow, o, heavy, nvisit, num_sms, launches, st);  \
+        *e = launch_reg<NP, SUM, G, STAMP>(a, nrow, o, heavy, nvisit, num_sms, launches, st);           \
         return true;                                                                                   \
     } while (0)
     if (seq) {
@@ -785,10 +700,7 @@ cudaError_t launch_join_emit(const JoinArgs<T>& a, const TileOut& o, const Heavy
                              int model, bool stamp, int num_sms, int* launches, cudaStream_t st) {
     uint32_t nrow = 1;  // neighbour rows: 3^(k-1)
     for (uint32_t j = 1; j < a.g.k; j++) nrow *= 3u;
-    if (o.stride == 0 || !heavy.list || heavy.cap != kHeavyCap || !a.gstart || a.gspan < 1u || a.gspan > 4u)
-        return cudaErrorInvalidValue;
-    if (a.gspan > 1u && (sizeof(T) != 4 || !join_reg_supported(a.n, a.npad, model, a.ilp)))
-        return cudaErrorInvalidValue;
+    if (o.stride == 0 || !heavy.list || heavy.cap != kHeavyCap || heavy.unit == 0) return cudaErrorInvalidValue;
     if (nvisit == 0) return cudaSuccess;
     if ((uint64_t)(nvisit - 1) * o.stride >= a.num_items) return cudaErrorInvalidValue;
     return stamp ? dispatch_model<T, true>(a, model, nrow, o, heavy, nvisit, num_sms, launches, st)

@@ -47,13 +47,6 @@ cudaError_t launch_row_table(const uint64_t* cell_key, uint32_t M, uint32_t n0, 
                              cudaStream_t st);
 cudaError_t launch_cell_plan(const uint64_t* cell_key, uint32_t M, const GridGeom& g, const uint32_t* ds,
                              uint2* plan, cudaStream_t st);
-// Query groups of up to `span` neighbouring cells of a grid row: flags[M] marks
-// their first cells, and with pos = the exclusive scan of flags (M + 1
-// entries) gstart[M + 1] receives their first slots (N past the last group).
-cudaError_t launch_group_flags(const uint64_t* cell_key, uint32_t M, uint32_t n0, uint32_t span, uint32_t* flags,
-                               cudaStream_t st);
-cudaError_t launch_group_starts_of(const uint32_t* flags, const uint32_t* pos, const uint32_t* cell_start, uint32_t M,
-                                   uint32_t N, uint32_t* gstart, cudaStream_t st);
 cudaError_t launch_item_counts(const uint32_t* cell_start, const uint32_t* order, uint32_t M, uint32_t qchunk,
                                uint32_t* nchunks, uint32_t* sizes, cudaStream_t st);
 cudaError_t launch_make_items(const uint32_t* order, const uint32_t* nchunks, const uint32_t* item_off,
@@ -75,11 +68,10 @@ struct HeavyList {
     uint32_t* count;  // slices found (may exceed cap; those entries are dropped)
     uint32_t* claim;  // the second launch's work counter
     uint32_t cap;
+    uint32_t unit;    // steps of a slice (join_unit_steps)
 };
 constexpr uint32_t kHeavyCap = 1u << 20;
-// Whether the join of float rows runs in registers (query groups of several
-// cells need that form).
-bool join_reg_supported(uint32_t n, uint32_t npad, int model, uint32_t ilp);
+uint32_t join_unit_steps(double cand, int num_sms);
 template <typename T>
 cudaError_t launch_join_emit(const JoinArgs<T>& a, const TileOut& o, const HeavyList& heavy, uint32_t nvisit,
                              int model, bool stamp, int num_sms, int* launches, cudaStream_t st);

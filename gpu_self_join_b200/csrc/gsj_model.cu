@@ -285,18 +285,19 @@ __device__ __forceinline__ float mlp_out(const float* __restrict__ w, const floa
     return o;
 }
 
-// out[c] = network output of row c; with cell_start, *est += size_c x
-// predicted list length (2^out - 1, clamped to [0, N]).
+// out[c] = network output of row c; with cell_start (row c is cell c * stride),
+// est[0] += size x predicted list length (2^out - 1, clamped to [0, N]) and
+// est[1] += size.
 __global__ void __launch_bounds__(256) k_model_predict(const float* __restrict__ X, uint32_t m,
                                                        const float* __restrict__ W, float* __restrict__ out,
-                                                       const uint32_t* __restrict__ cell_start, float nmax,
-                                                       double* __restrict__ est) {
+                                                       const uint32_t* __restrict__ cell_start, uint32_t stride,
+                                                       float nmax, double* __restrict__ est) {
     __shared__ __align__(16) float w[kModelWeights];
-    __shared__ double red[8];
+    __shared__ double red[8], red2[8];
     for (int i = threadIdx.x; i < kModelWeights; i += blockDim.x) w[i] = W[i];
     __syncthreads();
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    double part = 0.0;
+    double part = 0.0, pts = 0.0;
     if (c < m) {
         float x[kF];
 #pragma unroll
@@ -311,27 +312,40 @@ __global__ void __launch_bounds__(256) k_model_predict(const float* __restrict__
         if (out) out[c] = o;
         if (cell_start) {
             const float per = fminf(fmaxf(exp2f(fminf(o, 40.f)) - 1.f, 0.f), nmax);
-            part = (double)(cell_start[c + 1] - cell_start[c]) * (double)per;
+            pts = (double)(cell_start[c * stride + 1] - cell_start[c * stride]);
+            part = pts * (double)per;
         }
     }
     if (est) {
-        for (int o = 16; o > 0; o >>= 1) part += __shfl_down_sync(0xffffffffu, part, o);
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = part;
+        for (int o = 16; o > 0; o >>= 1) {
+            part += __shfl_down_sync(0xffffffffu, part, o);
+            pts += __shfl_down_sync(0xffffffffu, pts, o);
+        }
+        if ((threadIdx.x & 31) == 0) {
+            red[threadIdx.x >> 5] = part;
+            red2[threadIdx.x >> 5] = pts;
+        }
         __syncthreads();
         if (threadIdx.x == 0) {
-            double t = 0.0;
-            for (int i = 0; i < (int)(blockDim.x >> 5); i++) t += red[i];
+            double t = 0.0, p = 0.0;
+            for (int i = 0; i < (int)(blockDim.x >> 5); i++) {
+                t += red[i];
+                p += red2[i];
+            }
             atomicAdd(est, t);
+            atomicAdd(est + 1, p);
         }
     }
 }
 
 __device__ __forceinline__ float log2p1(float v) { return log2f(1.f + v); }
 
-__global__ void __launch_bounds__(256) k_model_features(const JoinArgs<float> a, uint32_t M, float log2_eps,
-                                                        uint32_t n, float* __restrict__ X) {
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= M) return;
+// Row i describes cell i * stride.
+__global__ void __launch_bounds__(256) k_model_features(const JoinArgs<float> a, uint32_t rows, uint32_t stride,
+                                                        float log2_eps, uint32_t n, float* __restrict__ X) {
+    const uint32_t row = blockIdx.x * blockDim.x + threadIdx.x;
+    if (row >= rows) return;
+    const uint32_t c = row * stride;
     const uint32_t k = a.g.k;
     const uint64_t key = a.cell_key[c];
     const uint32_t size = a.cell_start[c + 1] - a.cell_start[c];
@@ -356,7 +370,7 @@ __global__ void __launch_bounds__(256) k_model_features(const JoinArgs<float> a,
         }
     }
     const float inv = k ? 1.f / (2.f * (float)k) : 0.f;
-    float* x = X + (size_t)c * kF;
+    float* x = X + (size_t)row * kF;
     x[0] = log2p1((float)size) / 8.f;
 #pragma unroll
     for (int i = 0; i < 8; i++) x[1 + i] = hist[i] * inv;
@@ -415,10 +429,10 @@ cudaError_t model_init(float* W, float* M1, float* M2, uint32_t seed, cudaStream
     return cudaGetLastError();
 }
 
-cudaError_t model_features(const JoinArgs<float>& lookup, uint32_t M, float log2_eps, uint32_t n, float* X,
-                           cudaStream_t st) {
-    if (M == 0) return cudaSuccess;
-    k_model_features<<<blocks_for(M, 256), 256, 0, st>>>(lookup, M, log2_eps, n, X);
+cudaError_t model_features(const JoinArgs<float>& lookup, uint32_t rows, uint32_t stride, float log2_eps, uint32_t n,
+                           float* X, cudaStream_t st) {
+    if (rows == 0) return cudaSuccess;
+    k_model_features<<<blocks_for(rows, 256), 256, 0, st>>>(lookup, rows, stride, log2_eps, n, X);
     return cudaGetLastError();
 }
 
@@ -438,10 +452,10 @@ cudaError_t model_subsample(const float* X, const float* Y, uint32_t M, uint32_t
     return cudaGetLastError();
 }
 
-cudaError_t model_predict(const float* X, uint32_t m, const float* W, float* out, const uint32_t* cell_start,
+cudaError_t model_predict(const float* X, uint32_t m, const float* W, float* out, const uint32_t* cell_start, uint32_t stride,
                           float nmax, double* est, cudaStream_t st) {
     if (m == 0) return cudaSuccess;
-    k_model_predict<<<blocks_for(m, 256), 256, 0, st>>>(X, m, W, out, cell_start, nmax, est);
+    k_model_predict<<<blocks_for(m, 256), 256, 0, st>>>(X, m, W, out, cell_start, stride, nmax, est);
     return cudaGetLastError();
 }
 
