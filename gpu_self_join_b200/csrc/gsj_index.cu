@@ -19,44 +19,78 @@
 namespace gsj {
 
 // ------------------------------------------------------------ REORDER statistic
-// One block.  Thread i owns dimension i and adds the sampled values in the
-// reference's sequential order (rows 0, 100, 200, ...), unfused, in T.  The
-// sampled rows are staged through shared memory in chunks by the whole block
-// (up to 1024 threads, many loads in flight) so that the sequential chains run
-// on on-chip data.
+// Every dimension's sampled values (rows 0, 100, 200, ...) are added one after
+// another in the reference's order, unfused, in T: a chain of dependent additions
+// per dimension, twice (mean, then squared deviations).  A block takes 8
+// dimensions (a 32-byte sector of a row in FP32); its warps 1.. stage the next
+// chunk of samples, in the second pass already as squared deviations, while the
+// first 8 lanes of warp 0 add the current one from shared memory, 16 values read
+// ahead of the chain.
+// Bound by the additions' latency (4 cycles) and the staging of one block.
+constexpr uint32_t kVarDims = 8, kVarThreads = 1024, kVarUnroll = 16;
 template <typename T>
-__global__ void k_variance(const T* __restrict__ in, uint64_t N, uint32_t n, T denom,
-                           T* __restrict__ var_out) {
+constexpr uint32_t kVarChunk = 992u * 4u / sizeof(T);  // samples: 8 (FP32) or 4 loads a thread
+template <typename T>
+constexpr size_t kVarSmem = 2u * kVarChunk<T> * kVarDims * sizeof(T);
+
+template <typename T>
+__global__ void __launch_bounds__(kVarThreads, 1) k_variance(const T* __restrict__ in, uint64_t N, uint32_t n, T denom,
+                                                          T* __restrict__ var_out) {
     extern __shared__ unsigned char smem_raw[];
-    T* stage = reinterpret_cast<T*>(smem_raw);
-    const uint32_t chunk = (uint32_t)(kVarStageBytes / sizeof(T)) / n;  // samples per chunk
+    T* const stage = reinterpret_cast<T*>(smem_raw);
+    __shared__ T s_avg[kVarDims];
+    constexpr uint32_t C = kVarChunk<T>, E = C * kVarDims;
+    const uint32_t d0 = blockIdx.x * kVarDims, nd = min(kVarDims, n - d0);
     const uint64_t nsamp = (N + 99) / 100;
-    for (uint32_t d0 = 0; d0 < n; d0 += blockDim.x) {
-        const uint32_t d = d0 + threadIdx.x;
-        T sum = 0, avg = 0, ssq = 0;
-        for (int pass = 0; pass < 2; pass++) {
-            for (uint64_t s0 = 0; s0 < nsamp; s0 += chunk) {
-                const uint32_t cs = (uint32_t)((nsamp - s0) < chunk ? (nsamp - s0) : chunk);
-                __syncthreads();
-                for (uint32_t e = threadIdx.x; e < cs * n; e += blockDim.x) {
-                    const uint32_t s = e / n, c = e - s * n;
-                    stage[e] = in[(s0 + s) * 100ull * n + c];
-                }
-                __syncthreads();
-                if (d < n) {
-                    if (pass == 0) {
-                        for (uint32_t s = 0; s < cs; s++) sum = FP<T>::add(sum, stage[s * n + d]);
-                    } else {
-                        for (uint32_t s = 0; s < cs; s++) {
-                            const T dv = FP<T>::sub(stage[s * n + d], avg);
-                            ssq = FP<T>::add(ssq, FP<T>::mul(dv, dv));
-                        }
-                    }
-                }
+    const uint64_t nchunk = (nsamp + C - 1) / C;
+    T avg = 0;
+    // elements t, t + nt, ... of chunk c into its buffer
+    auto fill = [&](uint64_t c, int pass, uint32_t t, uint32_t nt) {
+        T* const dst = stage + (c & 1u) * E;
+        const uint64_t s0 = c * C;
+        const uint32_t cnt = (uint32_t)min((uint64_t)C, nsamp - s0) * kVarDims;
+        const T a = pass ? s_avg[t & (kVarDims - 1u)] : T(0);  // nt is a multiple of kVarDims
+#pragma unroll 4
+        for (uint32_t e = t; e < cnt; e += nt) {
+            const uint32_t d = e & (kVarDims - 1u);
+            T v = d < nd ? in[(s0 + e / kVarDims) * 100ull * n + d0 + d] : T(0);
+            if (pass) {
+                const T dv = FP<T>::sub(v, a);
+                v = FP<T>::mul(dv, dv);
             }
-            if (pass == 0) avg = FP<T>::div(sum, denom);
+            dst[e] = v;
         }
-        if (d < n) var_out[d] = FP<T>::div(ssq, denom);
+    };
+    for (int pass = 0; pass < 2; pass++) {
+        T sum = 0;
+        fill(0, pass, threadIdx.x, kVarThreads);
+        __syncthreads();
+        for (uint64_t c = 0; c < nchunk; c++) {
+            if (threadIdx.x < 32u) {
+                if (threadIdx.x < nd) {
+                    const T* const p = stage + (c & 1u) * E + threadIdx.x;
+                    const uint32_t cs = (uint32_t)min((uint64_t)C, nsamp - c * C);
+                    uint32_t s = 0;
+                    for (; s + kVarUnroll <= cs; s += kVarUnroll) {
+                        T v[kVarUnroll];
+#pragma unroll
+                        for (uint32_t u = 0; u < kVarUnroll; u++) v[u] = p[(s + u) * kVarDims];
+#pragma unroll
+                        for (uint32_t u = 0; u < kVarUnroll; u++) sum = FP<T>::add(sum, v[u]);
+                    }
+                    for (; s < cs; s++) sum = FP<T>::add(sum, p[s * kVarDims]);
+                }
+            } else if (c + 1 < nchunk) {
+                fill(c + 1, pass, threadIdx.x - 32u, kVarThreads - 32u);
+            }
+            __syncthreads();
+        }
+        if (threadIdx.x < nd) {
+            avg = FP<T>::div(sum, denom);
+            if (pass == 0) s_avg[threadIdx.x] = avg;
+            else var_out[d0 + threadIdx.x] = avg;
+        }
+        __syncthreads();
     }
 }
 
@@ -430,11 +464,10 @@ static inline unsigned blocks_for(uint64_t n, unsigned t) { return (unsigned)((n
 
 template <typename T>
 cudaError_t launch_variance(const T* in, uint64_t N, uint32_t n, T denom, T* var_out, cudaStream_t st) {
-    // the staging uses every thread; the sums use the first n (d0 loop above 1024)
-    const unsigned threads = 1024;
-    cudaError_t e = cudaFuncSetAttribute(k_variance<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kVarStageBytes);
+    const int smem = (int)kVarSmem<T>;
+    cudaError_t e = cudaFuncSetAttribute(k_variance<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    k_variance<T><<<1, threads, kVarStageBytes, st>>>(in, N, n, denom, var_out);
+    k_variance<T><<<(n + kVarDims - 1u) / kVarDims, kVarThreads, smem, st>>>(in, N, n, denom, var_out);
     return cudaGetLastError();
 }
 

@@ -800,6 +800,7 @@ __global__ void __launch_bounds__(256, 4) k_screen_recheck(const float* __restri
         uint32_t pos = x - cnt;
         for (uint32_t m = r.z; m; m &= m - 1u) wl[pos++] = (uint16_t)((lane << 5) | ((uint32_t)__ffs(m) - 1u));
         __syncwarp();
+        uint32_t nhit = 0, ncross = 0;
         for (uint32_t b = 0; b < total; b += 32u) {
             const bool valid = b + lane < total;
             const uint32_t e = valid ? wl[b + lane] : 0u;
@@ -809,19 +810,35 @@ __global__ void __launch_bounds__(256, 4) k_screen_recheck(const float* __restri
             bool hit = false;
             if (valid && qs < npoints && cs < npoints)
                 hit = exact_sqdist4<MODEL>(pts + (size_t)qs * npad, pts + (size_t)cs * npad, n, ilp, thr) <= thr;
-            const bool cross = STAMP && hit && ((crossm >> (e & 31u)) & 1u);
-            const unsigned hb = __ballot_sync(FULL, hit), cb = __ballot_sync(FULL, cross);
-            if (hb == 0u) continue;
-            const uint32_t wtotal = (uint32_t)__popc(hb) + (uint32_t)__popc(cb);
+            // the hits move to the front of the list (behind the entries still to be read)
+            const unsigned hb = __ballot_sync(FULL, hit);
+            if (hit) wl[nhit + (uint32_t)__popc(hb & lt)] = (uint16_t)e;
+            nhit += (uint32_t)__popc(hb);
+            if (STAMP)
+                ncross += (uint32_t)__popc(__ballot_sync(FULL, hit && ((crossm >> (e & 31u)) & 1u)));
+            __syncwarp();
+        }
+        // one reservation for the warp's 32 records
+        if (nhit) {
             unsigned long long base = 0;
-            if (lane == 0u) base = atomicAdd(o.cursor, (unsigned long long)wtotal);
+            if (lane == 0u) base = atomicAdd(o.cursor, (unsigned long long)(nhit + ncross));
             base = __shfl_sync(FULL, base, 0);
-            if (hit) {
-                unsigned long long p = base + (unsigned)__popc(hb & lt) + (unsigned)__popc(cb & lt);
-                const uint64_t qid = ids[qs], cid = ids[cs];
-                if (p < o.cap) o.pairs[p] = (qid << o.shift) | cid;
-                p++;
-                if (cross && p < o.cap) o.pairs[p] = (cid << o.shift) | qid;
+            for (uint32_t b = 0; b < nhit; b += 32u) {
+                const bool valid = b + lane < nhit;
+                const uint32_t e = valid ? wl[b + lane] : 0u;
+                const uint32_t qs = __shfl_sync(FULL, r.x, (int)(e >> 5));
+                const uint32_t cs = __shfl_sync(FULL, r.y, (int)(e >> 5)) + (e & 31u);
+                const uint32_t crossm = STAMP ? __shfl_sync(FULL, r.w, (int)(e >> 5)) : 0u;
+                const bool cross = STAMP && valid && ((crossm >> (e & 31u)) & 1u);
+                const unsigned cb = STAMP ? __ballot_sync(FULL, cross) : 0u;
+                if (valid) {
+                    unsigned long long p = base + lane + (unsigned)__popc(cb & lt);
+                    const uint64_t qid = ids[qs], cid = ids[cs];
+                    if (p < o.cap) o.pairs[p] = (qid << o.shift) | cid;
+                    p++;
+                    if (cross && p < o.cap) o.pairs[p] = (cid << o.shift) | qid;
+                }
+                base += 32u + (unsigned)__popc(cb);
             }
         }
         __syncwarp();

@@ -15,7 +15,6 @@ namespace gsj {
 // cached per (device, kernel, block size, dynamic shared memory).
 cudaError_t blocks_per_sm(const void* kern, int threads, size_t smem, int* per_sm);
 
-constexpr unsigned kVarStageBytes = 98304;  // shared staging of sampled rows (REORDER statistic)
 
 template <typename T>
 cudaError_t launch_variance(const T* in, uint64_t N, uint32_t n, T denom, T* var_out, cudaStream_t st);
