@@ -715,7 +715,7 @@ int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int mo
     const uint64_t entry = screen ? 2u : 1u;  // 64-bit words per buffer entry
     unsigned long long U = 0, R = 0, nlist = 0, used = 0;
     for (int attempt = 0; attempt < 3; attempt++) {
-        cap = retry_cap(attempt, estimate, used, screen ? reserve_bound(U, warps, kScreenBlock, 1u) : U);
+        cap = retry_cap(attempt, estimate, used, screen ? reserve_bound(U, warps, kScreenBlock, 32u) : U);
         GSJ_TRY(dev_get(c, screen ? c->unc : c->pairs, (cap ? cap : 1) * entry, &list));
         GSJ_TRY(reset());
         o.emit = true;

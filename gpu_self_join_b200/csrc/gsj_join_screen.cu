@@ -127,6 +127,17 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64
         "l"(adesc), "l"(bdesc), "r"(kIdesc), "r"(accumulate));
 }
 
+// True for one lane of a converged warp, the same one every time.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(p));
+    return p != 0;
+}
+
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                  : "memory");
@@ -188,6 +199,14 @@ __device__ __forceinline__ void tmem_wait_ld(uint32_t* r) {
                  :
                  : "memory");
     asm volatile("" : "+r"(r[30]), "+r"(r[31])::"memory");
+}
+
+// The same for 32 more registers, after the wait.
+__device__ __forceinline__ void tmem_named(uint32_t* r) {
+#pragma unroll
+    for (int j = 0; j < 32; j += 8)
+        asm volatile("" : "+r"(r[j]), "+r"(r[j + 1]), "+r"(r[j + 2]), "+r"(r[j + 3]), "+r"(r[j + 4]), "+r"(r[j + 5]),
+                          "+r"(r[j + 6]), "+r"(r[j + 7])::"memory");
 }
 
 // The reference's squared distance in its exact order, one thread, stopping
@@ -260,6 +279,16 @@ __device__ float exact_sqdist4(const float* __restrict__ q, const float* __restr
     return s;
 }
 
+// Bit c: slot gs + c lies outside [lo, hi); gs is a slot or, modulo 2^32, up to
+// 24 below slot 0.
+__device__ __forceinline__ uint32_t outside_mask(uint32_t gs, uint32_t lo, uint32_t hi) {
+    const int64_t g = gs > 0xffffffe0u ? (int64_t)gs - (1ll << 32) : (int64_t)gs;
+    const int64_t a = (int64_t)lo - g, b = (int64_t)hi - g;
+    const uint32_t l = a <= 0 ? 0u : a >= 32 ? 32u : (uint32_t)a, h = b <= 0 ? 0u : b >= 32 ? 32u : (uint32_t)b;
+    const uint32_t below_l = l == 32u ? 0xffffffffu : (1u << l) - 1u, below_h = h == 32u ? 0xffffffffu : (1u << h) - 1u;
+    return ~(below_h & ~below_l);
+}
+
 struct ScreenSmem {
     uint32_t a, nbs, nbe, nbg, mbase, mmask, misc, b, total;
 };
@@ -318,15 +347,20 @@ __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_
 // 128 consecutive query slots of one cell): slices give small joins and the
 // sampling pass enough units for the whole chip and shorten the last wave.
 //
-// What bounds it: the consumers' dependent instructions.  At K = 32 the tensor
-// pipe needs 128 cycles for a tile; a tile takes about 600 cycles of an SM (0.21
-// of the tensor pipe), 16 consumer warps an SM issuing 0.47 instructions a cycle
-// and scheduler, half of them on the 32-column blocks that hold an undecided
-// pair.  A consumer warp reads 32 columns at a time: with 64 the registers spill
-// at 2 CTAs an SM (133 against 105 ms on the 18-D workload).  Measured (both
-// launches of a join): 18-D 5M points 270 -> 105 ms, 90-D 515k 117 -> 40 ms, 32-D
-// 45k 2.0 -> 0.64 ms, against four warps staging rows one by one with cp.async
-// and a compare per pair with a bound per 32 candidates (1,720 cycles a tile).
+// What bounds it: the two accumulators of a CTA (all of tensor memory at 2 CTAs
+// an SM) alternate between the MMA and eight consumer warps that need them for
+// different times, since only some warps of a tile meet an undecided pair (about
+// 1 in 5 at 18 dims; such a warp takes some 1,000 cycles longer).  So a consumer
+// warp reads its 64 columns at once and frees the accumulator before it looks at
+// them, and the path of a warp with undecided pairs is kept short (one word of
+// metadata says whether four groups are consecutive, which makes one record a
+// query row; records go to a block that is never split).  A tile takes some 530
+// cycles of an SM at K = 32 (the tensor pipe needs 128) and 650 at K = 96 (384).
+// Measured (both launches of a join): 18-D 5M points 270 -> 97 ms, 90-D 515k 117
+// -> 33 ms, 32-D 45k 2.0 -> 0.61 ms, against four warps staging rows one by one
+// with cp.async and a compare per pair with a bound per 32 candidates (1,720
+// cycles a tile).  Tried without gain: 16 consumer warps a CTA reading 16 columns
+// at a time, an MMA warp per accumulator.
 template <bool STAMP>
 __global__ void __launch_bounds__(kSThreads, 2) k_tile_screen(const JoinArgs<float> a, const TileOut o,
                                                               const ScreenConst sc, uint32_t nrow, uint32_t stages,
@@ -379,8 +413,8 @@ __global__ void __launch_bounds__(kSThreads, 2) k_tile_screen(const JoinArgs<flo
     unsigned long long cand_total = 0;
     // consumer warps: the reserved block of records; undecided pairs and records
     // so far in shared memory
-    unsigned long long blk_base = 0;
-    uint32_t blk_used = kBlk;
+    uint4* blk = nullptr;
+    uint32_t blk_used = kBlk, blk_room = 0;
     uint4* recs = reinterpret_cast<uint4*>(o.pairs);
     unsigned long long* n_und = reinterpret_cast<unsigned long long*>(misc + 64) + warp;
     unsigned long long* n_rec = n_und + kConsumers / 32;
@@ -541,6 +575,7 @@ __global__ void __launch_bounds__(kSThreads, 2) k_tile_screen(const JoinArgs<flo
                 const uint32_t prev = __shfl_up_sync(FULL, gid, 1);
                 const bool head = mine && (half == 0u || gid != prev + 1u);
                 const unsigned heads = __ballot_sync(FULL, head);
+                const unsigned breaks = heads | __ballot_sync(FULL, !mine);
                 for (uint32_t u = 0; u < 2u && t + u < t1; u++) {
                     if (g >= stages) {
                         ok = warp_wait_bounded(drained + 8u * b, ph ^ 1u);
@@ -549,7 +584,8 @@ __global__ void __launch_bounds__(kSThreads, 2) k_tile_screen(const JoinArgs<flo
                     const uint32_t ng = min(kTileGrps, groups - (t + u) * kTileGrps);
                     const uint32_t bar = landed + 8u * b;
                     if (sub == u) {
-                        m_base[(g % kMeta) * kTileGrps + half] = gid * kGrp;
+                        // bit 0: the four groups of the aligned quad are consecutive
+                        m_base[(g % kMeta) * kTileGrps + half] = gid * kGrp | ((breaks >> (lane & ~3)) & 0xeu ? 0u : 1u);
                         m_mask[(g % kMeta) * kTileGrps + half] = mask;
                     }
                     __syncwarp();
@@ -581,31 +617,36 @@ __global__ void __launch_bounds__(kSThreads, 2) k_tile_screen(const JoinArgs<flo
                 }
             }
         } else if (warp == kMmaWarp) {
-            // ================= one thread: a landed tile and a free accumulator -> MMA
-            if (lane == 0) {
-                bool ok = true;
-                uint32_t b = g0 % stages, ph = (g0 / stages) & 1u;
-                for (uint32_t t = t0, g = g0; t < t1; t++, g++) {
-                    // the first use of an accumulator waits for the phase before its first
-                    const uint32_t s = g & 1u;
-                    ok = bar_wait_bounded(landed + 8u * b, ph) &&
-                         bar_wait_bounded(empty + 8u * s, ((g >> 1) & 1u) ^ 1u);
-                    if (!ok) break;
-                    fence_after();
-                    const uint32_t bt = b_addr + b * stage_bytes;
-                    for (uint32_t ks = 0; ks < (kpad >> 4); ks++)
-                        mma_bf16(tmem + s * kTmemCols, smem_desc(a_addr + ks * 256u, 128u, sbo),
-                                 smem_desc(bt + ks * 256u, 128u, sbo), ks > 0 ? 1u : 0u);
-                    mma_commit(drained + 8u * b);
+            // ================= a landed tile and a free accumulator -> MMA: the warp stays
+            // converged (waits, descriptors), one elected lane issues
+            bool ok = true;
+            uint32_t b = g0 % stages, ph = (g0 / stages) & 1u;
+            const uint64_t adesc = smem_desc(a_addr, 128u, sbo);
+            const uint32_t ksteps = kpad >> 4;
+            for (uint32_t t = t0, g = g0; t < t1; t++, g++) {
+                // the first use of an accumulator waits for the phase before its first
+                const uint32_t s = g & 1u;
+                ok = warp_wait_bounded(landed + 8u * b, ph) && warp_wait_bounded(empty + 8u * s, ((g >> 1) & 1u) ^ 1u);
+                if (!ok) break;
+                fence_after();
+                const uint64_t bdesc = smem_desc(b_addr + b * stage_bytes, 128u, sbo);
+                const uint32_t acc = tmem + s * kTmemCols;
+                if (elect_one()) {
+                    // a K step is 2 core matrices of 128 bytes on (in units of 16 bytes)
+                    mma_bf16(acc, adesc, bdesc, 0u);
+                    for (uint32_t ks = 1; ks < ksteps; ks++)
+                        mma_bf16(acc, adesc + 16u * ks, bdesc + 16u * ks, 1u);
                     mma_commit(full + 8u * s);
+                    mma_commit(drained + 8u * b);
                     bar_arrive(full + 8u * s);
-                    if (++b == stages) {
-                        b = 0;
-                        ph ^= 1u;
-                    }
                 }
-                if (!ok) misc[1] = 1u;
+                __syncwarp();
+                if (++b == stages) {
+                    b = 0;
+                    ph ^= 1u;
+                }
             }
+            if (!ok) misc[1] = 1u;
             __syncwarp();
         } else {
             // ================= consumer warps: query row i = TMEM lane i; warps w and
@@ -627,82 +668,85 @@ __global__ void __launch_bounds__(kSThreads, 2) k_tile_screen(const JoinArgs<flo
                     if (lane == 0) bar_arrive(empty + 8u * s);
                     continue;
                 }
+                // the accumulator is free as soon as the warp's 64 columns are in registers
+                uint32_t v[64];
+                tmem_ld32(ta, v);
+                tmem_ld32(ta + 32u, v + 32);
+                tmem_wait_ld(v);
+                tmem_named(v + 32);
+                fence_before();
+                __syncwarp();
+                if (lane == 0) bar_arrive(empty + 8u * s);
+                // common case: every value has its sign bit clear (independent chains: one
+                // chain of dependent operations would take several times the issue time)
+                uint32_t x[8];
+#pragma unroll
+                for (int c = 0; c < 8; c++) {
+                    x[c] = v[8 * c];
+#pragma unroll
+                    for (int j = 1; j < 8; j++) x[c] |= v[8 * c + j];
+                }
+                uint32_t signs[2] = {(x[0] | x[1]) | (x[2] | x[3]), (x[4] | x[5]) | (x[6] | x[7])};
+                if (!__any_sync(FULL, (int)(signs[0] | signs[1]) < 0)) continue;
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
-                    uint32_t v[32];
-                    tmem_ld32(ta + 32u * (uint32_t)h, v);
-                    tmem_wait_ld(v);
-                    if (h == 1) {  // the accumulator is read
-                        fence_before();
-                        __syncwarp();
-                        if (lane == 0) bar_arrive(empty + 8u * s);
+                    if (!__any_sync(FULL, (int)signs[h] < 0)) {
+                        signs[h] = 0u;
+                        continue;
                     }
-                    // common case: every value of the 32 columns has its sign bit clear
-                    // (independent chains: one chain of dependent operations would take
-                    // several times the issue time)
-                    uint32_t x[4];
-#pragma unroll
-                    for (int c = 0; c < 4; c++) {
-                        x[c] = v[8 * c];
-#pragma unroll
-                        for (int j = 1; j < 8; j++) x[c] |= v[8 * c + j];
-                    }
-                    if (!__any_sync(FULL, (int)((x[0] | x[1]) | (x[2] | x[3])) < 0)) continue;
-                    const uint32_t mg = (g % kMeta) * kTileGrps + colbase / kGrp + 4u * (uint32_t)h;  // first group
-                    uint32_t und = 0;
+                    signs[h] = 0u;
 #pragma unroll
                     for (int c = 0; c < 4; c++) {
                         uint32_t y = 0;
 #pragma unroll
-                        for (int j = 7; j >= 0; j--) y = __funnelshift_l(v[8 * c + j], y, 1);
-                        und |= y << (8 * c);
+                        for (int j = 7; j >= 0; j--) y = __funnelshift_l(v[32 * h + 8 * c + j], y, 1);
+                        signs[h] |= y << (8 * c);
                     }
-                    und &= *reinterpret_cast<const uint32_t*>(m_mask + mg);
+                }
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const uint32_t mg = (g % kMeta) * kTileGrps + colbase / kGrp + 4u * (uint32_t)h;  // first group
+                    const uint32_t und = signs[h] & *reinterpret_cast<const uint32_t*>(m_mask + mg);
+                    const uint32_t base = m_base[mg];
+                    unsigned have = __ballot_sync(FULL, und != 0u);
+                    if (!have) continue;
                     und_count += (uint32_t)__popc(und);
                     // a record per run of consecutive groups (nearly always all four)
-                    const uint4 gb = *reinterpret_cast<const uint4*>(m_base + mg);
-                    const uint32_t brk = (gb.y != gb.x + kGrp ? 1u : 0u) | (gb.z != gb.y + kGrp ? 2u : 0u) |
-                                         (gb.w != gb.z + kGrp ? 4u : 0u);
-                    for (uint32_t c0 = 0; c0 < 4u;) {
-                        // the run's groups [c0, c1), the slot gs of its first row
-                        const uint32_t cut = brk >> c0;
-                        const uint32_t c1 = cut ? c0 + (uint32_t)__ffs(cut) : 4u;
-                        const uint32_t gs = c0 == 0u ? gb.x : c0 == 1u ? gb.y : c0 == 2u ? gb.z : gb.w;
-                        const uint32_t col0 = kGrp * c0;
-                        const uint32_t mine = und & (0xffffffffu >> (32u - kGrp * c1)) & (0xffffffffu << col0);
-                        c0 = c1;
-                        const unsigned have = __ballot_sync(FULL, mine != 0u);
-                        if (!have) continue;
+                    uint32_t mine = und, gs = base & ~1u, left = 0, next_grp = 4u;
+                    if (!(base & 1u)) {
+                        left = und & 0xffffff00u;
+                        mine = und & 0xffu;
+                        next_grp = 1u;
+                        have = __ballot_sync(FULL, mine != 0u);
+                    }
+                    for (;;) {
+                        // gs: the slot of column 0 (modulo 2^32) for the groups of `mine`
                         const uint32_t cnt = (uint32_t)__popc(have);
                         rec_count += cnt;
-                        if (!o.emit) continue;
-                        // the warp's block first, the rest in the next one
-                        unsigned long long next = 0;
-                        const bool over = blk_used + cnt > kBlk;
-                        if (over) {
-                            if (lane == 0) next = atomicAdd(o.cursor, (unsigned long long)kBlk);
-                            next = __shfl_sync(FULL, next, 0);
-                        }
-                        if (mine) {
-                            uint32_t cross = 0;
-                            if (STAMP) {
-                                // columns outside the query's cell [cs0, ce)
-                                const uint32_t lo = cs0 > gs ? min(32u, col0 + (cs0 - gs)) : col0;
-                                const uint32_t hi = ce > gs ? min(32u, col0 + (ce - gs)) : col0;
-                                const uint32_t below_hi = hi >= 32u ? 0xffffffffu : (1u << hi) - 1u;
-                                const uint32_t below_lo = lo >= 32u ? 0xffffffffu : (1u << lo) - 1u;
-                                cross = ~(below_hi & ~below_lo);
+                        if (o.emit && cnt) {
+                            if (blk_used + cnt > kBlk) {  // the rest of the block stays empty records
+                                for (uint32_t e2 = blk_used + (uint32_t)lane; e2 < blk_room; e2 += 32u)
+                                    blk[e2] = make_uint4(0u, 0u, 0u, 0u);
+                                unsigned long long at = 0;
+                                if (lane == 0) at = atomicAdd(o.cursor, (unsigned long long)kBlk);
+                                at = __shfl_sync(FULL, at, 0);
+                                blk = recs + at;
+                                blk_room = at < o.cap ? (uint32_t)min((unsigned long long)kBlk, o.cap - at) : 0u;
+                                blk_used = 0u;
                             }
                             const uint32_t p = blk_used + (uint32_t)__popc(have & lt);
-                            const unsigned long long at = p < kBlk ? blk_base + p : next + (p - kBlk);
-                            // gs - col0: the slot of column 0 (modulo 2^32)
-                            if (at < o.cap) recs[at] = make_uint4(qslot, gs - col0, mine, cross);
+                            if (mine && p < blk_room) {
+                                uint32_t cross = 0;
+                                if (STAMP) cross = outside_mask(gs, cs0, ce);
+                                blk[p] = make_uint4(qslot, gs, mine, cross);
+                            }
+                            blk_used += cnt;
                         }
-                        blk_used += cnt;
-                        if (over) {
-                            blk_base = next;
-                            blk_used -= kBlk;
-                        }
+                        if (next_grp == 4u) break;
+                        mine = (left >> (kGrp * next_grp) & 0xffu) << (kGrp * next_grp);
+                        gs = (m_base[mg + next_grp] & ~1u) - kGrp * next_grp;
+                        have = __ballot_sync(FULL, mine != 0u);
+                        next_grp++;
                     }
                 }
             }
@@ -716,9 +760,7 @@ __global__ void __launch_bounds__(kSThreads, 2) k_tile_screen(const JoinArgs<flo
     }
     // ---- the consumer warps' last blocks and their counts
     if (tid < kConsumers) {
-        if (o.emit && blk_used < kBlk)
-            for (uint32_t e2 = blk_used + (uint32_t)lane; e2 < kBlk; e2 += 32u)
-                if (blk_base + e2 < o.cap) recs[blk_base + e2] = make_uint4(0u, 0u, 0u, 0u);
+        for (uint32_t e2 = blk_used + (uint32_t)lane; e2 < blk_room; e2 += 32u) blk[e2] = make_uint4(0u, 0u, 0u, 0u);
         if (lane == 0 && *n_und) atomicAdd(o.rechecks, *n_und);
         if (lane == 0 && !o.emit && *n_rec) atomicAdd(o.cursor, *n_rec);
     }

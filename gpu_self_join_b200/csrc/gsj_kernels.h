@@ -159,10 +159,10 @@ ScreenConst make_screen_const(uint32_t n, float thr);
 // Screen pass: the undecided pairs go to o.pairs as 16-byte records {query
 // slot, slot of column 0, mask of 32 columns, mask of the columns outside the
 // query's cell (unicomp)}, in blocks of kScreenBlock records that consumer warps
-// reserve on o.cursor and fill one after another, so that only a warp's last
-// block has unused records (mask 0); o.cap counts records; o.rechecks receives
-// the exact number of undecided pairs.  Without emission o.cursor receives the
-// number of records.
+// reserve on o.cursor and fill one after another; a block's end that cannot take
+// all records of a warp's 32 queries (up to 31) stays unused (mask 0); o.cap
+// counts records; o.rechecks receives the exact number of undecided pairs.
+// Without emission o.cursor receives the number of records.
 constexpr uint32_t kScreenBlock = 256;
 // Keys of the warp join: blocks of kScreenBlockSlack entries, unused tails kUndecidedPad.
 constexpr unsigned long long kUndecidedPad = ~0ull;
