@@ -209,47 +209,34 @@ __device__ __forceinline__ void tmem_named(uint32_t* r) {
                           "+r"(r[j + 6]), "+r"(r[j + 7])::"memory");
 }
 
-// The reference's squared distance in its exact order, one thread, stopping
-// as soon as the running value (which only grows) is above thr.
-template <int MODEL>
-__device__ float exact_sqdist(const float* __restrict__ q, const float* __restrict__ c, uint32_t n, uint32_t ilp,
-                              float thr) {
-    if (MODEL == kSeq || MODEL == kIlpSc) {
-        float s = 0.f;
-        uint32_t p = 0;
-        for (uint32_t l = 0; l < n; l++) {
+// The reference's squared distance of the ILP model without SHORTCIRCUIT (one
+// chain per register over the dims l = j mod ILP, the chains added in order), one
+// thread, stopping as soon as the running value (which only grows) is above thr.
+__device__ float exact_sqdist_ilp(const float* __restrict__ q, const float* __restrict__ c, uint32_t n, uint32_t ilp,
+                                  float thr) {
+    float s = 0.f;
+    for (uint32_t j = 0; j < ilp && j < n; j++) {
+        float r = 0.f;
+        for (uint32_t l = j; l < n; l += ilp) {
             const float d = __fsub_rn(c[l], q[l]);
-            s = (MODEL == kSeq || p == 0) ? __fmaf_rn(d, d, s) : __fadd_rn(s, __fmaf_rn(d, d, 0.f));
-            if (MODEL == kIlpSc && ++p == ilp) p = 0;
-            if (s > thr) break;
+            r = __fmaf_rn(d, d, r);
         }
-        return s;
-    } else {
-        float s = 0.f;
-        for (uint32_t j = 0; j < ilp && j < n; j++) {
-            float r = 0.f;
-            for (uint32_t l = j; l < n; l += ilp) {
-                const float d = __fsub_rn(c[l], q[l]);
-                r = __fmaf_rn(d, d, r);
-            }
-            s = j == 0 ? r : __fadd_rn(s, r);
-            if (s > thr) break;
-        }
-        return s;
+        s = j == 0 ? r : __fadd_rn(s, r);
+        if (s > thr) break;
     }
+    return s;
 }
 
-// Same arithmetic, rows read as float4 blocks of 16 dimensions loaded before
-// use (npad is a multiple of 4 here); the ILP model without SHORTCIRCUIT
-// walks its dimensions with stride ILP and keeps the scalar form.
+// The other models, rows read as float4 blocks of 16 dimensions loaded before use
+// (npad is a multiple of 4, the padding is 0 and adds nothing): the sequential
+// model fuses every term; with SHORTCIRCUIT the terms l = 0 mod ILP are fused,
+// the others rounded and added.  fused[b]: bit e, whether term 16 b + e is.
 template <int MODEL>
-__device__ float exact_sqdist4(const float* __restrict__ q, const float* __restrict__ c, uint32_t n, uint32_t ilp,
-                               float thr) {
-    if (MODEL == kIlp) return exact_sqdist<MODEL>(q, c, n, ilp, thr);
+__device__ __forceinline__ float exact_sqdist4(const float* __restrict__ q, const float* __restrict__ c, uint32_t n,
+                                               const uint32_t* __restrict__ fused, float thr) {
     const float4* q4 = reinterpret_cast<const float4*>(q);
     const float4* c4 = reinterpret_cast<const float4*>(c);
     float s = 0.f;
-    uint32_t p = 0;
     for (uint32_t l0 = 0; l0 < n; l0 += 16u) {
         float4 qa[4], ca[4];
 #pragma unroll
@@ -257,21 +244,19 @@ __device__ float exact_sqdist4(const float* __restrict__ q, const float* __restr
             if (l0 + 4u * b < n) {
                 qa[b] = q4[(l0 >> 2) + b];
                 ca[b] = c4[(l0 >> 2) + b];
-            } else {
-                qa[b] = ca[b] = make_float4(0.f, 0.f, 0.f, 0.f);
             }
         }
+        const uint32_t fm = MODEL == kIlpSc ? fused[l0 >> 4] : 0u;
 #pragma unroll
         for (int b = 0; b < 4; b++) {
+            if (l0 + 4u * b >= n) break;
             const float qv[4] = {qa[b].x, qa[b].y, qa[b].z, qa[b].w};
             const float cv[4] = {ca[b].x, ca[b].y, ca[b].z, ca[b].w};
 #pragma unroll
             for (int e = 0; e < 4; e++) {
-                if (l0 + 4u * b + (uint32_t)e < n) {
-                    const float d = __fsub_rn(cv[e], qv[e]);
-                    s = (MODEL == kSeq || p == 0) ? __fmaf_rn(d, d, s) : __fadd_rn(s, __fmaf_rn(d, d, 0.f));
-                    if (MODEL == kIlpSc && ++p == ilp) p = 0;
-                }
+                const float d = __fsub_rn(cv[e], qv[e]);
+                if (MODEL == kSeq || (fm & (1u << (4 * b + e)))) s = __fmaf_rn(d, d, s);
+                else s = __fadd_rn(s, __fmul_rn(d, d));
             }
         }
         if (s > thr) break;
@@ -818,12 +803,25 @@ cudaError_t launch_screen_one(const JoinArgs<float>& a, const TileOut& o, const 
 // the candidate outside the query's cell) also the reverse pair.  A warp takes
 // 32 records, lists their pairs in shared memory and checks 32 pairs at a time,
 // so that records of one pair and of 32 keep the lanes equally busy.
+// Bound by its instructions (0.75 issued a cycle and scheduler), the order of the
+// model's roundings among them: which terms are fused is a bit mask per 16 dims,
+// and a warp reserves output once for its 32 records.  18-D 5M points (524 M
+// pairs) 23.0 -> 15.6 ms, 8-D 120k 211 -> 124 us, 90-D 515k 3.15 -> 2.96 ms.
 template <int MODEL, bool STAMP>
 __global__ void __launch_bounds__(256, 4) k_screen_recheck(const float* __restrict__ pts, const uint32_t* __restrict__ ids,
                                                         uint32_t n, uint32_t npad, uint32_t ilp, float thr,
                                                         uint32_t npoints, const uint4* __restrict__ recs,
                                                         unsigned long long nrec, const TileOut o) {
     __shared__ uint16_t list[8][1024];  // record lane << 5 | column
+    __shared__ uint32_t fused[8];       // n <= 126
+    if (MODEL == kIlpSc) {
+        if (threadIdx.x < 8u) {
+            uint32_t m = 0;
+            for (uint32_t e = 0; e < 16u; e++) m |= (16u * threadIdx.x + e) % ilp == 0u ? 1u << e : 0u;
+            fused[threadIdx.x] = m;
+        }
+        __syncthreads();
+    }
     const unsigned FULL = 0xffffffffu;
     const unsigned lt = lanemask_lt_s();
     const uint32_t lane = threadIdx.x & 31u;
@@ -851,7 +849,9 @@ __global__ void __launch_bounds__(256, 4) k_screen_recheck(const float* __restri
             const uint32_t crossm = STAMP ? __shfl_sync(FULL, r.w, (int)(e >> 5)) : 0u;
             bool hit = false;
             if (valid && qs < npoints && cs < npoints)
-                hit = exact_sqdist4<MODEL>(pts + (size_t)qs * npad, pts + (size_t)cs * npad, n, ilp, thr) <= thr;
+                hit = (MODEL == kIlp
+                           ? exact_sqdist_ilp(pts + (size_t)qs * npad, pts + (size_t)cs * npad, n, ilp, thr)
+                           : exact_sqdist4<MODEL>(pts + (size_t)qs * npad, pts + (size_t)cs * npad, n, fused, thr)) <= thr;
             // the hits move to the front of the list (behind the entries still to be read)
             const unsigned hb = __ballot_sync(FULL, hit);
             if (hit) wl[nhit + (uint32_t)__popc(hb & lt)] = (uint16_t)e;
