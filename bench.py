@@ -164,10 +164,12 @@ def _roofline(stats: list, N: int, n: int, R: int, w) -> dict:
     paths: the estimate + the pair-emitting pass) and "fill" (ROWS: the fill
     pass; the other paths: pair placement + list sort).  Algorithmic bytes per
     launch (C = candidate evaluations):
-      join_fill   table 4R written, per-query list length, bit-mask offsets,
-                  id and list offset 24N, hit masks C/8 read
+      join_fill   table 4R written, coordinates and per-query data 24N, one
+                  decision bit per candidate C/8 (the passes share no decisions:
+                  the fill repeats the tests in registers, so this term is not
+                  memory traffic)
       join_count  coordinates 4Nn, ids 4N, list lengths 8N (by slot and by id),
-                  hit masks C/8 written
+                  decision bits C/8 (as above)
       join_emit   coordinates 4Nn + ids 4N + 8-byte pair keys 8R
       pair_place  keys 8R read + table 4R + offsets 8N written
     The screen is a tensor-core kernel: 2(n+2) FLOPs per screened pair (one

@@ -10,8 +10,10 @@
 //   index: cell keys -> radix sort -> runs -> cell table -> work items
 //   join, one of four paths (gsj_stats.join_path):
 //     ROWS   (dense, k <= 3, n <= 4): count pass -> list offsets -> fill pass
-//     WARP, TILE, SCREEN: one pass appending packed (query, candidate) keys,
-//       sized by a sampling pass -> radix sort -> table + offsets
+//     WARP, TILE, SCREEN: one pass appending packed (query, candidate) keys
+//       (SCREEN, and TILE unless plain: records of undecided pairs, then the
+//       exact check), sized by a sampling pass or the learned model -> list
+//       lengths, offsets, placement, each list sorted
 // The result stays on the device in the context's pool until fetched.
 #include <cuda_runtime.h>
 
