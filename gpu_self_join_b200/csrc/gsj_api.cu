@@ -1013,7 +1013,7 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
         const T inv_sample = (T)(1.0 / (100 * 1.0));
         const T denom = (T)N * inv_sample;
         S.kernel_launches += 1;
-    GSJ_CUDA(c, launch_variance<T>(d_in, N, n, denom, d_var, st));
+        GSJ_CUDA(c, launch_variance<T>(d_in, N, n, denom, d_var, st));
         std::vector<T> var(n);
         GSJ_TRY(d2h_small(c, var.data(), d_var, n));
         std::vector<dim_reorder_sort<T>> dv(n);

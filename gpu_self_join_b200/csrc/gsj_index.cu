@@ -26,7 +26,9 @@ namespace gsj {
 // chunk of samples, in the second pass already as squared deviations, while the
 // first 8 lanes of warp 0 add the current one from shared memory, 16 values read
 // ahead of the chain.
-// Bound by the additions' latency (4 cycles) and the staging of one block.
+// Bound by the additions' latency (4 cycles) and the staging of one block.  Against
+// one block that staged and added in turn: 18-D 5M points 1.38 -> 0.48 ms, 90-D
+// 515k 460 -> 66 us, 8-D 120k 26 -> 16 us.
 constexpr uint32_t kVarDims = 8, kVarThreads = 1024, kVarUnroll = 16;
 template <typename T>
 constexpr uint32_t kVarChunk = 992u * 4u / sizeof(T);  // samples: 8 (FP32) or 4 loads a thread
