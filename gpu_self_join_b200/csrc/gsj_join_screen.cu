@@ -47,12 +47,12 @@
 // belong to the range; only undecided pairs look at it.
 //
 // Roles: warps 0-7 consume, warp 8 copies candidate tiles (a bulk copy per run of
-// consecutive groups; most tiles are one run), one thread of warp 9 issues the
+// consecutive groups; most tiles are one run), an elected lane of warp 9 issues the
 // MMAs.  Candidate tiles rotate through up to kMaxStages buffers and two
 // accumulators alternate, handed over by mbarriers (landed: a buffer's bytes have
 // arrived; drained: its MMA has read it; full / empty: an accumulator).  Every
-// wait is a bounded poll by one thread whose outcome is shared before any
-// warp-collective; on time-out the error flag is raised and the CTA stops.
+// wait is a bounded poll by a whole warp, whose lanes agree on the outcome; on
+// time-out the error flag is raised and the CTA stops.
 // Tensor memory (2 x 128 columns) is allocated once per CTA; the shared-memory
 // request keeps at most 2 CTAs (512 columns) on an SM; it is released before
 // exit.
@@ -156,12 +156,6 @@ __device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
         : "r"(bar), "r"(parity), "r"(kWaitHintNs)
         : "memory");
     return ok != 0;
-}
-
-__device__ __forceinline__ bool bar_wait_bounded(uint32_t bar, uint32_t parity) {
-    for (uint32_t it = 0; it < kWaitPolls; it++)
-        if (bar_try(bar, parity)) return true;
-    return false;
 }
 
 // The whole warp waits; the outcome is the same for all lanes.

@@ -357,25 +357,6 @@ cudaError_t launch_tile_one(const JoinArgs<float>& a, const TileOut& o, uint32_t
     return cudaGetLastError();
 }
 
-// Packed sorted pairs -> neighbour table + list lengths.  Keys are sorted, so
-// the lanes of a warp that share a query add their count with one atomic.
-__global__ void k_pairs_to_table(const unsigned long long* __restrict__ keys, uint64_t R, uint32_t shift,
-                                 uint32_t* __restrict__ table, uint32_t* __restrict__ counts) {
-    const uint64_t mask = (1ull << shift) - 1ull;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < R; i0 += stride) {
-        const uint64_t i = i0 + threadIdx.x;
-        const bool v = i < R;
-        const unsigned act = __ballot_sync(0xffffffffu, v);
-        if (!v) continue;
-        const unsigned long long kk = keys[i];
-        table[i] = (uint32_t)(kk & mask);
-        const uint32_t q = (uint32_t)(kk >> shift);
-        const unsigned peers = __match_any_sync(act, q);
-        if ((threadIdx.x & 31) == (unsigned)(__ffs(peers) - 1)) atomicAdd(&counts[q], (uint32_t)__popc(peers));
-    }
-}
-
 }  // namespace
 
 bool tile_supported(uint32_t n, uint32_t npad, uint32_t k, int model, uint32_t ilp) {
@@ -399,16 +380,6 @@ cudaError_t launch_tile_join(const JoinArgs<float>& a, const TileOut& o, bool st
         case kIlpSc * 2 + 1: return launch_tile_one<kIlpSc, true>(a, o, nrow, nvisit, num_sms, st);
         default: return cudaErrorInvalidValue;
     }
-}
-
-cudaError_t launch_pairs_to_table(const unsigned long long* keys, uint64_t R, uint32_t shift, uint32_t* table,
-                                  uint32_t* counts, int num_sms, cudaStream_t st) {
-    if (R == 0) return cudaSuccess;
-    uint64_t blocks = (R + 255) / 256;
-    const uint64_t cap = (uint64_t)num_sms * 32;
-    if (blocks > cap) blocks = cap;
-    k_pairs_to_table<<<(unsigned)blocks, 256, 0, st>>>(keys, R, shift, table, counts);
-    return cudaGetLastError();
 }
 
 }  // namespace gsj

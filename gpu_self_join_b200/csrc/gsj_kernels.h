@@ -131,9 +131,6 @@ bool tile_supported(uint32_t n, uint32_t npad, uint32_t k, int model, uint32_t i
 // Visits items 0, stride, ..., (nvisit-1)*stride; a.work_counter must be zero.
 cudaError_t launch_tile_join(const JoinArgs<float>& a, const TileOut& o, bool stamp, int model, uint32_t nvisit,
                              int num_sms, cudaStream_t st);
-// Sorted packed pairs -> table (low bits) and counts[query] += pairs (counts zeroed by the caller).
-cudaError_t launch_pairs_to_table(const unsigned long long* keys, uint64_t R, uint32_t shift, uint32_t* table,
-                                  uint32_t* counts, int num_sms, cudaStream_t st);
 
 // Tensor-core screened tile join (gsj_join_screen.cu): BF16 tcgen05 dot
 // products with a proven rejection bound, exact FP32 check of the rest.
