@@ -33,6 +33,7 @@ EXPORTED_SYMBOLS = (
     "GDSJoinPy_f64", "copyResultIntoPythonArray64", "gsj_list_offsets_noalloc", "gsj_bruteforce_count",
     "gsj_join_host", "gsj_model_train", "gsj_model_reset", "gsj_model_weights", "gsj_model_features",
     "gsj_model_predict", "gsj_model_loss_grad", "gsj_autotune", "gsj_tuning_get", "gsj_tuning_set",
+    "gsj_test_slice_list",
 )
 MODEL_WEIGHTS = 3201
 MODEL_FEATURES = 16
@@ -145,6 +146,7 @@ def lib() -> ctypes.CDLL:
                                ctypes.POINTER(GsjTuning)]
     L.gsj_tuning_get.argtypes = [P, u32, u32, u32, ctypes.POINTER(GsjTuning)]
     L.gsj_tuning_set.argtypes = [P, u32, u32, u32, ctypes.POINTER(GsjTuning)]
+    L.gsj_test_slice_list.argtypes = [P, u32, u64, ctypes.POINTER(u64)]
     L.gsj_model_train.argtypes = [P, u32, P]
     L.gsj_model_reset.argtypes = [P]
     L.gsj_model_weights.argtypes = [P, P, u32, i32]

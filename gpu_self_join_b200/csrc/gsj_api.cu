@@ -155,8 +155,8 @@ bool compareByDimVariance(const dim_reorder_sort<T>& a, const dim_reorder_sort<T
 
 // Scalars of a join in the context's `misc` buffer (at least 512 bytes):
 // min/max per indexed dim (2 kMaxK values of T), then 32-bit words: run count,
-// work counter, error flag, candidate counter (64-bit), pair cursors (2 x
-// 64-bit); the pair placement's error flag and long-list count at words
+// work counter, error flag, candidate counter (64-bit), pair cursors and slice
+// counters (4 x 64-bit); the pair placement's error flag and long-list count at words
 // 4 kMaxK + 20 and + 24, the longest list at + 28 (bytes 240, 256 and 272).
 constexpr size_t kMiscWords = 128;
 
@@ -202,6 +202,10 @@ struct gsj_context {
     // tuned launch shapes by (path, dim, density_log2)
     std::map<std::tuple<uint32_t, uint32_t, uint32_t>, gsj_tuning> tuning;
     const gsj_tuning* forced = nullptr;  // the autotuner's candidate, in place of the table
+    // slices of the warp join's long items: the list's capacity, the slices counted
+    // before the first item (test hooks), those of the last join
+    uint32_t slice_cap = kHeavyCap;
+    uint64_t slices_before = 0, slices_found = 0;
     // last result
     bool have_result = false;
     uint64_t N = 0, R = 0;
@@ -565,15 +569,19 @@ int emit_join(gsj_context* c, JoinArgs<T>& a, uint64_t N, bool stamp, int model,
     const uint64_t warps = (uint64_t)c->num_sms * 128u;
     HeavyList heavy{};
     GSJ_TRY(dev_get(c, c->heavy, kHeavyCap, &heavy.list));
-    heavy.cap = kHeavyCap;
-    heavy.count = reinterpret_cast<uint32_t*>(cursor + 2);
-    heavy.claim = heavy.count + 1;
+    heavy.cap = c->slice_cap;
+    heavy.count = cursor + 2;
+    heavy.claim = reinterpret_cast<uint32_t*>(cursor + 3);
     int nl = 0;
     const uint64_t slack = warps * kScreenBlockSlack;
     auto reset = [&]() -> int {
         GSJ_CUDA(c, cudaMemsetAsync(a.work_counter, 0, 4 * sizeof(uint32_t), st));
         // the cursor and the key count, then the heavy list's counters
-        GSJ_CUDA(c, cudaMemsetAsync(cursor, 0, 3 * sizeof(unsigned long long), st));
+        GSJ_CUDA(c, cudaMemsetAsync(cursor, 0, 4 * sizeof(unsigned long long), st));
+        if (c->slices_before) {  // test hook: a list that some (empty) slices fill already
+            GSJ_CUDA(c, cudaMemsetAsync(heavy.list, 0xff, heavy.cap * sizeof(uint2), st));
+            GSJ_CUDA(c, cudaMemcpyAsync(heavy.count, &c->slices_before, sizeof(uint64_t), cudaMemcpyHostToDevice, st));
+        }
         return GSJ_OK;
     };
     GSJ_CUDA(c, cudaEventRecord(c->tev[2], st));
@@ -613,10 +621,11 @@ int emit_join(gsj_context* c, JoinArgs<T>& a, uint64_t N, bool stamp, int model,
         o.pairs = pairs;
         o.cap = cap;
         GSJ_CUDA(c, launch_join_emit<T>(a, o, heavy, ni, model, stamp, c->num_sms, &nl, st));
-        unsigned long long got[2] = {0, 0};  // entries reserved, keys
-        GSJ_TRY(d2h_small(c, got, cursor, 2));
+        unsigned long long got[3] = {0, 0, 0};  // entries reserved, keys, slices found
+        GSJ_TRY(d2h_small(c, got, cursor, 3));
         used = got[0];
         R = got[1];
+        c->slices_found = got[2];
         if (used <= cap) break;
         if (attempt == 2) return fail(c, GSJ_ERR_STATE, "warp join: pair buffer short at its proven bound");
         c->stats.reruns++;
@@ -1758,6 +1767,15 @@ int gsj_result_device(gsj_context* c, const uint32_t** counts, const uint64_t** 
     if (counts) *counts = static_cast<const uint32_t*>(c->counts.p);
     if (offsets) *offsets = static_cast<const uint64_t*>(c->offsets.p);
     if (table) *table = static_cast<const uint32_t*>(c->table.p);
+    return GSJ_OK;
+}
+
+int gsj_test_slice_list(gsj_context* c, uint32_t cap, uint64_t before, uint64_t* found) {
+    if (!c) return fail(c, GSJ_ERR_INVALID, "null context");
+    if (cap > kHeavyCap) return fail(c, GSJ_ERR_INVALID, "slice list: capacity above the built-in one");
+    if (found) *found = c->slices_found;
+    c->slice_cap = cap ? cap : kHeavyCap;
+    c->slices_before = before;
     return GSJ_OK;
 }
 

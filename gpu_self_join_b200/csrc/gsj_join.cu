@@ -438,7 +438,7 @@ __global__ void __launch_bounds__(256, 4) k_join_reg(const JoinArgs<float> a, ui
         __syncwarp();
     };
 
-    const uint32_t nunits = SLICES ? min(*heavy.count, heavy.cap) : nvisit;
+    const uint32_t nunits = SLICES ? (uint32_t)min(*heavy.count, (unsigned long long)heavy.cap) : nvisit;
     uint32_t* counter = SLICES ? heavy.claim : a.work_counter;
     // one claim at a time, the next one in flight while an item is processed (see k_join)
     uint32_t claim = 0;
@@ -469,13 +469,13 @@ __global__ void __launch_bounds__(256, 4) k_join_reg(const JoinArgs<float> a, ui
             cand_total += (unsigned long long)total * qn;
             if (g_hi > 2u * per) {
                 const uint32_t ns = (g_hi + per - 1u) / per;
-                uint32_t at = 0;
-                if (lane == 0) at = atomicAdd(heavy.count, ns);
+                unsigned long long at = 0;
+                if (lane == 0) at = atomicAdd(heavy.count, (unsigned long long)ns);
                 at = __shfl_sync(FULL, at, 0);
-                const bool fits = at < heavy.cap && ns <= heavy.cap - at;
-                for (uint32_t i = (uint32_t)lane; i < ns; i += 32u)
-                    if (at < heavy.cap && i < heavy.cap - at)
-                        heavy.list[at + i] = make_uint2(fits ? visit : 0xffffffffu, i);
+                const bool fits = at + ns <= heavy.cap;
+                const uint32_t room = at < heavy.cap ? min(ns, heavy.cap - (uint32_t)at) : 0u;
+                for (uint32_t i = (uint32_t)lane; i < room; i += 32u)
+                    heavy.list[at + i] = make_uint2(fits ? visit : 0xffffffffu, i);
                 if (fits) continue;
             }
         }
@@ -604,7 +604,7 @@ static cudaError_t launch_reg(const JoinArgs<float>& a, uint32_t nrow, const Til
     if (e != cudaSuccess) return e;
     k1<<<(unsigned)blocks, threads, smem, st>>>(a, nrow, o, heavy, nvisit);
     // the slices of the heavy items, whose number only the device knows
-    e = warp_grid((const void*)k2, L.total, a.shape_warps, a.shape_per_sm, kHeavyCap, num_sms, threads, smem, blocks);
+    e = warp_grid((const void*)k2, L.total, a.shape_warps, a.shape_per_sm, heavy.cap, num_sms, threads, smem, blocks);
     if (e != cudaSuccess) return e;
     k2<<<(unsigned)blocks, threads, smem, st>>>(a, nrow, o, heavy, nvisit);
     *launches += 2;
@@ -700,7 +700,7 @@ cudaError_t launch_join_emit(const JoinArgs<T>& a, const TileOut& o, const Heavy
                              int model, bool stamp, int num_sms, int* launches, cudaStream_t st) {
     uint32_t nrow = 1;  // neighbour rows: 3^(k-1)
     for (uint32_t j = 1; j < a.g.k; j++) nrow *= 3u;
-    if (o.stride == 0 || !heavy.list || heavy.cap != kHeavyCap || heavy.unit == 0) return cudaErrorInvalidValue;
+    if (o.stride == 0 || !heavy.list || heavy.cap == 0 || heavy.cap > kHeavyCap || heavy.unit == 0) return cudaErrorInvalidValue;
     if (nvisit == 0) return cudaSuccess;
     if ((uint64_t)(nvisit - 1) * o.stride >= a.num_items) return cudaErrorInvalidValue;
     return stamp ? dispatch_model<T, true>(a, model, nrow, o, heavy, nvisit, num_sms, launches, st)

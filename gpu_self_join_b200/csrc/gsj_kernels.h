@@ -61,13 +61,15 @@ cudaError_t launch_iota(uint32_t* out, uint32_t M, cudaStream_t st);
 // and heavy.claim must be zero.  The launcher picks the specialisation.
 struct TileOut;
 // Slices of the items that are too long for one warp: found by the first launch,
-// processed by a second one.
+// processed by a second one.  The items that find the list full are processed
+// where they are found.
 struct HeavyList {
-    uint2* list;      // [cap] (visit, slice)
-    uint32_t* count;  // slices found (may exceed cap; those entries are dropped)
-    uint32_t* claim;  // the second launch's work counter
-    uint32_t cap;
-    uint32_t unit;    // steps of a slice (join_unit_steps)
+    uint2* list;                // [cap] (visit, slice)
+    unsigned long long* count;  // slices found, the dropped ones of a full list included: a
+                                // join may find more than 2^32
+    uint32_t* claim;            // the second launch's work counter
+    uint32_t cap;               // 1 .. kHeavyCap
+    uint32_t unit;              // steps of a slice (join_unit_steps)
 };
 constexpr uint32_t kHeavyCap = 1u << 20;
 uint32_t join_unit_steps(double cand, int num_sms);

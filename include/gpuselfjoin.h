@@ -314,6 +314,14 @@ GSJ_API int gsj_model_predict(gsj_context* ctx, const float* features, uint32_t 
 GSJ_API int gsj_model_loss_grad(gsj_context* ctx, const float* features, const float* targets, uint32_t n,
                                 float* loss, float* grad);
 
+/* ---------------------------------------------------------------- testing
+ * The warp join (GSJ_PATH_WARP, float rows of up to 16 values) cuts its longest
+ * items into slices kept in a list.  For tests: *found (optional) receives the
+ * slices that the last join of ctx counted; later joins of ctx use a list of
+ * `cap` slices (0: the built-in capacity) and count from `before`.  No setting
+ * changes a result. */
+GSJ_API int gsj_test_slice_list(gsj_context* ctx, uint32_t cap, uint64_t before, uint64_t* found);
+
 /* ---------------------------------------------------------------- drop-in
  * The reference's shared-library ABI (built with -DPYTHON, Makefile:58-77).
  *
