@@ -258,6 +258,11 @@ int dev_get(gsj_context* c, Buf& b, size_t count, X** out) {
     return GSJ_OK;
 }
 
+void dev_release(Buf& b) {
+    if (b.p) cudaFree(b.p);
+    b = Buf{};
+}
+
 int pinned_get(gsj_context* c, PinnedBuf& b, size_t bytes) {
     if (b.cap < bytes) {
         if (b.p) cudaFreeHost(b.p);
@@ -644,6 +649,21 @@ int emit_join(gsj_context* c, JoinArgs<T>& a, uint64_t N, bool stamp, int model,
 // data).  A sampling pass over every kSampleStride-th item sizes the pair
 // buffer; the full pass counts every pair even past the buffer, so a short
 // buffer is re-sized to the exact count and the pass repeated.
+//
+// Below 16 dimensions a screen whose bound decides nothing gives up (returns
+// kTakePlain, nothing else done): the bound grows with a point's distance from the
+// data's mean, so clusters hundreds of eps apart, or one sentinel value that moves
+// the mean, leave every candidate undecided.  An undecided pair costs 0.72 npad ps
+// (5.8 at 8 columns, 11.5 at 16), a screened candidate 0.5 and one of the FP32 tiles
+// 0.22 npad (1.8, 3.5); a pair within eps costs about the same either way (8 to 10
+// ps).  So the FP32 tiles win once the undecided pairs that are not within eps
+// exceed a quarter of the candidates.  Measured with the screen / the tiles (ms,
+// undecided share): 8-D 16 ms / 8.4 (1.0), 15-D 29.2 / 9.2 (1.0), 8-D 4.7 / 10.0
+// (0.04), 8-D of pairs mostly within eps 10.3 / 12.2 (0.42).  Below
+// kFewUndecided pairs the exact check takes less than 0.1 ms.
+constexpr int kTakePlain = 1;
+constexpr double kFewUndecided = 16777216.0;
+
 int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int model, bool screen, bool exact_size,
               bool learned, uint32_t* counts, uint64_t* offsets, unsigned long long* cursor, double t_join,
               double t_start) {
@@ -674,7 +694,42 @@ int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int mo
         return screen ? launch_tile_screen(a, o, sc, stamp, model, nvisit, c->num_sms, st)
                       : launch_tile_join(a, o, stamp, model, nvisit, c->num_sms, st);
     };
-    GSJ_CUDA(c, cudaEventRecord(c->tev[2], st));
+    // The sampled items once more, their undecided pairs (about `expect` records)
+    // kept and checked: *useless when the FP32 tiles are the better choice.  The
+    // device counters are the sample's afterwards.
+    const uint32_t nsample = (ni + kSampleStride - 1) / kSampleStride;
+    auto check_bound = [&](double expect, bool* useless) -> int {
+        const uint64_t room = (uint64_t)(expect * 1.25) + slack;
+        uint4* recs = nullptr;
+        GSJ_TRY(dev_get(c, c->pairs, room * 2u, reinterpret_cast<unsigned long long**>(&recs)));
+        GSJ_TRY(reset());
+        o.emit = true;
+        o.stride = kSampleStride;
+        o.pairs = reinterpret_cast<unsigned long long*>(recs);
+        o.cap = room;
+        S.kernel_launches += 2;
+        GSJ_CUDA(c, launch(nsample));
+        unsigned long long got[2] = {0, 0}, C = 0, hits = 0;
+        uint32_t err = 0;
+        Readback rb(c);
+        GSJ_TRY(rb.add(got, cursor, 2));
+        GSJ_TRY(rb.add(&C, cand, 1));
+        GSJ_TRY(rb.add(&err, a.err_flag, 1));
+        GSJ_TRY(rb.wait());
+        if (err) return fail(c, GSJ_ERR_CUDA, "tile join: tensor-core wait timed out");
+        const uint64_t nrec = std::min<uint64_t>(got[0], room);
+        // no room for keys: the pairs within eps are counted only, one direction each
+        TileOut ro = o;
+        ro.pairs = nullptr;
+        ro.cap = 0;
+        GSJ_CUDA(c, cudaMemsetAsync(cursor, 0, sizeof(unsigned long long), st));
+        GSJ_CUDA(c, launch_screen_recheck(a, recs, nrec, ro, false, model, c->num_sms, st));
+        GSJ_TRY(d2h_small(c, &hits, cursor, 1));
+        const double within = nrec ? (double)hits * ((double)got[0] / (double)nrec) : 0.0;
+        *useless = 4.0 * ((double)got[1] - within) > (double)C;
+        return GSJ_OK;
+    };
+    bool guarded = screen && a.n < kScreenPathDims;  // the bound is still to be looked at
     if (screen) {
         // centred BF16 rows of all points, read by every candidate tile
         uint4* rows = nullptr;
@@ -700,21 +755,28 @@ int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int mo
         est_entries = est;
     } else if (!exact_size) {
         // sampled estimator: the exact pass over every kSampleStride-th item
-        const uint32_t nsample = (ni + kSampleStride - 1) / kSampleStride;
         GSJ_TRY(reset());
         o.emit = false;
         o.stride = kSampleStride;
         S.kernel_launches += 1;
         GSJ_CUDA(c, launch(nsample));
         unsigned long long sampled[2] = {0, 0};  // entries, and the screen's undecided pairs
+        unsigned long long C = 0;
         uint32_t err = 0;
         Readback rb(c);
         GSJ_TRY(rb.add(sampled, cursor, 2));
+        GSJ_TRY(rb.add(&C, cand, 1));
         GSJ_TRY(rb.add(&err, a.err_flag, 1));
         GSJ_TRY(rb.wait());
         if (err) return fail(c, GSJ_ERR_CUDA, "tile join: tensor-core wait timed out");
         est_entries = nsample ? (double)sampled[0] * (double)ni / (double)nsample : 0.0;
         est = screen && nsample ? (double)sampled[1] * (double)ni / (double)nsample : est_entries;
+        if (guarded && est >= kFewUndecided && 4.0 * (double)sampled[1] > (double)C) {
+            bool useless = false;
+            GSJ_TRY(check_bound((double)sampled[0], &useless));
+            if (useless) return kTakePlain;
+            guarded = false;
+        }
     }
     GSJ_CUDA(c, cudaEventRecord(c->tev[7], st));
     S.estimate = (uint64_t)est;
@@ -736,15 +798,24 @@ int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int mo
         S.kernel_launches += 1;
         GSJ_CUDA(c, launch(ni));
         // entries written (pairs), or reserved (records)
-        unsigned long long got[2] = {0, 0};
+        unsigned long long got[2] = {0, 0}, C = 0;
         uint32_t err = 0;
         Readback rb(c);
         GSJ_TRY(rb.add(got, cursor, 2));
+        GSJ_TRY(rb.add(&C, cand, 1));
         GSJ_TRY(rb.add(&err, a.err_flag, 1));
         GSJ_TRY(rb.wait());
         used = got[0];
         U = screen ? got[1] : used;
         if (err) return fail(c, GSJ_ERR_CUDA, "tile join: tensor-core wait timed out");
+        if (guarded && (double)U >= kFewUndecided && 4.0 * (double)U > (double)C) {
+            // no sampling pass was run, or its few items did not show it
+            bool useless = false;
+            GSJ_TRY(check_bound((double)used / kSampleStride, &useless));
+            if (useless) return kTakePlain;
+            guarded = false;
+            GSJ_CUDA(c, cudaMemcpyAsync(cand, &C, sizeof(C), cudaMemcpyHostToDevice, st));
+        }
         if (used <= cap) {
             nlist = used;
             break;
@@ -774,6 +845,54 @@ int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int mo
     S.join_path = a.n >= kScreenPathDims && screen ? GSJ_PATH_SCREEN : GSJ_PATH_TILE;
     S.ms_join = now_ms() - t_join;
     S.ms_total = now_ms() - t_start;
+    return GSJ_OK;
+}
+
+// ------------------------------------------------------------------ work items
+// Chunks of up to `qchunk` consecutive query slots of one cell, in cell order or
+// (QUERYREORDER) heaviest cells first, GPU.cu:1491-1525.
+int work_items(gsj_context* c, bool query_reorder, const uint32_t* cell_start, uint32_t M, uint32_t qchunk,
+               uint2** items, uint32_t* num_items) {
+    gsj_stats& S = c->stats;
+    cudaStream_t st = c->st;
+    uint32_t *order = nullptr, *nchunks = nullptr, *item_off = nullptr;
+    void* temp = nullptr;
+    GSJ_TRY(dev_get(c, c->nchunks, M + 1, &nchunks));
+    GSJ_TRY(dev_get(c, c->item_off, M + 1, &item_off));
+    if (query_reorder) {
+        uint32_t *sizes = nullptr, *sizes2 = nullptr, *iota = nullptr;
+        GSJ_TRY(dev_get(c, c->sizes, 2 * (size_t)M, &sizes));
+        sizes2 = sizes + M;
+        GSJ_TRY(dev_get(c, c->order, 2 * (size_t)M, &order));
+        iota = order + M;
+        // stable descending sort by cell size (ties keep ascending cell order):
+        // an ascending sort of the complemented sizes
+        S.kernel_launches += 2;
+        GSJ_CUDA(c, launch_item_counts(cell_start, nullptr, M, qchunk, nchunks, sizes, st));
+        GSJ_CUDA(c, launch_iota(iota, M, st));
+        GSJ_TRY(dev_get(c, c->temp, radix_sort_temp_bytes(M), (unsigned char**)&temp));
+        bool alt = false;
+        int nl = 0;
+        GSJ_CUDA(c, radix_sort<uint32_t>(sizes, sizes2, iota, order, M, 0, 32, temp, &alt, &nl, st));
+        S.kernel_launches += (uint64_t)nl;
+        if (!alt) {
+            // the sorted cell indices are in iota (order + M): move them to order[0, M)
+            GSJ_CUDA(c, cudaMemcpyAsync(order, iota, (size_t)M * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
+        }
+        S.kernel_launches += 1;
+        GSJ_CUDA(c, launch_item_counts(cell_start, order, M, qchunk, nchunks, nullptr, st));
+    } else {
+        S.kernel_launches += 1;
+        GSJ_CUDA(c, launch_item_counts(cell_start, nullptr, M, qchunk, nchunks, nullptr, st));
+    }
+    GSJ_TRY(dev_get(c, c->temp, scan_u32_u64_temp_bytes(M), (unsigned char**)&temp));
+    S.kernel_launches += (uint64_t)scan_launches(M);
+    GSJ_CUDA(c, scan_u32_u32(nchunks, item_off, M, temp, st));
+    GSJ_TRY(d2h_small(c, num_items, item_off + M, 1));
+    S.work_items = *num_items;
+    GSJ_TRY(dev_get(c, c->items, *num_items, items));
+    S.kernel_launches += 1;
+    GSJ_CUDA(c, launch_make_items(order, nchunks, item_off, M, *items, st));
     return GSJ_OK;
 }
 
@@ -1254,52 +1373,12 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
         }
     }
 
-    // ---- work items (QUERYREORDER: heaviest cells first, GPU.cu:1491-1525).
-    // The ROWS path has none: its passes claim 32 consecutive query slots at a
-    // time, and the order in which queries run changes no result.
+    // ---- work items.  The ROWS path has none: its passes claim 32 consecutive
+    // query slots at a time, and the order in which queries run changes no result.
     uint32_t num_items = 0;
     uint2* items = nullptr;
-    if (tpq) {
-        S.work_items = ((uint64_t)N + 31u) / 32u;
-    } else {
-        uint32_t *order = nullptr, *nchunks = nullptr, *item_off = nullptr;
-        GSJ_TRY(dev_get(c, c->nchunks, M + 1, &nchunks));
-        GSJ_TRY(dev_get(c, c->item_off, M + 1, &item_off));
-        if (cfg.query_reorder) {
-            uint32_t *sizes = nullptr, *sizes2 = nullptr, *iota = nullptr;
-            GSJ_TRY(dev_get(c, c->sizes, 2 * (size_t)M, &sizes));
-            sizes2 = sizes + M;
-            GSJ_TRY(dev_get(c, c->order, 2 * (size_t)M, &order));
-            iota = order + M;
-            // stable descending sort by cell size (ties keep ascending cell order):
-            // an ascending sort of the complemented sizes
-            S.kernel_launches += 2;
-            GSJ_CUDA(c, launch_item_counts(cell_start, nullptr, M, qchunk, nchunks, sizes, st));
-            GSJ_CUDA(c, launch_iota(iota, M, st));
-            GSJ_TRY(dev_get(c, c->temp, radix_sort_temp_bytes(M), (unsigned char**)&temp));
-            bool alt = false;
-            int nl2 = 0;
-            GSJ_CUDA(c, radix_sort<uint32_t>(sizes, sizes2, iota, order, M, 0, 32, temp, &alt, &nl2, st));
-            S.kernel_launches += (uint64_t)nl2;
-            if (!alt) {
-                // the sorted cell indices are in iota (order + M): move them to order[0, M)
-                GSJ_CUDA(c, cudaMemcpyAsync(order, iota, (size_t)M * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
-            }
-            S.kernel_launches += 1;
-            GSJ_CUDA(c, launch_item_counts(cell_start, order, M, qchunk, nchunks, nullptr, st));
-        } else {
-            S.kernel_launches += 1;
-            GSJ_CUDA(c, launch_item_counts(cell_start, nullptr, M, qchunk, nchunks, nullptr, st));
-        }
-        GSJ_TRY(dev_get(c, c->temp, scan_u32_u64_temp_bytes(M), (unsigned char**)&temp));
-        S.kernel_launches += (uint64_t)scan_launches(M);
-        GSJ_CUDA(c, scan_u32_u32(nchunks, item_off, M, temp, st));
-        GSJ_TRY(d2h_small(c, &num_items, item_off + M, 1));
-        S.work_items = num_items;
-        GSJ_TRY(dev_get(c, c->items, num_items, &items));
-        S.kernel_launches += 1;
-        GSJ_CUDA(c, launch_make_items(order, nchunks, item_off, M, items, st));
-    }
+    if (tpq) S.work_items = ((uint64_t)N + 31u) / 32u;
+    else GSJ_TRY(work_items(c, cfg.query_reorder != 0, cell_start, M, qchunk, &items, &num_items));
     GSJ_CUDA(c, cudaEventRecord(c->tev[1], st));
     const double t_join = now_ms();
     S.ms_index = t_join - t_index;
@@ -1355,7 +1434,23 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     if constexpr (std::is_same<T, float>::value) {
         if (tile) {
             unsigned long long* cursor = reinterpret_cast<unsigned long long*>(ctr + 4);
-            return tile_join(c, a, N, stamp, model, screen, exact_size, learned, counts, offsets, cursor, t_join,
+            GSJ_CUDA(c, cudaEventRecord(c->tev[2], st));
+            if (screen) {
+                const int r = tile_join(c, a, N, stamp, model, true, exact_size, learned, counts, offsets, cursor, t_join,
+                                        t_start);
+                if (r != kTakePlain && r != GSJ_ERR_NOMEM) return r;
+                // the bound decides nothing, or the undecided pairs do not fit: the FP32
+                // tiles, which need room for the result pairs alone
+                if (r == GSJ_ERR_NOMEM) {
+                    c->err.clear();
+                    dev_release(c->unc);
+                    dev_release(c->pairs);
+                }
+                GSJ_TRY(work_items(c, cfg.query_reorder != 0, cell_start, M, (uint32_t)kTileQ, &items, &num_items));
+                a.items = items;
+                a.num_items = num_items;
+            }
+            return tile_join(c, a, N, stamp, model, false, exact_size, learned, counts, offsets, cursor, t_join,
                              t_start);
         }
     }

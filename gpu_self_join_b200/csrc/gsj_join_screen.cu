@@ -752,7 +752,7 @@ __global__ void __launch_bounds__(kSThreads, 2) k_tile_screen(const JoinArgs<flo
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2u * kTmemCols)
                      : "memory");
-    if (tid == 0 && o.emit && cand_total) atomicAdd(a.cand_cnt, cand_total);
+    if (tid == 0 && cand_total) atomicAdd(a.cand_cnt, cand_total);
 }
 
 template <bool STAMP>
