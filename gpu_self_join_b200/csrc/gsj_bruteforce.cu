@@ -72,7 +72,7 @@ cudaError_t launch_bruteforce(const T* pts, uint32_t N, uint32_t n, T thr, uint3
     if (rows == 0) return cudaErrorInvalidValue;
     const size_t smem = (size_t)rows * row_bytes;
     auto kern = k_bruteforce<T, POL>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem((const void*)kern, smem);
     if (e != cudaSuccess) return e;
     const uint32_t blocks = (N + kBfThreads - 1) / kBfThreads;
     kern<<<blocks, kBfThreads, smem, st>>>(pts, N, n, thr, rows, counts, total);

@@ -552,7 +552,7 @@ static cudaError_t warp_grid(const void* kern, uint32_t per_warp, const uint32_t
     if (warps < 1) return cudaErrorInvalidValue;
     threads = warps * 32;
     smem = (size_t)warps * per_warp;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = blocks_per_sm(kern, threads, smem, &per_sm);

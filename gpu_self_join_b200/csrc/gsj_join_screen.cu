@@ -765,7 +765,7 @@ cudaError_t launch_screen_one(const JoinArgs<float>& a, const TileOut& o, const 
     while (stages < kMaxStages && screen_smem(sc.kpad, nrow, stages + 1u).total <= two) stages++;
     const ScreenSmem L = screen_smem(sc.kpad, nrow, stages);
     const uint32_t smem = L.total > kMinSmem ? L.total : kMinSmem;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem((const void*)kern, smem);
     if (e != cudaSuccess) return e;
     // the whole unified L1/shared array as shared memory, so that the CTAs the
     // occupancy calculation counts on are resident together

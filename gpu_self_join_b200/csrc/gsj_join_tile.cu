@@ -340,7 +340,7 @@ cudaError_t launch_tile_one(const JoinArgs<float>& a, const TileOut& o, uint32_t
                             cudaStream_t st) {
     auto kern = k_tile_join<MODEL, STAMP>;
     const TileSmem L = tile_smem(a.npad, nrow);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total);
+    cudaError_t e = allow_smem((const void*)kern, L.total);
     if (e != cudaSuccess) return e;
     // the whole unified L1/shared array as shared memory, so that the CTAs the
     // occupancy calculation counts on are resident together

@@ -14,6 +14,11 @@ namespace gsj {
 // since the calculation can come out below what the SM holds.  Results are
 // cached per (device, kernel, block size, dynamic shared memory).
 cudaError_t blocks_per_sm(const void* kern, int threads, size_t smem, int* per_sm);
+// Lets launches of `kern` take up to the device's limit of dynamic shared memory
+// (an error when `smem` is above it).  The attribute belongs to the kernel, not to
+// a launch: set to each launch's own size, another thread's context could lower
+// it between this thread's setting and launch, which then failed.
+cudaError_t allow_smem(const void* kern, size_t smem);
 
 
 template <typename T>

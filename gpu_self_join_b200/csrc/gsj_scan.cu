@@ -199,6 +199,20 @@ cudaError_t blocks_per_sm(const void* kern, int threads, size_t smem, int* per_s
     return cudaSuccess;
 }
 
+cudaError_t allow_smem(const void* kern, size_t smem) {
+    int dev = 0, optin = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e != cudaSuccess) return e;
+    cudaFuncAttributes fa{};
+    e = cudaFuncGetAttributes(&fa, kern);
+    if (e != cudaSuccess) return e;
+    const int limit = optin - (int)fa.sharedSizeBytes;
+    if (limit < 0 || smem > (size_t)limit) return cudaErrorInvalidValue;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+}
+
 // ---------------------------------------------------------------- no allocation
 // Scratch of gsj_list_offsets_noalloc: the per-tile sums of the scan live in
 // a fixed array in the library's device image instead of memory obtained
