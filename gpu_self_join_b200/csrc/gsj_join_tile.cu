@@ -96,7 +96,14 @@ __device__ __forceinline__ void tile_dists(const float* __restrict__ qs, const f
         // kSeq: s = fma(d, d, s) over l.  kIlpSc (kernel.cu:320-334): the first
         // dim of every ILP block is fused into s, the others are squared on
         // their own and added.
+        // Four dims a trip: how far the compiler unrolled by itself depended on the code
+        // around the loop, and with the neighbour rows in place of the cells it did
+        // worse (ms of the pass, cells / rows / rows with four a trip): 18-D 300k ILP 8
+        // with SHORTCIRCUIT 21.7 / 23.3 / 20.9, 90-D 100k 24.4 / 26.4 / 23.4, 128-D 50k
+        // 27.5 / 30.1 / 26.1, sequential 18-D 23.9 / 23.5 / 21.6, 12-D 16.3 / 15.9 / 14.7;
+        // two a trip 21.2, 23.7, 26.0, 23.2, 15.8.
         uint32_t p = 0;
+#pragma unroll 4
         for (uint32_t l = 0; l < n; l++) {
             const float4 qa = *reinterpret_cast<const float4*>(qs + (size_t)l * kTQ + ty * 4);
             const float4 ca = *reinterpret_cast<const float4*>(cs + (size_t)l * kTC + tx * 4);
