@@ -1021,7 +1021,8 @@ int rows_to_host(gsj_context* c, JoinArgs<T>& a, const gsj_config& cfg, uint64_t
         a.table = seg;
         GSJ_CUDA(c, cudaMemsetAsync(ctr, 0, sizeof(uint32_t), st));
         S.kernel_launches += 1;
-        GSJ_CUDA(c, launch_rows_fill<T>(a, slot_cell, qslots + h_gs[b], h_gs[b + 1] - h_gs[b], h_bo[b], c->num_sms, st));
+        GSJ_CUDA(c, launch_rows_fill<T>(a, slot_cell, qslots + h_gs[b], h_gs[b + 1] - h_gs[b], h_bo[b], R, S.candidates,
+                                        c->num_sms, st));
         GSJ_CUDA(c, cudaEventRecord(c->seg_filled[sg], st));
         const uint64_t rb = h_bo[b + 1] - h_bo[b];
         GSJ_CUDA(c, cudaStreamWaitEvent(c->cst[sg], c->seg_filled[sg], 0));
@@ -1513,7 +1514,7 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     a.err_flag = ctr + 1;  // zeroed with the counters before the count pass
     GSJ_CUDA(c, cudaEventRecord(c->tev[4], st));
     S.kernel_launches += 1;
-    GSJ_CUDA(c, launch_rows_fill<T>(a, slot_cell, nullptr, (uint32_t)N, 0, c->num_sms, st));
+    GSJ_CUDA(c, launch_rows_fill<T>(a, slot_cell, nullptr, (uint32_t)N, 0, R, ncand, c->num_sms, st));
     GSJ_CUDA(c, cudaEventRecord(c->tev[5], st));
     uint32_t errflag = 0, nlong[2] = {0, 0};
     // every list ascending

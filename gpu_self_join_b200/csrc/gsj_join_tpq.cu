@@ -26,6 +26,13 @@
 // double 250k 0.120 + 0.126 -> 0.080 + 0.101 ms.  Four CTAs an SM (64 registers)
 // for float: 2-D 20M 3.03 / 2.80 / 3.01 / 2.80 ms with 3 / 4 / 5 / 6; double
 // spills there (3-D 250k 0.101 / 0.114 with 2 / 4).
+//
+// Sparse cells leave most of a warp's lanes without a candidate and pay the cell's
+// set-up for one or two queries: k_rows_thread, a thread per query, takes their
+// count and, for short lists, their fill (launch_rows has the lines and both sides).
+// Against the passes with masks, whole joins on the device: 3-D double 5M points at 1.6 a cell 1.87
+// -> 1.29 ms, 2-D 10M at 1.2 2.08 -> 1.68, 4-D with 2 dims indexed 500k at 600 2.99 ->
+// 2.68; 2-D at 2 to 3 points a cell is 4 % above them.
 // The chunks are claimed dynamically (one atomic per warp, the next claim
 // issued before the current chunk is processed), since chunk costs vary with the
 // local density by orders of magnitude.
@@ -91,6 +98,10 @@ __device__ __forceinline__ double quiet_nan<double>() {
     return __longlong_as_double(0x7fffffffffffffffll);
 }
 
+// k_rows_join's passes: the count, and the fill where many or few of the candidates
+// are within eps.
+enum RowsPass : int { kCountOnly = 0, kFill = 1, kFillFew = 2 };
+
 // Where a query's list goes: read back with one 16-byte broadcast.
 struct alignas(16) FillList {
     unsigned long long dst;
@@ -101,7 +112,7 @@ struct alignas(16) FillList {
 // Count pass: counts_by_id[id] = list length.  Fill pass: the list of point id i
 // goes to a.table[offsets[i] - base]; a list that would leave the table or
 // differ from its counted length raises *err_flag and is not written past it.
-template <typename T, int NT, int NR, int POL, bool FILL>
+template <typename T, int NT, int NR, int POL, int FILL>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_rows_join(const JoinArgs<T> a, const uint32_t* __restrict__ slot_cell,
                                                    uint32_t* __restrict__ counts_by_id,
                                                    const uint32_t* __restrict__ qslots, uint32_t nq, uint64_t base) {
@@ -187,7 +198,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_rows_join(const
                     if (f0 + 32u * (uint32_t)t < total) {
                         const uint32_t slot = in ? f + d : s;
                         load_row<T, NT>(a.pts + (size_t)slot * npad, cx[t]);
-                        if (FILL) cid[t] = a.ids[slot];
+                        if (FILL) cid[t] = FILL == kFillFew ? slot : a.ids[slot];
                         if (!in) cx[t][0] = quiet_nan<T>();  // within no threshold
                     }
                 }
@@ -198,6 +209,12 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_rows_join(const
                         T q[NT];
 #pragma unroll
                         for (int l = 0; l < NT; l++) q[l] = sq[warp][j * NT + l];
+                        if (FILL == kFillFew) {
+                            bool any = false;
+#pragma unroll
+                            for (int t = 0; t < W; t++) any |= sqdist_seq_reg<T, NT, POL>(q, cx[t]) <= thr;
+                            if (!__any_sync(FULL, any)) continue;
+                        }
                         uint32_t rj = f0 ? __shfl_sync(FULL, run, (int)j) : 0u;
                         FillList fl{};
                         if (FILL) fl = slist[FILL ? warp : 0][j];
@@ -208,7 +225,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_rows_join(const
                             const unsigned b = __ballot_sync(FULL, hit);
                             if (FILL) {
                                 const uint32_t pos = rj + (uint32_t)__popc(b & lt);
-                                if (hit && pos < fl.len) list[pos] = cid[t];
+                                if (hit && pos < fl.len) list[pos] = FILL == kFillFew ? a.ids[cid[t]] : cid[t];
                             }
                             rj += (uint32_t)__popc(b);
                         }
@@ -232,43 +249,59 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_rows_join(const
     if (!FILL && lane == 0 && cand) atomicAdd(a.cand_cnt, cand);
 }
 
-// Count pass with a thread per query: the slots of a warp are consecutive in
-// cell order, so lanes of one cell walk the same ranges (broadcast loads).
-template <typename T, int NT, int NR, int POL>
-__global__ void __launch_bounds__(256) k_rows_count(const JoinArgs<T> a, const uint32_t* __restrict__ slot_cell,
-                                                    uint32_t* __restrict__ counts_by_id) {
+// A thread per query: the slots of a warp are consecutive in cell order, so lanes
+// of one cell walk the same ranges (broadcast loads).  Passes as for k_rows_join.
+template <typename T, int NT, int NR, int POL, bool FILL>
+__global__ void __launch_bounds__(256) k_rows_thread(const JoinArgs<T> a, const uint32_t* __restrict__ slot_cell,
+                                                     uint32_t* __restrict__ counts_by_id,
+                                                     const uint32_t* __restrict__ qslots, uint32_t nq, uint64_t base) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    const uint32_t N = a.n_points;
     const uint32_t npad = a.npad;
     const T thr = a.thr;
     unsigned long long cand = 0;
     uint32_t cur = __shfl_sync(FULL, claim32(a.work_counter, lane), 0);
-    while (cur < N) {
+    while (cur < nq) {
         const uint32_t nxt = claim32(a.work_counter, lane);  // in flight while this chunk runs
-        const uint32_t s = cur + (uint32_t)lane;
-        if (s < N) {
+        const uint32_t i = cur + (uint32_t)lane;
+        if (i < nq) {
+            const uint32_t s = FILL && qslots ? qslots[i] : i;
             const uint32_t cell = slot_cell[s];
+            const uint32_t id = a.ids[s];
             T q[NT];
             load_row<T, NT>(a.pts + (size_t)s * npad, q);
-            uint32_t cnt = 0;
+            uint32_t cnt = 0, len = 0;
+            uint32_t* list = nullptr;
+            if (FILL) {
+                const unsigned long long dst = a.offsets[id] - base;
+                len = (uint32_t)(a.offsets[id + 1] - a.offsets[id]);
+                if (dst + len > a.table_cap) {
+                    *a.err_flag = 1u;
+                    len = 0u;
+                }
+                list = a.table + dst;
+            }
 #pragma unroll
             for (int r = 0; r < NR; r++) {
                 const uint2 e = a.plan[(size_t)cell * NR + r];
                 const T* cp = a.pts + (size_t)e.x * npad;
-                cand += e.y;
+                if (!FILL) cand += e.y;
 #pragma unroll 4
                 for (uint32_t u = 0; u < e.y; u++) {
                     T cr[NT];
                     load_row<T, NT>(cp, cr);
                     cp += npad;
-                    cnt += sqdist_seq_reg<T, NT, POL>(q, cr) <= thr ? 1u : 0u;
+                    const bool hit = sqdist_seq_reg<T, NT, POL>(q, cr) <= thr;
+                    if (FILL && hit && cnt < len) list[cnt] = a.ids[e.x + u];
+                    cnt += hit ? 1u : 0u;
                 }
             }
-            counts_by_id[a.ids[s]] = cnt;
+            if (!FILL) counts_by_id[id] = cnt;
+            else if (cnt != len) *a.err_flag = 1u;
         }
         cur = __shfl_sync(FULL, nxt, 0);
     }
+    if (FILL) return;
     // one atomic per warp for the candidate statistic
     for (int o = 16; o > 0; o >>= 1) cand += __shfl_down_sync(FULL, cand, o);
     if (lane == 0 && cand) atomicAdd(a.cand_cnt, cand);
@@ -281,28 +314,11 @@ static int resident_blocks(const void* kern, int threads, size_t smem, int num_s
     return num_sms * per_sm;
 }
 
-template <typename T, int NT, int NR, bool FILL>
-static cudaError_t launch_rows(const JoinArgs<T>& a, const uint32_t* slot_cell, uint32_t* counts_by_id,
+// Launches one of the forms over nq queries.
+template <typename T, typename K>
+static cudaError_t launch_form(K kern, const JoinArgs<T>& a, const uint32_t* slot_cell, uint32_t* counts_by_id,
                                const uint32_t* qslots, uint32_t nq, uint64_t base, int num_sms, cudaStream_t st) {
-    constexpr int POL = sizeof(T) == 8 ? kPolF64 : kPolF32;
     const int threads = a.shape_threads ? (int)a.shape_threads : 256;
-    if constexpr (!FILL) {
-        // Sparse cells leave the lanes of k_rows_join's cells half empty and pay its
-        // set-up for few queries; from about 7 points a cell on (5 in double) the
-        // cell form is faster.  Count pass, cell form against thread per query: 2-D
-        // 20M at 3.1 points a cell 1.76 / 0.93 ms, 3-D 2M at 7.3 0.349 / 0.357,
-        // 3-D 250k double at 7.0 0.082 / 0.113, 3-D 2M with 2 dims indexed at 175
-        // 1.46 / 1.68.
-        if (a.n_points < (sizeof(T) == 8 ? 5u : 7u) * (uint64_t)a.num_cells) {
-            auto kern = k_rows_count<T, NT, NR, POL>;
-            uint64_t blocks = (uint64_t)resident_blocks((const void*)kern, threads, 0, num_sms);
-            const uint64_t needed = ((uint64_t)nq + threads - 1) / threads;
-            if (blocks > needed) blocks = needed ? needed : 1;
-            kern<<<(unsigned)blocks, threads, 0, st>>>(a, slot_cell, counts_by_id);
-            return cudaGetLastError();
-        }
-    }
-    auto kern = k_rows_join<T, NT, NR, POL, FILL>;
     uint64_t blocks = (uint64_t)resident_blocks((const void*)kern, threads, 0, num_sms);
     const uint64_t needed = ((uint64_t)nq + threads - 1) / threads;
     if (blocks > needed) blocks = needed ? needed : 1;
@@ -310,47 +326,93 @@ static cudaError_t launch_rows(const JoinArgs<T>& a, const uint32_t* slot_cell, 
     return cudaGetLastError();
 }
 
+template <typename T, int NT, int NR, bool FILL>
+static cudaError_t launch_rows(const JoinArgs<T>& a, const uint32_t* slot_cell, uint32_t* counts_by_id,
+                               const uint32_t* qslots, uint32_t nq, uint64_t base, uint64_t pairs, uint64_t cands,
+                               int num_sms, cudaStream_t st) {
+    constexpr int POL = sizeof(T) == 8 ? kPolF64 : kPolF32;
+    if constexpr (!FILL) {
+        // Sparse cells leave the lanes of k_rows_join's cells half empty and pay its
+        // set-up for few queries; from about 7 points a cell on (5 in double) the
+        // cell form is faster.  Count pass, cell form against thread per query: 2-D
+        // 20M at 3.1 points a cell 1.76 / 0.93 ms, 3-D 2M at 7.3 0.349 / 0.357,
+        // 3-D 250k double at 7.0 0.082 / 0.113, 3-D 2M with 2 dims indexed at 175
+        // 1.46 / 1.68.
+        if (a.n_points < (sizeof(T) == 8 ? 5u : 7u) * (uint64_t)a.num_cells)
+            return launch_form<T>(k_rows_thread<T, NT, NR, POL, false>, a, slot_cell, counts_by_id, qslots, nq, base,
+                                  num_sms, st);
+        return launch_form<T>(k_rows_join<T, NT, NR, POL, kCountOnly>, a, slot_cell, counts_by_id, qslots, nq, base,
+                              num_sms, st);
+    } else {
+        const uint64_t N = a.n_points;
+        // Fill pass, cell form against thread per query (ms): 2-D 4M points, 1.6 a cell
+        // and 4.1 result pairs a point 0.497 / 0.277, 2.3 and 7.3 0.402 / 0.418, 3.2 and
+        // 10.4 0.361 / 0.542; 3-D 2M at 1.6 and 5.2 0.359 / 0.201, 3.1 and 13.4 0.369 /
+        // 0.348, 4.0 and 17.5 0.403 / 0.437 (double 1.6 0.620 / 0.262); 1-D 4M at 2.3
+        // and 5.2 0.324 / 0.292, 4.1 and 9.2 0.259 / 0.482.  So sparse cells (the count
+        // pass's line) take a thread per query while it stores few ids, each to a sector
+        // of its own; with many candidates a point (4-D 500k, 130 of them and 1.5 pairs:
+        // 0.145 / 0.148, double 0.162 / 0.195) the cell form is the better one again.
+        if (N < (sizeof(T) == 8 ? 5u : 7u) * (uint64_t)a.num_cells && pairs <= (NR == 1 ? 6u : 4u + NR) * N &&
+            cands <= 96u * N)
+            return launch_form<T>(k_rows_thread<T, NT, NR, POL, true>, a, slot_cell, counts_by_id, qslots, nq, base,
+                                  num_sms, st);
+        // Where few candidates are within eps one vote a query skips four tiles, and an id
+        // is loaded for a hit alone.  Every candidate's id / the hits' ids, by the share
+        // of hits: 4-D 500k 0.0009 2.36 / 1.23 ms, 0.0084 0.348 / 0.286, 0.0117 0.145 /
+        // 0.144, 0.022 0.068 / 0.070, 2-D 4M 0.36 0.46 / 0.54; double 4-D 0.0009 2.64 /
+        // 2.21, 2-D 0.0021 0.247 / 0.213, 0.0044 2.22 / 2.24, 0.0084 0.334 / 0.392.
+        if (pairs * (sizeof(T) == 8 ? 256u : 64u) < cands)
+            return launch_form<T>(k_rows_join<T, NT, NR, POL, kFillFew>, a, slot_cell, counts_by_id, qslots, nq, base,
+                                  num_sms, st);
+        return launch_form<T>(k_rows_join<T, NT, NR, POL, kFill>, a, slot_cell, counts_by_id, qslots, nq, base,
+                              num_sms, st);
+    }
+}
+
 template <typename T, int NR, bool FILL>
 static cudaError_t rows_nr(const JoinArgs<T>& a, const uint32_t* slot_cell, uint32_t* counts_by_id,
-                           const uint32_t* qslots, uint32_t nq, uint64_t base, int num_sms, cudaStream_t st) {
+                           const uint32_t* qslots, uint32_t nq, uint64_t base, uint64_t pairs, uint64_t cands,
+                           int num_sms, cudaStream_t st) {
     switch (a.n) {
-        case 1: return launch_rows<T, 1, NR, FILL>(a, slot_cell, counts_by_id, qslots, nq, base, num_sms, st);
-        case 2: return launch_rows<T, 2, NR, FILL>(a, slot_cell, counts_by_id, qslots, nq, base, num_sms, st);
-        case 3: return launch_rows<T, 3, NR, FILL>(a, slot_cell, counts_by_id, qslots, nq, base, num_sms, st);
-        case 4: return launch_rows<T, 4, NR, FILL>(a, slot_cell, counts_by_id, qslots, nq, base, num_sms, st);
+        case 1: return launch_rows<T, 1, NR, FILL>(a, slot_cell, counts_by_id, qslots, nq, base, pairs, cands, num_sms, st);
+        case 2: return launch_rows<T, 2, NR, FILL>(a, slot_cell, counts_by_id, qslots, nq, base, pairs, cands, num_sms, st);
+        case 3: return launch_rows<T, 3, NR, FILL>(a, slot_cell, counts_by_id, qslots, nq, base, pairs, cands, num_sms, st);
+        case 4: return launch_rows<T, 4, NR, FILL>(a, slot_cell, counts_by_id, qslots, nq, base, pairs, cands, num_sms, st);
         default: return cudaErrorInvalidValue;
     }
 }
 
 template <typename T, bool FILL>
 static cudaError_t rows_any(const JoinArgs<T>& a, const uint32_t* slot_cell, uint32_t* counts_by_id,
-                            const uint32_t* qslots, uint32_t nq, uint64_t base, int num_sms, cudaStream_t st) {
+                            const uint32_t* qslots, uint32_t nq, uint64_t base, uint64_t pairs, uint64_t cands,
+                            int num_sms, cudaStream_t st) {
     if (a.n < 1 || a.n > 4 || a.ilp != 0 || a.g.k > 3 || !a.plan) return cudaErrorInvalidValue;
     if (nq == 0) return cudaSuccess;
-    if (a.g.k == 1) return rows_nr<T, 1, FILL>(a, slot_cell, counts_by_id, qslots, nq, base, num_sms, st);
-    if (a.g.k == 2) return rows_nr<T, 3, FILL>(a, slot_cell, counts_by_id, qslots, nq, base, num_sms, st);
-    return rows_nr<T, 9, FILL>(a, slot_cell, counts_by_id, qslots, nq, base, num_sms, st);
+    if (a.g.k == 1) return rows_nr<T, 1, FILL>(a, slot_cell, counts_by_id, qslots, nq, base, pairs, cands, num_sms, st);
+    if (a.g.k == 2) return rows_nr<T, 3, FILL>(a, slot_cell, counts_by_id, qslots, nq, base, pairs, cands, num_sms, st);
+    return rows_nr<T, 9, FILL>(a, slot_cell, counts_by_id, qslots, nq, base, pairs, cands, num_sms, st);
 }
 
 template <typename T>
 cudaError_t launch_rows_count(const JoinArgs<T>& a, const uint32_t* slot_cell, uint32_t* counts_by_id, int num_sms,
                               cudaStream_t st) {
-    return rows_any<T, false>(a, slot_cell, counts_by_id, nullptr, a.n_points, 0, num_sms, st);
+    return rows_any<T, false>(a, slot_cell, counts_by_id, nullptr, a.n_points, 0, 0, 0, num_sms, st);
 }
 
 template <typename T>
 cudaError_t launch_rows_fill(const JoinArgs<T>& a, const uint32_t* slot_cell, const uint32_t* qslots, uint32_t nq,
-                             uint64_t base, int num_sms, cudaStream_t st) {
-    return rows_any<T, true>(a, slot_cell, nullptr, qslots, nq, base, num_sms, st);
+                             uint64_t base, uint64_t pairs, uint64_t cands, int num_sms, cudaStream_t st) {
+    return rows_any<T, true>(a, slot_cell, nullptr, qslots, nq, base, pairs, cands, num_sms, st);
 }
 
 template cudaError_t launch_rows_count<float>(const JoinArgs<float>&, const uint32_t*, uint32_t*, int, cudaStream_t);
 template cudaError_t launch_rows_count<double>(const JoinArgs<double>&, const uint32_t*, uint32_t*, int,
                                                cudaStream_t);
 template cudaError_t launch_rows_fill<float>(const JoinArgs<float>&, const uint32_t*, const uint32_t*, uint32_t,
-                                             uint64_t, int, cudaStream_t);
+                                             uint64_t, uint64_t, uint64_t, int, cudaStream_t);
 template cudaError_t launch_rows_fill<double>(const JoinArgs<double>&, const uint32_t*, const uint32_t*, uint32_t,
-                                              uint64_t, int, cudaStream_t);
+                                              uint64_t, uint64_t, uint64_t, int, cudaStream_t);
 
 // ---------------------------------------------------------------- result batches
 // Batch b of the host-result pipeline holds the point ids [bound[b],

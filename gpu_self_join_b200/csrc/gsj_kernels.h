@@ -91,10 +91,11 @@ cudaError_t launch_rows_count(const JoinArgs<T>& a, const uint32_t* slot_cell, u
 // Fill pass (a.work_counter zeroed, a.offsets/table/table_cap/err_flag set):
 // the lists of the queries at slots qslots[0 .. nq) (slots 0 .. nq-1 when
 // qslots is null) into the point-id-ordered table; the list of point id i lands
-// at a.table[offsets[i] - base].
+// at a.table[offsets[i] - base].  pairs, cands: the whole join's result pairs and
+// candidates, which choose the kernel.
 template <typename T>
 cudaError_t launch_rows_fill(const JoinArgs<T>& a, const uint32_t* slot_cell, const uint32_t* qslots, uint32_t nq,
-                             uint64_t base, int num_sms, cudaStream_t st);
+                             uint64_t base, uint64_t pairs, uint64_t cands, int num_sms, cudaStream_t st);
 // Result batches by point-id range: bound[0..nb] (ids) and boff[0..nb] (their
 // table offsets), each batch's lists at most `step` + the longest list
 // entries; per-slot batch keys (with the slot index as value, for a stable
