@@ -1380,9 +1380,6 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     uint2* items = nullptr;
     if (tpq) S.work_items = ((uint64_t)N + 31u) / 32u;
     else GSJ_TRY(work_items(c, cfg.query_reorder != 0, cell_start, M, qchunk, &items, &num_items));
-    GSJ_CUDA(c, cudaEventRecord(c->tev[1], st));
-    const double t_join = now_ms();
-    S.ms_index = t_join - t_index;
 
     // ---- join arguments (every path)
     uint32_t* ctr = reinterpret_cast<uint32_t*>(d_mm + 2 * kMaxK) + 2;  // work counter
@@ -1415,6 +1412,20 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     a.shape_per_sm = shape.ctas_per_sm;
     const bool stamp = cfg.stamp != 0 && !(cfg.flags & GSJ_FLAG_NO_UNICOMP);
     const bool exact_size = (cfg.flags & GSJ_FLAG_EXACT_SIZE) != 0;
+    if (!dense && k <= 3 && !tile && !cfg.sort) {
+        // the warp join's neighbour rows; without room for them it looks them up itself
+        uint2* rplan = nullptr;
+        if (dev_get(c, c->plan, (size_t)M * (k == 1 ? 1u : (k == 2 ? 3u : 9u)), &rplan) == GSJ_OK) {
+            S.kernel_launches += 1;
+            GSJ_CUDA(c, launch_row_plan<T>(a, stamp, rplan, st));
+            a.plan = rplan;
+        } else {
+            c->err.clear();
+        }
+    }
+    GSJ_CUDA(c, cudaEventRecord(c->tev[1], st));
+    const double t_join = now_ms();
+    S.ms_index = t_join - t_index;
     // the cell table of this join, for the model's features (estimate now,
     // training after the join)
     c->last.valid = true;

@@ -32,7 +32,9 @@ struct JoinArgs {
     const uint32_t* cell_start;   // [M+1]
     const uint64_t* cell_key;     // [M]
     const uint32_t* ds;           // [totalCells+1] slot prefix over all linear ids (dense grids), or null
-    const uint2* plan;            // [M][3^(k-1)] (slot start, count) of each neighbour row (dense, k <= 3)
+    const uint2* plan;            // [M][3^(k-1)] (slot start, count) of each neighbour row, or null: the ROWS
+                                  // path's (whole rows), the warp join's on hashed grids of k <= 3 (rows as
+                                  // its traversal takes them)
     const uint4* htab;            // [hcap] hash table of the grid rows that hold a cell {linear id of the row's
                                   // cell 0 (lo, hi; kEmptyKey = empty), first cell, cells}, or null
     uint64_t hmask;               // hcap - 1

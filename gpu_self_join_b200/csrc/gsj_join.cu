@@ -128,12 +128,33 @@ __device__ __forceinline__ uint32_t cand_slot(const uint32_t* nb_start, const ui
 // The neighbour rows of `cell` (first slot cs; kernel.cu:180-303; stamploops.h
 // for STAMP) as slot ranges in nb_start and the exclusive prefix of their sizes
 // in nb_pref (nb_pref[rows] = total).  Returns the number of rows; the whole
-// warp calls.
-template <typename T, bool STAMP>
+// warp calls.  PLAN: a.plan holds them (as a template argument: a branch on the
+// pointer cost the 8-D register form 1 %).
+template <typename T, bool STAMP, bool PLAN>
 __device__ __forceinline__ uint32_t enumerate_rows(const JoinArgs<T>& a, uint32_t cell, uint32_t cs, uint32_t nrow,
                                                    uint32_t* nb_start, uint32_t* nb_pref, int lane, unsigned lt,
                                                    uint32_t& total) {
     const unsigned FULL = 0xffffffffu;
+    if (PLAN) {  // at most 9 rows, looked up before (k_row_plan)
+        uint2 e = make_uint2(0u, 0u);
+        if ((uint32_t)lane < nrow) e = a.plan[(size_t)cell * nrow + (uint32_t)lane];
+        const unsigned m = __ballot_sync(FULL, e.y != 0u);
+        uint32_t x = e.y;
+#pragma unroll
+        for (int s = 1; s < 16; s <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULL, x, s);
+            if (lane >= s) x += y;
+        }
+        total = __shfl_sync(FULL, x, 15);
+        const uint32_t nnb = (uint32_t)__popc(m);
+        if (e.y) {
+            const uint32_t pos = (uint32_t)__popc(m & lt);
+            nb_start[pos] = e.x;
+            nb_pref[pos] = x - e.y;
+        }
+        if (lane == 0) nb_pref[nnb] = total;
+        return nnb;
+    }
     // own cell coordinates, from the first query of the cell with the formula the
     // keys were built with (main.cu:744, kernel.cu:184)
     uint32_t own[kMaxK];
@@ -176,7 +197,7 @@ __device__ __forceinline__ uint32_t enumerate_rows(const JoinArgs<T>& a, uint32_
     return nnb;
 }
 
-template <typename T, int NT, int MODEL, int POL, bool STAMP>
+template <typename T, int NT, int MODEL, int POL, bool STAMP, bool PLAN>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_join(const JoinArgs<T> a, uint32_t nrow,
                                                                        const TileOut o, uint32_t nvisit) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -215,7 +236,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_join(const Join
         const uint32_t q0 = cs + wi.y * kQChunk;
         const uint32_t qn = min((uint32_t)kQChunk, ce - q0);
         uint32_t total;
-        const uint32_t nnb = enumerate_rows<T, STAMP>(a, wi.x, cs, nrow, nb_start, nb_pref, lane, lt, total);
+        const uint32_t nnb = enumerate_rows<T, STAMP, PLAN>(a, wi.x, cs, nrow, nb_start, nb_pref, lane, lt, total);
 
         // ---- queries
         for (uint32_t e = lane; e < qn * npad; e += 32) q_s[e] = a.pts[(size_t)q0 * npad + e];
@@ -402,7 +423,7 @@ __host__ __device__ inline RegSmem reg_smem(uint32_t np4, uint32_t nrow) {
 // Short units balance a small join (142k points in 8-D, 32 queries an item in the
 // dense cells: unsliced, the longest items held the launch for two thirds of its
 // time), long ones repeat the enumeration less often: see join_unit_steps.
-template <int NP, int SUM, int G, bool STAMP, bool SLICES>
+template <int NP, int SUM, int G, bool STAMP, bool PLAN, bool SLICES>
 __global__ void __launch_bounds__(256, 4) k_join_reg(const JoinArgs<float> a, uint32_t nrow, const TileOut o,
                                                      const HeavyList heavy, uint32_t nvisit) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -459,7 +480,7 @@ __global__ void __launch_bounds__(256, 4) k_join_reg(const JoinArgs<float> a, ui
         const uint32_t q0 = cs + wi.y * kQChunk;
         const uint32_t qn = min((uint32_t)kQChunk, ce - q0);
         uint32_t total;
-        const uint32_t nnb = enumerate_rows<float, STAMP>(a, wi.x, cs, nrow, nb_start, nb_pref, lane, lt, total);
+        const uint32_t nnb = enumerate_rows<float, STAMP, PLAN>(a, wi.x, cs, nrow, nb_start, nb_pref, lane, lt, total);
         uint32_t g_lo = 0, g_hi = (total + 32u * G - 1u) / (32u * G);  // candidate groups of this unit
         const uint32_t per = (heavy.unit + qn - 1u) / qn;              // groups of a slice
         if (SLICES) {
@@ -574,10 +595,11 @@ static cudaError_t warp_grid(const void* kern, uint32_t per_warp, const uint32_t
     return cudaSuccess;
 }
 
-template <typename T, int NT, int MODEL, int POL, bool STAMP>
+template <typename T, int NT, int MODEL, int POL, bool STAMP, bool PLAN = false>
 static cudaError_t launch_one(const JoinArgs<T>& a, uint32_t nrow, const TileOut& o, uint32_t nvisit, int num_sms,
                               int* launches, cudaStream_t st) {
-    auto kern = k_join<T, NT, MODEL, POL, STAMP>;
+    if (!PLAN && a.plan) return launch_one<T, NT, MODEL, POL, STAMP, true>(a, nrow, o, nvisit, num_sms, launches, st);
+    auto kern = k_join<T, NT, MODEL, POL, STAMP, PLAN>;
     const WarpSmem L = warp_smem_layout(a.npad, sizeof(T), nrow, NT == 0);
     int threads = 0;
     size_t smem = 0;
@@ -590,11 +612,13 @@ static cudaError_t launch_one(const JoinArgs<T>& a, uint32_t nrow, const TileOut
     return cudaGetLastError();
 }
 
-template <int NP, int SUM, int G, bool STAMP>
+template <int NP, int SUM, int G, bool STAMP, bool PLAN = false>
 static cudaError_t launch_reg(const JoinArgs<float>& a, uint32_t nrow, const TileOut& o, const HeavyList& heavy,
                               uint32_t nvisit, int num_sms, int* launches, cudaStream_t st) {
-    auto k1 = k_join_reg<NP, SUM, G, STAMP, false>;
-    auto k2 = k_join_reg<NP, SUM, G, STAMP, true>;
+    if (!PLAN && a.plan)
+        return launch_reg<NP, SUM, G, STAMP, true>(a, nrow, o, heavy, nvisit, num_sms, launches, st);
+    auto k1 = k_join_reg<NP, SUM, G, STAMP, PLAN, false>;
+    auto k2 = k_join_reg<NP, SUM, G, STAMP, PLAN, true>;
     const RegSmem L = reg_smem((NP + 3) / 4 * 4, nrow);
     int threads = 0;
     size_t smem = 0;

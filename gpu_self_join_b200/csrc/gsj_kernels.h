@@ -51,6 +51,10 @@ cudaError_t launch_row_table(const uint64_t* cell_key, uint32_t M, uint32_t n0, 
                              cudaStream_t st);
 cudaError_t launch_cell_plan(const uint64_t* cell_key, uint32_t M, const GridGeom& g, const uint32_t* ds,
                              uint2* plan, cudaStream_t st);
+// The same for the warp join on a hashed grid with k <= 3 (a: cell table, grid and
+// neighbour offsets), the rows of the unicomp half-space with `stamp`.
+template <typename T>
+cudaError_t launch_row_plan(const JoinArgs<T>& a, bool stamp, uint2* plan, cudaStream_t st);
 cudaError_t launch_item_counts(const uint32_t* cell_start, const uint32_t* order, uint32_t M, uint32_t qchunk,
                                uint32_t* nchunks, uint32_t* sizes, cudaStream_t st);
 cudaError_t launch_make_items(const uint32_t* order, const uint32_t* nchunks, const uint32_t* item_off,
