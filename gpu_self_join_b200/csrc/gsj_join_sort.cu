@@ -31,9 +31,15 @@ namespace gsj {
 
 namespace {
 
+// Bound by the dependent loads of the windows.  Count + fill (ms) of single cells
+// hashed / each cell searched in its row / a row searched once / the last with
+// registers for 4 CTAs an SM (52 to 68, no spills; left to itself the compiler took
+// 40 to 48 with up to 84 bytes spilled): 18-D 50k points, 6 dims indexed 41.4 + 42.9 /
+// 45.9 + 43.1 / 45.8 + 40.0 / 38.1 + 38.6, 6-D 100k 1.85 + 1.88 / 1.58 + 1.61 / 0.85 +
+// 0.88 / 0.84 + 0.87; 8, 10 and 12 CTAs an SM 18-D 37.7 + 39.7, 38.9 + 40.0, 39.5 + 40.4.
 template <typename T, int MODEL, int POL, bool FILL>
-__global__ void __launch_bounds__(128) k_sort_join(const JoinArgs<T> a, const uint32_t* __restrict__ slot_cell,
-                                                   uint32_t noff, uint32_t* __restrict__ counts_by_id) {
+__global__ void __launch_bounds__(128, 4) k_sort_join(const JoinArgs<T> a, const uint32_t* __restrict__ slot_cell,
+                                                   uint32_t nrow, uint32_t* __restrict__ counts_by_id) {
     const uint32_t N = a.n_points;
     const uint32_t n = a.n, npad = a.npad, k = a.g.k;
     const T eps = a.eps, thr = a.thr;
@@ -64,42 +70,66 @@ __global__ void __launch_bounds__(128) k_sort_join(const JoinArgs<T> a, const ui
                 cnt++;
             }
         };
-        for (uint32_t o = 0; o < noff; o++) {
-            uint64_t lin;
-            if (!nb_offset<T, false>(a, o, key, lowmask, highmask, oddmask, lin)) continue;
-            uint32_t start, num;
-            if (!lookup_range(a, lin, start, num)) continue;
-            if (indexed) {
-                // the neighbour's step in dim 0 is digit 0 of the offset
-                const int dl0 = (int)(o % 3u) - 1;
-                const bool mid = dl0 == 0, left = dl0 < 0;
-                for (uint32_t kk = 0; kk < num; kk++) {
-                    const uint32_t pos = left ? num - 1u - kk : kk;
-                    const T dv = FP<T>::sub(a.pts[(size_t)(start + pos) * npad], p[0]);
-                    if (!mid && fabs(dv) > eps) break;
-                    eval(start + pos);
+        // neighbour cells in offset order: the grid row of dims 1.. once, then its cells
+        // x-1, x, x+1.  On hashed grids a row's cells follow one another in the sorted
+        // list: the first at or past x-1 is searched, the others come after it.
+        for (uint32_t r = 0; r < nrow; r++) {
+            uint64_t centre;
+            if (!nb_offset<T, false>(a, 3u * r + 1u, key, lowmask, highmask, oddmask, centre)) continue;
+            uint32_t at = 0, end = 0;
+            if (!a.ds) {
+                const uint64_t base = centre - own[0], klo = centre - (lowmask & 1u ? 0u : 1u);
+                row_entry(a, base, a.htab[mix64(base) & a.hmask], at, end);
+                end = end ? at + end : at;
+                uint32_t hi = end;
+                while (at < hi) {
+                    const uint32_t m = at + (hi - at) / 2u;
+                    if (a.cell_key[m] < klo) at = m + 1u;
+                    else hi = m;
                 }
-            } else {
-                const int length = (int)num - 1;
-                auto db = [&](int pos) { return a.pts[(size_t)(start + (uint32_t)pos) * npad + sd]; };
-                int idx = length / 2;
-                for (int step = (length + 3) / 4; step > 1; step = (step + 1) / 2) {
-                    if (FP<T>::sub(p[sd], db(idx)) >= eps) {
-                        idx += step;
-                        if (idx > length) idx = length;
-                    } else {
-                        idx -= step;
-                        if (idx < 0) {
-                            idx = 0;
-                            step = 0;
+            }
+            for (int dl0 = lowmask & 1u ? 0 : -1; dl0 <= (highmask & 1u ? 0 : 1); dl0++) {
+                const uint64_t lin = centre + (uint64_t)(int64_t)dl0;
+                uint32_t start, num;
+                if (a.ds) {
+                    start = a.ds[lin];
+                    num = a.ds[lin + 1u] - start;
+                    if (num == 0u) continue;
+                } else {
+                    if (at >= end || a.cell_key[at] != lin) continue;
+                    start = a.cell_start[at];
+                    num = a.cell_start[++at] - start;
+                }
+                if (indexed) {
+                    const bool mid = dl0 == 0, left = dl0 < 0;
+                    for (uint32_t kk = 0; kk < num; kk++) {
+                        const uint32_t pos = left ? num - 1u - kk : kk;
+                        const T dv = FP<T>::sub(a.pts[(size_t)(start + pos) * npad], p[0]);
+                        if (!mid && fabs(dv) > eps) break;
+                        eval(start + pos);
+                    }
+                } else {
+                    const int length = (int)num - 1;
+                    auto db = [&](int pos) { return a.pts[(size_t)(start + (uint32_t)pos) * npad + sd]; };
+                    int idx = length / 2;
+                    for (int step = (length + 3) / 4; step > 1; step = (step + 1) / 2) {
+                        if (FP<T>::sub(p[sd], db(idx)) >= eps) {
+                            idx += step;
+                            if (idx > length) idx = length;
+                        } else {
+                            idx -= step;
+                            if (idx < 0) {
+                                idx = 0;
+                                step = 0;
+                            }
                         }
                     }
-                }
-                if (idx > 0 && FP<T>::sub(p[sd], db(idx - 1)) <= eps) idx--;
-                if (idx > 0 && FP<T>::sub(p[sd], db(idx - 1)) <= eps) idx--;
-                while (idx <= length && FP<T>::sub(db(idx), p[sd]) < eps) {
-                    eval(start + (uint32_t)idx);
-                    idx++;
+                    if (idx > 0 && FP<T>::sub(p[sd], db(idx - 1)) <= eps) idx--;
+                    if (idx > 0 && FP<T>::sub(p[sd], db(idx - 1)) <= eps) idx--;
+                    while (idx <= length && FP<T>::sub(db(idx), p[sd]) < eps) {
+                        eval(start + (uint32_t)idx);
+                        idx++;
+                    }
                 }
             }
         }
@@ -113,14 +143,14 @@ __global__ void __launch_bounds__(128) k_sort_join(const JoinArgs<T> a, const ui
 }
 
 template <typename T, int MODEL, int POL>
-cudaError_t sort_launch(const JoinArgs<T>& a, const uint32_t* slot_cell, uint32_t noff, uint32_t* counts_by_id,
+cudaError_t sort_launch(const JoinArgs<T>& a, const uint32_t* slot_cell, uint32_t nrow, uint32_t* counts_by_id,
                         bool fill, int num_sms, cudaStream_t st) {
     uint64_t blocks = ((uint64_t)a.n_points + 127) / 128;
     const uint64_t cap = (uint64_t)num_sms * 16;
     if (blocks > cap) blocks = cap;
     if (blocks == 0) blocks = 1;
-    if (fill) k_sort_join<T, MODEL, POL, true><<<(unsigned)blocks, 128, 0, st>>>(a, slot_cell, noff, counts_by_id);
-    else k_sort_join<T, MODEL, POL, false><<<(unsigned)blocks, 128, 0, st>>>(a, slot_cell, noff, counts_by_id);
+    if (fill) k_sort_join<T, MODEL, POL, true><<<(unsigned)blocks, 128, 0, st>>>(a, slot_cell, nrow, counts_by_id);
+    else k_sort_join<T, MODEL, POL, false><<<(unsigned)blocks, 128, 0, st>>>(a, slot_cell, nrow, counts_by_id);
     return cudaGetLastError();
 }
 
@@ -138,11 +168,11 @@ template <typename T>
 cudaError_t launch_sort_join(const JoinArgs<T>& a, const uint32_t* slot_cell, uint32_t* counts_by_id, int model,
                              bool fill, int num_sms, cudaStream_t st) {
     constexpr int POL = sizeof(T) == 8 ? kPolF64 : kPolF32;
-    uint32_t noff = 1;
-    for (uint32_t j = 0; j < a.g.k; j++) noff *= 3u;
-    if (model == kSeq) return sort_launch<T, kSeq, POL>(a, slot_cell, noff, counts_by_id, fill, num_sms, st);
-    if (model == kIlp) return sort_launch<T, kIlp, POL>(a, slot_cell, noff, counts_by_id, fill, num_sms, st);
-    return sort_launch<T, kIlpSc, POL>(a, slot_cell, noff, counts_by_id, fill, num_sms, st);
+    uint32_t nrow = 1;  // neighbour rows: 3^(k-1)
+    for (uint32_t j = 1; j < a.g.k; j++) nrow *= 3u;
+    if (model == kSeq) return sort_launch<T, kSeq, POL>(a, slot_cell, nrow, counts_by_id, fill, num_sms, st);
+    if (model == kIlp) return sort_launch<T, kIlp, POL>(a, slot_cell, nrow, counts_by_id, fill, num_sms, st);
+    return sort_launch<T, kIlpSc, POL>(a, slot_cell, nrow, counts_by_id, fill, num_sms, st);
 }
 
 template <typename T>
