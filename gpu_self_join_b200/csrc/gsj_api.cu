@@ -199,8 +199,10 @@ struct gsj_context {
         float log2_eps = 0;
         JoinArgs<float> lookup{};
     } last;
-    // tuned launch shapes by (path, dim, density_log2)
-    std::map<std::tuple<uint32_t, uint32_t, uint32_t>, gsj_tuning> tuning;
+    // tuned launch shapes by (path, dim, density_log2, screened): GSJ_PATH_TILE stands
+    // for two kernels below 16 dimensions
+    std::map<std::tuple<uint32_t, uint32_t, uint32_t, bool>, gsj_tuning> tuning;
+    bool screened = false;  // the last join went through the screen
     const gsj_tuning* forced = nullptr;  // the autotuner's candidate, in place of the table
     // slices of the warp join's long items: the list's capacity, the slices counted
     // before the first item (test hooks), those of the last join
@@ -842,6 +844,7 @@ int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int mo
     GSJ_CUDA(c, cudaEventRecord(c->tev[3], st));
     GSJ_TRY(pairs_to_csr(c, pairs, R, R, shift, N, counts, offsets, cand));
     S.screen_rechecks = screen ? U : 0;
+    c->screened = screen;
     S.join_path = a.n >= kScreenPathDims && screen ? GSJ_PATH_SCREEN : GSJ_PATH_TILE;
     S.ms_join = now_ms() - t_join;
     S.ms_total = now_ms() - t_start;
@@ -1097,6 +1100,7 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     c->have_result = false;
     c->table_on_device = true;
     c->last.valid = false;
+    c->screened = false;
     S.batches = 1;
     c->N = N;
     c->R = 0;
@@ -1362,17 +1366,15 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     uint32_t dlog = 0;
     while (dlog < 31 && (N / std::max<uint32_t>(M, 1u)) >> (dlog + 1)) dlog++;
     S.density_log2 = dlog;
-    gsj_tuning shape{};
-    if (c->forced) {
-        shape = *c->forced;
+    auto shape_of = [&](uint32_t path, bool screened) -> gsj_tuning {
         S.tuned = 1;
-    } else {
-        auto it = c->tuning.find(std::make_tuple(path_id, n, dlog));
-        if (it != c->tuning.end()) {
-            shape = it->second;
-            S.tuned = 1;
-        }
-    }
+        if (c->forced) return *c->forced;
+        auto it = c->tuning.find(std::make_tuple(path, n, dlog, screened));
+        if (it != c->tuning.end()) return it->second;
+        S.tuned = 0;
+        return gsj_tuning{};
+    };
+    gsj_tuning shape = shape_of(path_id, screen);
 
     // ---- work items.  The ROWS path has none: its passes claim 32 consecutive
     // query slots at a time, and the order in which queries run changes no result.
@@ -1461,6 +1463,8 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
                 GSJ_TRY(work_items(c, cfg.query_reorder != 0, cell_start, M, (uint32_t)kTileQ, &items, &num_items));
                 a.items = items;
                 a.num_items = num_items;
+                shape = shape_of(GSJ_PATH_TILE, false);
+                a.shape_per_sm = shape.ctas_per_sm;
             }
             return tile_join(c, a, N, stamp, model, false, exact_size, learned, counts, offsets, cursor, t_join,
                              t_start);
@@ -1714,7 +1718,8 @@ static int tuning_valid(gsj_context* c, const gsj_tuning& t) {
 
 int gsj_tuning_get(gsj_context* c, uint32_t path, uint32_t dim, uint32_t dlog, gsj_tuning* t) {
     if (!c || !t) return fail(c, GSJ_ERR_INVALID, "null argument");
-    auto it = c->tuning.find(std::make_tuple(path, dim, dlog));
+    auto it = c->tuning.find(std::make_tuple(path, dim, dlog, path == GSJ_PATH_TILE || path == GSJ_PATH_SCREEN));
+    if (it == c->tuning.end()) it = c->tuning.find(std::make_tuple(path, dim, dlog, false));
     if (it == c->tuning.end()) return fail(c, GSJ_ERR_STATE, "no tuning entry for this key");
     *t = it->second;
     return GSJ_OK;
@@ -1723,7 +1728,8 @@ int gsj_tuning_get(gsj_context* c, uint32_t path, uint32_t dim, uint32_t dlog, g
 int gsj_tuning_set(gsj_context* c, uint32_t path, uint32_t dim, uint32_t dlog, const gsj_tuning* t) {
     if (!c || !t) return fail(c, GSJ_ERR_INVALID, "null argument");
     GSJ_TRY(tuning_valid(c, *t));
-    c->tuning[std::make_tuple(path, dim, dlog)] = *t;
+    if (path != GSJ_PATH_SCREEN) c->tuning[std::make_tuple(path, dim, dlog, false)] = *t;
+    if (path == GSJ_PATH_SCREEN || path == GSJ_PATH_TILE) c->tuning[std::make_tuple(path, dim, dlog, true)] = *t;
     return GSJ_OK;
 }
 
@@ -1736,9 +1742,10 @@ int gsj_autotune(gsj_context* c, const void* data, uint64_t num_points, double e
     GSJ_TRY(gsj_join(c, data, num_points, eps, cfg, data_on_device, &st));
     if (num_points == 0) return fail(c, GSJ_ERR_INVALID, "nothing to tune on an empty input");
     const uint32_t path = (uint32_t)st.join_path, dlog = (uint32_t)st.density_log2;
+    const auto key = std::make_tuple(path, cfg->dim, dlog, c->screened);
     gsj_tuning cur{};
     {
-        auto it = c->tuning.find(std::make_tuple(path, cfg->dim, dlog));
+        auto it = c->tuning.find(key);
         if (it != c->tuning.end()) cur = it->second;
     }
     auto timed = [&](const gsj_tuning& t, double* ms) -> int {
@@ -1760,8 +1767,9 @@ int gsj_autotune(gsj_context* c, const void* data, uint64_t num_points, double e
         knobs.push_back({&gsj_tuning::warps, {0, 4, 2}});
         knobs.push_back({&gsj_tuning::ctas_per_sm, {0, 4, 2}});
     }
-    if (path == GSJ_PATH_TILE) knobs.push_back({&gsj_tuning::ctas_per_sm, {0, 2, 1}});
-    if (path == GSJ_PATH_SCREEN) knobs.push_back({&gsj_tuning::ctas_per_sm, {0, 1}});
+    // the screen holds 2 CTAs an SM at most
+    if (std::get<3>(key)) knobs.push_back({&gsj_tuning::ctas_per_sm, {0, 1}});
+    else if (path == GSJ_PATH_TILE) knobs.push_back({&gsj_tuning::ctas_per_sm, {0, 2, 1}});
     double best_ms = 0.0;
     GSJ_TRY(timed(cur, &best_ms));
     for (auto& kv : knobs) {
@@ -1777,7 +1785,7 @@ int gsj_autotune(gsj_context* c, const void* data, uint64_t num_points, double e
             }
         }
     }
-    c->tuning[std::make_tuple(path, cfg->dim, dlog)] = cur;
+    c->tuning[key] = cur;
     *best = cur;
     return GSJ_OK;
 }

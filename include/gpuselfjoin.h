@@ -260,7 +260,9 @@ GSJ_API int gsj_list_offsets_noalloc(const uint32_t* d_counts, uint64_t n, uint6
  * reference fixes them at compile time (BLOCKSIZE, params.h:17; GPUSTREAMS,
  * params.h:85).  A context keeps a table of tuned shapes; a join whose
  * (path, dim, density_log2) has an entry launches with it (gsj_stats.tuned).
- * Shapes never change results, only speed. */
+ * GSJ_PATH_TILE stands for two kernels (screened and plain joins): gsj_autotune
+ * keeps their shapes apart, gsj_tuning_set sets both, gsj_tuning_get returns the
+ * screened one where there is one.  Shapes never change results, only speed. */
 typedef struct gsj_tuning {
     uint32_t threads;     /* ROWS path: CTA size of the count and fill passes
                              (64..256, a multiple of 32; 0: 256)              */
