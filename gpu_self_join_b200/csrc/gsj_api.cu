@@ -571,15 +571,18 @@ int emit_join(gsj_context* c, JoinArgs<T>& a, uint64_t N, bool stamp, int model,
     o.rechecks = cursor + 1; // keys emitted (exact)
     o.shift = shift;
     unsigned long long* cand = reinterpret_cast<unsigned long long*>(a.work_counter + 2);
-    // a warp appends at most 64 keys at once (32 hits and their reverse keys);
-    // at most 64 warps per SM are resident, in each of the two launches of a pass
-    const uint64_t warps = (uint64_t)c->num_sms * 128u;
     HeavyList heavy{};
     GSJ_TRY(dev_get(c, c->heavy, kHeavyCap, &heavy.list));
     heavy.cap = c->slice_cap;
     heavy.count = cursor + 2;
     heavy.claim = reinterpret_cast<uint32_t*>(cursor + 3);
+    heavy.unit = 32u;  // the sampling pass's: few items, short units
+    o.stride = 1;
     int nl = 0;
+    // a warp appends at most 64 keys at once (32 hits and their reverse keys) and may
+    // leave one block of kScreenBlockSlack keys partly filled
+    uint64_t warps = 0;
+    GSJ_CUDA(c, launch_join_emit<T>(a, o, heavy, ni, model, stamp, WarpLaunch{c->num_sms, st, &nl, &warps}));
     const uint64_t slack = warps * kScreenBlockSlack;
     auto reset = [&]() -> int {
         GSJ_CUDA(c, cudaMemsetAsync(a.work_counter, 0, 4 * sizeof(uint32_t), st));
@@ -602,8 +605,7 @@ int emit_join(gsj_context* c, JoinArgs<T>& a, uint64_t N, bool stamp, int model,
         GSJ_TRY(reset());
         o.emit = false;
         o.stride = kSampleStride;
-        heavy.unit = 32u;  // few items: short units
-        GSJ_CUDA(c, launch_join_emit<T>(a, o, heavy, nsample, model, stamp, c->num_sms, &nl, st));
+        GSJ_CUDA(c, launch_join_emit<T>(a, o, heavy, nsample, model, stamp, WarpLaunch{c->num_sms, st, &nl, nullptr}));
         unsigned long long sampled = 0, sampled_cand = 0;
         Readback rb(c);
         GSJ_TRY(rb.add(&sampled, o.rechecks, 1));
@@ -627,7 +629,7 @@ int emit_join(gsj_context* c, JoinArgs<T>& a, uint64_t N, bool stamp, int model,
         o.stride = 1;
         o.pairs = pairs;
         o.cap = cap;
-        GSJ_CUDA(c, launch_join_emit<T>(a, o, heavy, ni, model, stamp, c->num_sms, &nl, st));
+        GSJ_CUDA(c, launch_join_emit<T>(a, o, heavy, ni, model, stamp, WarpLaunch{c->num_sms, st, &nl, nullptr}));
         unsigned long long got[3] = {0, 0, 0};  // entries reserved, keys, slices found
         GSJ_TRY(d2h_small(c, got, cursor, 3));
         used = got[0];
@@ -679,9 +681,9 @@ int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int mo
     o.cursor = cursor;
     o.shift = shift;
     o.rechecks = cursor + 1;  // the screen's exact count of undecided pairs
-    // the screen's consumer warps reserve blocks and fill them (at most 64 warps
-    // per SM are resident); the tile join appends exactly
-    const uint64_t warps = (uint64_t)c->num_sms * 64u;
+    // the screen's consumer warps (8 in each of at most 2 CTAs an SM, by its tensor
+    // memory) reserve blocks and fill them; the tile join appends exactly
+    const uint64_t warps = (uint64_t)c->num_sms * 16u;
     const uint64_t slack = screen ? warps * kScreenBlock : 0u;
     unsigned long long* cand = reinterpret_cast<unsigned long long*>(a.work_counter + 2);
     a.err_flag = a.work_counter + 1;

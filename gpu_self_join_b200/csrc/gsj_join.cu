@@ -596,42 +596,50 @@ static cudaError_t warp_grid(const void* kern, uint32_t per_warp, const uint32_t
 }
 
 template <typename T, int NT, int MODEL, int POL, bool STAMP, bool PLAN = false>
-static cudaError_t launch_one(const JoinArgs<T>& a, uint32_t nrow, const TileOut& o, uint32_t nvisit, int num_sms,
-                              int* launches, cudaStream_t st) {
-    if (!PLAN && a.plan) return launch_one<T, NT, MODEL, POL, STAMP, true>(a, nrow, o, nvisit, num_sms, launches, st);
+static cudaError_t launch_one(const JoinArgs<T>& a, uint32_t nrow, const TileOut& o, uint32_t nvisit, const WarpLaunch& w) {
+    if (!PLAN && a.plan) return launch_one<T, NT, MODEL, POL, STAMP, true>(a, nrow, o, nvisit, w);
     auto kern = k_join<T, NT, MODEL, POL, STAMP, PLAN>;
     const WarpSmem L = warp_smem_layout(a.npad, sizeof(T), nrow, NT == 0);
     int threads = 0;
     size_t smem = 0;
     uint64_t blocks = 0;
-    const cudaError_t e = warp_grid((const void*)kern, L.total, a.shape_warps, a.shape_per_sm, nvisit, num_sms,
+    const cudaError_t e = warp_grid((const void*)kern, L.total, a.shape_warps, a.shape_per_sm, nvisit, w.num_sms,
                                     threads, smem, blocks);
     if (e != cudaSuccess) return e;
-    kern<<<(unsigned)blocks, threads, smem, st>>>(a, nrow, o, nvisit);
-    *launches += 1;
+    if (w.warps) {
+        *w.warps = blocks * (uint64_t)(threads / 32);
+        return cudaSuccess;
+    }
+    kern<<<(unsigned)blocks, threads, smem, w.st>>>(a, nrow, o, nvisit);
+    *w.launches += 1;
     return cudaGetLastError();
 }
 
 template <int NP, int SUM, int G, bool STAMP, bool PLAN = false>
 static cudaError_t launch_reg(const JoinArgs<float>& a, uint32_t nrow, const TileOut& o, const HeavyList& heavy,
-                              uint32_t nvisit, int num_sms, int* launches, cudaStream_t st) {
+                              uint32_t nvisit, const WarpLaunch& w) {
     if (!PLAN && a.plan)
-        return launch_reg<NP, SUM, G, STAMP, true>(a, nrow, o, heavy, nvisit, num_sms, launches, st);
+        return launch_reg<NP, SUM, G, STAMP, true>(a, nrow, o, heavy, nvisit, w);
     auto k1 = k_join_reg<NP, SUM, G, STAMP, PLAN, false>;
     auto k2 = k_join_reg<NP, SUM, G, STAMP, PLAN, true>;
     const RegSmem L = reg_smem((NP + 3) / 4 * 4, nrow);
     int threads = 0;
     size_t smem = 0;
     uint64_t blocks = 0;
-    cudaError_t e = warp_grid((const void*)k1, L.total, a.shape_warps, a.shape_per_sm, nvisit, num_sms, threads, smem,
+    cudaError_t e = warp_grid((const void*)k1, L.total, a.shape_warps, a.shape_per_sm, nvisit, w.num_sms, threads, smem,
                               blocks);
     if (e != cudaSuccess) return e;
-    k1<<<(unsigned)blocks, threads, smem, st>>>(a, nrow, o, heavy, nvisit);
+    if (w.warps) *w.warps = blocks * (uint64_t)(threads / 32);
+    else k1<<<(unsigned)blocks, threads, smem, w.st>>>(a, nrow, o, heavy, nvisit);
     // the slices of the heavy items, whose number only the device knows
-    e = warp_grid((const void*)k2, L.total, a.shape_warps, a.shape_per_sm, heavy.cap, num_sms, threads, smem, blocks);
+    e = warp_grid((const void*)k2, L.total, a.shape_warps, a.shape_per_sm, heavy.cap, w.num_sms, threads, smem, blocks);
     if (e != cudaSuccess) return e;
-    k2<<<(unsigned)blocks, threads, smem, st>>>(a, nrow, o, heavy, nvisit);
-    *launches += 2;
+    if (w.warps) {
+        *w.warps += blocks * (uint64_t)(threads / 32);
+        return cudaSuccess;
+    }
+    k2<<<(unsigned)blocks, threads, smem, w.st>>>(a, nrow, o, heavy, nvisit);
+    *w.launches += 2;
     return cudaGetLastError();
 }
 
@@ -648,14 +656,14 @@ uint32_t join_unit_steps(double cand, int num_sms) {
 // The register form's dispatch: false when the join takes k_join.
 template <bool STAMP>
 static bool try_reg(const JoinArgs<float>& a, int model, uint32_t nrow, const TileOut& o, const HeavyList& heavy,
-                    uint32_t nvisit, int num_sms, int* launches, cudaStream_t st, cudaError_t* e) {
+                    uint32_t nvisit, const WarpLaunch& w, cudaError_t* e) {
     if (a.n > 16 || a.npad != npad_for(a.n, 4u) || a.npad < 4u || (a.npad & 3u)) return false;
     const bool seq = model == kSeq || a.ilp <= 1u;
     const bool first = !seq && a.ilp >= a.n;
     if (!seq && !first && model != kIlpSc) return false;  // ILP chains of several dims
 #define GSJ_REG(NP, SUM, G)                                                                            \
     do {                                                                                               \
-        *e = launch_reg<NP, SUM, G, STAMP>(a, nrow, o, heavy, nvisit, num_sms, launches, st);           \
+        *e = launch_reg<NP, SUM, G, STAMP>(a, nrow, o, heavy, nvisit, w);           \
         return true;                                                                                   \
     } while (0)
     if (seq) {
@@ -679,61 +687,59 @@ static bool try_reg(const JoinArgs<float>& a, int model, uint32_t nrow, const Ti
 }
 
 template <typename T, int MODEL, int POL, bool STAMP>
-static cudaError_t dispatch_nt(const JoinArgs<T>& a, uint32_t nrow, const TileOut& o, uint32_t nvisit, int num_sms,
-                               int* launches, cudaStream_t st) {
+static cudaError_t dispatch_nt(const JoinArgs<T>& a, uint32_t nrow, const TileOut& o, uint32_t nvisit, const WarpLaunch& w) {
     if constexpr (MODEL == kSeq) {
         if (a.npad == npad_for(a.n, sizeof(T))) {
             switch (a.n) {
-                case 1: return launch_one<T, 1, MODEL, POL, STAMP>(a, nrow, o, nvisit, num_sms, launches, st);
-                case 2: return launch_one<T, 2, MODEL, POL, STAMP>(a, nrow, o, nvisit, num_sms, launches, st);
+                case 1: return launch_one<T, 1, MODEL, POL, STAMP>(a, nrow, o, nvisit, w);
+                case 2: return launch_one<T, 2, MODEL, POL, STAMP>(a, nrow, o, nvisit, w);
                 default: break;
             }
             if constexpr (sizeof(T) == 8) {
                 switch (a.n) {
-                    case 3: return launch_one<T, 3, MODEL, POL, STAMP>(a, nrow, o, nvisit, num_sms, launches, st);
-                    case 4: return launch_one<T, 4, MODEL, POL, STAMP>(a, nrow, o, nvisit, num_sms, launches, st);
-                    case 6: return launch_one<T, 6, MODEL, POL, STAMP>(a, nrow, o, nvisit, num_sms, launches, st);
-                    case 8: return launch_one<T, 8, MODEL, POL, STAMP>(a, nrow, o, nvisit, num_sms, launches, st);
+                    case 3: return launch_one<T, 3, MODEL, POL, STAMP>(a, nrow, o, nvisit, w);
+                    case 4: return launch_one<T, 4, MODEL, POL, STAMP>(a, nrow, o, nvisit, w);
+                    case 6: return launch_one<T, 6, MODEL, POL, STAMP>(a, nrow, o, nvisit, w);
+                    case 8: return launch_one<T, 8, MODEL, POL, STAMP>(a, nrow, o, nvisit, w);
                     default: break;
                 }
             }
         }
     }
-    return launch_one<T, 0, MODEL, POL, STAMP>(a, nrow, o, nvisit, num_sms, launches, st);
+    return launch_one<T, 0, MODEL, POL, STAMP>(a, nrow, o, nvisit, w);
 }
 
 template <typename T, bool STAMP>
 static cudaError_t dispatch_model(const JoinArgs<T>& a, int model, uint32_t nrow, const TileOut& o,
-                                  const HeavyList& heavy, uint32_t nvisit, int num_sms, int* launches,
-                                  cudaStream_t st) {
+                                  const HeavyList& heavy, uint32_t nvisit, const WarpLaunch& w) {
     constexpr int P = sizeof(T) == 8 ? kPolF64 : kPolF32;
     if constexpr (sizeof(T) == 4) {
         cudaError_t e = cudaSuccess;
-        if (try_reg<STAMP>(a, model, nrow, o, heavy, nvisit, num_sms, launches, st, &e)) return e;
+        if (try_reg<STAMP>(a, model, nrow, o, heavy, nvisit, w, &e)) return e;
     }
     switch (model) {
-        case kSeq: return dispatch_nt<T, kSeq, P, STAMP>(a, nrow, o, nvisit, num_sms, launches, st);
-        case kIlp: return dispatch_nt<T, kIlp, P, STAMP>(a, nrow, o, nvisit, num_sms, launches, st);
-        case kIlpSc: return dispatch_nt<T, kIlpSc, P, STAMP>(a, nrow, o, nvisit, num_sms, launches, st);
+        case kSeq: return dispatch_nt<T, kSeq, P, STAMP>(a, nrow, o, nvisit, w);
+        case kIlp: return dispatch_nt<T, kIlp, P, STAMP>(a, nrow, o, nvisit, w);
+        case kIlpSc: return dispatch_nt<T, kIlpSc, P, STAMP>(a, nrow, o, nvisit, w);
         default: return cudaErrorInvalidValue;
     }
 }
 
 template <typename T>
 cudaError_t launch_join_emit(const JoinArgs<T>& a, const TileOut& o, const HeavyList& heavy, uint32_t nvisit,
-                             int model, bool stamp, int num_sms, int* launches, cudaStream_t st) {
+                             int model, bool stamp, const WarpLaunch& w) {
     uint32_t nrow = 1;  // neighbour rows: 3^(k-1)
     for (uint32_t j = 1; j < a.g.k; j++) nrow *= 3u;
     if (o.stride == 0 || !heavy.list || heavy.cap == 0 || heavy.cap > kHeavyCap || heavy.unit == 0) return cudaErrorInvalidValue;
     if (nvisit == 0) return cudaSuccess;
     if ((uint64_t)(nvisit - 1) * o.stride >= a.num_items) return cudaErrorInvalidValue;
-    return stamp ? dispatch_model<T, true>(a, model, nrow, o, heavy, nvisit, num_sms, launches, st)
-                 : dispatch_model<T, false>(a, model, nrow, o, heavy, nvisit, num_sms, launches, st);
+    return stamp ? dispatch_model<T, true>(a, model, nrow, o, heavy, nvisit, w)
+                 : dispatch_model<T, false>(a, model, nrow, o, heavy, nvisit, w);
 }
 
 template cudaError_t launch_join_emit<float>(const JoinArgs<float>&, const TileOut&, const HeavyList&, uint32_t, int,
-                                             bool, int, int*, cudaStream_t);
+                                             bool, const WarpLaunch&);
 template cudaError_t launch_join_emit<double>(const JoinArgs<double>&, const TileOut&, const HeavyList&, uint32_t, int,
-                                              bool, int, int*, cudaStream_t);
+                                              bool, const WarpLaunch&);
 
 }  // namespace gsj

@@ -82,9 +82,15 @@ struct HeavyList {
 };
 constexpr uint32_t kHeavyCap = 1u << 20;
 uint32_t join_unit_steps(double cand, int num_sms);
+struct WarpLaunch {
+    int num_sms;
+    cudaStream_t st;
+    int* launches;    // advanced by the kernels launched
+    uint64_t* warps;  // not null: nothing is launched, *warps = warps of the pass's launches
+};
 template <typename T>
 cudaError_t launch_join_emit(const JoinArgs<T>& a, const TileOut& o, const HeavyList& heavy, uint32_t nvisit,
-                             int model, bool stamp, int num_sms, int* launches, cudaStream_t st);
+                             int model, bool stamp, const WarpLaunch& w);
 
 // ROWS path: dense low-dimensional grids (k <= 3, n <= 4), full neighbourhood.
 // slot_cell[s] = cell of slot s; a.plan holds 3^(k-1) rows a cell.
