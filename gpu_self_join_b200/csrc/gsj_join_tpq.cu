@@ -333,12 +333,20 @@ static cudaError_t launch_rows(const JoinArgs<T>& a, const uint32_t* slot_cell, 
     constexpr int POL = sizeof(T) == 8 ? kPolF64 : kPolF32;
     if constexpr (!FILL) {
         // Sparse cells leave the lanes of k_rows_join's cells half empty and pay its
-        // set-up for few queries; from about 7 points a cell on (5 in double) the
-        // cell form is faster.  Count pass, cell form against thread per query: 2-D
-        // 20M at 3.1 points a cell 1.76 / 0.93 ms, 3-D 2M at 7.3 0.349 / 0.357,
-        // 3-D 250k double at 7.0 0.082 / 0.113, 3-D 2M with 2 dims indexed at 175
-        // 1.46 / 1.68.
-        if (a.n_points < (sizeof(T) == 8 ? 5u : 7u) * (uint64_t)a.num_cells)
+        // set-up for few queries.  Count pass, cell form / thread per query (ms, uniform
+        // points, points a non-empty cell): nine rows: 3-D 2M at 5.0 0.293 / 0.267, 5.9 0.312 /
+        // 0.306, 7.0 0.314 / 0.344, 250k at 4.0 0.057 / 0.053, 5.9 0.064 / 0.068, 4-D 1M at
+        // 6.0 0.181 / 0.177, 6.8 0.189 / 0.195; in double 3-D 2M at 5.0 0.480 / 0.428, 5.9
+        // 0.496 / 0.484, 250k at 3.1 0.074 / 0.068, 5.0 0.074 / 0.089, 4-D 1M at 4.1 0.234 /
+        // 0.246.  Three rows: 2-D 4M at 7.0 0.228 / 0.158, 10 0.226 / 0.195, in double at 7.0
+        // 0.269 / 0.250, 8.0 0.271 / 0.277, a 2-D mixture 8M at 9.1 1.14 / 1.18; 4-D 1M at 6.0 0.080 / 0.074, 7.0 0.080 / 0.082, in
+        // double at 6.0 0.119 / 0.119.  One row: 1-D 4M at 10 0.129 / 0.119, in double 0.160 /
+        // 0.123.
+        constexpr uint32_t line = NR == 9   ? (sizeof(T) == 8 ? 5u : 6u)
+                                  : NR == 1 ? 10u
+                                  : NT <= 2 ? (sizeof(T) == 8 ? 7u : 8u)
+                                            : 6u;
+        if (a.n_points < line * (uint64_t)a.num_cells)
             return launch_form<T>(k_rows_thread<T, NT, NR, POL, false>, a, slot_cell, counts_by_id, qslots, nq, base,
                                   num_sms, st);
         return launch_form<T>(k_rows_join<T, NT, NR, POL, kCountOnly>, a, slot_cell, counts_by_id, qslots, nq, base,
@@ -349,10 +357,10 @@ static cudaError_t launch_rows(const JoinArgs<T>& a, const uint32_t* slot_cell, 
         // and 4.1 result pairs a point 0.497 / 0.277, 2.3 and 7.3 0.402 / 0.418, 3.2 and
         // 10.4 0.361 / 0.542; 3-D 2M at 1.6 and 5.2 0.359 / 0.201, 3.1 and 13.4 0.369 /
         // 0.348, 4.0 and 17.5 0.403 / 0.437 (double 1.6 0.620 / 0.262); 1-D 4M at 2.3
-        // and 5.2 0.324 / 0.292, 4.1 and 9.2 0.259 / 0.482.  So sparse cells (the count
-        // pass's line) take a thread per query while it stores few ids, each to a sector
-        // of its own; with many candidates a point (4-D 500k, 130 of them and 1.5 pairs:
-        // 0.145 / 0.148, double 0.162 / 0.195) the cell form is the better one again.
+        // and 5.2 0.324 / 0.292, 4.1 and 9.2 0.259 / 0.482.  So sparse cells take a
+        // thread per query while it stores few ids, each to a sector of its own; with
+        // many candidates a point (4-D 500k, 130 of them and 1.5 pairs: 0.145 / 0.148,
+        // double 0.162 / 0.195) the cell form is the better one again.
         if (N < (sizeof(T) == 8 ? 5u : 7u) * (uint64_t)a.num_cells && pairs <= (NR == 1 ? 6u : 4u + NR) * N &&
             cands <= 96u * N)
             return launch_form<T>(k_rows_thread<T, NT, NR, POL, true>, a, slot_cell, counts_by_id, qslots, nq, base,
