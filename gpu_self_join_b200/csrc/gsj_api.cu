@@ -418,6 +418,15 @@ int stage_times(gsj_context* c, bool estimate) {
     return GSJ_OK;
 }
 
+// Host times of the join that began at t_start: the host does not wait for the index
+// build's last kernels, so their device time belongs to ms_index too.
+void host_times(gsj_stats& S, double t_join, double t_start) {
+    const double late = std::max(0.0, S.dev_ms_index - S.ms_index);
+    S.ms_index += late;
+    S.ms_join = now_ms() - t_join - late;
+    S.ms_total = now_ms() - t_start;
+}
+
 // Entries a block-reserving pass may take for `real` entries: each warp
 // reserves blocks of `block` entries and abandons its block (padding the tail)
 // when the next chunk of at most `max_chunk` entries does not fit (1: chunks
@@ -643,8 +652,7 @@ int emit_join(gsj_context* c, JoinArgs<T>& a, uint64_t N, bool stamp, int model,
     GSJ_CUDA(c, cudaEventRecord(c->tev[3], st));
     GSJ_TRY(pairs_to_csr(c, pairs, used, R, shift, N, counts, offsets, cand));
     S.join_path = GSJ_PATH_WARP;
-    S.ms_join = now_ms() - t_join;
-    S.ms_total = now_ms() - t_start;
+    host_times(S, t_join, t_start);
     return GSJ_OK;
 }
 
@@ -848,8 +856,7 @@ int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int mo
     S.screen_rechecks = screen ? U : 0;
     c->screened = screen;
     S.join_path = a.n >= kScreenPathDims && screen ? GSJ_PATH_SCREEN : GSJ_PATH_TILE;
-    S.ms_join = now_ms() - t_join;
-    S.ms_total = now_ms() - t_start;
+    host_times(S, t_join, t_start);
     return GSJ_OK;
 }
 
@@ -1086,8 +1093,7 @@ int sort_join(gsj_context* c, JoinArgs<T>& a, uint64_t N, int model, uint32_t* c
     S.join_path = GSJ_PATH_SORT;
     c->R = R;
     c->have_result = true;
-    S.ms_join = now_ms() - t_join;
-    S.ms_total = now_ms() - t_start;
+    host_times(S, t_join, t_start);
     return GSJ_OK;
 }
 
@@ -1514,12 +1520,11 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
         uint32_t errflag = 0;
         GSJ_TRY(d2h_small(c, &errflag, ctr + 1, 1));
         if (errflag) return fail(c, GSJ_ERR_STATE, "fill pass: a list would leave its segment (internal error)");
-        S.ms_join = now_ms() - t_join;
         S.total_pairs = R;
         S.join_path = GSJ_PATH_ROWS;
         c->R = R;
         c->have_result = true;
-        S.ms_total = now_ms() - t_start;
+        host_times(S, t_join, t_start);
         return GSJ_OK;
     }
     uint32_t* table = nullptr;
@@ -1545,12 +1550,11 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
         GSJ_CUDA(c, cudaStreamSynchronize(st));
     }
     GSJ_TRY(stage_times(c, false));
-    S.ms_join = now_ms() - t_join;
     S.total_pairs = R;
     S.join_path = GSJ_PATH_ROWS;
     c->R = R;
     c->have_result = true;
-    S.ms_total = now_ms() - t_start;
+    host_times(S, t_join, t_start);
     return GSJ_OK;
 }
 
