@@ -461,6 +461,8 @@ int validate(gsj_context* c, const gsj_config& cfg, uint64_t N) {
 }
 
 // ------------------------------------------------------------------ lists ascending
+// (The counters and flags of this and the next section start at zero: run_join
+// clears `misc` at its start and before any second try at a join's pairs.)
 // Sorts every list of the table ascending (ids below N): a warp per list up
 // to 256 entries, a CTA bitonic network up to 4096, CTA radix passes with a
 // scratch copy of the table above.  The numbers of long lists are queued on `rb`
@@ -1462,7 +1464,9 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
                                         t_start);
                 if (r != kTakePlain && r != GSJ_ERR_NOMEM) return r;
                 // the bound decides nothing, or the undecided pairs do not fit: the FP32
-                // tiles, which need room for the result pairs alone
+                // tiles, which need room for the result pairs alone.  The first try may
+                // have come as far as the table's lists: their counters start over too
+                GSJ_CUDA(c, cudaMemsetAsync(d_mm, 0, kMiscWords * sizeof(uint32_t), st));
                 if (r == GSJ_ERR_NOMEM) {
                     c->err.clear();
                     dev_release(c->unc);
