@@ -1485,8 +1485,17 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     // Every other grid except the thread-per-query rows: one emit pass + pair sort.
     if (!tpq) {
         unsigned long long* cursor = reinterpret_cast<unsigned long long*>(ctr + 4);
-        return emit_join<T>(c, a, N, stamp, model, exact_size, learned, counts, offsets, cursor, t_join,
-                            t_start);
+        int r = emit_join<T>(c, a, N, stamp, model, exact_size, learned, counts, offsets, cursor, t_join, t_start);
+        if (r == GSJ_ERR_NOMEM && a.plan) {
+            // the row plan is the one buffer that the join can do without
+            GSJ_CUDA(c, cudaMemsetAsync(d_mm, 0, kMiscWords * sizeof(uint32_t), st));
+            c->err.clear();
+            dev_release(c->plan);
+            dev_release(c->pairs);
+            a.plan = nullptr;
+            r = emit_join<T>(c, a, N, stamp, model, exact_size, learned, counts, offsets, cursor, t_join, t_start);
+        }
+        return r;
     }
     // Dense low-dimensional grids (the ROWS path): the distance work is cheap, so
     // a count pass gives every list its place and a fill pass repeats the tests.
@@ -1898,6 +1907,7 @@ int gsj_result_device(gsj_context* c, const uint32_t** counts, const uint64_t** 
 int gsj_test_slice_list(gsj_context* c, uint32_t cap, uint64_t before, uint64_t* found) {
     if (!c) return fail(c, GSJ_ERR_INVALID, "null context");
     if (cap > kHeavyCap) return fail(c, GSJ_ERR_INVALID, "slice list: capacity above the built-in one");
+    if (before >> 62) return fail(c, GSJ_ERR_INVALID, "slice list: count beyond what a join can reach");
     if (found) *found = c->slices_found;
     c->slice_cap = cap ? cap : kHeavyCap;
     c->slices_before = before;
