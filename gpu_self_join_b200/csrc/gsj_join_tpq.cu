@@ -267,12 +267,12 @@ __global__ void __launch_bounds__(256) k_rows_thread(const JoinArgs<T> a, const 
         if (i < nq) {
             const uint32_t s = FILL && qslots ? qslots[i] : i;
             const uint32_t cell = slot_cell[s];
-            const uint32_t id = a.ids[s];
             T q[NT];
             load_row<T, NT>(a.pts + (size_t)s * npad, q);
             uint32_t cnt = 0, len = 0;
             uint32_t* list = nullptr;
             if (FILL) {
+                const uint32_t id = a.ids[s];
                 const unsigned long long dst = a.offsets[id] - base;
                 len = (uint32_t)(a.offsets[id + 1] - a.offsets[id]);
                 if (dst + len > a.table_cap) {
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(256) k_rows_thread(const JoinArgs<T> a, const 
                     cnt += hit ? 1u : 0u;
                 }
             }
-            if (!FILL) counts_by_id[id] = cnt;
+            if (!FILL) counts_by_id[a.ids[s]] = cnt;
             else if (cnt != len) *a.err_flag = 1u;
         }
         cur = __shfl_sync(FULL, nxt, 0);
