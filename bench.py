@@ -164,12 +164,11 @@ def _roofline(stats: list, N: int, n: int, R: int, w) -> dict:
     paths: the estimate + the pair-emitting pass) and "fill" (ROWS: the fill
     pass; the other paths: pair placement + list sort).  Algorithmic bytes per
     launch (C = candidate evaluations):
-      join_fill   table 4R written, coordinates and per-query data 24N, one
-                  decision bit per candidate C/8 (the passes share no decisions:
-                  the fill repeats the tests in registers, so this term is not
-                  memory traffic)
-      join_count  coordinates 4Nn, ids 4N, list lengths 8N (by slot and by id),
-                  decision bits C/8 (as above)
+      join_fill   table 4R written, coordinates and per-query data 24N
+      join_count  coordinates 4Nn, ids 4N, list lengths 8N (by slot and by id)
+                  (both figures of `algorithmic_bytes` and what follows from them also
+                  hold a decision bit per candidate, C/8, which the passes once shared
+                  through memory; `memory` is without it)
       join_emit   coordinates 4Nn + ids 4N + 8-byte pair keys 8R
       pair_place  keys 8R read + table 4R + offsets 8N written
     The screen is a tensor-core kernel: 2(n+2) FLOPs per screened pair (one
@@ -201,12 +200,16 @@ def _roofline(stats: list, N: int, n: int, R: int, w) -> dict:
             kwork = 2.0 * (n + 2) * C
             pk, peak_kind = _tensor_peak()
     achieved = kwork / (kms / 1e3) / (1e12 if unit == "TFLOP/s" else 1e9)
+    # the bytes that must move: the ROWS passes keep every decision in registers
+    moved = kwork - (C / 8.0 if path == 1 else 0.0)
     join_ms = index_ms + count_ms + fill_ms
     b_alg = b_coords + 4.0 * N + 4.0 * R
     roof = {"bound": bound, "kernel": kname, "achieved": achieved, "peak": pk, "unit": unit,
             "frac": achieved / pk, "peak_source": peak_kind,
             ("algorithmic_flops" if unit == "TFLOP/s" else "algorithmic_bytes"): kwork,
             "kernel_ms": kms, "traffic": _traffic_from_profile(kname, w.name),
+            **({"memory": {"bytes": moved, "gbs": moved / (kms / 1e3) / 1e9, "frac": moved / (kms / 1e3) / 1e9 / pk}}
+               if unit == "GB/s" else {}),
             "stage_ms": {"index": index_ms, "count": count_ms, "fill": fill_ms},
             "join": {"ms": join_ms, "algorithmic_bytes": b_alg, "achieved_gbs": b_alg / (join_ms / 1e3) / 1e9,
                      "frac": b_alg / (join_ms / 1e3) / 1e9 / peak}}

@@ -464,7 +464,7 @@ int validate(gsj_context* c, const gsj_config& cfg, uint64_t N) {
 // (The counters and flags of this and the next section start at zero: run_join
 // clears `misc` at its start and before any second try at a join's pairs.)
 // Sorts every list of the table ascending (ids below N): a warp per list up
-// to 256 entries, a CTA bitonic network up to 4096, CTA radix passes with a
+// to 512 entries, a CTA (its warps' runs merged) up to 4096, CTA radix passes with a
 // scratch copy of the table above.  The numbers of long lists are queued on `rb`
 // (nlong); the caller waits and calls sort_very_long.
 int sort_table_lists(gsj_context* c, uint32_t* table, const uint64_t* offsets, uint64_t N, Readback& rb,
@@ -591,10 +591,10 @@ int emit_join(gsj_context* c, JoinArgs<T>& a, uint64_t N, bool stamp, int model,
     o.stride = 1;
     int nl = 0;
     // a warp appends at most 64 keys at once (32 hits and their reverse keys) and may
-    // leave one block of kScreenBlockSlack keys partly filled
+    // leave one block of kKeyBlock keys partly filled
     uint64_t warps = 0;
     GSJ_CUDA(c, launch_join_emit<T>(a, o, heavy, ni, model, stamp, WarpLaunch{c->num_sms, st, &nl, &warps}));
-    const uint64_t slack = warps * kScreenBlockSlack;
+    const uint64_t slack = warps * kKeyBlock;
     auto reset = [&]() -> int {
         GSJ_CUDA(c, cudaMemsetAsync(a.work_counter, 0, 4 * sizeof(uint32_t), st));
         // the cursor and the key count, then the heavy list's counters
@@ -633,7 +633,7 @@ int emit_join(gsj_context* c, JoinArgs<T>& a, uint64_t N, bool stamp, int model,
     unsigned long long* pairs = nullptr;
     unsigned long long used = 0, R = 0;
     for (int attempt = 0; attempt < 3; attempt++) {
-        cap = retry_cap(attempt, estimate, used, reserve_bound(R, warps, kScreenBlockSlack, 64u));
+        cap = retry_cap(attempt, estimate, used, reserve_bound(R, warps, kKeyBlock, 64u));
         GSJ_TRY(dev_get(c, c->pairs, cap ? cap : 1, &pairs));
         GSJ_TRY(reset());
         o.emit = true;

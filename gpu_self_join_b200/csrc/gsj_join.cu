@@ -73,9 +73,9 @@ __host__ __device__ inline WarpSmem warp_smem_layout(uint32_t npad, uint32_t tsi
 // The warp appends its hits as packed (query id << shift |
 // candidate id) keys, and with unicomp the reverse key of a hit in another
 // cell, into blocks of kEmitBlk entries it reserves on o.cursor (unused tails
-// padded with kUndecidedPad, which sorts after every key); emitted counts the
+// padded with kKeyPad, which sorts after every key); emitted counts the
 // keys exactly.  hit / cr are this lane's flags, b / cb their ballots.
-constexpr uint32_t kEmitBlk = (uint32_t)kScreenBlockSlack;
+constexpr uint32_t kEmitBlk = (uint32_t)kKeyBlock;
 
 __device__ __forceinline__ void emit_keys(const TileOut& o, unsigned long long& blk_base, uint32_t& blk_used,
                                           unsigned long long& emitted, bool hit, bool cr, unsigned b, unsigned cb,
@@ -85,7 +85,7 @@ __device__ __forceinline__ void emit_keys(const TileOut& o, unsigned long long& 
     if (!o.emit) return;
     if (blk_used + cnt > kEmitBlk) {
         for (uint32_t e = blk_used + (uint32_t)lane; e < kEmitBlk; e += 32u)
-            if (blk_base + e < o.cap) o.pairs[blk_base + e] = kUndecidedPad;
+            if (blk_base + e < o.cap) o.pairs[blk_base + e] = kKeyPad;
         unsigned long long nb = 0;
         if (lane == 0) nb = atomicAdd(o.cursor, (unsigned long long)kEmitBlk);
         blk_base = __shfl_sync(0xffffffffu, nb, 0);
@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_join(const Join
     if (lane == 0 && cand_total) atomicAdd(a.cand_cnt, cand_total);
     if (o.emit && blk_used < kEmitBlk)
         for (uint32_t e = blk_used + (uint32_t)lane; e < kEmitBlk; e += 32u)
-            if (blk_base + e < o.cap) o.pairs[blk_base + e] = kUndecidedPad;
+            if (blk_base + e < o.cap) o.pairs[blk_base + e] = kKeyPad;
     if (lane == 0 && emitted) atomicAdd(o.rechecks, emitted);
 }
 
@@ -558,7 +558,7 @@ __global__ void __launch_bounds__(256, 4) k_join_reg(const JoinArgs<float> a, ui
     if (!SLICES && lane == 0 && cand_total) atomicAdd(a.cand_cnt, cand_total);
     if (o.emit && blk_used < kEmitBlk)
         for (uint32_t e = blk_used + (uint32_t)lane; e < kEmitBlk; e += 32u)
-            if (blk_base + e < o.cap) o.pairs[blk_base + e] = kUndecidedPad;
+            if (blk_base + e < o.cap) o.pairs[blk_base + e] = kKeyPad;
     if (lane == 0 && emitted) atomicAdd(o.rechecks, emitted);
 }
 

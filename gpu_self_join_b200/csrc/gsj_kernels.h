@@ -179,9 +179,10 @@ ScreenConst make_screen_const(uint32_t n, float thr);
 // counts records; o.rechecks receives the exact number of undecided pairs.
 // Without emission o.cursor receives the number of records.
 constexpr uint32_t kScreenBlock = 256;
-// Keys of the warp join: blocks of kScreenBlockSlack entries, unused tails kUndecidedPad.
-constexpr unsigned long long kUndecidedPad = ~0ull;
-constexpr uint64_t kScreenBlockSlack = 1024;
+// Keys of the warp join: its warps reserve blocks of kKeyBlock entries; the unused
+// tails hold kKeyPad, which no key equals.
+constexpr unsigned long long kKeyPad = ~0ull;
+constexpr uint64_t kKeyBlock = 1024;
 cudaError_t launch_tile_screen(const JoinArgs<float>& a, const TileOut& o, const ScreenConst& sc, bool stamp,
                                int model, uint32_t nvisit, int num_sms, cudaStream_t st);
 // Exact check of the undecided pairs; hits go to o as packed (query id, candidate id) keys.

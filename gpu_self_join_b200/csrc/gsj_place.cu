@@ -184,7 +184,7 @@ __device__ __forceinline__ void warp_sort_list(uint32_t* __restrict__ list, uint
     }
 }
 
-// Every list of min_len+1..kWarpSortMax entries sorted by one warp (the
+// Every list of 2..kWarpSortMax entries sorted by one warp (the
 // network sized to the list: 32, 64, ... 512 entries); lists above
 // kWarpSortMax are gathered into long_lists (*nlong, warp-aggregated), those
 // above kCtaSortMax counted in *nvery.  List l: table[offsets[l] ..
@@ -192,7 +192,7 @@ __device__ __forceinline__ void warp_sort_list(uint32_t* __restrict__ list, uint
 template <typename OffT>
 __global__ void __launch_bounds__(256) k_list_sort_short(uint32_t* __restrict__ table,
                                                          const OffT* __restrict__ offsets, uint32_t nlists,
-                                                         uint32_t min_len, uint32_t* __restrict__ long_lists,
+                                                         uint32_t* __restrict__ long_lists,
                                                          uint32_t* __restrict__ nlong) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(256) k_list_sort_short(uint32_t* __restrict__ 
             const unsigned vl = __ballot_sync(FULL, len > kCtaSortMax);
             if (vl && lane == 0) atomicAdd(nlong + 1, (uint32_t)__popc(vl));
         }
-        unsigned mine = __ballot_sync(FULL, len > min_len && len > 1u && len <= kWarpSortMax);
+        unsigned mine = __ballot_sync(FULL, len > 1u && len <= kWarpSortMax);
         while (mine) {
             const int j = __ffs(mine) - 1;
             mine &= mine - 1u;
@@ -397,7 +397,7 @@ cudaError_t sort_lists(uint32_t* table, const OffT* offsets, uint32_t nlists, vo
     if (nlists == 0) return cudaSuccess;
     uint32_t* ll = static_cast<uint32_t*>(temp);
     const unsigned g = grid_for((uint64_t)nlists, 256, (uint64_t)num_sms * 64);
-    k_list_sort_short<OffT><<<g, 256, 0, st>>>(table, offsets, nlists, 1u, ll, d_nlong);
+    k_list_sort_short<OffT><<<g, 256, 0, st>>>(table, offsets, nlists, ll, d_nlong);
     // the longer lists' number stays on the device: a CTA that finds none ends at once
     k_list_sort_cta<OffT><<<grid_for(nlists, 1, (uint64_t)num_sms * 6), kCtaSortThreads, 0, st>>>(table, offsets, ll,
                                                                                                  d_nlong);

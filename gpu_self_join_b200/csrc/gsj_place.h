@@ -7,7 +7,7 @@
 
 namespace gsj {
 
-// Temporary bytes of place_pairs / find_long_lists for nlists lists.
+// Temporary bytes of place_pairs, sort_lists and sort_very_long_lists for nlists lists.
 size_t place_temp_bytes(uint64_t nlists);
 
 // Lists of the packed keys (query id << shift | neighbour id; entries equal
@@ -20,10 +20,10 @@ cudaError_t place_pairs(const unsigned long long* keys, uint64_t nkeys, uint32_t
                         uint32_t* counts, uint64_t* offsets, uint32_t* table, uint64_t cap, uint32_t* cursor,
                         uint32_t* err, void* temp, int num_sms, int* launches, cudaStream_t st);
 
-// Sorts every list of up to 4096 entries ascending (a warp per list up to 256
-// entries, a CTA above) and gathers the indices of the lists above 256 into
+// Sorts every list of up to 4096 entries ascending (a warp per list up to 512
+// entries, a CTA above) and gathers the indices of the lists above 512 into
 // temp.  List l is table[offsets[l] .. offsets[l+1]).  d_nlong: two device
-// words, zeroed by the caller, which receive the number of lists above 256 and
+// words, zeroed by the caller, which receive the number of lists above 512 and
 // above 4096 entries.
 template <typename OffT>
 cudaError_t sort_lists(uint32_t* table, const OffT* offsets, uint32_t nlists, void* temp, uint32_t* d_nlong,

@@ -111,13 +111,13 @@ typedef struct gsj_stats {
     double ms_h2d;            /* host->device copy of the dataset               */
     double ms_index;          /* REORDER + grid extents + on-device index build */
     double ms_join;           /* join: count + offsets + fill (ROWS), or pair
-                                 emission + pair sort + table (other paths)     */
+                                 emission + placement + list sort (other paths) */
     double ms_d2h;            /* result copies to the host                      */
     double ms_total;          /* whole call                                     */
     /* device time (CUDA events on the context's stream) */
     double dev_ms_index;      /* index build: keys, sort, cells, lookup, items  */
     double dev_ms_count;      /* count pass (other paths: the distance pass)    */
-    double dev_ms_fill;       /* fill pass (other paths: pair sort + table)     */
+    double dev_ms_fill;       /* fill pass (other paths: placement + list sort) */
     uint64_t kernel_launches; /* launches of this library's own kernels         */
     uint64_t join_path;       /* GSJ_PATH_* taken by the last join              */
     uint64_t screen_rechecks; /* GSJ_PATH_TILE, GSJ_PATH_SCREEN: pairs the BF16 screen
@@ -135,15 +135,19 @@ typedef struct gsj_stats {
 } gsj_stats;
 
 /* Join paths (gsj_stats.join_path). */
-#define GSJ_PATH_WARP 0u  /* warp per (cell, 32 queries): pair keys + on-device sort */
-#define GSJ_PATH_ROWS 1u  /* dense k <= 3, n <= 4: thread-per-query count + fill   */
+#define GSJ_PATH_WARP 0u  /* warp per (cell, 32 queries): pair keys, placed into
+                             their lists, every list sorted                   */
+#define GSJ_PATH_ROWS 1u  /* dense k <= 3, n <= 4: count + fill, a warp per cell
+                             or a thread per query                            */
 #define GSJ_PATH_TILE 2u  /* float, 5 <= n <= 128, k <= 6, >= 8 points per cell:
-                             screened below 16 dimensions like GSJ_PATH_SCREEN, with
-                             GSJ_FLAG_PLAIN (or above 126) 64 x 64 register tiles
-                             of the exact arithmetic                          */
-#define GSJ_PATH_SCREEN 3u /* float, 16 <= n <= 128, k <= 6, >= 8 points per cell:
+                             screened below 16 dimensions like GSJ_PATH_SCREEN; 64 x
+                             64 register tiles of the exact arithmetic with
+                             GSJ_FLAG_PLAIN, above 126 dimensions, below 16 where
+                             the screen's bound decides nothing, and where the
+                             undecided pairs do not fit the device            */
+#define GSJ_PATH_SCREEN 3u /* float, 16 <= n <= 126, k <= 6, >= 8 points per cell:
                              BF16 tcgen05 screen with a proven bound, exact FP32
-                             check of the rest, pair buffer, on-device sort   */
+                             check of the rest, then as GSJ_PATH_WARP         */
 #define GSJ_PATH_SORT 4u  /* cfg.sort: thread per query, the reference's pruned
                              scans of sorted cells, count + fill              */
 
