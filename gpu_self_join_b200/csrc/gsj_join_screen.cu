@@ -335,9 +335,10 @@ __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_
 // metadata says whether four groups are consecutive, which makes one record a
 // query row; records go to a block that is never split).  A tile takes some 530
 // cycles of an SM at K = 32 (the tensor pipe needs 128) and 650 at K = 96 (384).
-// Measured (both launches of a join): 18-D 5M points 270 -> 97 ms, 90-D 515k 117
-// -> 33 ms, 32-D 45k 2.0 -> 0.61 ms, against four warps staging rows one by one
-// with cp.async and a compare per pair with a bound per 32 candidates (1,720
+// Measured (count stage of a join, the exact check included): 18-D 5M points 380 ->
+// 145 ms (126 of it this kernel, 3 its sampling pass), 90-D 515k 121 -> 38 ms, 32-D
+// 45k 2.0 -> 0.61 ms (both launches alone), against four warps staging rows one by
+// one with cp.async and a compare per pair with a bound per 32 candidates (1,720
 // cycles a tile).  Tried without gain: 16 consumer warps a CTA reading 16 columns
 // at a time, an MMA warp per accumulator.
 template <bool STAMP>
