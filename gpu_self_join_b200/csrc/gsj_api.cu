@@ -594,7 +594,9 @@ int emit_join(gsj_context* c, JoinArgs<T>& a, uint64_t N, bool stamp, int model,
     // leave one block of kKeyBlock keys partly filled
     uint64_t warps = 0;
     GSJ_CUDA(c, launch_join_emit<T>(a, o, heavy, ni, model, stamp, WarpLaunch{c->num_sms, st, &nl, &warps}));
-    const uint64_t slack = warps * kKeyBlock;
+    // the estimate's margin: the partly filled blocks, and for small joins, of which the
+    // sample sees a handful of items, what it misses
+    const uint64_t slack = std::max<uint64_t>(warps, (uint64_t)c->num_sms * 64u) * kKeyBlock;
     auto reset = [&]() -> int {
         GSJ_CUDA(c, cudaMemsetAsync(a.work_counter, 0, 4 * sizeof(uint32_t), st));
         // the cursor and the key count, then the heavy list's counters
@@ -703,6 +705,10 @@ int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int mo
         GSJ_CUDA(c, cudaMemsetAsync(a.work_counter, 0, 4 * sizeof(uint32_t), st));
         GSJ_CUDA(c, cudaMemsetAsync(cursor, 0, 2 * sizeof(unsigned long long), st));
         return GSJ_OK;
+    // the estimate's margin: for small joins, of which the sample sees a handful of
+    // items, also what it misses (6,000 points in 15-D: 2.6 M estimated, 8.8 M undecided;
+    // the repeated pass 0.64 -> 0.82 ms)
+    const uint64_t margin = 4u * slack;
     };
     auto launch = [&](uint32_t nvisit) -> cudaError_t {
         return screen ? launch_tile_screen(a, o, sc, stamp, model, nvisit, c->num_sms, st)
@@ -794,7 +800,7 @@ int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int mo
     }
     GSJ_CUDA(c, cudaEventRecord(c->tev[7], st));
     S.estimate = (uint64_t)est;
-    const uint64_t estimate = exact_size ? 0u : (uint64_t)(est_entries * 1.25) + N + (1u << 16) + slack;
+    const uint64_t estimate = exact_size ? 0u : (uint64_t)(est_entries * 1.25) + N + (1u << 16) + margin;
     uint64_t cap = estimate;
     // ---- full pass (repeated with a larger buffer if the buffer was short):
     // the tile join's hits, or the screen's records of undecided pairs
