@@ -678,6 +678,14 @@ int emit_join(gsj_context* c, JoinArgs<T>& a, uint64_t N, bool stamp, int model,
 // (0.04), 8-D of pairs mostly within eps 10.3 / 12.2 (0.42).  Below
 // kFewUndecided pairs the exact check takes less than 0.1 ms.
 constexpr int kTakePlain = 1;
+
+// The counters of a tile pass as they lie in `misc`, read back with one copy.
+struct PassCounters {
+    uint32_t claims, err;
+    unsigned long long cand, cursor[2];  // candidates; entries, the screen's undecided pairs
+};
+static_assert(sizeof(PassCounters) == 32, "work counter, error flag, candidates, cursors");
+
 constexpr double kFewUndecided = 16777216.0;
 
 int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int model, bool screen, bool exact_size,
@@ -697,6 +705,10 @@ int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int mo
     // memory) reserve blocks and fill them; the tile join appends exactly
     const uint64_t warps = (uint64_t)c->num_sms * 16u;
     const uint64_t slack = screen ? warps * kScreenBlock : 0u;
+    // the estimate's margin: for small joins, of which the sample sees a handful of
+    // items, also what it misses (6,000 points in 15-D: 2.6 M estimated, 8.8 M undecided;
+    // the repeated pass 0.64 -> 0.82 ms)
+    const uint64_t margin = 4u * slack;
     unsigned long long* cand = reinterpret_cast<unsigned long long*>(a.work_counter + 2);
     a.err_flag = a.work_counter + 1;
     ScreenConst sc = make_screen_const(a.n, a.thr);
@@ -705,21 +717,23 @@ int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int mo
         GSJ_CUDA(c, cudaMemsetAsync(a.work_counter, 0, 4 * sizeof(uint32_t), st));
         GSJ_CUDA(c, cudaMemsetAsync(cursor, 0, 2 * sizeof(unsigned long long), st));
         return GSJ_OK;
-    // the estimate's margin: for small joins, of which the sample sees a handful of
-    // items, also what it misses (6,000 points in 15-D: 2.6 M estimated, 8.8 M undecided;
-    // the repeated pass 0.64 -> 0.82 ms)
-    const uint64_t margin = 4u * slack;
     };
     auto launch = [&](uint32_t nvisit) -> cudaError_t {
         return screen ? launch_tile_screen(a, o, sc, stamp, model, nvisit, c->num_sms, st)
                       : launch_tile_join(a, o, stamp, model, nvisit, c->num_sms, st);
     };
-    // The sampled items once more, their undecided pairs (about `expect` records)
-    // kept and checked: *useless when the FP32 tiles are the better choice.  The
-    // device counters are the sample's afterwards.
+    auto counters = [&](PassCounters* pc) -> int {
+        GSJ_TRY(d2h_small(c, pc, reinterpret_cast<const PassCounters*>(a.work_counter), 1));
+        if (pc->err) return fail(c, GSJ_ERR_CUDA, "tile join: tensor-core wait timed out");
+        return GSJ_OK;
+    };
+    // The sampled items once more, some 65,536 records of their undecided pairs kept
+    // and checked (2 million pairs at most; all of the sample's took up to a tenth of
+    // the join): *useless when the FP32 tiles are the better choice.  The device
+    // counters are the sample's afterwards.
     const uint32_t nsample = (ni + kSampleStride - 1) / kSampleStride;
-    auto check_bound = [&](double expect, bool* useless) -> int {
-        const uint64_t room = (uint64_t)(expect * 1.25) + slack;
+    auto check_bound = [&](bool* useless) -> int {
+        const uint64_t room = (1u << 16) + slack;
         uint4* recs = nullptr;
         GSJ_TRY(dev_get(c, c->pairs, room * 2u, reinterpret_cast<unsigned long long**>(&recs)));
         GSJ_TRY(reset());
@@ -729,15 +743,10 @@ int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int mo
         o.cap = room;
         S.kernel_launches += 2;
         GSJ_CUDA(c, launch(nsample));
-        unsigned long long got[2] = {0, 0}, C = 0, hits = 0;
-        uint32_t err = 0;
-        Readback rb(c);
-        GSJ_TRY(rb.add(got, cursor, 2));
-        GSJ_TRY(rb.add(&C, cand, 1));
-        GSJ_TRY(rb.add(&err, a.err_flag, 1));
-        GSJ_TRY(rb.wait());
-        if (err) return fail(c, GSJ_ERR_CUDA, "tile join: tensor-core wait timed out");
-        const uint64_t nrec = std::min<uint64_t>(got[0], room);
+        PassCounters pc{};
+        GSJ_TRY(counters(&pc));
+        unsigned long long hits = 0;
+        const uint64_t nrec = std::min<uint64_t>(pc.cursor[0], 1u << 16);
         // no room for keys: the pairs within eps are counted only, one direction each
         TileOut ro = o;
         ro.pairs = nullptr;
@@ -745,8 +754,8 @@ int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int mo
         GSJ_CUDA(c, cudaMemsetAsync(cursor, 0, sizeof(unsigned long long), st));
         GSJ_CUDA(c, launch_screen_recheck(a, recs, nrec, ro, false, model, c->num_sms, st));
         GSJ_TRY(d2h_small(c, &hits, cursor, 1));
-        const double within = nrec ? (double)hits * ((double)got[0] / (double)nrec) : 0.0;
-        *useless = 4.0 * ((double)got[1] - within) > (double)C;
+        const double within = nrec ? (double)hits * ((double)pc.cursor[0] / (double)nrec) : 0.0;
+        *useless = 4.0 * ((double)pc.cursor[1] - within) > (double)pc.cand;
         return GSJ_OK;
     };
     bool guarded = screen && a.n < kScreenPathDims;  // the bound is still to be looked at
@@ -780,20 +789,13 @@ int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int mo
         o.stride = kSampleStride;
         S.kernel_launches += 1;
         GSJ_CUDA(c, launch(nsample));
-        unsigned long long sampled[2] = {0, 0};  // entries, and the screen's undecided pairs
-        unsigned long long C = 0;
-        uint32_t err = 0;
-        Readback rb(c);
-        GSJ_TRY(rb.add(sampled, cursor, 2));
-        GSJ_TRY(rb.add(&C, cand, 1));
-        GSJ_TRY(rb.add(&err, a.err_flag, 1));
-        GSJ_TRY(rb.wait());
-        if (err) return fail(c, GSJ_ERR_CUDA, "tile join: tensor-core wait timed out");
-        est_entries = nsample ? (double)sampled[0] * (double)ni / (double)nsample : 0.0;
-        est = screen && nsample ? (double)sampled[1] * (double)ni / (double)nsample : est_entries;
-        if (guarded && est >= kFewUndecided && 4.0 * (double)sampled[1] > (double)C) {
+        PassCounters pc{};
+        GSJ_TRY(counters(&pc));
+        est_entries = nsample ? (double)pc.cursor[0] * (double)ni / (double)nsample : 0.0;
+        est = screen && nsample ? (double)pc.cursor[1] * (double)ni / (double)nsample : est_entries;
+        if (guarded && est >= kFewUndecided && 4.0 * (double)pc.cursor[1] > (double)pc.cand) {
             bool useless = false;
-            GSJ_TRY(check_bound((double)sampled[0], &useless));
+            GSJ_TRY(check_bound(&useless));
             if (useless) return kTakePlain;
             guarded = false;
         }
@@ -818,23 +820,17 @@ int tile_join(gsj_context* c, JoinArgs<float>& a, uint64_t N, bool stamp, int mo
         S.kernel_launches += 1;
         GSJ_CUDA(c, launch(ni));
         // entries written (pairs), or reserved (records)
-        unsigned long long got[2] = {0, 0}, C = 0;
-        uint32_t err = 0;
-        Readback rb(c);
-        GSJ_TRY(rb.add(got, cursor, 2));
-        GSJ_TRY(rb.add(&C, cand, 1));
-        GSJ_TRY(rb.add(&err, a.err_flag, 1));
-        GSJ_TRY(rb.wait());
-        used = got[0];
-        U = screen ? got[1] : used;
-        if (err) return fail(c, GSJ_ERR_CUDA, "tile join: tensor-core wait timed out");
-        if (guarded && (double)U >= kFewUndecided && 4.0 * (double)U > (double)C) {
+        PassCounters pc{};
+        GSJ_TRY(counters(&pc));
+        used = pc.cursor[0];
+        U = screen ? pc.cursor[1] : used;
+        if (guarded && (double)U >= kFewUndecided && 4.0 * (double)U > (double)pc.cand) {
             // no sampling pass was run, or its few items did not show it
             bool useless = false;
-            GSJ_TRY(check_bound((double)used / kSampleStride, &useless));
+            GSJ_TRY(check_bound(&useless));
             if (useless) return kTakePlain;
             guarded = false;
-            GSJ_CUDA(c, cudaMemcpyAsync(cand, &C, sizeof(C), cudaMemcpyHostToDevice, st));
+            GSJ_CUDA(c, cudaMemcpyAsync(cand, &pc.cand, sizeof(pc.cand), cudaMemcpyHostToDevice, st));
         }
         if (used <= cap) {
             nlist = used;
