@@ -326,6 +326,11 @@ static cudaError_t launch_form(K kern, const JoinArgs<T>& a, const uint32_t* slo
     return cudaGetLastError();
 }
 
+// From about this many queries on a thread per query fills the chip (148 SMs hold
+// 303,104 threads): the lines below were drawn on both sides of it, from 3,000
+// points to 4 million.
+constexpr uint32_t kManyQueries = 400000u;
+
 template <typename T, int NT, int NR, bool FILL>
 static cudaError_t launch_rows(const JoinArgs<T>& a, const uint32_t* slot_cell, uint32_t* counts_by_id,
                                const uint32_t* qslots, uint32_t nq, uint64_t base, uint64_t pairs, uint64_t cands,
@@ -341,11 +346,16 @@ static cudaError_t launch_rows(const JoinArgs<T>& a, const uint32_t* slot_cell, 
         // 0.246.  Three rows: 2-D 4M at 7.0 0.228 / 0.158, 10 0.226 / 0.195, in double at 7.0
         // 0.269 / 0.250, 8.0 0.271 / 0.277, a 2-D mixture 8M at 9.1 1.14 / 1.18; 4-D 1M at 6.0 0.080 / 0.074, 7.0 0.080 / 0.082, in
         // double at 6.0 0.119 / 0.119.  One row: 1-D 4M at 10 0.129 / 0.119, in double 0.160 /
-        // 0.123.
-        constexpr uint32_t line = NR == 9   ? (sizeof(T) == 8 ? 5u : 6u)
-                                  : NR == 1 ? 10u
-                                  : NT <= 2 ? (sizeof(T) == 8 ? 7u : 8u)
-                                            : 6u;
+        // 0.123.  Fewer points than the chip holds threads for leave a thread's serial
+        // candidates in plain sight, in double above all: us for 3-D double 10k at 3.8 31.0 /
+        // 37.1, 100k at 3.9 47.3 / 47.2, at 4.8 47.4 / 51.4, 2-D double 10k at 5.0 14.5 / 16.4,
+        // 300k at 6.0 32.8 / 35.2; 3-D float 10k at 5.8 22.8 / 20.6, 300k at 5.9 65.6 / 67.9.
+        const bool many = a.n_points >= kManyQueries;
+        const uint32_t line = sizeof(T) == 8 ? (many ? (NR == 9 ? 5u : NR == 1 ? 10u : NT <= 2 ? 7u : 6u)
+                                                     : (NR == 9 ? 4u : 5u))
+                              : NR == 1      ? (many ? 10u : 7u)
+                              : NR == 3 && NT <= 2 ? 8u
+                                                   : 6u;
         if (a.n_points < line * (uint64_t)a.num_cells)
             return launch_form<T>(k_rows_thread<T, NT, NR, POL, false>, a, slot_cell, counts_by_id, qslots, nq, base,
                                   num_sms, st);
@@ -360,9 +370,12 @@ static cudaError_t launch_rows(const JoinArgs<T>& a, const uint32_t* slot_cell, 
         // and 5.2 0.324 / 0.292, 4.1 and 9.2 0.259 / 0.482.  So sparse cells take a
         // thread per query while it stores few ids, each to a sector of its own; with
         // many candidates a point (4-D 500k, 130 of them and 1.5 pairs: 0.145 / 0.148,
-        // double 0.162 / 0.195) the cell form is the better one again.
-        if (N < (sizeof(T) == 8 ? 5u : 7u) * (uint64_t)a.num_cells && pairs <= (NR == 1 ? 6u : 4u + NR) * N &&
-            cands <= 96u * N)
+        // double 0.162 / 0.195) the cell form is the better one again, and on fewer points
+        // sooner (us; 3-D 100k, 28 candidates and 5.1 pairs 53.8 / 48.0, 54 and 9.1 51.7 /
+        // 58.3, in double 51.5 / 53.3 and 49.3 / 65.7; 2-D 100k, 19 and 7.3 33.5 / 24.6).
+        const bool many = N >= kManyQueries;
+        if (N < (sizeof(T) == 8 ? 5u : 7u) * (uint64_t)a.num_cells &&
+            pairs <= (NR == 1 ? 6u : NR == 3 ? 7u : many ? 14u : 6u) * N && cands <= (many ? 96u : 32u) * N)
             return launch_form<T>(k_rows_thread<T, NT, NR, POL, true>, a, slot_cell, counts_by_id, qslots, nq, base,
                                   num_sms, st);
         // Where few candidates are within eps one vote a query skips four tiles, and an id
