@@ -1426,7 +1426,7 @@ int run_join(gsj_context* c, const void* data, uint64_t N, double eps_d, const g
     a.shape_per_sm = shape.ctas_per_sm;
     const bool stamp = cfg.stamp != 0 && !(cfg.flags & GSJ_FLAG_NO_UNICOMP);
     const bool exact_size = (cfg.flags & GSJ_FLAG_EXACT_SIZE) != 0;
-    if (!dense && k <= 3 && !tile && !cfg.sort) {
+    if (!dense && k <= 3 && !tile && !cfg.sort && M >= kRowPlanCells) {
         // the warp join's neighbour rows; without room for them it looks them up itself
         uint2* rplan = nullptr;
         if (dev_get(c, c->plan, (size_t)M * (k == 1 ? 1u : (k == 2 ? 3u : 9u)), &rplan) == GSJ_OK) {

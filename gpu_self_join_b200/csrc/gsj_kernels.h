@@ -53,6 +53,11 @@ cudaError_t launch_cell_plan(const uint64_t* cell_key, uint32_t M, const GridGeo
                              uint2* plan, cudaStream_t st);
 // The same for the warp join on a hashed grid with k <= 3 (a: cell table, grid and
 // neighbour offsets), the rows of the unicomp half-space with `stamp`.
+// On fewer cells than kRowPlanCells the join's own warps have lanes and time for it,
+// and the launch costs more than it gives (whole joins, us, without / with: 3-D float
+// 2,000 cells 290 / 299, 4,000 352 / 370, 30,000 379 / 391, 100,000 445 / 445; double
+// 2,000 274 / 284, 30,000 367 / 360, 100,000 488 / 433; 2-D double 30,000 356 / 338).
+constexpr uint32_t kRowPlanCells = 32768;
 template <typename T>
 cudaError_t launch_row_plan(const JoinArgs<T>& a, bool stamp, uint2* plan, cudaStream_t st);
 cudaError_t launch_item_counts(const uint32_t* cell_start, const uint32_t* order, uint32_t M, uint32_t qchunk,
